@@ -347,7 +347,6 @@ k_seg_topology(const int64_t* __restrict__ part_off, const int64_t* __restrict__
     __shared__ int64_t cnt_lo[kMaxDepth];
     __shared__ int64_t internal[kMaxDepth][2];
     __shared__ int depth_s;
-    __shared__ unsigned leaf_ctr;
     if (threadIdx.x == 0) {
         int depth = 0;
         while (((n + (1ll << depth) - 1) >> depth) > L && depth < kMaxDepth - 2) depth++;
@@ -361,12 +360,11 @@ k_seg_topology(const int64_t* __restrict__ part_off, const int64_t* __restrict__
                 internal[d][v] = 1 + internal[d + 1][h - lo] + internal[d + 1][r - lo];
             }
         }
-        leaf_ctr = 0;
     }
     __syncthreads();
     const int depth = depth_s;
     const int64_t nodes = node_off[s + 1] - node_off[s];
-    const int64_t leaves = leaf_off[s + 1] - leaf_off[s];
+    const int64_t leaf_slots = leaf_off[s + 1] - leaf_off[s];   // at least 2^depth
     const int64_t slots = (2ll << depth) - 1;
     const int64_t nb = node_off[s], pb = part_off[s];
     for (int64_t slot = threadIdx.x; slot < slots; slot += blockDim.x) {
@@ -397,8 +395,8 @@ k_seg_topology(const int64_t* __restrict__ part_off, const int64_t* __restrict__
         parent[nb + id] = par < 0 ? -1 : (int32_t)(nb + par);
         if (c <= L) {
             first_child[nb + id] = -1;
-            const unsigned li = atomicAdd(&leaf_ctr, 1u);
-            if (li < leaves) leaf_list[leaf_off[s] + li] = (int32_t)(nb + id);
+            const int64_t li = j << (depth - d);   // slot order, as k_topology
+            if (li < leaf_slots) leaf_list[leaf_off[s] + li] = (int32_t)(nb + id);
             else atomicOr(err, kErrBadNode);
         } else {
             first_child[nb + id] = (int32_t)(nb + 2 * k + 1);
@@ -968,13 +966,16 @@ int plan_layout(bhut_batch* b, const int64_t* offsets, int64_t nsys)
         TopoTables tt;
         BHUT_TRY(make_topo_tables(n, b->leaf, &tt));
         b->node_off[s + 1] = b->node_off[s] + tt.num_nodes;
-        b->leaf_off[s + 1] = b->leaf_off[s] + tt.num_leaves;
+        // leaf slots, aligned so that k_bottom_up's groups merge whole subtrees
+        const int64_t align = std::min<int64_t>(tt.leaf_slots, kLeafSlotAlign);
+        b->leaf_off[s] = (b->leaf_off[s] + align - 1) / align * align;
+        b->leaf_off[s + 1] = b->leaf_off[s] + tt.leaf_slots;
     }
     b->nsys = nsys;
     b->ntot = offsets[nsys];
     b->mtot = b->node_off[nsys];
     b->ltot = b->leaf_off[nsys];
-    if (b->ntot > 0x7fffffffLL || b->mtot > 0x7fffffffLL) {
+    if (b->ntot > 0x7fffffffLL || b->mtot > 0x7fffffffLL || b->ltot > 0x7fffffffLL) {
         set_error("batch too large: at most 2^31-1 particles and nodes");
         return kInvalid;
     }
@@ -1207,15 +1208,13 @@ int enqueue_solve(bhut_batch* b, double theta, double eps, double G, double* out
 int ensure_topology(bhut_batch* b)
 {
     if (b->topo_valid) return kOk;
+    BHUT_CUDA(cudaMemsetAsync(b->leaf_list.p, 0xff, sizeof(int32_t) * (size_t)b->ltot, b->stream));
     k_seg_topology<<<(unsigned)b->nsys, kSegThreads, 0, b->stream>>>(
         b->d_part_off.as<int64_t>(), b->d_node_off.as<int64_t>(), b->d_leaf_off.as<int64_t>(),
         b->leaf, b->first_child.as<int32_t>(), b->start.as<int32_t>(), b->count.as<int32_t>(),
         b->parent.as<int32_t>(), b->leaf_list.as<int32_t>(), b->err.as<unsigned>());
     BHUT_CUDA(cudaGetLastError());
     note_launches(1);
-    // leaves in particle order (the particle keys are free until the solve)
-    BHUT_TRY(order_leaves(b->leaf_list.as<int32_t>(), b->ltot, b->start.as<int32_t>(),
-                          b->keys.as<uint64_t>(), b->sort_scratch.p, b->stream));
     b->topo_valid = true;
     return kOk;
 }

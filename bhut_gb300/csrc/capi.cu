@@ -218,7 +218,7 @@ int enqueue_build(bhut_tree* t, int64_t n)
     BHUT_TRY(launch_gather(t->pos.as<double>(), t->mass.as<double>(), t->perm.as<int32_t>(), n, dim,
                            t->sx.as<double>(), t->sy.as<double>(), t->sz.as<double>(),
                            t->sm.as<double>(), s));
-    BHUT_TRY(launch_bottom_up(t->dev(), t->leaf_list.as<int32_t>(), t->tt.num_leaves,
+    BHUT_TRY(launch_bottom_up(t->dev(), t->leaf_list.as<int32_t>(), t->tt.leaf_slots,
                               t->first_child.as<int32_t>(), t->start.as<int32_t>(),
                               t->count.as<int32_t>(), t->parent.as<int32_t>(),
                               t->arrive.as<unsigned>(), t->nodes(), false, nullptr, nullptr,
@@ -239,7 +239,7 @@ void build_graph_key(const bhut_tree* t, int64_t n, const void** key)
     int k = 0;
     for (const DevBuf* b : bufs) key[k++] = b->p;
     key[k++] = (const void*)(intptr_t)n;
-    key[k++] = (const void*)(intptr_t)t->tt.num_leaves;
+    key[k++] = (const void*)(intptr_t)t->tt.leaf_slots;
     key[k++] = (const void*)t->stream;
 }
 
@@ -271,15 +271,10 @@ int do_build(bhut_tree* t, int64_t n)
     if (!t->topo_valid) {
         for (DevBuf* b : {&t->first_child, &t->start, &t->count, &t->parent})
             BHUT_TRY(b->ensure(sizeof(int32_t) * m, s));
-        BHUT_TRY(t->leaf_list.ensure(sizeof(int32_t) * t->tt.num_leaves, s));
+        BHUT_TRY(t->leaf_list.ensure(sizeof(int32_t) * t->tt.leaf_slots, s));
         BHUT_TRY(launch_topology(t->tt, t->first_child.as<int32_t>(), t->start.as<int32_t>(),
                                  t->count.as<int32_t>(), t->parent.as<int32_t>(),
-                                 t->leaf_list.as<int32_t>(), t->counters.as<unsigned>() + 1,
-                                 t->err.as<unsigned>(), s));
-        BHUT_TRY(t->tkeys.ensure(sizeof(uint64_t) * t->tt.num_leaves, s));
-        BHUT_TRY(order_leaves(t->leaf_list.as<int32_t>(), t->tt.num_leaves,
-                              t->start.as<int32_t>(), t->tkeys.as<uint64_t>(),
-                              t->sort_scratch.p, s));
+                                 t->leaf_list.as<int32_t>(), t->err.as<unsigned>(), s));
         t->topo_valid = true;
     }
     // the box of these positions was computed while they were staged
@@ -462,7 +457,7 @@ int prepare_fast(bhut_tree* t)
         BHUT_TRY(t->quad.ensure(sizeof(double) * 6 * t->m, s));
         BHUT_TRY(t->nq0.ensure(sizeof(float4) * t->m, s));
         BHUT_TRY(t->nq1.ensure(sizeof(float2) * t->m, s));
-        BHUT_TRY(launch_quadrupoles(t->dev(), t->leaf_list.as<int32_t>(), t->tt.num_leaves,
+        BHUT_TRY(launch_quadrupoles(t->dev(), t->leaf_list.as<int32_t>(), t->tt.leaf_slots,
                                     t->first_child.as<int32_t>(), t->start.as<int32_t>(),
                                     t->count.as<int32_t>(), t->parent.as<int32_t>(),
                                     t->arrive.as<unsigned>(), t->quad.as<double>(),
@@ -632,7 +627,7 @@ int bhut_tree_refit(bhut_tree* t, const double* positions, const double* masses,
     BHUT_TRY(launch_gather(t->pos.as<double>(), t->mass.as<double>(), t->perm.as<int32_t>(), n,
                            t->dim, t->sx.as<double>(), t->sy.as<double>(), t->sz.as<double>(),
                            t->sm.as<double>(), s));
-    BHUT_TRY(launch_bottom_up(t->dev(), t->leaf_list.as<int32_t>(), t->tt.num_leaves,
+    BHUT_TRY(launch_bottom_up(t->dev(), t->leaf_list.as<int32_t>(), t->tt.leaf_slots,
                               t->first_child.as<int32_t>(), t->start.as<int32_t>(),
                               t->count.as<int32_t>(), t->parent.as<int32_t>(),
                               t->arrive.as<unsigned>(), t->nodes(), true, t->pos.as<double>(),
@@ -659,7 +654,7 @@ int bhut_tree_refit_only(bhut_tree* t, const double* positions, const double* ma
     BHUT_TRY(launch_gather(t->pos.as<double>(), t->mass.as<double>(), t->perm.as<int32_t>(), n,
                            t->dim, t->sx.as<double>(), t->sy.as<double>(), t->sz.as<double>(),
                            t->sm.as<double>(), s));
-    BHUT_TRY(launch_bottom_up(t->dev(), t->leaf_list.as<int32_t>(), t->tt.num_leaves,
+    BHUT_TRY(launch_bottom_up(t->dev(), t->leaf_list.as<int32_t>(), t->tt.leaf_slots,
                               t->first_child.as<int32_t>(), t->start.as<int32_t>(),
                               t->count.as<int32_t>(), t->parent.as<int32_t>(),
                               t->arrive.as<unsigned>(), t->nodes(), true, t->pos.as<double>(),
@@ -1240,6 +1235,7 @@ int bhut_tree_import(bhut_tree* t, const double* positions, const double* masses
     t->tt.leaf_size = t->leaf;
     t->tt.num_nodes = m;
     t->tt.num_leaves = nleaves;
+    t->tt.leaf_slots = nleaves;            // an unordered list without holes
     t->ff_valid = false;
     t->built = true;
     return kOk;

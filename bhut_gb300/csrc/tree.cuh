@@ -45,9 +45,15 @@ struct TopoTables {
     int64_t num_nodes;
     int64_t num_leaves;
     int64_t slots;                 // 2^(depth+1) - 1 BFS slots
+    int64_t leaf_slots;            // entries of the leaf list: 2^depth (see k_topology)
 };
 
 int make_topo_tables(int64_t n, int leaf_size, TopoTables* t);
+
+// Leaf lists are merged in aligned groups of this many entries (k_bottom_up);
+// a batch starts each system's list at a multiple of it, or of the list's
+// own length when that is smaller.
+constexpr int kLeafSlotAlign = 256;
 
 // Normalisation of the "fast" traversal: u = (x - c) * s with s a power of
 // two mapping the box into [-1, 1]; masses scaled by ms (a power of two, or
@@ -203,22 +209,17 @@ int launch_morton(const double* pos, int64_t n, int dim, const double* box, uint
 int launch_gather(const double* pos, const double* mass, const int32_t* perm, int64_t n, int dim,
                   double* sx, double* sy, double* sz, double* sm, cudaStream_t s);
 int launch_topology(const TopoTables& tt, int32_t* first_child, int32_t* start, int32_t* count,
-                    int32_t* parent, int32_t* leaf_list, unsigned* leaf_counter, unsigned* err,
-                    cudaStream_t s);
-// Reorders the leaf list by first particle (siblings end up in neighbouring
-// entries, which the bottom-up pass merges inside a block).  `keys` holds
-// num_leaves entries; the scratch sort_scratch_bytes(num_leaves).
-int order_leaves(int32_t* leaf_list, int64_t num_leaves, const int32_t* start, uint64_t* keys,
-                 void* sort_scratch, cudaStream_t s);
+                    int32_t* parent, int32_t* leaf_list, unsigned* err, cudaStream_t s);
 // Node boxes and moments from the leaves up (build, or refit with opos /
-// omass in input order); quadrupoles the same way.  `frontier` holds
-// num_leaves entries of scratch, `frontier_count` one counter.
-int launch_bottom_up(const TreeDev& t, const int32_t* leaf_list, int64_t num_leaves,
+// omass in input order); quadrupoles the same way.  The leaf list holds
+// `entries` leaves and holes (-1); `frontier` holds as many entries of
+// scratch, `frontier_count` one counter.
+int launch_bottom_up(const TreeDev& t, const int32_t* leaf_list, int64_t entries,
                      const int32_t* first_child, const int32_t* start, const int32_t* count,
                      const int32_t* parent, unsigned* arrive, NodeOut o, bool refit,
                      const double* opos, const double* omass, int32_t* frontier,
                      unsigned* frontier_count, unsigned* err, cudaStream_t s);
-int launch_quadrupoles(const TreeDev& t, const int32_t* leaf_list, int64_t num_leaves,
+int launch_quadrupoles(const TreeDev& t, const int32_t* leaf_list, int64_t entries,
                        const int32_t* first_child, const int32_t* start, const int32_t* count,
                        const int32_t* parent, unsigned* arrive, double* quad, int32_t* frontier,
                        unsigned* frontier_count, unsigned* err, cudaStream_t s);
