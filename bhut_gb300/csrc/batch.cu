@@ -405,7 +405,7 @@ k_seg_topology(const int64_t* __restrict__ part_off, const int64_t* __restrict__
 }
 
 // Float-float copies of every particle and node in its system's frame.
-__global__ void k_seg_ff_particles(TreeDev t, const int32_t* __restrict__ sys_of,
+__global__ void k_seg_ff_particles(TreeDev t, bool fine, const int32_t* __restrict__ sys_of,
                                    const FastFrame* __restrict__ frames, float4* __restrict__ ph,
                                    float4* __restrict__ pl)
 {
@@ -414,9 +414,9 @@ __global__ void k_seg_ff_particles(TreeDev t, const int32_t* __restrict__ sys_of
          i += (int64_t)gridDim.x * blockDim.x) {
         const FastFrame& f = frames[sys_of[i]];
         float4 h, l;
-        split_grid(__dmul_rn(__dsub_rn(t.sx[i], f.c[0]), f.s), h.x, l.x);
-        split_grid(__dmul_rn(__dsub_rn(t.sy[i], f.c[1]), f.s), h.y, l.y);
-        if (dim == 3) split_grid(__dmul_rn(__dsub_rn(t.sz[i], f.c[2]), f.s), h.z, l.z);
+        split_grid(__dmul_rn(__dsub_rn(t.sx[i], f.c[0]), f.s), fine, h.x, l.x);
+        split_grid(__dmul_rn(__dsub_rn(t.sy[i], f.c[1]), f.s), fine, h.y, l.y);
+        if (dim == 3) split_grid(__dmul_rn(__dsub_rn(t.sz[i], f.c[2]), f.s), fine, h.z, l.z);
         else h.z = l.z = 0.0f;
         if (f.unit) { h.w = 1.0f; l.w = 0.0f; }   // every mass is m0: exactly 1 in units of m0
         else split_plain(__dmul_rn(t.sm[i], f.ms), h.w, l.w);
@@ -425,13 +425,13 @@ __global__ void k_seg_ff_particles(TreeDev t, const int32_t* __restrict__ sys_of
     }
 }
 
-__global__ void k_seg_ff_nodes(TreeDev t, const int32_t* __restrict__ node_sys,
+__global__ void k_seg_ff_nodes(TreeDev t, bool fine, const int32_t* __restrict__ node_sys,
                                const FastFrame* __restrict__ frames,
                                const double* __restrict__ center, float4* __restrict__ nh,
                                float4* __restrict__ nl, float* __restrict__ nsize,
                                float* __restrict__ ndelta, const double* __restrict__ quad,
                                float4* __restrict__ nq0, float2* __restrict__ nq1,
-                               int4* __restrict__ nhdr)
+                               int4* __restrict__ nhdr, const float4* __restrict__ ph)
 {
     const int dim = t.dim;
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < t.m;
@@ -439,11 +439,13 @@ __global__ void k_seg_ff_nodes(TreeDev t, const int32_t* __restrict__ node_sys,
         const FastFrame& f = frames[node_sys[k]];
         const NodeCM c = t.cm[k];
         float4 h, l;
-        split_grid(__dmul_rn(__dsub_rn(c.x, f.c[0]), f.s), h.x, l.x);
-        split_grid(__dmul_rn(__dsub_rn(c.y, f.c[1]), f.s), h.y, l.y);
-        if (dim == 3) split_grid(__dmul_rn(__dsub_rn(c.z, f.c[2]), f.s), h.z, l.z);
+        split_grid(__dmul_rn(__dsub_rn(c.x, f.c[0]), f.s), fine, h.x, l.x);
+        split_grid(__dmul_rn(__dsub_rn(c.y, f.c[1]), f.s), fine, h.y, l.y);
+        if (dim == 3) split_grid(__dmul_rn(__dsub_rn(c.z, f.c[2]), f.s), fine, h.z, l.z);
         else h.z = l.z = 0.0f;
+        const int fc = t.first_child[k];
         split_plain(__dmul_rn(c.w, f.ms), h.w, l.w);
+        if (fc < 0) leaf_box(ph, t.start[k], t.count[k], h, l);   // (LeafBox in a leaf's place)
         nh[k] = h;
         nl[k] = l;
         nsize[k] = __double2float_rn(__dmul_rn(t.size[k], f.s));
@@ -454,12 +456,11 @@ __global__ void k_seg_ff_nodes(TreeDev t, const int32_t* __restrict__ node_sys,
             dd += v * v;
         }
         ndelta[k] = __double2float_ru(sqrt(dd) * f.s);
-        // header: leaf (-1, start, count, mass != 0); internal (first child,
-        // size, |com - centre| as float bits, mass != 0)
-        const int fc = t.first_child[k];
+        // header: leaf (-1, start, count, flag); internal (first child, size,
+        // |com - centre| as float bits, flag)
         nhdr[k] = fc < 0 ? make_int4(fc, t.start[k], t.count[k], c.w != 0.0)
                          : make_int4(fc, __float_as_int(nsize[k]), __float_as_int(ndelta[k]),
-                                     c.w != 0.0);
+                                     node_flag(c, h));
         if (quad) {   // mass x length^2: scale by ms s^2
             const double qs = f.ms * f.s * f.s;
             const double* q = quad + 6 * k;
@@ -486,7 +487,7 @@ struct BatchDev {
     const float* ndelta;
     const float4* nq0;            // quadrupoles (FP32 form); NULL: monopoles
     const float2* nq1;
-    const int4* nhdr;             // (first_child, start, count, mass != 0)
+    const int4* nhdr;             // (first_child, start, count, flag)
 };
 
 struct BatchArgs {
@@ -581,7 +582,10 @@ k_batch_traverse(BatchDev b, BatchArgs a)
 {
     constexpr int LPT = kWarp / TPW;            // lanes per target
     __shared__ int2 stack[STK == 0 ? kBatchWarps : 1][kStackDepth];
+    // the fast form's two-lane tasks and the FP32 form read source by source
+    constexpr bool kStaged = !FP32 && TPW == 32;
     __shared__ float4 sh[kBatchWarps][kWarp], sl[kBatchWarps][kWarp];
+    __shared__ LeafStage stage[kStaged ? kBatchWarps : 1];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int sub = lane % LPT;
     const unsigned FULL = 0xffffffffu;
@@ -636,27 +640,39 @@ k_batch_traverse(BatchDev b, BatchArgs a)
             const int node = e.x;
             const bool act = ((unsigned)e.y >> lane) & 1u;
             cnt[2] += act && sub == 0;
-            const int4 hd = b.nhdr[node];   // (first_child, start, count, mass != 0)
+            const int4 hd = b.nhdr[node];   // (first_child, start, count, flag)
             if (!hd.w) continue;
             const int fc = hd.x;
             if (fc < 0) {
                 const int s0 = hd.y, c = hd.z;
+                LeafBox box;
+                if (kStaged && soft) {
+                    box.c = b.nh[node];
+                    box.h = b.nl[node];
+                }
                 for (int bb = 0; bb < c; bb += kWarp) {
                     const int jj = bb + lane;
+                    const bool staged = kStaged && soft;
                     if (jj < c) {
-                        sh[w][lane] = b.ph[s0 + jj];
-                        sl[w][lane] = b.pl[s0 + jj];
+                        const float4 h = b.ph[s0 + jj], l = b.pl[s0 + jj];
+                        if (staged) {
+                            stage[kStaged ? w : 0].put(lane, h, l);
+                        } else {
+                            sh[w][lane] = h;
+                            sl[w][lane] = l;
+                        }
                     }
                     __syncwarp();
                     const int cn = min(kWarp, c - bb);
                     if (act && sub == 0) cnt[0] += cn - (i >= s0 + bb && i < s0 + bb + cn);
-                    if (!FP32 && LPT == 1 && soft) {   // as the single-tree walk
+                    if (staged) {   // as the single-tree walk
+                        const LeafStage& sg = stage[kStaged ? w : 0];
                         if (unit)
-                            leaf_block_soft<DIM, true>((unsigned)e.y, lane, Th, Tl, sh[w], sl[w],
-                                                       cn, e2h, e2l, ah, al);
+                            leaf_block_soft<DIM, true>((unsigned)e.y, lane, Th, Tl, sg, cn, box,
+                                                       e2h, e2l, ah, al);
                         else
-                            leaf_block_soft<DIM, false>((unsigned)e.y, lane, Th, Tl, sh[w], sl[w],
-                                                        cn, e2h, e2l, ah, al);
+                            leaf_block_soft<DIM, false>((unsigned)e.y, lane, Th, Tl, sg, cn, box,
+                                                        e2h, e2l, ah, al);
                     } else if (act) {
                         if (FP32) {   // <= 32 terms in FP32, then one Kahan step
                             float2 pxy = make_float2(0.f, 0.f);
@@ -755,9 +771,9 @@ k_batch_traverse(BatchDev b, BatchArgs a)
                                                ah, al);
                         else
                             pair_f32<DIM>(Th, Tl, nhv, nlv, e2h, ah, al);
-                    } else if (soft) {
+                    } else if (soft && hd.w == 1) {
                         pair_ff_soft<DIM, false>(Th, Tl, nhv, nlv, e2h, e2l, ah, al);
-                    } else if (!pair_ff<DIM, false>(Th, Tl, nhv, nlv, e2h, e2l, ah, al)) {
+                    } else if (hd.w == 2 || !pair_ff<DIM, false>(Th, Tl, nhv, nlv, e2h, e2l, ah, al)) {
                         const NodeCM cm = t.cm[node];
                         pair_fp64<DIM>(x, y, z, cm.x, cm.y, cm.z, cm.w, eps2, a64);
                         cnt[4]++;
@@ -1167,14 +1183,15 @@ int enqueue_solve(bhut_batch* b, double theta, double eps, double G, double* out
                                     b->arrive.as<unsigned>(), b->quad.as<double>(),
                                     b->frontier.as<int32_t>(), b->counter.as<unsigned>() + 2,
                                     b->err.as<unsigned>(), s));
-    k_seg_ff_particles<<<grid_for(n, 256), 256, 0, s>>>(b->dev(), b->sys_of.as<int32_t>(),
+    const bool fine = b->form == BHUT_FORM_FAST;
+    k_seg_ff_particles<<<grid_for(n, 256), 256, 0, s>>>(b->dev(), fine, b->sys_of.as<int32_t>(),
                                                         b->frames.as<FastFrame>(),
                                                         b->ph.as<float4>(), b->pl.as<float4>());
     k_seg_ff_nodes<<<grid_for(b->mtot, 256), 256, 0, s>>>(
-        b->dev(), b->node_sys.as<int32_t>(), b->frames.as<FastFrame>(), b->center.as<double>(),
+        b->dev(), fine, b->node_sys.as<int32_t>(), b->frames.as<FastFrame>(), b->center.as<double>(),
         b->nh.as<float4>(), b->nl.as<float4>(), b->nsize.as<float>(), b->ndelta.as<float>(),
         quad ? b->quad.as<double>() : nullptr, b->nq0.as<float4>(), b->nq1.as<float2>(),
-        b->nhdr.as<int4>());
+        b->nhdr.as<int4>(), b->ph.as<float4>());
     BHUT_CUDA(cudaGetLastError());
     note_launches(2);
     // traversal

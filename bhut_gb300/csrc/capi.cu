@@ -133,11 +133,12 @@ struct bhut_tree {
     bool graph_unsupported = false;
     unsigned long long last_stats[5] = {0, 0, 0, 0, 0};
     // traversal targets
-    DevBuf tpos, tkeys, tperm, tx, ty, tz, tbox, out;
+    DevBuf tpos, tkeys, tperm, tx, ty, tz, tbox, out, split_partial;
     // float-float copies for the fast form
     DevBuf frame, ph, pl, nh, nl, nsize, ndelta, th, tl, quad, nq0, nq1, nhdr;
     bool ff_valid = false;
     bool ff_quad = false;
+    bool ff_fine = false;     // lo parts of form "fast"
     int mac = 0;
     int multipole = BHUT_MULTIPOLE_MONO;
 
@@ -442,7 +443,8 @@ int finish_out(bhut_tree* t, const OutTarget& o, size_t bytes, const char* what)
 int prepare_fast(bhut_tree* t)
 {
     const bool want_quad = t->multipole == BHUT_MULTIPOLE_QUAD && t->form == BHUT_FORM_FP32;
-    if (t->ff_valid && t->ff_quad == want_quad) return kOk;
+    const bool fine = t->form == BHUT_FORM_FAST;
+    if (t->ff_valid && t->ff_quad == want_quad && t->ff_fine == fine) return kOk;
     cudaStream_t s = t->stream;
     BHUT_TRY(t->frame.ensure(sizeof(FastFrame), s));
     BHUT_TRY(t->ph.ensure(sizeof(float4) * t->n, s));
@@ -464,13 +466,14 @@ int prepare_fast(bhut_tree* t)
                                     t->frontier.as<int32_t>(), t->counters.as<unsigned>() + 6,
                                     t->err.as<unsigned>(), s));
     }
-    BHUT_TRY(launch_fast_prepare(t->box.as<double>(), t->dim, t->frame.as<FastFrame>(), t->dev(),
+    BHUT_TRY(launch_fast_prepare(t->box.as<double>(), t->dim, fine, t->frame.as<FastFrame>(), t->dev(),
                                  t->center.as<double>(), t->ph.as<float4>(), t->pl.as<float4>(),
                                  t->nh.as<float4>(), t->nl.as<float4>(), t->nsize.as<float>(),
                                  t->ndelta.as<float>(), quad ? t->quad.as<double>() : nullptr,
                                  t->nq0.as<float4>(), t->nq1.as<float2>(), t->nhdr.as<int4>(),
                                  s));
     t->ff_quad = quad;
+    t->ff_fine = fine;
     t->ff_valid = true;
     return kOk;
 }
@@ -513,16 +516,21 @@ int traverse(bhut_tree* t, const double* tx, const double* ty, const double* tz,
         if (!self_targets) {
             BHUT_TRY(t->th.ensure(sizeof(float4) * nt, t->stream));
             BHUT_TRY(t->tl.ensure(sizeof(float4) * nt, t->stream));
-            BHUT_TRY(launch_fast_targets(tx, ty, tz, nt, t->dim, t->frame.as<FastFrame>(),
+            BHUT_TRY(launch_fast_targets(tx, ty, tz, nt, t->dim, t->ff_fine, t->frame.as<FastFrame>(),
                                          t->th.as<float4>(), t->tl.as<float4>(), t->stream));
             th = t->th.as<float4>();
             tl = t->tl.as<float4>();
         }
+        const int levels = t->form == BHUT_FORM_FAST ? fast_split_levels(nt, t->m, self_targets)
+                                                      : 0;
+        const int64_t part = fast_split_partial(nt, t->dim, levels);
+        if (part > 0) BHUT_TRY(t->split_partial.ensure(sizeof(double) * part, t->stream));
         const double es = eps * sc;
         BHUT_TRY(launch_traverse_fast(d, fast_tree(t), th, tl, tx, ty, tz, self_id, out_idx, nt,
                                       theta, eps, G, es * es, out, t->err.as<unsigned>(), st,
                                       t->stream, t->form == BHUT_FORM_FP32,
-                                      t->form == BHUT_FORM_FP32 ? t->mac : 0));
+                                      t->form == BHUT_FORM_FP32 ? t->mac : 0, levels,
+                                      t->split_partial.as<double>()));
         break;
     }
     case BHUT_FORM_EXACT:
@@ -825,6 +833,7 @@ void bhut_tree_destroy(bhut_tree* t)
                      &t->start, &t->count, &t->parent, &t->leaf_list, &t->arrive,
                      &t->sort_scratch, &t->box_partial, &t->box, &t->counters, &t->err, &t->stats,
                      &t->tpos, &t->tkeys, &t->tperm, &t->tx, &t->ty, &t->tz, &t->tbox, &t->out,
+                     &t->split_partial,
                      &t->frame, &t->ph, &t->pl, &t->nh, &t->nl, &t->nsize, &t->ndelta, &t->th,
                      &t->tl, &t->quad, &t->nq0, &t->nq1, &t->nhdr, &t->pos_in, &t->mass_in,
                      &t->box_in, &t->frontier};

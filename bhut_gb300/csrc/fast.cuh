@@ -11,33 +11,17 @@
 #ifndef BHUT_FF_KNUTH_ACC
 #define BHUT_FF_KNUTH_ACC 0
 #endif
-// Unroll factor of the float-float leaf pair loops (swept on GB300 at 1M
-// Plummer: 4 beats 1-2 by 2-10 %).
-#ifndef BHUT_FF_UNROLL
-#define BHUT_FF_UNROLL 4
-#endif
 
 namespace bhut {
 
-constexpr int kFFUnroll = BHUT_FF_UNROLL;
-// leaf_block_soft: leaf visits with at most BHUT_SPLIT_MAXK active lanes are
-// split across the idle lanes; the split pair loop is unrolled
-// BHUT_SPLIT_UNROLL times.  Swept on GB300 at 1M Plummer (theta 0.5, leaf
-// 32): split at <= 16 active lanes 173.8 ms, at <= 8 178.9 ms, no split
-// 187.2 ms; split-loop unroll 2 173.8 ms, 1 174.0 ms, 4 175.7 ms.  The FP32
-// form's pair term is too cheap for the split to pay (63.9-64.1 ms against
-// 62.7 ms unsplit), so it keeps one lane per target.
-#ifndef BHUT_SPLIT_MAXK
-#define BHUT_SPLIT_MAXK 16
-#endif
-#ifndef BHUT_SPLIT_UNROLL
-#define BHUT_SPLIT_UNROLL 2
-#endif
-constexpr int kSplitMaxK = BHUT_SPLIT_MAXK;
-constexpr int kSplitUnroll = BHUT_SPLIT_UNROLL;
+// leaf_block_soft: leaf visits with at most kSplitMaxK active lanes are split
+// across the idle lanes.  (The FP32 form's pair term is too cheap for the
+// split to pay, 63.9-64.1 ms against 62.7 ms unsplit at 1M Plummer, so it
+// keeps one lane per target.)
+constexpr int kSplitMaxK = 16;
 static_assert(kSplitMaxK <= 16, "a split gives every active target at least two lanes");
 
-// The coordinates are represented to 2^-48 (normalised units), so a pair's
+// A displacement is known to about 2^-48 (normalised units), so a pair's
 // relative error is about 2^-48 / sqrt(R), R = r^2 + eps^2.
 // Softened path: every R is at least eps^2, and the range test is compiled
 // out when (eps s)^2 >= 2 kTinyR.
@@ -86,16 +70,32 @@ static __device__ void frame_unit_mass(double m0, bool uniform, FastFrame* f)
 }
 
 
-// hi on the 2^-23 grid and lo on the 2^-47 grid (both exact in FP32 for
-// |u| <= 1): differences of hi parts, and of lo parts, are then exact in
-// FP32; u is represented to within 2^-48.
-static __device__ __forceinline__ void split_grid(double u, float& h, float& l)
+// hi on the 2^-23 grid (differences of hi parts are exact in FP32 for |u| <=
+// 1) and lo the rest, |lo| <= 2^-24:
+//  * rounded to FP32 (`fine`, form "fast"): u is represented to within 2^-49,
+//    differences of lo parts are rounded to within 2^-48;
+//  * on the 2^-47 grid (form "fp32"): u to within 2^-48, differences exact.
+// The grid's own error was the largest of a float-float solve (200k Plummer,
+// softening 0.01: 9.6e-13 relative L2 against IEEE FP64, rounded lo parts
+// 5.5e-13); the FP32 form, at 3e-8, keeps the grid and its results.
+static __device__ __forceinline__ void split_grid(double u, bool fine, float& h, float& l)
 {
     double H = rint(__dmul_rn(u, 8388608.0));
     double hd = __dmul_rn(H, 1.0 / 8388608.0);
     h = __double2float_rn(hd);
-    double L = rint(__dmul_rn(__dsub_rn(u, hd), 140737488355328.0));   // 2^47
-    l = __double2float_rn(__dmul_rn(L, 1.0 / 140737488355328.0));
+    double r = __dsub_rn(u, hd);
+    if (!fine)
+        r = __dmul_rn(rint(__dmul_rn(r, 140737488355328.0)), 1.0 / 140737488355328.0);   // 2^47
+    l = __double2float_rn(r);
+}
+
+// A node's header flag: 0 without mass (skipped), 1, or 2 when its centre of
+// mass lies outside the box (masses of both signs): its coordinates are not
+// on the grid and its monopole is taken in FP64.
+static __device__ __forceinline__ int node_flag(const NodeCM& c, const float4& h)
+{
+    const bool out = !(fabsf(h.x) <= 1.0f && fabsf(h.y) <= 1.0f && fabsf(h.z) <= 1.0f);
+    return c.w == 0.0 ? 0 : (out ? 2 : 1);
 }
 
 static __device__ __forceinline__ void split_plain(double u, float& h, float& l)
@@ -135,7 +135,7 @@ static __device__ __forceinline__ float comp(const float4& v, int k)
 // selects, so the pair loop has no branch).
 //
 // d = hi_src - hi_tgt is exact on the grid and l = lo_src - lo_tgt is small
-// (|l| <= 2^-23), so (d, l) is renormalised with FastTwoSum into (gh, gl),
+// (|l| <= 2^-23, rounded to 2^-48), so (d, l) is renormalised with FastTwoSum into (gh, gl),
 // |gl| <= ulp(gh) / 2; every later product of a float-float with g then
 // keeps ~2^-47 relative accuracy.  A pair at zero displacement (the target
 // itself, or a duplicate) contributes exactly zero, as in the reference.
@@ -235,7 +235,7 @@ __device__ __forceinline__ void pair_ff_soft(const float* Th, const float* Tl, f
 #pragma unroll
     for (int k = 0; k < DIM; k++) {
         const float d = __fsub_rn(comp(sh, k), Th[k]);   // exact on the grid
-        const float l = __fsub_rn(comp(sl, k), Tl[k]);   // exact on the lo grid
+        const float l = __fsub_rn(comp(sl, k), Tl[k]);
         const float h = __fadd_rn(d, l);                  // FastTwoSum(d, l)
         gl[k] = __fsub_rn(l, __fsub_rn(h, d));
         gh[k] = h;
@@ -313,73 +313,356 @@ static __device__ __forceinline__ int nth_set_bit(unsigned m, int r)
     return pos;
 }
 
-// One block of cn <= 32 leaf particles, staged in sh/sl, for the targets of
-// the lanes in `mask` (those that opened the leaf's parent), float-float
-// soft path (pair_ff_soft).  Called by all 32 lanes.
+// ---------------------------------------------------------------------------
+// float-float pair term of a distant leaf
+// ---------------------------------------------------------------------------
+// The bounding box of a leaf gives a target bounds on everything the pair
+// term adds up, and a bound makes a compensated sum cheap: with an
+// accumulator s known to be at least as large as the term, t = fma(a, b, s)
+// has t - s exact (Sterbenz) and fma(a, b, -(t - s)) is the exact rounding
+// error -- three FP32 operations to add a PRODUCT without error, no ordering
+// of the operands and no separate two-product.  The biases cost bits where
+// the bounds are loose, so the term serves leaves whose max R is at most
+// kFarRatio times their min R.
+//   * r^2 starts at s0 >= max R (subtracted again exactly: R <= s0), so its
+//     three squares cost 5 operations each (with the cross term of the lo
+//     parts) instead of 9 and two min/max;
+//   * the leaf's force sums start at +-B, B a power of two above twice any
+//     term plus what the terms can take off it, on the side of the box
+//     (terms of the other sign come from |d_k| <= h_k - |g_k| only); B comes
+//     off exactly after the leaf.  6 operations per component instead of 9 and three of the
+//     ALU pipe;
+//   * the displacement stays (d, l) without renormalisation: |l| <= 2^-23,
+//     and the products with l are rounded once at 2^-24 of themselves, i.e.
+//     2^-47 / D of the pair -- the error that the coordinates have anyway
+//     (r^2 alone is renormalised);
+//   * y is the rsqrt of 2 R / 3: then w = y^3 (1 - A), A = R y^2 - 3/2, has
+//     no constant left (A^2 terms below 2^-43); the leaf's sums carry the
+//     factor (3/2)^(3/2), taken off at its end.
+// 56 FP32 operations and one MUFU per pair with unit masses, against 77, 15
+// on the ALU pipe and one MUFU of pair_ff_soft.
+constexpr float kFarScale = 0.54433105395181735517;   // (2/3)^(3/2), float-float
+constexpr float kFarScaleLo = 0.54433105395181735517 - (double)kFarScale;
+
 //
-// With more than 16 active lanes each lane adds its pairs in order to its
-// accumulator.  With k <= 16 active lanes the idle lanes are put to work:
-// every active target gets f lanes (f = 2..32, the largest power of two with
-// f k <= 32); lane j works for the active target of rank j / f, on the pairs
-// q = j mod f, j mod f + f, ..., into a float-float partial sum that starts
-// at zero; the f partials are added in a fixed tree order (shuffles down by
-// f/2, f/4, ..., 1) and the group's sum is added to the target's
-// accumulator with ff_add.  Leaf visits with at most 16 active lanes carry
-// most of the warp's idle lanes (a CPU replay of the walk at 1M Plummer,
-// theta 0.5, leaf 32: 16 % of the leaf steps, 84 % of the idle lane-steps),
-// and the split cuts the pair steps of a solve by about a tenth.  The order
-// of every addition depends only on the mask and cn, so a result does not
-// depend on which kernel (single tree or batched) evaluates it.
+// Two sources go through each operation together (f32x2: FADD2 / FFMA2, the
+// same IEEE operations; a difference is an FFMA2 by -1): half the issue slots
+// and two independent chains per lane.
+constexpr float kFarRatio = 16.0f;
+struct FarLeaf {
+    float s0;      // bias of r^2, at least max R
+    float si, li;  // s0 + eps^2 as si + li
+    float b[3];    // bias of the force sums
+};
+
+// One leaf block staged for a warp, two sources to a row: source 2p in the
+// even and 2p + 1 in the odd components.
+struct LeafStage {
+    float4 a[kWarp / 2];   // (x hi, x hi', y hi, y hi')
+    float4 b[kWarp / 2];   // (x lo, x lo', y lo, y lo')
+    float4 c[kWarp / 2];   // (z hi, z hi', z lo, z lo')
+    float4 d[kWarp / 2];   // (m hi, m hi', m lo, m lo')
+    __device__ __forceinline__ void put(int q, float4 h, float4 l)
+    {
+        const int p = q >> 1, o = q & 1;
+        float* A = reinterpret_cast<float*>(&a[p]) + o;
+        float* B = reinterpret_cast<float*>(&b[p]) + o;
+        float* C = reinterpret_cast<float*>(&c[p]) + o;
+        float* D = reinterpret_cast<float*>(&d[p]) + o;
+        A[0] = h.x; A[2] = h.y; B[0] = l.x; B[2] = l.y;
+        C[0] = h.z; C[2] = l.z; D[0] = h.w; D[2] = l.w;
+    }
+    // source 2p (odd = 0) or 2p + 1 as (x, y, z, m) hi and lo
+    __device__ __forceinline__ void get(int p, int odd, float4& h, float4& l) const
+    {
+        const float4 A = a[p], B = b[p], C = c[p], D = d[p];
+        h = odd ? make_float4(A.y, A.w, C.y, D.y) : make_float4(A.x, A.z, C.x, D.x);
+        l = odd ? make_float4(B.y, B.w, C.w, D.w) : make_float4(B.x, B.z, C.z, D.z);
+    }
+};
+
+// A leaf's bounding box (c, h: centre and half extents, with a margin of
+// 2^-21 for the lo parts of particles and targets and for rounding) and its
+// largest |mass| (negative when some mass is).
+struct LeafBox {
+    float4 c;   // w: mass
+    float4 h;
+};
+
+// For sums of at most np terms.  False: the leaf is not distant (max R over
+// min R may exceed kFarRatio, or min R < r_floor).
+template <int DIM>
+__device__ __forceinline__ bool far_setup(const float* T, const LeafBox& box, int np, float e2h,
+                                          float e2l, float r_floor, FarLeaf& f)
+{
+    float g[3] = {0.f, 0.f, 0.f}, rmin = e2h, rmax = e2h;
+#pragma unroll
+    for (int k = 0; k < DIM; k++) {
+        g[k] = __fsub_rn(comp(box.c, k), T[k]);
+        const float h = comp(box.h, k);
+        const float near = fmaxf(fabsf(g[k]) - h, 0.0f), away = fabsf(g[k]) + h;
+        rmin = fmaf(near, near, rmin);
+        rmax = fmaf(away, away, rmax);
+    }
+    rmax *= 1.0f + 0x1p-20f;
+    f.s0 = rmax;
+    f.si = __fadd_rn(rmax, e2h);
+    f.li = __fadd_rn(__fsub_rn(e2h, __fsub_rn(f.si, rmax)), e2l);
+    // |term k| <= 1.84 |m| |d_k| / rmin^(3/2), |d_k| <= away_k; terms of the
+    // other sign only where the target is inside the box's slab, and then
+    // |d_k| <= h_k - |g_k| (any |d_k| with masses of both signs)
+    const float ri = rsqrt_mufu(fmaxf(rmin, 0x1p-80f));
+    const float u = 3.69f * fabsf(box.c.w) * (ri * ri * ri);
+    const float n = (float)np;
+#pragma unroll
+    for (int k = 0; k < DIM; k++) {
+        const float ak = fabsf(g[k]), h = comp(box.h, k);
+        const float take = box.c.w < 0.0f ? ak + h : fmaxf(h - ak, 0.0f);
+        const float B = u * fmaf(n, take, ak + h);
+        f.b[k] = copysignf(
+            __int_as_float((__float_as_int(B) & 0x7f800000) + 0x00800000), g[k]);
+    }
+    return rmin * kFarRatio >= rmax && rmin >= r_floor;
+}
+
+static __device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+
+// -v by the sign bits: two ALU instructions, where the FP32 pipe is the
+// scarce one.
+static __device__ __forceinline__ float2 neg2(float2 v)
+{
+    return make_float2(__int_as_float(__float_as_int(v.x) ^ 0x80000000),
+                       __int_as_float(__float_as_int(v.y) ^ 0x80000000));
+}
+
+// Rows p = sub, sub + step, ... of a staged distant leaf of cn sources, as an
+// unbiased float-float sum.
+template <int DIM, bool UNIT>
+__device__ __forceinline__ void far_pairs(const float* Th, const float* Tl, const LeafStage& st,
+                                          int sub, int step, int cn, const FarLeaf& f, float* ph,
+                                          float* pl)
+{
+    float2 ah[3], al[3], nT[3], nL[3];
+#pragma unroll
+    for (int k = 0; k < DIM; k++) {
+        ah[k] = both(f.b[k]);
+        al[k] = both(0.0f);
+        nT[k] = both(-Th[k]);
+        nL[k] = both(-Tl[k]);
+    }
+    const float2 m1 = both(-1.0f), two = both(2.0f);
+    const int np = (cn + 1) >> 1;
+    // from the last row down: its odd source may not exist (a lane beyond the
+    // rows has none)
+#pragma unroll 1
+    for (int p = sub < np ? sub + (np - 1 - sub) / step * step : -1; p >= 0; p -= step) {
+        const float4 A = st.a[p], B = st.b[p];
+        float4 C = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (DIM == 3) C = st.c[p];
+        const float2 xh[3] = {make_float2(A.x, A.y), make_float2(A.z, A.w), make_float2(C.x, C.y)};
+        const float2 xl[3] = {make_float2(B.x, B.y), make_float2(B.z, B.w), make_float2(C.z, C.w)};
+        float2 d[3], l[3], s = both(f.si), lo = both(f.li);
+#pragma unroll
+        for (int k = 0; k < DIM; k++) {
+            d[k] = __fadd2_rn(xh[k], nT[k]);              // exact on the grid
+            l[k] = __fadd2_rn(xl[k], nL[k]);
+            const float2 t = __ffma2_rn(d[k], d[k], s);
+            const float2 q = __ffma2_rn(d[k], d[k], __ffma2_rn(t, m1, s));
+            lo = __ffma2_rn(__ffma2_rn(two, d[k], l[k]), l[k], lo);
+            lo = __fadd2_rn(lo, q);
+            s = t;
+        }
+        const float2 R0 = __fadd2_rn(s, both(-f.s0));     // exact: s <= 2 s0
+        const float2 R = __fadd2_rn(R0, lo);              // FastTwoSum(R0, lo)
+        lo = __fadd2_rn(lo, __ffma2_rn(R, m1, R0));
+        const float2 rs = __fmul2_rn(R, both(2.0f / 3.0f));
+        const float2 y = make_float2(rsqrt_mufu(rs.x), rsqrt_mufu(rs.y));
+        const float2 Y = __fmul2_rn(y, y);
+        const float2 Ye = __ffma2_rn(y, y, neg2(Y));
+        const float2 A1 = __ffma2_rn(R, Ye, __ffma2_rn(lo, Y, __ffma2_rn(R, Y, both(-1.5f))));
+        const float2 W = __fmul2_rn(Y, y), nW = neg2(W);
+        const float2 We = __ffma2_rn(Ye, y, __ffma2_rn(Y, y, nW));
+        float2 fh = W, fl = __ffma2_rn(nW, A1, We);
+        if (!UNIT) {
+            const float4 M = st.d[p];
+            const float2 mh = make_float2(M.x, M.y), ml = make_float2(M.z, M.w);
+            fh = __fmul2_rn(mh, W);
+            fl = __ffma2_rn(mh, fl, __ffma2_rn(ml, W, __ffma2_rn(mh, W, neg2(fh))));
+        }
+#pragma unroll
+        for (int k = 0; k < DIM; k++) {
+            const float2 t = __ffma2_rn(fh, d[k], ah[k]);
+            float2 r = __ffma2_rn(fh, d[k], __ffma2_rn(t, m1, ah[k]));
+            r = __ffma2_rn(fl, d[k], r);
+            r = __ffma2_rn(fh, l[k], r);
+            al[k] = __fadd2_rn(al[k], r);
+            ah[k] = t;
+        }
+        if (2 * p + 1 >= cn) {   // no odd source (this lane's first row): start over
+#pragma unroll
+            for (int k = 0; k < DIM; k++) { ah[k].y = f.b[k]; al[k].y = 0.0f; }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < DIM; k++) {
+        const float hx = __fsub_rn(ah[k].x, f.b[k]), hy = __fsub_rn(ah[k].y, f.b[k]);
+        const float h = __fadd_rn(hx, hy);
+        const float l = __fadd_rn(two_sum_err(hx, hy, h), __fadd_rn(al[k].x, al[k].y));
+        ph[k] = __fmul_rn(h, kFarScale);
+        pl[k] = __fmaf_rn(l, kFarScale, __fmaf_rn(h, kFarScaleLo, __fmaf_rn(h, kFarScale, -ph[k])));
+    }
+}
+
+// The same rows of a near leaf with pair_ff_soft, added to (ph, pl).
+template <int DIM, bool UNIT>
+__device__ __forceinline__ void near_pairs(const float* Th, const float* Tl, const LeafStage& st,
+                                           int sub, int step, int cn, float e2h, float e2l,
+                                           float* ph, float* pl)
+{
+#pragma unroll 1
+    for (int p = sub; 2 * p < cn; p += step) {
+        float4 h, l;
+        st.get(p, 0, h, l);
+        pair_ff_soft<DIM, UNIT>(Th, Tl, h, l, e2h, e2l, ph, pl);
+        if (2 * p + 1 < cn) {
+            st.get(p, 1, h, l);
+            pair_ff_soft<DIM, UNIT>(Th, Tl, h, l, e2h, e2l, ph, pl);
+        }
+    }
+}
+
+// Lanes of a leaf visit.  More than kSplitMaxK active targets: every lane
+// works for itself.  Fewer, k: f lanes for each active target; lane j works
+// for the active target of rank j / f.
+struct LaneSplit {
+    int f = 1, sub = 0, owner, leader;
+    bool work;
+    __device__ __forceinline__ LaneSplit(unsigned mask, int lane)
+    {
+        const int k = __popc(mask);
+        owner = leader = lane;
+        work = (mask >> lane) & 1u;
+        if (k <= kSplitMaxK) {
+            const bool mine = work;
+            f = 2;
+            while (f * 2 * k <= kWarp) f *= 2;
+            const int r = lane / f;
+            sub = lane & (f - 1);
+            work = r < k;
+            owner = nth_set_bit(mask, work ? r : 0);
+            leader = mine ? __popc(mask & ((1u << lane) - 1u)) * f : 0;
+        }
+    }
+};
+
+// The lanes' partial sums (ph, pl) of a visit, added in a fixed order per
+// target and to the accumulators (ah, al) of the active lanes.
+template <int DIM>
+__device__ __forceinline__ void split_add(const LaneSplit& sp, bool mine, float* ph, float* pl,
+                                          float* ah, float* al)
+{
+    const unsigned FULL = 0xffffffffu;
+    if (sp.f > 1) {
+        for (int o = sp.f >> 1; o >= 1; o >>= 1) {
+#pragma unroll
+            for (int c = 0; c < DIM; c++) {
+                const float bh = __shfl_down_sync(FULL, ph[c], o);
+                const float bl = __shfl_down_sync(FULL, pl[c], o);
+                ff_add(ph[c], pl[c], bh, bl);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < DIM; c++) {
+            ph[c] = __shfl_sync(FULL, ph[c], sp.leader);
+            pl[c] = __shfl_sync(FULL, pl[c], sp.leader);
+        }
+    }
+    if (mine) {
+#pragma unroll
+        for (int c = 0; c < DIM; c++) ff_add(ah[c], al[c], ph[c], pl[c]);
+    }
+}
+
+// The coordinates a lane works on in a visit: its own target's, or those of
+// the target it was given.
+template <int DIM>
+__device__ __forceinline__ void split_target(const LaneSplit& sp, const float* Th, const float* Tl,
+                                             float* T, float* L)
+{
+#pragma unroll
+    for (int c = 0; c < DIM; c++) {
+        T[c] = Th[c];
+        L[c] = Tl[c];
+        if (sp.f > 1) {
+            T[c] = __shfl_sync(0xffffffffu, Th[c], sp.owner);
+            L[c] = __shfl_sync(0xffffffffu, Tl[c], sp.owner);
+        }
+    }
+}
+
+// One staged block of cn <= 32 leaf particles for the targets of the lanes in
+// `mask` (those that opened the leaf's parent), float-float soft path
+// (far_pairs when the leaf is distant for every working lane, else
+// pair_ff_soft).  Called by all 32 lanes.
+//
+// With more than 16 active lanes each lane sums its own target's pairs.  With
+// k <= 16 active lanes the idle lanes are put to work: every active target
+// gets f lanes (f = 2..32, the largest power of two with f k <= 32); lane j
+// works for the active target of rank j / f, on the rows (two sources)
+// j mod f, j mod f + f, ..., into a float-float partial sum; the f partials
+// are added in a fixed tree order (shuffles down by f/2, f/4, ..., 1) and the
+// sum is added to the target's accumulator with ff_add.  Leaf visits with at
+// most 16 active lanes carry most of the warp's idle lanes (a CPU replay of
+// the walk at 1M Plummer, theta 0.5, leaf 32: 16 % of the leaf steps, 84 % of
+// the idle lane-steps), and the split cuts the pair steps of a solve by about
+// a tenth.  The order of every addition depends only on the mask and cn, so a
+// result does not depend on which kernel (single tree or batched) evaluates
+// it.  One loop serves full and split visits: the loops' code competes for
+// the instruction cache.
 template <int DIM, bool UNIT>
 __device__ __forceinline__ void leaf_block_soft(unsigned mask, int lane, const float* Th,
-                                                const float* Tl, const float4* sh,
-                                                const float4* sl, int cn, float e2h, float e2l,
+                                                const float* Tl, const LeafStage& st, int cn,
+                                                const LeafBox& box, float e2h, float e2l,
                                                 float* ah, float* al)
 {
     const unsigned FULL = 0xffffffffu;
-    const bool mine = (mask >> lane) & 1u;
-    const int k = __popc(mask);
-    if (k == 0) return;
-    if (k > kSplitMaxK) {
-        if (mine) {
-#pragma unroll (kFFUnroll)
-            for (int q = 0; q < cn; q++)
-                pair_ff_soft<DIM, UNIT>(Th, Tl, sh[q], sl[q], e2h, e2l, ah, al);
-        }
-        return;
-    }
-    int f = 2;
-    while (f * 2 * k <= kWarp) f *= 2;
-    const int r = lane / f, sub = lane & (f - 1);
-    const bool work = r < k;
-    const int owner = nth_set_bit(mask, work ? r : 0);
+    if (mask == 0) return;
+    const LaneSplit sp(mask, lane);
     float T[3] = {0.f, 0.f, 0.f}, L[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-    for (int c = 0; c < DIM; c++) {
-        T[c] = __shfl_sync(FULL, Th[c], owner);
-        L[c] = __shfl_sync(FULL, Tl[c], owner);
-    }
+    split_target<DIM>(sp, Th, Tl, T, L);
     float ph[3] = {0.f, 0.f, 0.f}, pl[3] = {0.f, 0.f, 0.f};
-    if (work) {
-#pragma unroll (kSplitUnroll)
-        for (int q = sub; q < cn; q += f)
-            pair_ff_soft<DIM, UNIT>(T, L, sh[q], sl[q], e2h, e2l, ph, pl);
+    FarLeaf f;
+    const bool far = far_setup<DIM>(T, box, (cn + 1) >> 1, e2h, e2l, 0.0f, f);
+    if (__all_sync(FULL, far || !sp.work)) {
+        if (sp.work) far_pairs<DIM, UNIT>(T, L, st, sp.sub, sp.f, cn, f, ph, pl);
+    } else {
+        if (sp.work) near_pairs<DIM, UNIT>(T, L, st, sp.sub, sp.f, cn, e2h, e2l, ph, pl);
     }
-    for (int o = f >> 1; o >= 1; o >>= 1) {
+    split_add<DIM>(sp, (mask >> lane) & 1u, ph, pl, ah, al);
+}
+
+// The LeafBox of particles [start, start + count).
+static __device__ __forceinline__ void leaf_box(const float4* __restrict__ ph, int start,
+                                                int count, float4& c, float4& h)
+{
+    float lo[3] = {4.f, 4.f, 4.f}, hi[3] = {-4.f, -4.f, -4.f}, mx = 0.0f;
+    bool neg = false;
+#pragma unroll 8
+    for (int i = start; i < start + count; i++) {
+        const float4 p = ph[i];
 #pragma unroll
-        for (int c = 0; c < DIM; c++) {
-            const float bh = __shfl_down_sync(FULL, ph[c], o);
-            const float bl = __shfl_down_sync(FULL, pl[c], o);
-            ff_add(ph[c], pl[c], bh, bl);
+        for (int k = 0; k < 3; k++) {
+            lo[k] = fminf(lo[k], comp(p, k));
+            hi[k] = fmaxf(hi[k], comp(p, k));
         }
+        mx = fmaxf(mx, fabsf(p.w));
+        neg |= p.w < 0.0f;
     }
-    const int leader = mine ? __popc(mask & ((1u << lane) - 1u)) * f : 0;
-#pragma unroll
-    for (int c = 0; c < DIM; c++) {
-        const float gh = __shfl_sync(FULL, ph[c], leader);
-        const float gl = __shfl_sync(FULL, pl[c], leader);
-        if (mine) ff_add(ah[c], al[c], gh, gl);
-    }
+    c = make_float4(0.5f * (lo[0] + hi[0]), 0.5f * (lo[1] + hi[1]), 0.5f * (lo[2] + hi[2]),
+                    neg ? -mx : mx);
+    const float s = 1.0f + 0x1p-20f, o = 0x1p-21f;
+    h = make_float4(fmaf(0.5f * (hi[0] - lo[0]), s, o), fmaf(0.5f * (hi[1] - lo[1]), s, o),
+                    fmaf(0.5f * (hi[2] - lo[2]), s, o), 0.0f);
 }
 
 // FP64 pair in physical units, G-less (the Numba loop arithmetic).

@@ -9,24 +9,23 @@
 //
 //  * Coordinates are shifted to the tree's box centre and scaled by a power
 //    of two into [-1/2, 1/2]; each coordinate is stored as hi + lo with hi on
-//    the 2^-23 grid and lo on the 2^-47 grid (|lo| <= 2^-24), so hi_j - hi_i
-//    and lo_j - lo_i are exact in FP32 and the displacement is exact up to
-//    the 2^-48 representation of the coordinates.  Masses are scaled by a power
-//    of two into [-1, 1] and split hi + lo.  Scales are undone in FP64.
-//  * r^2 + eps^2 is summed error-free (two-product squares, TwoSum of the
-//    high parts); (r^2)^(-3/2) is the hardware rsqrt refined by one
-//    correction step, w = y^3 (1 + 3e/2 + 15e^2/8) with e = 1 - r^2 y^2
-//    computed exactly (Newton-Raphson for the inverse square root, carried
-//    to second order; the softened term pair_ff_soft stops at first order);
-//    m * w * dx and the accumulation are float-float (Dekker/Knuth
-//    two-product and TwoSum).
-//  * A pair's relative error is dominated by the 2^-48 coordinate
-//    representation: about 2^-48 / sqrt(r^2 + eps^2).  With a softening
-//    that bounds r^2 + eps^2 from below ((eps s)^2 >= 2^-33) every pair is
-//    float-float and the range test is compiled out; otherwise pairs with
-//    r^2 + eps^2 below 2^-26 in normalised units (softened distance under
-//    2^-13 of the box half-size), or outside the FP32 range, are evaluated
-//    in FP64 from the FP64 arrays, so a float-float pair stays below 2^-35.
+//    the 2^-23 grid and lo the rest in FP32 (|lo| <= 2^-24), so hi_j - hi_i
+//    is exact in FP32 and the displacement is known to about 2^-48.  Masses
+//    are scaled by a power of two into [-1, 1] and split hi + lo.  Scales are
+//    undone in FP64.
+//  * r^2 + eps^2 is summed error-free; (r^2)^(-3/2) is the hardware rsqrt
+//    refined by one correction step from the exactly computed residual
+//    (Newton-Raphson for the inverse square root; carried to second order
+//    in the checked term); m * w * dx and the accumulation are float-float
+//    (Dekker/Knuth two-product and TwoSum, or sums biased by a leaf's bounds:
+//    pair terms and figures in fast.cuh).
+//  * A pair's relative error is dominated by the coordinates: about
+//    2^-48 / sqrt(r^2 + eps^2).  With a softening that bounds r^2 + eps^2
+//    from below ((eps s)^2 >= 2^-33) every pair is float-float and the range
+//    test is compiled out; otherwise pairs with r^2 + eps^2 below 2^-26 in
+//    normalised units (softened distance under 2^-13 of the box half-size),
+//    or outside the FP32 range, are evaluated in FP64 from the FP64 arrays,
+//    so a float-float pair stays below 2^-35.
 //  * The opening decision is the reference's, bit for bit: a FP32 test
 //    decides every node whose ratio is clearly above or below theta, and
 //    nodes inside a small error band are decided by the exact FP64 test of
@@ -38,30 +37,41 @@ namespace bhut {
 
 constexpr int kFastWarps = 4;
 constexpr int kFastThreads = kFastWarps * kWarp;
+constexpr int kSplitMaxLevels = 10;
 // Tuning (overridable at build time): resident blocks per SM for the fast
-// form (6: 24 warps per SM, registers capped at 80) and the unroll factors
-// of the leaf pair loops.  Swept on GB300 at 1M Plummer: unroll 4 / 8 beat
-// 1-2 / 1-4 by 2-10 %; 5 blocks per SM (96 registers) gains nothing.
+// form (5: 20 warps per SM, registers capped at 96; 4 / 5 / 6 blocks at 1M
+// Plummer 142.4 / 140.5 / 139.1 ms, at 200k 22.5 / 23.0 / 23.8 ms, without
+// softening at 200k 11.0 / 10.6 / 11.3 ms) and the unroll factor of the FP32
+// form's leaf pair loop (8 beats 1-4 by 2-10 %).
 #ifndef BHUT_FAST_BLOCKS
-#define BHUT_FAST_BLOCKS 6
+#define BHUT_FAST_BLOCKS 5
 #endif
 #ifndef BHUT_F32_UNROLL
 #define BHUT_F32_UNROLL 8
 #endif
-// Self accelerations of few targets: up to this many lanes per target (1, 2
-// or 4; k_traverse_fast_lpt).
-#ifndef BHUT_FAST_MAX_LPT
-#define BHUT_FAST_MAX_LPT 4
+// Split traversals (fast_split_levels): split while fewer warps than this walk
+// and their subtrees hold more nodes than that.  Swept on GB300:
+//   warps (ms)            none   6144  12288  24576  49152  98304
+//   10k self              1.26   0.34   0.33   0.35   0.34   0.33
+//   60k self              6.31   5.08   4.74   4.66   4.55   4.48
+//   200k self             23.0      -      -      -   23.3   24.5
+//   2,000 targets of 1M   28.8   1.56   1.28   1.20   1.16   1.17
+//   100k targets of 1M    21.2   21.2   17.2   16.2   14.5   17.2
+//   250k targets of 1M    31.0   31.0   30.7   30.6   29.4   30.4
+//   1M self                139      -      -      -    139    181
+//   nodes                 4 / 8 / 16 / 32: 10k self 0.42 / 0.35 / 0.34 / 0.33,
+//                         1,000 self 0.10 / 0.10 / 0.11 / 0.20
+// Self targets that fill the GPU once (kWaveWarps) are not split: neighbours
+// then share what the walk reads, and a split gives it up (100k uniform cube
+// without softening 5.04 ms unsplit, 5.87 to 6.58 split; 100k Plummer 10.3,
+// 9.3 to 10.0).  External targets vary more from group to group, and the
+// shorter walks balance.
+#ifndef BHUT_SPLIT_WARPS
+#define BHUT_SPLIT_WARPS 49152
 #endif
-// ... chosen so that at least this many warps per SM share the work
-#ifndef BHUT_FAST_LPT_WARPS_PER_SM
-#define BHUT_FAST_LPT_WARPS_PER_SM 8
-#endif
-static_assert(BHUT_FAST_MAX_LPT == 1 || BHUT_FAST_MAX_LPT == 2 || BHUT_FAST_MAX_LPT == 4 ||
-              BHUT_FAST_MAX_LPT == 8, "lanes per target: 1, 2, 4 or 8");
-// Checked path (small or no softening): split sparse leaf visits (1) or not.
-#ifndef BHUT_CHECK_SPLIT
-#define BHUT_CHECK_SPLIT 1
+constexpr int64_t kWaveWarps = 152 * 4 * 5;   // resident warps of k_traverse_fast
+#ifndef BHUT_SPLIT_NODES
+#define BHUT_SPLIT_NODES 16
 #endif
 constexpr int kFastBlocksPerSM = BHUT_FAST_BLOCKS;
 constexpr int kF32Unroll = BHUT_F32_UNROLL;
@@ -79,16 +89,16 @@ __global__ void k_frame(const double* __restrict__ box, int dim, FastFrame* __re
 
 __global__ void k_ff_particles(const double* __restrict__ sx, const double* __restrict__ sy,
                                const double* __restrict__ sz, const double* __restrict__ sm,
-                               int64_t n, int dim, const FastFrame* __restrict__ fr,
+                               int64_t n, int dim, bool fine, const FastFrame* __restrict__ fr,
                                float4* __restrict__ ph, float4* __restrict__ pl)
 {
     const FastFrame f = *fr;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
         float4 h, l;
-        split_grid(__dmul_rn(__dsub_rn(sx[i], f.c[0]), f.s), h.x, l.x);
-        split_grid(__dmul_rn(__dsub_rn(sy[i], f.c[1]), f.s), h.y, l.y);
-        if (dim == 3) split_grid(__dmul_rn(__dsub_rn(sz[i], f.c[2]), f.s), h.z, l.z);
+        split_grid(__dmul_rn(__dsub_rn(sx[i], f.c[0]), f.s), fine, h.x, l.x);
+        split_grid(__dmul_rn(__dsub_rn(sy[i], f.c[1]), f.s), fine, h.y, l.y);
+        if (dim == 3) split_grid(__dmul_rn(__dsub_rn(sz[i], f.c[2]), f.s), fine, h.z, l.z);
         else h.z = l.z = 0.0f;
         if (f.unit) { h.w = 1.0f; l.w = 0.0f; }   // every mass is m0: exactly 1 in units of m0
         else split_plain(__dmul_rn(sm[i], f.ms), h.w, l.w);
@@ -97,12 +107,12 @@ __global__ void k_ff_particles(const double* __restrict__ sx, const double* __re
     }
 }
 
-__global__ void k_ff_nodes(TreeDev t, const double* __restrict__ center,
+__global__ void k_ff_nodes(TreeDev t, bool fine, const double* __restrict__ center,
                            const FastFrame* __restrict__ fr, float4* __restrict__ nh,
                            float4* __restrict__ nl, float* __restrict__ nsize,
                            float* __restrict__ ndelta, const double* __restrict__ quad,
                            float4* __restrict__ nq0, float2* __restrict__ nq1,
-                           int4* __restrict__ nhdr)
+                           int4* __restrict__ nhdr, const float4* __restrict__ ph)
 {
     const FastFrame f = *fr;
     const int dim = t.dim;
@@ -111,12 +121,13 @@ __global__ void k_ff_nodes(TreeDev t, const double* __restrict__ center,
         NodeCM c = t.cm[k];
 
         float4 h, l;
-        // a node's COM lies inside the box: |u| <= 1 up to rounding
-        split_grid(__dmul_rn(__dsub_rn(c.x, f.c[0]), f.s), h.x, l.x);
-        split_grid(__dmul_rn(__dsub_rn(c.y, f.c[1]), f.s), h.y, l.y);
-        if (dim == 3) split_grid(__dmul_rn(__dsub_rn(c.z, f.c[2]), f.s), h.z, l.z);
+        split_grid(__dmul_rn(__dsub_rn(c.x, f.c[0]), f.s), fine, h.x, l.x);
+        split_grid(__dmul_rn(__dsub_rn(c.y, f.c[1]), f.s), fine, h.y, l.y);
+        if (dim == 3) split_grid(__dmul_rn(__dsub_rn(c.z, f.c[2]), f.s), fine, h.z, l.z);
         else h.z = l.z = 0.0f;
+        const int fc = t.first_child[k];
         split_plain(__dmul_rn(c.w, f.ms), h.w, l.w);
+        if (fc < 0) leaf_box(ph, t.start[k], t.count[k], h, l);   // (LeafBox in a leaf's place)
         nh[k] = h;
         nl[k] = l;
         nsize[k] = __double2float_rn(__dmul_rn(t.size[k], f.s));
@@ -128,12 +139,11 @@ __global__ void k_ff_nodes(TreeDev t, const double* __restrict__ center,
             dd += v * v;
         }
         ndelta[k] = __double2float_ru(sqrt(dd) * f.s);
-        // header: leaf (-1, start, count, mass != 0); internal (first child,
-        // size, |com - centre| as float bits, mass != 0)
-        const int fc = t.first_child[k];
+        // header: leaf (-1, start, count, flag); internal (first child, size,
+        // |com - centre| as float bits, flag)
         nhdr[k] = fc < 0 ? make_int4(fc, t.start[k], t.count[k], c.w != 0.0)
                          : make_int4(fc, __float_as_int(nsize[k]), __float_as_int(ndelta[k]),
-                                     c.w != 0.0);
+                                     node_flag(c, h));
         if (quad) {   // mass x length^2: scale by ms s^2
             const double qs = f.ms * f.s * f.s;
             const double* q = quad + 6 * k;
@@ -147,7 +157,7 @@ __global__ void k_ff_nodes(TreeDev t, const double* __restrict__ center,
 // Targets: grid split when inside the box (|u| <= 1), plain split otherwise;
 // th.w = 1 marks a target outside the box, tl.w = max |u|.
 __global__ void k_ff_targets(const double* __restrict__ tx, const double* __restrict__ ty,
-                             const double* __restrict__ tz, int64_t nt, int dim,
+                             const double* __restrict__ tz, int64_t nt, int dim, bool fine,
                              const FastFrame* __restrict__ fr, float4* __restrict__ th,
                              float4* __restrict__ tl)
 {
@@ -161,7 +171,7 @@ __global__ void k_ff_targets(const double* __restrict__ tx, const double* __rest
         bool inside = amax <= 1.0;
         float hh[3], ll[3];
         for (int d = 0; d < 3; d++) {
-            if (inside) split_grid(u[d], hh[d], ll[d]);
+            if (inside) split_grid(u[d], fine, hh[d], ll[d]);
             else split_plain(u[d], hh[d], ll[d]);
         }
         th[i] = make_float4(hh[0], hh[1], hh[2], inside ? 0.0f : 1.0f);
@@ -190,61 +200,53 @@ struct FastArgs {
 };
 
 // leaf_block_soft for the checked path (targets inside the box, softening
-// too small to bound r^2 + eps^2 from below: pair_ff with the range test,
-// pairs below kTinyRCheck taken in FP64 from the FP64 particle arrays).  The
-// split is the same; a lane that works for another lane's target also
-// takes that target's FP64 pairs (the target's FP64 coordinates come by
-// shuffle) and the group adds its FP64 partial sums like the float-float
-// ones.  `nfb` counts the FP64 pairs a lane evaluated.
-template <int DIM>
+// too small to bound r^2 + eps^2 from below: near leaves take pair_ff with
+// the range test, pairs below kTinyRCheck in FP64 from the FP64 particle
+// arrays).  The split is the same; a lane that works for another lane's
+// target also takes that target's FP64 pairs (the target's FP64 coordinates
+// are read from memory) and the group adds its FP64 partial sums like the
+// float-float ones.  `nfb` counts the FP64 pairs a lane evaluated.
+template <int DIM, bool UNIT>
 __device__ __forceinline__ void leaf_block_check(unsigned mask, int lane, const float* Th,
-                                                 const float* Tl, double x, double y, double z,
-                                                 const float4* sh, const float4* sl, int cn,
-                                                 int first, const TreeDev& t, float e2h,
-                                                 float e2l, double eps2, float* ah, float* al,
-                                                 double* a64, unsigned& nfb)
+                                                 const float* Tl, const FastArgs& a, int64_t base,
+                                                 const LeafStage& st, int cn, int first,
+                                                 const TreeDev& t, const LeafBox& box, double eps2,
+                                                 float* ah, float* al, double* a64, unsigned& nfb)
 {
     const unsigned FULL = 0xffffffffu;
+    if (mask == 0) return;
+    const LaneSplit sp(mask, lane);
     const bool mine = (mask >> lane) & 1u;
-    const int k = __popc(mask);
-    if (k == 0) return;
-    if (k > kSplitMaxK || !BHUT_CHECK_SPLIT) {
-        if (mine) {
-            unsigned fb = 0;
-#pragma unroll (kFFUnroll)
-            for (int q = 0; q < cn; q++)
-                fb |= (unsigned)!pair_ff<DIM, false, true>(Th, Tl, sh[q], sl[q], e2h, e2l, ah,
-                                                           al) << q;
-            while (fb) {
-                const int gi = first + __ffs(fb) - 1;
-                fb &= fb - 1;
-                pair_fp64<DIM>(x, y, z, t.sx[gi], t.sy[gi], DIM == 3 ? t.sz[gi] : 0.0, t.sm[gi],
-                               eps2, a64);
-                nfb++;
-            }
-        }
+    float T[3] = {0.f, 0.f, 0.f}, L[3] = {0.f, 0.f, 0.f};
+    split_target<DIM>(sp, Th, Tl, T, L);
+    float ph[3] = {0.f, 0.f, 0.f}, pl[3] = {0.f, 0.f, 0.f};
+    FarLeaf f;
+    const bool far = far_setup<DIM>(T, box, (cn + 1) >> 1, a.e2h, a.e2l, kTinyRCheck, f);
+    if (__all_sync(FULL, far || !sp.work)) {
+        if (sp.work) far_pairs<DIM, UNIT>(T, L, st, sp.sub, sp.f, cn, f, ph, pl);
+        split_add<DIM>(sp, mine, ph, pl, ah, al);
         return;
     }
-    int f = 2;
-    while (f * 2 * k <= kWarp) f *= 2;
-    const int r = lane / f, sub = lane & (f - 1);
-    const bool work = r < k;
-    const int owner = nth_set_bit(mask, work ? r : 0);
-    float T[3] = {0.f, 0.f, 0.f}, L[3] = {0.f, 0.f, 0.f};
+    unsigned fb = 0;
+    if (sp.work) {
+#pragma unroll 1
+        for (int p = sp.sub; 2 * p < cn; p += sp.f) {
 #pragma unroll
-    for (int c = 0; c < DIM; c++) {
-        T[c] = __shfl_sync(FULL, Th[c], owner);
-        L[c] = __shfl_sync(FULL, Tl[c], owner);
+            for (int o = 0; o < 2; o++) {
+                const int q = 2 * p + o;
+                if (q >= cn) break;
+                float4 h, l;
+                st.get(p, o, h, l);
+                fb |= (unsigned)!pair_ff<DIM, false, true>(T, L, h, l, a.e2h, a.e2l, ph, pl) << q;
+            }
+        }
     }
-    const double X = __shfl_sync(FULL, x, owner), Y = __shfl_sync(FULL, y, owner);
-    const double Z = __shfl_sync(FULL, z, owner);
-    float ph[3] = {0.f, 0.f, 0.f}, pl[3] = {0.f, 0.f, 0.f};
+    split_add<DIM>(sp, mine, ph, pl, ah, al);
+    if (!__any_sync(FULL, fb != 0)) return;
     double p64[3] = {0.0, 0.0, 0.0};
-    if (work) {
-        unsigned fb = 0;
-#pragma unroll (kSplitUnroll)
-        for (int q = sub; q < cn; q += f)
-            fb |= (unsigned)!pair_ff<DIM, false, true>(T, L, sh[q], sl[q], e2h, e2l, ph, pl) << q;
+    if (fb) {
+        const int64_t i = base + sp.owner;
+        const double X = a.tx[i], Y = a.ty[i], Z = DIM == 3 ? a.tz[i] : 0.0;
         while (fb) {
             const int gi = first + __ffs(fb) - 1;
             fb &= fb - 1;
@@ -253,109 +255,92 @@ __device__ __forceinline__ void leaf_block_check(unsigned mask, int lane, const 
             nfb++;
         }
     }
-    for (int o = f >> 1; o >= 1; o >>= 1) {
+    for (int o = sp.f >> 1; o >= 1; o >>= 1) {
 #pragma unroll
-        for (int c = 0; c < DIM; c++) {
-            const float bh = __shfl_down_sync(FULL, ph[c], o);
-            const float bl = __shfl_down_sync(FULL, pl[c], o);
-            ff_add(ph[c], pl[c], bh, bl);
+        for (int c = 0; c < DIM; c++)
             p64[c] = __dadd_rn(p64[c], __shfl_down_sync(FULL, p64[c], o));
-        }
     }
-    const int leader = mine ? __popc(mask & ((1u << lane) - 1u)) * f : 0;
 #pragma unroll
     for (int c = 0; c < DIM; c++) {
-        const float gh = __shfl_sync(FULL, ph[c], leader);
-        const float gl = __shfl_sync(FULL, pl[c], leader);
-        const double g64 = __shfl_sync(FULL, p64[c], leader);
-        if (mine) {
-            ff_add(ah[c], al[c], gh, gl);
-            a64[c] = __dadd_rn(a64[c], g64);
-        }
+        const double g64 = __shfl_sync(FULL, p64[c], sp.leader);
+        if (mine) a64[c] = __dadd_rn(a64[c], g64);
     }
 }
 
-// SOFT_PATH (= !FAR && !CHECK): every pair is taken by pair_ff_soft (no
-// FP64 fallback); UNIT: leaf pairs skip the mass product (unit masses).
-// LPT > 1 (soft path only): LPT consecutive lanes hold the same target; they
-// take the same opening decisions, share its leaf pairs (lane j of the group
-// takes pairs j, j + LPT, ...), the group's first lane alone adds monopoles
-// and counts, and the caller adds the lanes' sums.
-template <int DIM, bool FAR, bool CHECK, bool UNIT = false, int LPT = 1>
+// SOFT_PATH (= !FAR && !CHECK): every pair is float-float (no FP64
+// fallback); UNIT: leaf pairs skip the mass product (unit masses).
+// SPLIT: 2^levels warps share the targets; a warp follows the bits of `path`
+// (highest first) through the top `levels` levels and walks the subtree it
+// reaches.  A node of those levels is worked on (leaf, monopoles, counts) by
+// the warp whose remaining bits are zero.
+template <int DIM, bool FAR, bool CHECK, bool UNIT, bool SPLIT>
 __device__ __forceinline__ void walk(const TreeDev& t, const FastTree& ft, const FastArgs& a,
-                                     int w, int lane, bool valid, int64_t me_sorted, const float* Th,
-                                     const float* Tl, float band_abs, double x, double y, double z,
-                                     float* ah, float* al, double* a64, int2 (*stack)[kStackDepth],
-                                     float4 (*sh)[kWarp], float4 (*sl)[kWarp],
-                                     unsigned* cnt, bool& overflow)
+                                     int w, int lane, bool valid, int64_t base, int64_t me_sorted,
+                                     const float* Th, const float* Tl, float band_abs, float* ah,
+                                     float* al, double* a64, int2 (*stack)[kStackDepth],
+                                     LeafStage* stage, unsigned* cnt, bool& overflow,
+                                     int levels = 0, int path = 0)
 {
-    static_assert(LPT == 1 || (!FAR && !CHECK), "lane groups serve the soft path only");
     const unsigned FULL = 0xffffffffu;
-    const float theta_f = (float)a.theta;
+    const float theta_f = (float)a.theta, theta2 = theta_f * theta_f;
     const double eps2 = __dmul_rn(a.eps, a.eps);
-    const bool lead = (lane & (LPT - 1)) == 0;   // first lane of the target's group
-    const int sub = lane & (LPT - 1);
-    const unsigned live = __ballot_sync(FULL, valid);
-    if (lane == 0) stack[w][0] = make_int2(0, (int)live);
-    int sp = 1;
-    __syncwarp();
-    while (sp > 0) {
-        const int2 e = stack[w][--sp];
-        __syncwarp();
-        const int node = e.x;
-        const unsigned mask = (unsigned)e.y;
+    const int64_t me = base + lane;              // the lane's target
+    bool own = !SPLIT || path == 0;              // this warp works on the node
+    // The right child of an opened node is visited next, straight from
+    // registers; only left children go through the stack.  A visit's three
+    // loads (a leaf's box lies where an internal node has its centre of mass)
+    // are issued together.
+    int node = 0, sp = 0;
+    unsigned mask = __ballot_sync(FULL, valid);
+    while (true) {
         const bool act = (mask >> lane) & 1u;
-        cnt[2] += act && lead;
-        const int4 hd = ft.nhdr[node];   // (first_child, start, count, mass != 0)
-        if (!hd.w) continue;              // mass == 0 skip (bh.py:514)
+        cnt[2] += act && own;
+        const int4 hd = ft.nhdr[node];   // (first_child, start, count, flag)
+        const float4 nh = ft.nh[node], nl = ft.nl[node];
         const int fc = hd.x;
-        if (fc < 0) {
-            const int s = hd.y, c = hd.z;
+        if (!hd.w) {                      // mass == 0 skip (bh.py:514)
+        } else if (fc < 0) {
+            const int s = hd.y, c = own ? hd.z : 0;
+            LeafBox box{nh, nl};
+            if (UNIT) box.c.w = 1.0f;
             for (int b = 0; b < c; b += kWarp) {
                 const int jj = b + lane;
-                if (jj < c) {
-                    sh[w][lane] = ft.ph[s + jj];
-                    sl[w][lane] = ft.pl[s + jj];
-                }
+                if (jj < c) stage[w].put(lane, ft.ph[s + jj], ft.pl[s + jj]);
                 __syncwarp();
                 const int cn = min(kWarp, c - b);
-                if (act && lead) {
+                if (act) {
                     // The target itself (self mode: sorted index `me_sorted`)
                     // sits at zero displacement and adds exactly zero, so it
                     // is not skipped; it is only left out of the pair count
                     // (bh.py:254).
                     cnt[0] += cn - (me_sorted >= s + b && me_sorted < s + b + cn);
                 }
-                if (!FAR && !CHECK && LPT == 1) {
-                    leaf_block_soft<DIM, UNIT>(mask, lane, Th, Tl, sh[w], sl[w], cn, a.e2h, a.e2l,
+                if (!FAR && !CHECK) {
+                    leaf_block_soft<DIM, UNIT>(mask, lane, Th, Tl, stage[w], cn, box, a.e2h, a.e2l,
                                                ah, al);
-                } else if (!FAR && !CHECK) {
-                    if (act) {
-#pragma unroll (kSplitUnroll)
-                        for (int q = sub; q < cn; q += LPT)
-                            pair_ff_soft<DIM, UNIT>(Th, Tl, sh[w][q], sl[w][q], a.e2h, a.e2l, ah,
-                                                    al);
-                    }
                 } else if (!FAR) {
-                    leaf_block_check<DIM>(mask, lane, Th, Tl, x, y, z, sh[w], sl[w], cn, s + b, t,
-                                          a.e2h, a.e2l, eps2, ah, al, a64, cnt[4]);
+                    leaf_block_check<DIM, UNIT>(mask, lane, Th, Tl, a, base, stage[w], cn, s + b, t,
+                                                box, eps2, ah, al, a64, cnt[4]);
                 } else if (act) {
                     unsigned fb = 0;   // pairs left to FP64 (rare), taken after the loop
-#pragma unroll (kFFUnroll)
-                    for (int q = 0; q < cn; q++)
-                        fb |= (unsigned)!pair_ff<DIM, FAR, CHECK>(Th, Tl, sh[w][q], sl[w][q],
-                                                                  a.e2h, a.e2l, ah, al) << q;
+#pragma unroll 1
+                    for (int q = 0; q < cn; q++) {
+                        float4 h, l;
+                        stage[w].get(q >> 1, q & 1, h, l);
+                        fb |= (unsigned)!pair_ff<DIM, FAR, CHECK>(Th, Tl, h, l, a.e2h, a.e2l, ah,
+                                                                  al) << q;
+                    }
                     while (fb) {
                         const int gi = s + b + __ffs(fb) - 1;
                         fb &= fb - 1;
-                        pair_fp64<DIM>(x, y, z, t.sx[gi], t.sy[gi], DIM == 3 ? t.sz[gi] : 0.0,
-                                       t.sm[gi], eps2, a64);
+                        pair_fp64<DIM>(a.tx[me], a.ty[me], DIM == 3 ? a.tz[me] : 0.0, t.sx[gi],
+                                       t.sy[gi], DIM == 3 ? t.sz[gi] : 0.0, t.sm[gi], eps2, a64);
                         cnt[4]++;
                     }
                 }
                 __syncwarp();
             }
-            if (act) {   // renormalise the accumulators once per leaf
+            if (FAR && act) {   // renormalise once per leaf (ff_add did)
 #pragma unroll
                 for (int k = 0; k < DIM; k++) {
                     float hsum = __fadd_rn(ah[k], al[k]);
@@ -364,77 +349,127 @@ __device__ __forceinline__ void walk(const TreeDev& t, const FastTree& ft, const
                 }
             }
         } else {
-            bool open = false;
-            float4 nh = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (act) {
-                nh = ft.nh[node];
-                const float4 nlo = ft.nl[node];
+            // The hi parts alone decide outside a band of 2^-14 of d^2 plus
+            // 2^-28 (the lo parts move d by delta <= 2^-22, and 2 d delta <=
+            // 2^-15 d^2 + 2^15 delta^2); inside it the distance with the lo
+            // parts, and inside that one's band FP64.
+            float h2 = 0.0f;
+#pragma unroll
+            for (int k = 0; k < DIM; k++) {
+                const float d = __fsub_rn(comp(nh, k), Th[k]);
+                h2 = fmaf(d, d, h2);
+            }
+            const float size_f = __int_as_float(hd.y);
+            const float s2 = size_f * size_f, td2 = theta2 * h2;
+            bool open = act && s2 >= td2;
+            if (act && (FAR || !(fabsf(s2 - td2) > fmaf(0x1p-14f, td2, 0x1p-28f * theta2)))) {
                 float d2 = 0.0f;
 #pragma unroll
                 for (int k = 0; k < DIM; k++) {
-                    // hi and lo differences (both exact inside the box), rounded once
-                    float d = __fadd_rn(__fsub_rn(comp(nh, k), Th[k]), __fsub_rn(comp(nlo, k), Tl[k]));
+                    // hi and lo differences, rounded once
+                    const float d = __fadd_rn(__fsub_rn(comp(nh, k), Th[k]),
+                                              __fsub_rn(comp(nl, k), Tl[k]));
                     d2 = fmaf(d, d, d2);
                 }
-                const float dist = d2 > 0.0f ? d2 * rsqrtf(d2) : 0.0f;
+                // (below 2^-50 the absolute part of the band decides)
+                const float dist = d2 > 0x1p-100f ? d2 * rsqrt_mufu(d2) : 0.0f;
                 const float td = theta_f * dist;
                 const float band = theta_f * fmaf(kBandRel, dist, band_abs);
-                const float size_f = __int_as_float(hd.y);
                 if (size_f >= td + band) {
                     open = true;
                 } else if (size_f < td - band) {
                     open = false;
                 } else {
-                    open = open_exact64<DIM>(x, y, z, t.cm[node], t.size[node], a.theta);
-                    cnt[3] += lead;
+                    open = open_exact64<DIM>(a.tx[me], a.ty[me], DIM == 3 ? a.tz[me] : 0.0,
+                                             t.cm[node], t.size[node], a.theta);
+                    cnt[3] += own;
                 }
             }
             const unsigned omask = __ballot_sync(FULL, act && open);
-            if (act && !open && lead) {
-                const float4 nl = ft.nl[node];   // (cached: read by the opening test)
-                if (!FAR && !CHECK) {
+            if (act && !open && own) {
+                if (!FAR && !CHECK && hd.w == 1) {
                     pair_ff_soft<DIM, false>(Th, Tl, nh, nl, a.e2h, a.e2l, ah, al);
-                } else if (!pair_ff<DIM, FAR, CHECK>(Th, Tl, nh, nl, a.e2h, a.e2l, ah, al)) {
+                } else if (!FAR && !CHECK) {   // (into the sums: the soft path has no a64)
                     const NodeCM cm = t.cm[node];
-                    pair_fp64<DIM>(x, y, z, cm.x, cm.y, cm.z, cm.w, eps2, a64);
+                    double f[3] = {0.0, 0.0, 0.0};
+                    pair_fp64<DIM>(a.tx[me], a.ty[me], DIM == 3 ? a.tz[me] : 0.0, cm.x, cm.y,
+                                   cm.z, cm.w, eps2, f);
+#pragma unroll
+                    for (int k = 0; k < DIM; k++) {
+                        float h, l;
+                        split_plain(__ddiv_rn(f[k], ft.frame->conv), h, l);
+                        ff_add(ah[k], al[k], h, l);
+                    }
+                    cnt[4]++;
+                } else if (hd.w == 2 || !pair_ff<DIM, FAR, CHECK>(Th, Tl, nh, nl, a.e2h, a.e2l, ah, al)) {
+                    const NodeCM cm = t.cm[node];
+                    pair_fp64<DIM>(a.tx[me], a.ty[me], DIM == 3 ? a.tz[me] : 0.0, cm.x, cm.y,
+                                   cm.z, cm.w, eps2, a64);
                     cnt[4]++;
                 }
                 cnt[1]++;
             }
+            if (SPLIT && omask && levels > 0) {
+                levels--;
+                node = fc + ((path >> levels) & 1);
+                own = (path & ((1 << levels) - 1)) == 0;
+                mask = omask;
+                continue;
+            }
             if (omask) {
                 if (sp + 2 > kStackDepth) { overflow = true; break; }
-                if (lane == 0) {
-                    stack[w][sp] = make_int2(fc, (int)omask);
-                    stack[w][sp + 1] = make_int2(fc + 1, (int)omask);
-                }
-                sp += 2;
-                __syncwarp();
+                if (lane == 0) stack[w][sp] = make_int2(fc, (int)omask);
+                sp++;
+                node = fc + 1;
+                mask = omask;
+                continue;
             }
         }
+        if (sp == 0) break;
+        __syncwarp();
+        const int2 e = stack[w][--sp];
+        __syncwarp();
+        node = e.x;
+        mask = (unsigned)e.y;
     }
 }
 
 // SOFT: (eps s)^2 >= 2 kTinyR, so a warp of targets inside the box needs no
 // small-R test (pair_ff's CHECK).
-template <int DIM, bool SOFT>
+//
+// One warp per 32 targets; with SPLIT (few targets) 2^levels warps per 32
+// targets, the block's four among them.  A warp's walk is a chain of
+// dependent loads and short loops: it takes its time however few warps run,
+// so few targets leave the GPU idle for most of a solve.  Splitting the tree
+// shortens the chain itself (figures at BHUT_SPLIT_WARPS).  More warps than
+// the GPU holds several times over only repeat the top levels and, with the
+// group's warps in different blocks, lose the nodes that they share in L1.
+// A block adds its four sums in FP64; with more than four warps per group the blocks' sums go to `partial`
+// and k_split_sum adds them (fixed order, no atomics).
+template <int DIM, bool SOFT, bool SPLIT>
 __global__ void __launch_bounds__(kFastThreads, kFastBlocksPerSM)
-k_traverse_fast(TreeDev t, FastTree ft, FastArgs a)
+k_traverse_fast(TreeDev t, FastTree ft, FastArgs a, int levels, double* __restrict__ partial)
 {
     __shared__ int2 stack[kFastWarps][kStackDepth];
-    __shared__ float4 sh[kFastWarps][kWarp], sl[kFastWarps][kWarp];
+    __shared__ LeafStage stage[kFastWarps];
+    __shared__ double sum[SPLIT ? kFastWarps : 1][SPLIT ? DIM : 1][kWarp];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned FULL = 0xffffffffu;
     const FastFrame fr = *ft.frame;
     const double conv = __dmul_rn(fr.conv, a.G);
+    const int shares = SPLIT ? (1 << levels) / kFastWarps : 1;   // blocks per group
+    const int64_t step = SPLIT ? gridDim.x / shares : (int64_t)gridDim.x * kFastWarps;
+    const int share = SPLIT ? (int)(blockIdx.x % (unsigned)shares) : 0;
 
-    for (int64_t base = ((int64_t)blockIdx.x * kFastWarps + w) * kWarp; base < a.nt;
-         base += (int64_t)gridDim.x * kFastWarps * kWarp) {
+    for (int64_t g = SPLIT ? blockIdx.x / (unsigned)shares
+                           : (int64_t)blockIdx.x * kFastWarps + w;
+         g * kWarp < a.nt; g += step) {
+        const int64_t base = g * kWarp;
         const int64_t i = base + lane;
         const bool valid = i < a.nt;
         float Th[3] = {0.f, 0.f, 0.f}, Tl[3] = {0.f, 0.f, 0.f};
         bool far = false;
         float amax = 0.f;
-        double x = 0.0, y = 0.0, z = 0.0;
         if (valid) {
             // self targets are the sorted particles themselves (inside the box)
             const float4 h = a.th ? a.th[i] : ft.ph[i];
@@ -443,9 +478,6 @@ k_traverse_fast(TreeDev t, FastTree ft, FastArgs a)
             Tl[0] = l.x; Tl[1] = l.y; Tl[2] = l.z;
             far = a.th ? h.w != 0.0f : false;
             amax = a.th ? l.w : 1.0f;
-            x = a.tx[i];
-            y = a.ty[i];
-            z = DIM == 3 ? a.tz[i] : 0.0;
         }
         const float band_abs = kBandAbs * (1.0f + amax);
         float ah[3] = {0.f, 0.f, 0.f}, al[3] = {0.f, 0.f, 0.f};
@@ -454,15 +486,19 @@ k_traverse_fast(TreeDev t, FastTree ft, FastArgs a)
         // self mode: targets are the sorted particles, target i is particle i
         const int64_t me_sorted = (valid && a.th == nullptr) ? i : -1;
         bool overflow = false;
+        const int path = SPLIT ? share * kFastWarps + w : 0;
         if (__any_sync(FULL, far))
-            walk<DIM, true, true>(t, ft, a, w, lane, valid, me_sorted, Th, Tl, band_abs, x, y, z,
-                                  ah, al, a64, stack, sh, sl, cnt, overflow);
-        else if (SOFT && fr.unit)
-            walk<DIM, false, false, true>(t, ft, a, w, lane, valid, me_sorted, Th, Tl, band_abs, x,
-                                          y, z, ah, al, a64, stack, sh, sl, cnt, overflow);
+            walk<DIM, true, true, false, SPLIT>(t, ft, a, w, lane, valid, base, me_sorted, Th, Tl,
+                                                band_abs, ah, al, a64, stack, stage, cnt, overflow,
+                                                levels, path);
+        else if (fr.unit)
+            walk<DIM, false, !SOFT, true, SPLIT>(t, ft, a, w, lane, valid, base, me_sorted, Th, Tl,
+                                                 band_abs, ah, al, a64, stack, stage, cnt,
+                                                 overflow, levels, path);
         else
-            walk<DIM, false, !SOFT>(t, ft, a, w, lane, valid, me_sorted, Th, Tl, band_abs, x, y, z,
-                                    ah, al, a64, stack, sh, sl, cnt, overflow);
+            walk<DIM, false, !SOFT, false, SPLIT>(t, ft, a, w, lane, valid, base, me_sorted, Th,
+                                                  Tl, band_abs, ah, al, a64, stack, stage, cnt,
+                                                  overflow, levels, path);
         if (overflow && lane == 0) atomicOr(a.err, kErrStackOverflow);
         if (a.stats) {
 #pragma unroll
@@ -472,86 +508,37 @@ k_traverse_fast(TreeDev t, FastTree ft, FastArgs a)
                 if (lane == 0 && v) atomicAdd(&a.stats[k], v);
             }
         }
-        if (valid) {
-            const int64_t o = a.out_idx ? a.out_idx[i] : i;
 #pragma unroll
-            for (int k = 0; k < DIM; k++) {
-                double v = __dadd_rn((double)ah[k], (double)al[k]);
-                a.out[o * DIM + k] = __dadd_rn(__dmul_rn(v, conv), __dmul_rn(a64[k], a.G));
+        for (int k = 0; k < DIM; k++) {
+            const double v = __dadd_rn(
+                __dmul_rn(__dadd_rn((double)ah[k], (double)al[k]), conv), __dmul_rn(a64[k], a.G));
+            if (SPLIT) sum[SPLIT ? w : 0][SPLIT ? k : 0][lane] = v;
+            else if (valid) a.out[(a.out_idx ? a.out_idx[i] : i) * DIM + k] = v;
+        }
+        if (SPLIT) {
+            __syncthreads();
+            if (w < DIM && valid) {
+                double v = sum[0][SPLIT ? w : 0][lane];
+                for (int u = 1; u < kFastWarps; u++)
+                    v = __dadd_rn(v, sum[SPLIT ? u : 0][SPLIT ? w : 0][lane]);
+                if (shares > 1) partial[((int64_t)share * a.nt + i) * DIM + w] = v;
+                else a.out[(a.out_idx ? a.out_idx[i] : i) * DIM + w] = v;
             }
+            __syncthreads();
         }
     }
 }
 
-// Self accelerations of few targets (fewer warps than two per SM
-// sub-partition): LPT lanes per target, so that LPT times as many warps
-// share the work (soft path only; the group's partial sums are added by
-// shuffles in a fixed order at the end).
-template <int DIM, int LPT>
-__global__ void __launch_bounds__(kFastThreads, kFastBlocksPerSM)
-k_traverse_fast_lpt(TreeDev t, FastTree ft, FastArgs a)
+__global__ void k_split_sum(const double* __restrict__ partial, int64_t nt, int dim, int shares,
+                            const int32_t* __restrict__ out_idx, double* __restrict__ out)
 {
-    constexpr int kTargets = kWarp / LPT;   // targets per warp
-    __shared__ int2 stack[kFastWarps][kStackDepth];
-    __shared__ float4 sh[kFastWarps][kWarp], sl[kFastWarps][kWarp];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const unsigned FULL = 0xffffffffu;
-    const FastFrame fr = *ft.frame;
-    const double conv = __dmul_rn(fr.conv, a.G);
-    for (int64_t base = ((int64_t)blockIdx.x * kFastWarps + w) * kTargets; base < a.nt;
-         base += (int64_t)gridDim.x * kFastWarps * kTargets) {
-        const int64_t i = base + lane / LPT;
-        const bool valid = i < a.nt;
-        float Th[3] = {0.f, 0.f, 0.f}, Tl[3] = {0.f, 0.f, 0.f};
-        double x = 0.0, y = 0.0, z = 0.0;
-        if (valid) {
-            const float4 h = ft.ph[i], l = ft.pl[i];
-            Th[0] = h.x; Th[1] = h.y; Th[2] = h.z;
-            Tl[0] = l.x; Tl[1] = l.y; Tl[2] = l.z;
-            x = a.tx[i];
-            y = a.ty[i];
-            z = DIM == 3 ? a.tz[i] : 0.0;
-        }
-        const float band_abs = kBandAbs * 2.0f;
-        float ah[3] = {0.f, 0.f, 0.f}, al[3] = {0.f, 0.f, 0.f};
-        double a64[3] = {0.0, 0.0, 0.0};
-        unsigned cnt[5] = {0, 0, 0, 0, 0};
-        const int64_t me_sorted = valid ? i : -1;
-        bool overflow = false;
-        if (fr.unit)
-            walk<DIM, false, false, true, LPT>(t, ft, a, w, lane, valid, me_sorted, Th, Tl,
-                                               band_abs, x, y, z, ah, al, a64, stack, sh, sl, cnt,
-                                               overflow);
-        else
-            walk<DIM, false, false, false, LPT>(t, ft, a, w, lane, valid, me_sorted, Th, Tl,
-                                                band_abs, x, y, z, ah, al, a64, stack, sh, sl,
-                                                cnt, overflow);
-        if (overflow && lane == 0) atomicOr(a.err, kErrStackOverflow);
-#pragma unroll
-        for (int o = LPT / 2; o >= 1; o >>= 1) {
-#pragma unroll
-            for (int k = 0; k < DIM; k++) {
-                const float bh = __shfl_down_sync(FULL, ah[k], o);
-                const float bl = __shfl_down_sync(FULL, al[k], o);
-                ff_add(ah[k], al[k], bh, bl);
-            }
-        }
-        if (a.stats) {
-#pragma unroll
-            for (int k = 0; k < 5; k++) {
-                unsigned long long v = cnt[k];
-                for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(FULL, v, o);
-                if (lane == 0 && v) atomicAdd(&a.stats[k], v);
-            }
-        }
-        if (valid && (lane & (LPT - 1)) == 0) {
-            const int64_t o = a.out_idx ? a.out_idx[i] : i;
-#pragma unroll
-            for (int k = 0; k < DIM; k++) {
-                double v = __dadd_rn((double)ah[k], (double)al[k]);
-                a.out[o * DIM + k] = __dmul_rn(v, conv);
-            }
-        }
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nt * dim;
+         j += (int64_t)gridDim.x * blockDim.x) {
+        double v = partial[j];
+#pragma unroll 8
+        for (int y = 1; y < shares; y++) v = __dadd_rn(v, partial[(int64_t)y * nt * dim + j]);
+        const int64_t i = j / dim;
+        out[(out_idx ? out_idx[i] : i) * dim + j % dim] = v;
     }
 }
 
@@ -586,7 +573,7 @@ __device__ __forceinline__ void walk_f32(const TreeDev& t, const FastTree& ft, c
         const unsigned mask = (unsigned)e.y;
         const bool act = (mask >> lane) & 1u;
         cnt[2] += act;
-        const int4 hd = ft.nhdr[node];   // (first_child, start, count, mass != 0)
+        const int4 hd = ft.nhdr[node];   // (first_child, start, count, flag)
         if (!hd.w) continue;
         const int fc = hd.x;
         if (fc < 0) {
@@ -716,35 +703,56 @@ k_traverse_fp32(TreeDev t, FastTree ft, FastArgs a)
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-int launch_fast_prepare(const double* box, int dim, FastFrame* frame, const TreeDev& t,
+int launch_fast_prepare(const double* box, int dim, bool fine, FastFrame* frame, const TreeDev& t,
                         const double* center, float4* ph, float4* pl, float4* nh, float4* nl,
                         float* nsize, float* ndelta, const double* quad, float4* nq0,
                         float2* nq1, int4* nhdr, cudaStream_t s)
 {
     k_frame<<<1, 32, 0, s>>>(box, dim, frame);
-    k_ff_particles<<<grid_for(t.n, 256), 256, 0, s>>>(t.sx, t.sy, t.sz, t.sm, t.n, dim, frame, ph,
+    k_ff_particles<<<grid_for(t.n, 256), 256, 0, s>>>(t.sx, t.sy, t.sz, t.sm, t.n, dim, fine, frame,
+                                                      ph,
                                                       pl);
-    k_ff_nodes<<<grid_for(t.m, 256), 256, 0, s>>>(t, center, frame, nh, nl, nsize, ndelta, quad,
-                                                  nq0, nq1, nhdr);
+    k_ff_nodes<<<grid_for(t.m, 256), 256, 0, s>>>(t, fine, center, frame, nh, nl, nsize, ndelta, quad,
+                                                  nq0, nq1, nhdr, ph);
     BHUT_CUDA(cudaGetLastError());
     note_launches(3);
     return kOk;
 }
 
 int launch_fast_targets(const double* tx, const double* ty, const double* tz, int64_t nt, int dim,
-                        const FastFrame* frame, float4* th, float4* tl, cudaStream_t s)
+                        bool fine, const FastFrame* frame, float4* th, float4* tl, cudaStream_t s)
 {
-    k_ff_targets<<<grid_for(nt, 256), 256, 0, s>>>(tx, ty, tz, nt, dim, frame, th, tl);
+    k_ff_targets<<<grid_for(nt, 256), 256, 0, s>>>(tx, ty, tz, nt, dim, fine, frame, th, tl);
     BHUT_CUDA(cudaGetLastError());
     note_launches(1);
     return kOk;
+}
+
+// Levels of the tree to split a fast traversal of nt targets by (0: none, else
+// 2 to kSplitMaxLevels), and the doubles of `partial` it needs.
+int fast_split_levels(int64_t nt, int64_t nodes, bool self)
+{
+    const int64_t groups = (nt + kWarp - 1) / kWarp;
+    if (self && groups >= kWaveWarps) return 0;
+    int levels = 0;
+    while (levels < kSplitMaxLevels && (groups << levels) < BHUT_SPLIT_WARPS &&
+           (nodes >> levels) > BHUT_SPLIT_NODES)
+        levels++;
+    return levels < 2 ? 0 : levels;
+}
+
+int64_t fast_split_partial(int64_t nt, int dim, int levels)
+{
+    const int64_t shares = (1 << levels) / kFastWarps;
+    return levels > 0 && shares > 1 ? shares * nt * dim : 0;
 }
 
 int launch_traverse_fast(const TreeDev& t, const FastTree& ft, const float4* th, const float4* tl,
                          const double* tx, const double* ty, const double* tz,
                          const int32_t* self_id, const int32_t* out_idx, int64_t nt, double theta,
                          double eps, double G, double eps_scaled_sq, double* out, unsigned* err,
-                         unsigned long long* stats, cudaStream_t s, bool fp32, int mac)
+                         unsigned long long* stats, cudaStream_t s, bool fp32, int mac,
+                         int levels, double* partial)
 {
     if (nt <= 0) return kOk;
     FastArgs a;
@@ -761,33 +769,27 @@ int launch_traverse_fast(const TreeDev& t, const FastTree& ft, const float4* th,
         else k_traverse_fp32<2><<<grid, kFastThreads, 0, s>>>(t, ft, a);
     } else {
         const bool soft = a.e2h >= 2.0f * kTinyR;
-        // few self targets: lanes per target so that about two warps run on
-        // each SM sub-partition (self targets lie in the box: soft path)
-        int lpt = 1;
-        if (soft && th == nullptr && BHUT_FAST_MAX_LPT > 1) {
-            int dev = 0, sms = 0;
-            BHUT_CUDA(cudaGetDevice(&dev));
-            BHUT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-            const int64_t want = (int64_t)BHUT_FAST_LPT_WARPS_PER_SM * sms;
-            while (lpt < BHUT_FAST_MAX_LPT && (nt * lpt + kWarp - 1) / kWarp < want) lpt *= 2;
-        }
-        if (lpt > 1) {
-            const unsigned g = grid_for((nt * lpt + kWarp - 1) / kWarp, kFastWarps, 152u * 64u);
+        if (levels > 0) {
+            const int shares = (1 << levels) / kFastWarps;
+            const unsigned g = (unsigned)warps * (unsigned)shares;
             if (t.dim == 3) {
-                if (lpt == 2) k_traverse_fast_lpt<3, 2><<<g, kFastThreads, 0, s>>>(t, ft, a);
-                else if (lpt == 4) k_traverse_fast_lpt<3, 4><<<g, kFastThreads, 0, s>>>(t, ft, a);
-                else k_traverse_fast_lpt<3, 8><<<g, kFastThreads, 0, s>>>(t, ft, a);
+                if (soft) k_traverse_fast<3, true, true><<<g, kFastThreads, 0, s>>>(t, ft, a, levels, partial);
+                else k_traverse_fast<3, false, true><<<g, kFastThreads, 0, s>>>(t, ft, a, levels, partial);
             } else {
-                if (lpt == 2) k_traverse_fast_lpt<2, 2><<<g, kFastThreads, 0, s>>>(t, ft, a);
-                else if (lpt == 4) k_traverse_fast_lpt<2, 4><<<g, kFastThreads, 0, s>>>(t, ft, a);
-                else k_traverse_fast_lpt<2, 8><<<g, kFastThreads, 0, s>>>(t, ft, a);
+                if (soft) k_traverse_fast<2, true, true><<<g, kFastThreads, 0, s>>>(t, ft, a, levels, partial);
+                else k_traverse_fast<2, false, true><<<g, kFastThreads, 0, s>>>(t, ft, a, levels, partial);
+            }
+            if (shares > 1) {
+                k_split_sum<<<grid_for(nt * t.dim, 128), 128, 0, s>>>(partial, nt, t.dim, shares,
+                                                                      out_idx, out);
+                note_launches(1);
             }
         } else if (t.dim == 3) {
-            if (soft) k_traverse_fast<3, true><<<grid, kFastThreads, 0, s>>>(t, ft, a);
-            else k_traverse_fast<3, false><<<grid, kFastThreads, 0, s>>>(t, ft, a);
+            if (soft) k_traverse_fast<3, true, false><<<grid, kFastThreads, 0, s>>>(t, ft, a, 0, nullptr);
+            else k_traverse_fast<3, false, false><<<grid, kFastThreads, 0, s>>>(t, ft, a, 0, nullptr);
         } else {
-            if (soft) k_traverse_fast<2, true><<<grid, kFastThreads, 0, s>>>(t, ft, a);
-            else k_traverse_fast<2, false><<<grid, kFastThreads, 0, s>>>(t, ft, a);
+            if (soft) k_traverse_fast<2, true, false><<<grid, kFastThreads, 0, s>>>(t, ft, a, 0, nullptr);
+            else k_traverse_fast<2, false, false><<<grid, kFastThreads, 0, s>>>(t, ft, a, 0, nullptr);
         }
     }
     BHUT_CUDA(cudaGetLastError());

@@ -73,14 +73,15 @@ struct FastTree {
     const FastFrame* frame;
     const float4* ph;   // (x, y, z, m) hi
     const float4* pl;   // (x, y, z, m) lo
-    const float4* nh;   // (com, mass) hi per node
-    const float4* nl;   // (com, mass) lo per node
+    const float4* nh;   // (com, mass) hi per internal node, LeafBox::c per leaf
+    const float4* nl;   // (com, mass) lo per internal node, LeafBox::h per leaf
     const float* nsize; // 2 * half_size, normalised, per node
     const float* ndelta; // |com - AABB centre|, normalised, per node (offset criterion)
     const float4* nq0;   // quadrupole (xx, yy, zz, xy), normalised, per node; NULL: monopoles
     const float2* nq1;   // quadrupole (xz, yz)
-    const int4* nhdr;    // per node, one load per visit: leaf (-1, start, count, mass != 0),
-                         // internal (first child, size, |com - centre| as float bits, mass != 0)
+    const int4* nhdr;    // per node, one load per visit: leaf (-1, start, count, flag),
+                         // internal (first child, size, |com - centre| as float bits, flag);
+                         // the flag is 0 for a node without mass (node_flag)
 };
 
 // Morton encoding (bhut/utils/morton.py:14-45, 183-198) and the quantisation
@@ -229,17 +230,21 @@ int launch_traverse_exact(const TreeDev& t, const double* tx, const double* ty, 
                           const int32_t* self_id, const int32_t* out_idx, int64_t nt, double theta,
                           double eps, double G, double* out, unsigned* err,
                           unsigned long long* stats, cudaStream_t s);
-int launch_fast_prepare(const double* box, int dim, FastFrame* frame, const TreeDev& t,
+// `fine`: the lo parts of form "fast" (split_grid), else those of "fp32".
+int launch_fast_prepare(const double* box, int dim, bool fine, FastFrame* frame, const TreeDev& t,
                         const double* center, float4* ph, float4* pl, float4* nh, float4* nl,
                         float* nsize, float* ndelta, const double* quad, float4* nq0,
                         float2* nq1, int4* nhdr, cudaStream_t s);
 int launch_fast_targets(const double* tx, const double* ty, const double* tz, int64_t nt, int dim,
-                        const FastFrame* frame, float4* th, float4* tl, cudaStream_t s);
+                        bool fine, const FastFrame* frame, float4* th, float4* tl, cudaStream_t s);
 int launch_traverse_fast(const TreeDev& t, const FastTree& ft, const float4* th, const float4* tl,
                          const double* tx, const double* ty, const double* tz,
                          const int32_t* self_id, const int32_t* out_idx, int64_t nt, double theta,
                          double eps, double G, double eps_scaled_sq, double* out, unsigned* err,
-                         unsigned long long* stats, cudaStream_t s, bool fp32, int mac);
+                         unsigned long long* stats, cudaStream_t s, bool fp32, int mac,
+                         int levels, double* partial);
+int fast_split_levels(int64_t nt, int64_t nodes, bool self);
+int64_t fast_split_partial(int64_t nt, int dim, int levels);
 // TreeData arrays as the reference lays them out (bhut/tree/node.py:15-77):
 // int64 indices, com (m, dim), for compute_tree_statistics.
 struct StatTree {
