@@ -505,6 +505,12 @@ int traverse(bhut_tree* t, const double* tx, const double* ty, const double* tz,
     BHUT_TRY(t->stats.ensure(sizeof(unsigned long long) * 8, t->stream));
     BHUT_CUDA(cudaMemsetAsync(t->stats.p, 0, sizeof(unsigned long long) * 8, t->stream));
     unsigned long long* st = t->stats.as<unsigned long long>();
+    // (form fp32 keeps one order of its sums)
+    const int levels = t->form == BHUT_FORM_FP32
+                           ? 0
+                           : split_levels(nt, t->m, self_targets, t->form == BHUT_FORM_EXACT);
+    const int64_t part = split_partial_doubles(nt, t->dim, levels);
+    if (part > 0) BHUT_TRY(t->split_partial.ensure(sizeof(double) * part, t->stream));
     switch (t->form) {
     case BHUT_FORM_FAST:
     case BHUT_FORM_FP32: {
@@ -521,10 +527,6 @@ int traverse(bhut_tree* t, const double* tx, const double* ty, const double* tz,
             th = t->th.as<float4>();
             tl = t->tl.as<float4>();
         }
-        const int levels = t->form == BHUT_FORM_FAST ? fast_split_levels(nt, t->m, self_targets)
-                                                      : 0;
-        const int64_t part = fast_split_partial(nt, t->dim, levels);
-        if (part > 0) BHUT_TRY(t->split_partial.ensure(sizeof(double) * part, t->stream));
         const double es = eps * sc;
         BHUT_TRY(launch_traverse_fast(d, fast_tree(t), th, tl, tx, ty, tz, self_id, out_idx, nt,
                                       theta, eps, G, es * es, out, t->err.as<unsigned>(), st,
@@ -536,7 +538,8 @@ int traverse(bhut_tree* t, const double* tx, const double* ty, const double* tz,
     case BHUT_FORM_EXACT:
     default:
         BHUT_TRY(launch_traverse_exact(d, tx, ty, tz, self_id, out_idx, nt, theta, eps, G, out,
-                                       t->err.as<unsigned>(), st, t->stream));
+                                       t->err.as<unsigned>(), st, t->stream, levels,
+                                       t->split_partial.as<double>()));
     }
     BHUT_CUDA(cudaMemcpyAsync(t->last_stats, st, sizeof(unsigned long long) * 5,
                               cudaMemcpyDeviceToHost, t->stream));

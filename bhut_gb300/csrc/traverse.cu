@@ -11,6 +11,12 @@
 // loop (bh.py:226-280) with explicit round-to-nearest intrinsics and IEEE
 // sqrt/division, so P2P terms match the reference's bit for bit; monopoles
 // use r2^1.5 = r2 * sqrt(r2) in place of pow (kernels.py:66), within 2 ulp.
+// Products, square roots and reciprocals run on the integer and FP32 pipes
+// (fp64int.cuh), correctly rounded all the same; the FP64 pipe keeps a pair's
+// nine additions.  100k Plummer traversal 243 -> 96 ms, direct sum of 20,000
+// 28.6 -> 9.4 ms, bit for bit the same (with the products left to the FP64 pipe
+// 138 and 16.2 ms).  Bound now by the ALU and FP64 pipes, 71 and 70 % busy.
+#include "fp64int.cuh"
 #include "tree.cuh"
 
 namespace bhut {
@@ -18,62 +24,167 @@ namespace bhut {
 constexpr int kTravWarps = 4;
 constexpr int kTravThreads = kTravWarps * kWarp;
 
-// bh.py:576-601 with np.linalg.norm = sqrt(fma chain) (OpenBLAS ddot).
+// Products of a pair on the integer pipes: the squares and the force
+// components (tuning: 0 takes the FP64 pipe; 100k Plummer traversal both 95.9
+// ms, squares alone 103.3, forces alone 104.9, neither 122.4).
+#ifndef BHUT_INT_SQUARES
+#define BHUT_INT_SQUARES 1
+#endif
+#ifndef BHUT_INT_FORCE
+#define BHUT_INT_FORCE 1
+#endif
+template <bool INT>
+static __device__ __forceinline__ double mul_rn(const fp64int::Parts& a, const fp64int::Parts& b,
+                                                double x, double y)
+{
+    return INT ? fp64int::mul(a, b) : __dmul_rn(x, y);
+}
+
+// v, kept in registers (a product of two kernel arguments would otherwise be
+// formed again for every pair).
+static __device__ __forceinline__ double held(double v)
+{
+    asm volatile("" : "+d"(v));
+    return v;
+}
+
+// The leaf loop's force (bh.py:262-278) in FP64 instructions; false: none
+// (r^2 + eps^2 == 0).
+template <int DIM>
+static __device__ __noinline__ bool pair_fp64_force(double dx, double dy, double dz, double gm,
+                                                    double eps2, double3* F)
+{
+    double r2 = __dmul_rn(dx, dx);
+    r2 = __dadd_rn(r2, __dmul_rn(dy, dy));
+    if (DIM == 3) r2 = __dadd_rn(r2, __dmul_rn(dz, dz));
+    r2 = __dadd_rn(r2, eps2);
+    if (r2 == 0.0) return false;
+    const double ri = __ddiv_rn(1.0, __dsqrt_rn(r2));
+    const double f = __dmul_rn(gm, __dmul_rn(__dmul_rn(ri, ri), ri));
+    F->x = __dmul_rn(f, dx);
+    F->y = __dmul_rn(f, dy);
+    F->z = DIM == 3 ? __dmul_rn(f, dz) : 0.0;
+    return true;
+}
+
+// The leaf loop's term at displacement (dx, dy, dz), added to (ax, ay, az);
+// gm = G m.  Returns whether it counts (r^2 + eps^2 != 0).
+template <int DIM>
+static __device__ __forceinline__ bool pair_exact(double dx, double dy, double dz, double gm,
+                                                  double eps2, double& ax, double& ay, double& az)
+{
+    using fp64int::parts;
+    using fp64int::within;
+    // ranges in which no product below leaves the normal numbers: |d| within
+    // 2^+-250, |G m| within 2^+-200, r^2 + eps^2 within 2^-340 .. 2^300
+    const auto X = parts(dx), Y = parts(dy), Z = parts(DIM == 3 ? dz : 0.0), M = parts(gm);
+    bool ok = within(X, -250, 250) && within(Y, -250, 250) && within(Z, -250, 250) &&
+              within(M, -200, 200);
+    double r2 = mul_rn<BHUT_INT_SQUARES>(X, X, dx, dx);
+    r2 = __dadd_rn(r2, mul_rn<BHUT_INT_SQUARES>(Y, Y, dy, dy));
+    if (DIM == 3) r2 = __dadd_rn(r2, mul_rn<BHUT_INT_SQUARES>(Z, Z, dz, dz));
+    r2 = __dadd_rn(r2, eps2);
+    const auto R = parts(r2);
+    if (ok && R.zero) return false;   // (never -0)
+    ok = ok && within(R, -340, 300);
+    const auto I = fp64int::rsqrt(R);
+    const auto W = fp64int::product(M, fp64int::product(fp64int::product(I, I), I));
+    const double f = BHUT_INT_FORCE ? 0.0 : fp64int::whole(W);
+    double3 F = make_double3(mul_rn<BHUT_INT_FORCE>(W, X, f, dx),
+                             mul_rn<BHUT_INT_FORCE>(W, Y, f, dy),
+                             DIM == 3 ? mul_rn<BHUT_INT_FORCE>(W, Z, f, dz) : 0.0);
+    if (!ok) {   // something beyond those ranges
+        double3 G;
+        if (!pair_fp64_force<DIM>(dx, dy, dz, gm, eps2, &G)) return false;
+        F = G;
+    }
+    ax = __dadd_rn(ax, F.x);
+    ay = __dadd_rn(ay, F.y);
+    if (DIM == 3) az = __dadd_rn(az, F.z);
+    return true;
+}
+
+// size / sqrt(s) >= theta (bh.py:576-601) for s = |x - com|^2 as np.linalg.norm
+// sums it (fma chain, OpenBLAS ddot).  The squares decide outside 2^-39 of
+// each other (both sides are within a few 2^-53 of the exact ones, and
+// positive doubles order as integers); inside, or outside the normal range,
+// the reference's own square root and division.
+static __device__ __forceinline__ bool opens(double s, double size, double theta)
+{
+    const int64_t a = (int64_t)fp64int::bits(__dmul_rn(size, size));
+    const int64_t b = (int64_t)fp64int::bits(__dmul_rn(__dmul_rn(theta, theta), s));
+    const int64_t gap = a - b;
+    if ((gap > 8192 || gap < -8192) && fp64int::normal_positive(a) && fp64int::normal_positive(b))
+        return gap > 0;
+    const double d = __dsqrt_rn(s);
+    return d == 0.0 || __ddiv_rn(size, d) >= theta;
+}
+
+template <int DIM>
+static __device__ __forceinline__ double norm2_fma(double dx, double dy, double dz)
+{
+    const double s = __fma_rn(dy, dy, __dmul_rn(dx, dx));
+    return DIM == 3 ? __fma_rn(dz, dz, s) : s;
+}
+
 template <int DIM>
 __device__ __forceinline__ bool open_exact(double x, double y, double z, NodeCM cm, double size,
                                            double theta)
 {
-    double dx = __dsub_rn(x, cm.x), dy = __dsub_rn(y, cm.y);
-    double s;
-    if (DIM == 3) {
-        double dz = __dsub_rn(z, cm.z);
-        s = __fma_rn(dz, dz, __fma_rn(dy, dy, __dmul_rn(dx, dx)));
-    } else {
-        s = __fma_rn(dy, dy, __dmul_rn(dx, dx));
-    }
-    double d = __dsqrt_rn(s);
-    if (d == 0.0) return true;
-    return __ddiv_rn(size, d) >= theta;
+    return opens(norm2_fma<DIM>(__dsub_rn(x, cm.x), __dsub_rn(y, cm.y),
+                                DIM == 3 ? __dsub_rn(z, cm.z) : 0.0), size, theta);
 }
 
-// kernels.py:52-69 acc_monopole (single vector) via acc_monopole_node.
+// kernels.py:52-69 acc_monopole (single vector) via acc_monopole_node, at
+// displacement (dx, dy, dz) from the target.
 template <int DIM>
-__device__ __forceinline__ void monopole_exact(double x, double y, double z, NodeCM cm,
+__device__ __forceinline__ void monopole_exact(double dx, double dy, double dz, double m,
                                                double eps2, double G, double& ax, double& ay,
                                                double& az)
 {
-    double dx = __dsub_rn(cm.x, x), dy = __dsub_rn(cm.y, y);
-    double dz = DIM == 3 ? __dsub_rn(cm.z, z) : 0.0;
-    double r2 = __dadd_rn(__dadd_rn(-0.0, __dmul_rn(dx, dx)), __dmul_rn(dy, dy));
+    double r2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
     if (DIM == 3) r2 = __dadd_rn(r2, __dmul_rn(dz, dz));
-    r2 = __dadd_rn(0.0, r2);
     double r2s = __dadd_rn(r2, eps2);
     if (r2s == 0.0) return;
-    double f = __ddiv_rn(__dmul_rn(G, cm.w), __dmul_rn(r2s, __dsqrt_rn(r2s)));
+    double f = __ddiv_rn(__dmul_rn(G, m), __dmul_rn(r2s, fp64int::sqrt(r2s)));
     ax = __dadd_rn(ax, __dmul_rn(f, dx));
     ay = __dadd_rn(ay, __dmul_rn(f, dy));
     if (DIM == 3) az = __dadd_rn(az, __dmul_rn(f, dz));
 }
 
-template <int DIM>
+// SPLIT: 2^levels warps share 32 targets as in k_traverse_fast (few targets;
+// a warp follows the bits of its path through the top levels and walks the
+// subtree it reaches), so a target's pair terms are the same bit for bit but
+// are summed per subtree first.
+template <int DIM, bool SPLIT>
 __global__ void __launch_bounds__(kTravThreads)
 k_traverse_exact(TreeDev t, const double* __restrict__ tx, const double* __restrict__ ty,
                  const double* __restrict__ tz, const int32_t* __restrict__ self_id,
                  const int32_t* __restrict__ out_idx, int64_t nt, double theta, double eps,
                  double G, double* __restrict__ out, unsigned* __restrict__ err,
-                 unsigned long long* __restrict__ stats)
+                 unsigned long long* __restrict__ stats, int levels0,
+                 double* __restrict__ partial)
 {
     __shared__ int2 stack[kTravWarps][kStackDepth];
     __shared__ double px[kTravWarps][kWarp], py[kTravWarps][kWarp], pz[kTravWarps][kWarp],
         pm[kTravWarps][kWarp];
     __shared__ int32_t pid[kTravWarps][kWarp];
+    __shared__ double sum[SPLIT ? kTravWarps : 1][SPLIT ? DIM : 1][kWarp];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const double eps2 = __dmul_rn(eps, eps);
+    const double eps2 = held(__dmul_rn(eps, eps));
     const unsigned FULL = 0xffffffffu;
 
-    for (int64_t base = ((int64_t)blockIdx.x * kTravWarps + w) * kWarp; base < nt;
-         base += (int64_t)gridDim.x * kTravWarps * kWarp) {
-        const int64_t i = base + lane;
+    const int shares = SPLIT ? (1 << levels0) / kTravWarps : 1;   // blocks per group
+    const int64_t step = SPLIT ? gridDim.x / shares : (int64_t)gridDim.x * kTravWarps;
+    const int share = SPLIT ? (int)(blockIdx.x % (unsigned)shares) : 0;
+
+    for (int64_t g = SPLIT ? blockIdx.x / (unsigned)shares
+                           : (int64_t)blockIdx.x * kTravWarps + w;
+         g * kWarp < nt; g += step) {
+        const int64_t i = g * kWarp + lane;
+        const int path = SPLIT ? share * kTravWarps + w : 0;
+        int levels = levels0;
+        bool own = path == 0;                                // works on the node
         const bool valid = i < nt;
         const double x = valid ? tx[i] : 0.0, y = valid ? ty[i] : 0.0;
         const double z = (valid && DIM == 3) ? tz[i] : 0.0;
@@ -91,12 +202,12 @@ k_traverse_exact(TreeDev t, const double* __restrict__ tx, const double* __restr
             const int node = e.x;
             const unsigned mask = (unsigned)e.y;
             const bool act = (mask >> lane) & 1u;
-            n_visit += act;
+            n_visit += act && own;
             const NodeCM cm = t.cm[node];
             if (cm.w == 0.0) continue;                       // bh.py:514
             const int fc = t.first_child[node];
             if (fc < 0) {                                    // leaf: bh.py:520-524
-                const int s = t.start[node], c = t.count[node];
+                const int s = t.start[node], c = own ? t.count[node] : 0;
                 double lx = 0.0, ly = 0.0, lz = 0.0;
                 for (int b = 0; b < c; b += kWarp) {
                     const int jj = b + lane;
@@ -104,47 +215,50 @@ k_traverse_exact(TreeDev t, const double* __restrict__ tx, const double* __restr
                         px[w][lane] = t.sx[s + jj];
                         py[w][lane] = t.sy[s + jj];
                         if (DIM == 3) pz[w][lane] = t.sz[s + jj];
-                        pm[w][lane] = t.sm[s + jj];
+                        pm[w][lane] = __dmul_rn(G, t.sm[s + jj]);
                         pid[w][lane] = t.perm[s + jj];
                     }
                     __syncwarp();
                     const int cnt = min(kWarp, c - b);
                     if (act) {
+#pragma unroll 1
                         for (int q = 0; q < cnt; q++) {
                             if (pid[w][q] == me) continue;   // self skip, bh.py:254
-                            const double dx = __dsub_rn(px[w][q], x);
-                            const double dy = __dsub_rn(py[w][q], y);
-                            const double dz = DIM == 3 ? __dsub_rn(pz[w][q], z) : 0.0;
-                            double r2 = __dmul_rn(dx, dx);
-                            r2 = __dadd_rn(r2, __dmul_rn(dy, dy));
-                            if (DIM == 3) r2 = __dadd_rn(r2, __dmul_rn(dz, dz));
-                            r2 = __dadd_rn(r2, eps2);
-                            if (r2 == 0.0) continue;
-                            const double ri = __ddiv_rn(1.0, __dsqrt_rn(r2));
-                            const double ri3 = __dmul_rn(__dmul_rn(ri, ri), ri);
-                            const double f = __dmul_rn(__dmul_rn(G, pm[w][q]), ri3);
-                            lx = __dadd_rn(lx, __dmul_rn(f, dx));
-                            ly = __dadd_rn(ly, __dmul_rn(f, dy));
-                            if (DIM == 3) lz = __dadd_rn(lz, __dmul_rn(f, dz));
-                            n_p2p++;
+                            n_p2p += pair_exact<DIM>(
+                                __dsub_rn(px[w][q], x), __dsub_rn(py[w][q], y),
+                                DIM == 3 ? __dsub_rn(pz[w][q], z) : 0.0, pm[w][q], eps2, lx, ly,
+                                lz);
                         }
                     }
                     __syncwarp();
                 }
-                if (act) {
+                if (act && own) {
                     ax = __dadd_rn(ax, lx);
                     ay = __dadd_rn(ay, ly);
                     az = __dadd_rn(az, lz);
                 }
             } else {                                         // internal: bh.py:525-546
                 bool open = false;
-                if (act) open = open_exact<DIM>(x, y, z, cm, t.size[node], theta);
+                double dx = 0.0, dy = 0.0, dz = 0.0;
+                if (act) {
+                    dx = __dsub_rn(cm.x, x);
+                    dy = __dsub_rn(cm.y, y);
+                    if (DIM == 3) dz = __dsub_rn(cm.z, z);
+                    open = opens(norm2_fma<DIM>(dx, dy, dz), t.size[node], theta);
+                }
                 const unsigned omask = __ballot_sync(FULL, act && open);
-                if (act && !open) {
-                    monopole_exact<DIM>(x, y, z, cm, eps2, G, ax, ay, az);
+                if (act && !open && own) {
+                    monopole_exact<DIM>(dx, dy, dz, cm.w, eps2, G, ax, ay, az);
                     n_m2p++;
                 }
-                if (omask) {
+                if (SPLIT && omask && levels > 0) {
+                    levels--;
+                    own = (path & ((1 << levels) - 1)) == 0;
+                    if (lane == 0)
+                        stack[w][sp] = make_int2(fc + ((path >> levels) & 1), (int)omask);
+                    sp++;
+                    __syncwarp();
+                } else if (omask) {
                     if (sp + 2 > kStackDepth) { overflow = true; break; }
                     if (lane == 0) {
                         stack[w][sp] = make_int2(fc, (int)omask);        // left pushed first
@@ -168,7 +282,20 @@ k_traverse_exact(TreeDev t, const double* __restrict__ tx, const double* __restr
                 atomicAdd(&stats[2], n_visit);
             }
         }
-        if (valid) {
+        if (SPLIT) {
+            sum[SPLIT ? w : 0][0][lane] = ax;
+            sum[SPLIT ? w : 0][SPLIT ? 1 : 0][lane] = ay;
+            if (DIM == 3) sum[SPLIT ? w : 0][SPLIT ? DIM - 1 : 0][lane] = az;
+            __syncthreads();
+            if (w < DIM && valid) {
+                double v = sum[0][SPLIT ? w : 0][lane];
+                for (int u = 1; u < kTravWarps; u++)
+                    v = __dadd_rn(v, sum[SPLIT ? u : 0][SPLIT ? w : 0][lane]);
+                if (shares > 1) partial[((int64_t)share * nt + i) * DIM + w] = v;
+                else out[(out_idx ? out_idx[i] : i) * DIM + w] = v;
+            }
+            __syncthreads();
+        } else if (valid) {
             const int64_t o = out_idx ? out_idx[i] : i;
             out[o * DIM] = ax;
             out[o * DIM + 1] = ay;
@@ -184,6 +311,13 @@ k_traverse_exact(TreeDev t, const double* __restrict__ tx, const double* __restr
 // more than one chunk, per-chunk partial sums go to `partial` and
 // k_direct_reduce adds them in chunk order (deterministic).
 constexpr int kDirectThreads = 256;
+// Sources per chunk, at least: small sums need the blocks (2,000 / 5,000 /
+// 20,000 particles, ms: 4096 2.59 / 3.20 / 10.6, 1024 1.47 / 1.48 / 9.4, 512
+// 0.91 / 1.23 / 9.4, 256 0.64 / 1.01 / 9.4).
+#ifndef BHUT_DIRECT_CHUNK
+#define BHUT_DIRECT_CHUNK 256
+#endif
+constexpr int64_t kDirectChunk = BHUT_DIRECT_CHUNK;
 
 template <int DIM>
 __global__ void __launch_bounds__(kDirectThreads)
@@ -203,7 +337,7 @@ k_direct(const double* __restrict__ pos, const double* __restrict__ mass, int64_
         y = p[1];
         if (DIM == 3) z = p[2];
     }
-    const double eps2 = __dmul_rn(eps, eps);
+    const double eps2 = held(__dmul_rn(eps, eps));
     double ax = 0.0, ay = 0.0, az = 0.0;
     const int64_t j0 = (int64_t)blockIdx.y * chunk;
     const int64_t j1 = j0 + chunk < n ? j0 + chunk : n;
@@ -214,25 +348,16 @@ k_direct(const double* __restrict__ pos, const double* __restrict__ mass, int64_
             sx[threadIdx.x] = pos[j * DIM];
             sy[threadIdx.x] = pos[j * DIM + 1];
             sz[threadIdx.x] = DIM == 3 ? pos[j * DIM + 2] : 0.0;
-            sm[threadIdx.x] = mass[j];
+            sm[threadIdx.x] = __dmul_rn(G, mass[j]);
         }
         __syncthreads();
         const int cnt = (int)((j1 - b) < kDirectThreads ? (j1 - b) : kDirectThreads);
         if (valid) {
+#pragma unroll 1
             for (int q = 0; q < cnt; q++) {
                 if (b + q == me) continue;
-                const double dx = __dsub_rn(sx[q], x), dy = __dsub_rn(sy[q], y);
-                const double dz = DIM == 3 ? __dsub_rn(sz[q], z) : 0.0;
-                double r2 = __dmul_rn(dx, dx);
-                r2 = __dadd_rn(r2, __dmul_rn(dy, dy));
-                if (DIM == 3) r2 = __dadd_rn(r2, __dmul_rn(dz, dz));
-                r2 = __dadd_rn(r2, eps2);
-                if (r2 == 0.0) continue;
-                const double ri = __ddiv_rn(1.0, __dsqrt_rn(r2));
-                const double f = __dmul_rn(__dmul_rn(G, sm[q]), __dmul_rn(__dmul_rn(ri, ri), ri));
-                ax = __dadd_rn(ax, __dmul_rn(f, dx));
-                ay = __dadd_rn(ay, __dmul_rn(f, dy));
-                if (DIM == 3) az = __dadd_rn(az, __dmul_rn(f, dz));
+                pair_exact<DIM>(__dsub_rn(sx[q], x), __dsub_rn(sy[q], y),
+                                DIM == 3 ? __dsub_rn(sz[q], z) : 0.0, sm[q], eps2, ax, ay, az);
             }
         }
     }
@@ -258,20 +383,21 @@ __global__ void k_direct_reduce(const double* __restrict__ partial, int64_t nt, 
 int launch_traverse_exact(const TreeDev& t, const double* tx, const double* ty, const double* tz,
                           const int32_t* self_id, const int32_t* out_idx, int64_t nt, double theta,
                           double eps, double G, double* out, unsigned* err,
-                          unsigned long long* stats, cudaStream_t s)
+                          unsigned long long* stats, cudaStream_t s, int levels, double* partial)
 {
     if (nt <= 0) return kOk;
-    int64_t warps = (nt + kWarp - 1) / kWarp;
-    unsigned grid = grid_for(warps, kTravWarps, 152u * 64u);
-    if (t.dim == 3)
-        k_traverse_exact<3><<<grid, kTravThreads, 0, s>>>(t, tx, ty, tz, self_id, out_idx, nt, theta,
-                                                         eps, G, out, err, stats);
-    else
-        k_traverse_exact<2><<<grid, kTravThreads, 0, s>>>(t, tx, ty, tz, self_id, out_idx, nt, theta,
-                                                         eps, G, out, err, stats);
+    const int64_t groups = (nt + kWarp - 1) / kWarp;
+    const int shares = levels > 0 ? (1 << levels) / kTravWarps : 1;
+    const unsigned grid = levels > 0 ? (unsigned)(groups * shares)
+                                     : grid_for(groups, kTravWarps, 152u * 64u);
+    auto* kernel = t.dim == 3
+                       ? (levels > 0 ? k_traverse_exact<3, true> : k_traverse_exact<3, false>)
+                       : (levels > 0 ? k_traverse_exact<2, true> : k_traverse_exact<2, false>);
+    kernel<<<grid, kTravThreads, 0, s>>>(t, tx, ty, tz, self_id, out_idx, nt, theta, eps, G, out,
+                                         err, stats, levels, partial);
     BHUT_CUDA(cudaGetLastError());
     note_launches(1);
-    return kOk;
+    return shares > 1 ? launch_split_sum(partial, nt, t.dim, shares, out_idx, out, s) : kOk;
 }
 
 // ---------------------------------------------------------------------------
@@ -353,7 +479,7 @@ int direct_chunks(int64_t n, int64_t nt)
 {
     const int64_t tblocks = (nt + kDirectThreads - 1) / kDirectThreads;
     int64_t want = (152 * 8 + tblocks - 1) / tblocks;        // fill the GPU ~8 blocks per SM
-    int64_t maxc = (n + 4095) / 4096;                         // at least 4096 sources a chunk
+    int64_t maxc = (n + kDirectChunk - 1) / kDirectChunk;
     int64_t c = want < maxc ? want : maxc;
     return (int)(c < 1 ? 1 : (c > 1024 ? 1024 : c));
 }

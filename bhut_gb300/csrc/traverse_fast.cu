@@ -49,7 +49,7 @@ constexpr int kSplitMaxLevels = 10;
 #ifndef BHUT_F32_UNROLL
 #define BHUT_F32_UNROLL 8
 #endif
-// Split traversals (fast_split_levels): split while fewer warps than this walk
+// Split traversals (split_levels): split while fewer warps than this walk
 // and their subtrees hold more nodes than that.  Swept on GB300:
 //   warps (ms)            none   6144  12288  24576  49152  98304
 //   10k self              1.26   0.34   0.33   0.35   0.34   0.33
@@ -69,7 +69,15 @@ constexpr int kSplitMaxLevels = 10;
 #ifndef BHUT_SPLIT_WARPS
 #define BHUT_SPLIT_WARPS 49152
 #endif
-constexpr int64_t kWaveWarps = 152 * 4 * 5;   // resident warps of k_traverse_fast
+// Form "exact" (pairs are dearer, the walk matters less): ms for none / 12501 /
+// 25000 / 50001 warps, Plummer: 10k self 10.5 / 2.0 / 2.0 / 2.0, 30k 32.4 /
+// 14.6 / 13.7 / 13.3, 60k 62.6 / 42.4 / 40.9 / 40.8, 100k 95.7 / 85.3 / 86.5 /
+// 82.5, 200k 208 / 218 / 218 / 213, 2,000 targets of 100k 70.1 / 2.9 / 2.8 /
+// 2.8, 100k targets of 200k 121 / 115 / 115 / 125.
+#ifndef BHUT_SPLIT_WARPS_EXACT
+#define BHUT_SPLIT_WARPS_EXACT 25000
+#endif
+constexpr int64_t kWaveWarps = 152 * 4 * 5;   // resident warps of the traversals
 #ifndef BHUT_SPLIT_NODES
 #define BHUT_SPLIT_NODES 16
 #endif
@@ -728,20 +736,30 @@ int launch_fast_targets(const double* tx, const double* ty, const double* tz, in
     return kOk;
 }
 
-// Levels of the tree to split a fast traversal of nt targets by (0: none, else
+int launch_split_sum(const double* partial, int64_t nt, int dim, int shares,
+                     const int32_t* out_idx, double* out, cudaStream_t s)
+{
+    k_split_sum<<<grid_for(nt * dim, 128), 128, 0, s>>>(partial, nt, dim, shares, out_idx, out);
+    BHUT_CUDA(cudaGetLastError());
+    note_launches(1);
+    return kOk;
+}
+
+// Levels of the tree to split a traversal of nt targets by (0: none, else
 // 2 to kSplitMaxLevels), and the doubles of `partial` it needs.
-int fast_split_levels(int64_t nt, int64_t nodes, bool self)
+int split_levels(int64_t nt, int64_t nodes, bool self, bool exact)
 {
     const int64_t groups = (nt + kWarp - 1) / kWarp;
-    if (self && groups >= kWaveWarps) return 0;
+    if (self && groups >= (exact ? 2 : 1) * kWaveWarps) return 0;
+    const int64_t warps = exact ? BHUT_SPLIT_WARPS_EXACT : BHUT_SPLIT_WARPS;
     int levels = 0;
-    while (levels < kSplitMaxLevels && (groups << levels) < BHUT_SPLIT_WARPS &&
+    while (levels < kSplitMaxLevels && (groups << levels) < warps &&
            (nodes >> levels) > BHUT_SPLIT_NODES)
         levels++;
     return levels < 2 ? 0 : levels;
 }
 
-int64_t fast_split_partial(int64_t nt, int dim, int levels)
+int64_t split_partial_doubles(int64_t nt, int dim, int levels)
 {
     const int64_t shares = (1 << levels) / kFastWarps;
     return levels > 0 && shares > 1 ? shares * nt * dim : 0;
@@ -779,11 +797,7 @@ int launch_traverse_fast(const TreeDev& t, const FastTree& ft, const float4* th,
                 if (soft) k_traverse_fast<2, true, true><<<g, kFastThreads, 0, s>>>(t, ft, a, levels, partial);
                 else k_traverse_fast<2, false, true><<<g, kFastThreads, 0, s>>>(t, ft, a, levels, partial);
             }
-            if (shares > 1) {
-                k_split_sum<<<grid_for(nt * t.dim, 128), 128, 0, s>>>(partial, nt, t.dim, shares,
-                                                                      out_idx, out);
-                note_launches(1);
-            }
+            if (shares > 1) BHUT_TRY(launch_split_sum(partial, nt, t.dim, shares, out_idx, out, s));
         } else if (t.dim == 3) {
             if (soft) k_traverse_fast<3, true, false><<<grid, kFastThreads, 0, s>>>(t, ft, a, 0, nullptr);
             else k_traverse_fast<3, false, false><<<grid, kFastThreads, 0, s>>>(t, ft, a, 0, nullptr);

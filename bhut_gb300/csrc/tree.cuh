@@ -229,7 +229,7 @@ int launch_outside_root(const double* pos, int64_t n, int dim, const double* cen
 int launch_traverse_exact(const TreeDev& t, const double* tx, const double* ty, const double* tz,
                           const int32_t* self_id, const int32_t* out_idx, int64_t nt, double theta,
                           double eps, double G, double* out, unsigned* err,
-                          unsigned long long* stats, cudaStream_t s);
+                          unsigned long long* stats, cudaStream_t s, int levels, double* partial);
 // `fine`: the lo parts of form "fast" (split_grid), else those of "fp32".
 int launch_fast_prepare(const double* box, int dim, bool fine, FastFrame* frame, const TreeDev& t,
                         const double* center, float4* ph, float4* pl, float4* nh, float4* nl,
@@ -243,8 +243,12 @@ int launch_traverse_fast(const TreeDev& t, const FastTree& ft, const float4* th,
                          double eps, double G, double eps_scaled_sq, double* out, unsigned* err,
                          unsigned long long* stats, cudaStream_t s, bool fp32, int mac,
                          int levels, double* partial);
-int fast_split_levels(int64_t nt, int64_t nodes, bool self);
-int64_t fast_split_partial(int64_t nt, int dim, int levels);
+// Few targets: 2^levels warps per 32 targets (0: one), the doubles of scratch
+// that takes, and the sum of the blocks' partial results.
+int split_levels(int64_t nt, int64_t nodes, bool self, bool exact);
+int64_t split_partial_doubles(int64_t nt, int dim, int levels);
+int launch_split_sum(const double* partial, int64_t nt, int dim, int shares,
+                     const int32_t* out_idx, double* out, cudaStream_t s);
 // TreeData arrays as the reference lays them out (bhut/tree/node.py:15-77):
 // int64 indices, com (m, dim), for compute_tree_statistics.
 struct StatTree {
