@@ -501,9 +501,10 @@ struct BatchArgs {
     unsigned long long* stats;
 };
 
-// The warp's traversal stack of (node, lane mask) entries, two placements:
-//  STK 0: in shared memory, lane 0 writes, every lane reads (one __syncwarp
-//         per pop and per push);
+// The warp's traversal stack of (node, lane mask) entries (left children; the
+// right child of an opened node is visited next), two placements:
+//  STK 0: in shared memory, lane 0 writes, every lane reads (__syncwarp
+//         around each pop);
 //  STK 1: in registers, entry j held by lane j % 32 in register j / 32;
 //         a pop is two shuffles from the owning lane, a push a predicated
 //         register write; no shared memory, no __syncwarp.
@@ -514,28 +515,19 @@ template <> struct WarpStack<0> {
     int2* s;
     int sp = 0, lane;
     __device__ WarpStack(int2* s_, int lane_) : s(s_), lane(lane_) {}
-    __device__ void init(int node, unsigned mask)
-    {
-        if (lane == 0) s[0] = make_int2(node, (int)mask);
-        sp = 1;
-        __syncwarp();
-    }
     __device__ bool empty() const { return sp == 0; }
     __device__ int2 pop()
     {
+        __syncwarp();
         const int2 e = s[--sp];
         __syncwarp();
         return e;
     }
-    __device__ bool push2(int fc, unsigned m)
+    __device__ bool push(int node, unsigned m)
     {
         if (sp + 2 > kStackDepth) return false;
-        if (lane == 0) {
-            s[sp] = make_int2(fc, (int)m);
-            s[sp + 1] = make_int2(fc + 1, (int)m);
-        }
-        sp += 2;
-        __syncwarp();
+        if (lane == 0) s[sp] = make_int2(node, (int)m);
+        sp++;
         return true;
     }
 };
@@ -552,11 +544,6 @@ template <> struct WarpStack<1> {
             else { n1 = node; m1 = mask; }
         }
     }
-    __device__ void init(int node, unsigned mask)
-    {
-        put(0, node, (int)mask);
-        sp = 1;
-    }
     __device__ bool empty() const { return sp == 0; }
     __device__ int2 pop()
     {
@@ -566,32 +553,41 @@ template <> struct WarpStack<1> {
         const int mask = __shfl_sync(0xffffffffu, hi ? m1 : m0, sp & 31);
         return make_int2(node, mask);
     }
-    __device__ bool push2(int fc, unsigned m)
+    __device__ bool push(int node, unsigned m)
     {
         if (sp + 2 > kStackDepth) return false;
-        put(sp, fc, (int)m);
-        put(sp + 1, fc + 1, (int)m);
-        sp += 2;
+        put(sp, node, (int)m);
+        sp++;
         return true;
     }
 };
 
+// Resident blocks per SM of the FP32 form (1 / 8 / 9 / 10 at 256 systems:
+// 61.0 / 45.9 / 46.8 / 44.8 ms; 24 systems with quadrupoles 11.3 / 8.9 / 9.0 /
+// 8.7 ms).
+#ifndef BHUT_BATCH_BLOCKS
+#define BHUT_BATCH_BLOCKS 10
+#endif
 template <int DIM, bool FP32, int TPW, int STK>
-__global__ void __launch_bounds__(kBatchThreads)
+__global__ void __launch_bounds__(kBatchThreads, FP32 ? BHUT_BATCH_BLOCKS : 1)
 k_batch_traverse(BatchDev b, BatchArgs a)
 {
     constexpr int LPT = kWarp / TPW;            // lanes per target
     __shared__ int2 stack[STK == 0 ? kBatchWarps : 1][kStackDepth];
-    // the fast form's two-lane tasks and the FP32 form read source by source
-    constexpr bool kStaged = !FP32 && TPW == 32;
-    __shared__ float4 sh[kBatchWarps][kWarp], sl[kBatchWarps][kWarp];
+    // two-lane tasks read source by source, the others row by row (LeafStage)
+    constexpr bool kStaged = TPW == 32;
+    constexpr bool SCALAR = !kStaged || !FP32;   // (form fast without a large softening)
+    __shared__ float4 sh_all[SCALAR ? kBatchWarps : 1][kWarp], sl_all[SCALAR ? kBatchWarps : 1][kWarp];
     __shared__ LeafStage stage[kStaged ? kBatchWarps : 1];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    float4* const sh = sh_all[SCALAR ? w : 0];
+    float4* const sl = sl_all[SCALAR ? w : 0];
     const int sub = lane % LPT;
     const unsigned FULL = 0xffffffffu;
     const TreeDev& t = b.t;
     const float theta_f = (float)a.theta;
     const double eps2 = __dmul_rn(a.eps, a.eps);
+    const OpenF32 opener(a.theta, a.mac);
     unsigned long long tot[5] = {0, 0, 0, 0, 0};
 
     while (true) {
@@ -626,52 +622,65 @@ k_batch_traverse(BatchDev b, BatchArgs a)
             }
         }
         const TargetF32x2 tx = target_f32x2(Th, Tl);
+        const float2 nT[3] = {both(-Th[0]), both(-Th[1]), both(-Th[2])};
+        const float2 nL[3] = {both(-Tl[0]), both(-Tl[1]), both(-Tl[2])};
         const bool unit = fr.unit != 0;   // every particle mass of this system exactly 1
         float ah[3] = {0.f, 0.f, 0.f}, al[3] = {0.f, 0.f, 0.f};   // ff sum, or (sum, Kahan comp)
         double a64[3] = {0.0, 0.0, 0.0};
         unsigned cnt[5] = {0, 0, 0, 0, 0};
         bool overflow = false;
 
-        const unsigned live = __ballot_sync(FULL, valid);
         WarpStack<STK> st(stack[STK == 0 ? w : 0], lane);
-        st.init(root, live);
-        while (!st.empty()) {
-            const int2 e = st.pop();
-            const int node = e.x;
-            const bool act = ((unsigned)e.y >> lane) & 1u;
+        int node = root;
+        unsigned mask = __ballot_sync(FULL, valid);
+        while (true) {
+            const bool act = (mask >> lane) & 1u;
             cnt[2] += act && sub == 0;
             const int4 hd = b.nhdr[node];   // (first_child, start, count, flag)
-            if (!hd.w) continue;
+            const float4 nhv = b.nh[node];
             const int fc = hd.x;
-            if (fc < 0) {
+            if (!hd.w) {
+            } else if (fc < 0) {
                 const int s0 = hd.y, c = hd.z;
                 LeafBox box;
                 if (kStaged && soft) {
-                    box.c = b.nh[node];
+                    box.c = nhv;
                     box.h = b.nl[node];
                 }
                 for (int bb = 0; bb < c; bb += kWarp) {
                     const int jj = bb + lane;
-                    const bool staged = kStaged && soft;
-                    if (jj < c) {
+                    const int cn = min(kWarp, c - bb);
+                    const bool staged = kStaged && (FP32 || soft);
+                    int np = 0;
+                    if (FP32 && kStaged) {
+                        np = stage_f32(stage[kStaged ? w : 0], lane, b.ph, b.pl, s0 + bb, cn, false);
+                    } else if (jj < c) {
                         const float4 h = b.ph[s0 + jj], l = b.pl[s0 + jj];
                         if (staged) {
                             stage[kStaged ? w : 0].put(lane, h, l);
                         } else {
-                            sh[w][lane] = h;
-                            sl[w][lane] = l;
+                            sh[lane] = h;
+                            sl[lane] = l;
                         }
                     }
                     __syncwarp();
-                    const int cn = min(kWarp, c - bb);
                     if (act && sub == 0) cnt[0] += cn - (i >= s0 + bb && i < s0 + bb + cn);
-                    if (staged) {   // as the single-tree walk
+                    if (FP32 && kStaged) {   // <= 32 terms in FP32, then one Kahan step
+                        if (act) {
+                            const LeafStage& sg = stage[kStaged ? w : 0];
+                            float part[3] = {0.f, 0.f, 0.f};
+                            if (soft && unit) rows_f32<DIM, false, true>(sg, np, nT, nL, e2h, part);
+                            else if (soft) rows_f32<DIM, false, false>(sg, np, nT, nL, e2h, part);
+                            else rows_f32<DIM, true, false>(sg, np, nT, nL, e2h, part);
+                            kahan_add_f32<DIM>(part, ah, al);
+                        }
+                    } else if (staged) {   // as the single-tree walk
                         const LeafStage& sg = stage[kStaged ? w : 0];
                         if (unit)
-                            leaf_block_soft<DIM, true>((unsigned)e.y, lane, Th, Tl, sg, cn, box,
+                            leaf_block_soft<DIM, true>(mask, lane, Th, Tl, sg, cn, box,
                                                        e2h, e2l, ah, al);
                         else
-                            leaf_block_soft<DIM, false>((unsigned)e.y, lane, Th, Tl, sg, cn, box,
+                            leaf_block_soft<DIM, false>(mask, lane, Th, Tl, sg, cn, box,
                                                         e2h, e2l, ah, al);
                     } else if (act) {
                         if (FP32) {   // <= 32 terms in FP32, then one Kahan step
@@ -680,18 +689,18 @@ k_batch_traverse(BatchDev b, BatchArgs a)
                             if (soft && unit) {
 #pragma unroll 8
                                 for (int q = sub; q < cn; q += LPT)
-                                    pair_f32_partial2<DIM, false, true>(tx, sh[w][q], sl[w][q],
-                                                                        e2h, pxy, pz);
+                                    pair_f32_partial2<DIM, false, true>(
+                                        tx, sh[q], sl[q], e2h, pxy, pz);
                             } else if (soft) {
 #pragma unroll 8
                                 for (int q = sub; q < cn; q += LPT)
-                                    pair_f32_partial2<DIM, false, false>(tx, sh[w][q], sl[w][q],
-                                                                         e2h, pxy, pz);
+                                    pair_f32_partial2<DIM, false, false>(
+                                        tx, sh[q], sl[q], e2h, pxy, pz);
                             } else {
 #pragma unroll 8
                                 for (int q = sub; q < cn; q += LPT)
-                                    pair_f32_partial2<DIM, true, false>(tx, sh[w][q], sl[w][q],
-                                                                        e2h, pxy, pz);
+                                    pair_f32_partial2<DIM, true, false>(
+                                        tx, sh[q], sl[q], e2h, pxy, pz);
                             }
                             const float part[3] = {pxy.x, pxy.y, pz};
                             kahan_add_f32<DIM>(part, ah, al);
@@ -699,17 +708,14 @@ k_batch_traverse(BatchDev b, BatchArgs a)
                             unsigned fb = 0;   // pairs left to FP64, taken after the loop
                             if (soft && unit) {
                                 for (int q = sub; q < cn; q += LPT)
-                                    pair_ff_soft<DIM, true>(Th, Tl, sh[w][q], sl[w][q], e2h, e2l,
-                                                            ah, al);
+                                    pair_ff_soft<DIM, true>(Th, Tl, sh[q], sl[q], e2h, e2l, ah, al);
                             } else if (soft) {
                                 for (int q = sub; q < cn; q += LPT)
-                                    pair_ff_soft<DIM, false>(Th, Tl, sh[w][q], sl[w][q], e2h, e2l,
-                                                             ah, al);
+                                    pair_ff_soft<DIM, false>(Th, Tl, sh[q], sl[q], e2h, e2l, ah, al);
                             } else {
                                 for (int q = sub; q < cn; q += LPT)
-                                    fb |= (unsigned)!pair_ff<DIM, false>(Th, Tl, sh[w][q],
-                                                                         sl[w][q], e2h, e2l, ah,
-                                                                         al) << q;
+                                    fb |= (unsigned)!pair_ff<DIM, false>(Th, Tl, sh[q], sl[q], e2h,
+                                                                         e2l, ah, al) << q;
                             }
                             while (fb) {
                                 const int gi = s0 + bb + __ffs(fb) - 1;
@@ -732,34 +738,33 @@ k_batch_traverse(BatchDev b, BatchArgs a)
                 }
             } else {
                 bool open = false;
-                float4 nhv = make_float4(0.f, 0.f, 0.f, 0.f), nlv = nhv;
-                if (act) {
-                    nhv = b.nh[node];
-                    if (!FP32) nlv = b.nl[node];
+                float4 nlv = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (FP32) {   // hi coordinates only, as the single-tree walk
                     float d2 = 0.0f;
 #pragma unroll
                     for (int k = 0; k < DIM; k++) {
-                        // FP32 form: hi coordinates only (exact differences),
-                        // as the single-tree FP32 walk
-                        const float d = FP32 ? __fsub_rn(comp(nhv, k), Th[k])
-                                             : __fadd_rn(__fsub_rn(comp(nhv, k), Th[k]),
-                                                         __fsub_rn(comp(nlv, k), Tl[k]));
+                        const float d = __fsub_rn(comp(nhv, k), Th[k]);
+                        d2 = fmaf(d, d, d2);
+                    }
+                    open = opener(d2, __int_as_float(hd.y), __int_as_float(hd.z), act);
+                } else if (act) {
+                    nlv = b.nl[node];
+                    float d2 = 0.0f;
+#pragma unroll
+                    for (int k = 0; k < DIM; k++) {
+                        const float d = __fadd_rn(__fsub_rn(comp(nhv, k), Th[k]),
+                                                  __fsub_rn(comp(nlv, k), Tl[k]));
                         d2 = fmaf(d, d, d2);
                     }
                     const float dist = d2 > 0.0f ? d2 * rsqrtf(d2) : 0.0f;
                     const float size_f = __int_as_float(hd.y);
-                    if (FP32) {
-                        open = a.mac == 1 ? size_f >= theta_f * (dist - __int_as_float(hd.z))
-                                          : (dist == 0.0f || size_f >= theta_f * dist);
-                    } else {
-                        const float td = theta_f * dist;
-                        const float band = theta_f * fmaf(kBandRel, dist, 2.0f * kBandAbs);
-                        if (size_f >= td + band) open = true;
-                        else if (size_f < td - band) open = false;
-                        else {
-                            open = open_exact64<DIM>(x, y, z, t.cm[node], t.size[node], a.theta);
-                            cnt[3]++;
-                        }
+                    const float td = theta_f * dist;
+                    const float band = theta_f * fmaf(kBandRel, dist, 2.0f * kBandAbs);
+                    if (size_f >= td + band) open = true;
+                    else if (size_f < td - band) open = false;
+                    else {
+                        open = open_exact64<DIM>(x, y, z, t.cm[node], t.size[node], a.theta);
+                        cnt[3]++;
                     }
                 }
                 const unsigned omask = __ballot_sync(FULL, act && open);
@@ -780,11 +785,20 @@ k_batch_traverse(BatchDev b, BatchArgs a)
                     }
                     cnt[1]++;
                 }
-                if (omask && !st.push2(fc, omask)) {
-                    overflow = true;
-                    break;
+                if (omask) {
+                    if (!st.push(fc, omask)) {
+                        overflow = true;
+                        break;
+                    }
+                    node = fc + 1;
+                    mask = omask;
+                    continue;
                 }
             }
+            if (st.empty()) break;
+            const int2 e = st.pop();
+            node = e.x;
+            mask = (unsigned)e.y;
         }
         if (overflow && lane == 0) atomicOr(a.err, kErrStackOverflow);
         // fold the lanes that share a target

@@ -796,6 +796,69 @@ __device__ __forceinline__ void pair_f32_partial2(const TargetF32x2& t, float4 s
     if (DIM == 3) pz = fmaf(f, dz, pz);
 }
 
+// Rows 0 .. np - 1 of a staged leaf block (two sources to a row) for a target
+// with negated coordinates (nT, nL): displacements, r^2 and w = r^-3 of both
+// sources in f32x2 instructions, the forces added to the partial sum p one
+// source after the other.  Every operation and its order are those of
+// pair_f32_partial (x - y is x + (-y) exactly), so the sums are the same bit
+// for bit.  UNIT: masses are exactly 1 and their products are skipped, also
+// exactly.  np is a multiple of four; places past the last source hold
+// stand-ins that add exactly zero.
+template <int DIM, bool CHECK, bool UNIT>
+__device__ __forceinline__ void rows_f32(const LeafStage& st, int np, const float2* nT,
+                                         const float2* nL, float e2, float* p)
+{
+    for (int r0 = 0; r0 < np; r0 += 4)
+#pragma unroll
+    for (int r = r0; r < r0 + 4; r++) {
+        const float4 A = st.a[r], B = st.b[r];
+        const float2 dx = __fadd2_rn(__fadd2_rn(make_float2(A.x, A.y), nT[0]),
+                                     __fadd2_rn(make_float2(B.x, B.y), nL[0]));
+        const float2 dy = __fadd2_rn(__fadd2_rn(make_float2(A.z, A.w), nT[1]),
+                                     __fadd2_rn(make_float2(B.z, B.w), nL[1]));
+        float2 dz = both(0.0f), r2 = __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, both(e2)));
+        if (DIM == 3) {
+            const float4 C = st.c[r];
+            dz = __fadd2_rn(__fadd2_rn(make_float2(C.x, C.y), nT[2]),
+                            __fadd2_rn(make_float2(C.z, C.w), nL[2]));
+            r2 = __ffma2_rn(dz, dz, r2);
+        }
+        const bool ok0 = !CHECK || r2.x >= 0x1p-126f, ok1 = !CHECK || r2.y >= 0x1p-126f;
+        const float2 ri = make_float2(rsqrt_mufu(ok0 ? r2.x : 1.0f), rsqrt_mufu(ok1 ? r2.y : 1.0f));
+        float2 f = __fmul2_rn(__fmul2_rn(ri, ri), ri);
+        if (!UNIT) {
+            const float4 M = st.d[r];
+            f = __fmul2_rn(make_float2(M.x, M.y), f);
+        }
+        if (CHECK) f = make_float2(ok0 ? f.x : 0.0f, ok1 ? f.y : 0.0f);
+        p[0] = fmaf(f.x, dx.x, p[0]);
+        p[1] = fmaf(f.x, dy.x, p[1]);
+        if (DIM == 3) p[2] = fmaf(f.x, dz.x, p[2]);
+        p[0] = fmaf(f.y, dx.y, p[0]);
+        p[1] = fmaf(f.y, dy.y, p[1]);
+        if (DIM == 3) p[2] = fmaf(f.y, dz.y, p[2]);
+    }
+}
+
+// Stages sources [first, first + cn) of a leaf, cn <= 32, for rows_f32 and
+// returns the rows.  Stand-ins: for targets in the box (|T| <= 1) far away, so
+// that r^2 is about 3e36 and r^-3 rounds to zero; when some target lies
+// outside, without mass (the masses must then be used), at a point off every
+// grid.
+static __device__ __forceinline__ int stage_f32(LeafStage& st, int lane, const float4* ph,
+                                                const float4* pl, int first, int cn, bool outside)
+{
+    const int np = ((cn + 7) >> 3) << 2;
+    const float v = outside ? 3.14159265f : 1e18f;
+    float4 h = make_float4(v, v * 1.25f, v * 1.5f, 0.0f), l = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (lane < cn) {
+        h = ph[first + lane];
+        l = pl[first + lane];
+    }
+    if (lane < 2 * np) st.put(lane, h, l);
+    return np;
+}
+
 template <int DIM>
 __device__ __forceinline__ void kahan_add_f32(const float* p, float* acc, float* cmp)
 {
@@ -807,6 +870,32 @@ __device__ __forceinline__ void kahan_add_f32(const float* p, float* acc, float*
         acc[k] = t;
     }
 }
+
+// Opening test of the FP32 form, on the hi coordinates (exact differences on
+// the 2^-23 grid).  The criterion is a heuristic, so a decision at the margin
+// may go either way, but always the same way: `opens` is the definition, and
+// the squares, which need no square root, decide where they are further apart
+// than both forms' rounding (2^-18 of them; each is a handful of roundings).
+// mac 1: the offset criterion, open when d < size / theta + |com - centre|.
+struct OpenF32 {
+    float theta, inv, mac;   // mac: 1 or 0, the weight of |com - centre|
+    __device__ __forceinline__ OpenF32(double th, int m)
+        : theta((float)th), inv(1.0f / (float)th), mac(m == 1 ? 1.0f : 0.0f) {}
+    __device__ __forceinline__ bool opens(float d2, float size, float off) const
+    {
+        const float dist = d2 > 0.0f ? d2 * rsqrtf(d2) : 0.0f;
+        if (mac != 0.0f) return size >= theta * (dist - off);
+        return dist == 0.0f || size >= theta * dist;
+    }
+    // lanes outside `act` return anything
+    __device__ __forceinline__ bool operator()(float d2, float size, float off, bool act) const
+    {
+        const float r = fmaf(off, mac, size * inv), r2 = r * r;
+        bool open = r2 >= d2;
+        if (act && !(fabsf(r2 - d2) > 0x1p-18f * d2)) open = opens(d2, size, off);
+        return open;
+    }
+};
 
 // A node's monopole plus its Plummer-softened traceless quadrupole (FP32
 // form, multipole "quad"), Kahan-added.  With d = com - x (target to node),

@@ -41,13 +41,9 @@ constexpr int kSplitMaxLevels = 10;
 // Tuning (overridable at build time): resident blocks per SM for the fast
 // form (5: 20 warps per SM, registers capped at 96; 4 / 5 / 6 blocks at 1M
 // Plummer 142.4 / 140.5 / 139.1 ms, at 200k 22.5 / 23.0 / 23.8 ms, without
-// softening at 200k 11.0 / 10.6 / 11.3 ms) and the unroll factor of the FP32
-// form's leaf pair loop (8 beats 1-4 by 2-10 %).
+// softening at 200k 11.0 / 10.6 / 11.3 ms).
 #ifndef BHUT_FAST_BLOCKS
 #define BHUT_FAST_BLOCKS 5
-#endif
-#ifndef BHUT_F32_UNROLL
-#define BHUT_F32_UNROLL 8
 #endif
 // Split traversals (split_levels): split while fewer warps than this walk
 // and their subtrees hold more nodes than that.  Swept on GB300:
@@ -82,7 +78,6 @@ constexpr int64_t kWaveWarps = 152 * 4 * 5;   // resident warps of the traversal
 #define BHUT_SPLIT_NODES 16
 #endif
 constexpr int kFastBlocksPerSM = BHUT_FAST_BLOCKS;
-constexpr int kF32Unroll = BHUT_F32_UNROLL;
 
 // ---------------------------------------------------------------------------
 // frame (normalisation) derived from the tree's bounding box
@@ -555,93 +550,63 @@ __global__ void k_split_sum(const double* __restrict__ partial, int64_t nt, int 
 // test in FP32 on hi + lo displacements (each difference exact, rounded
 // once); per-target sums Kahan-compensated: every monopole, and every leaf
 // block of at most 32 pair terms (summed in FP32 first), is one Kahan step.
+// 2M galaxy, theta 0.7, leaf 16: 119 -> 109 ms with two sources to a row, the
+// opening test on squares and the right child from registers; of that about 71
+// ms are the walk (node loads, tests, monopoles), 16 staging leaves, the rest
+// pairs.  Prefetching the next nodes' headers: 122 to 126 ms, not kept.
 // FP64 stays in the tree build (bounding box, Morton keys, masses and
 // centres of mass, quadrupoles) and in the final scaling.
 // ---------------------------------------------------------------------------
 template <int DIM>
 __device__ __forceinline__ void walk_f32(const TreeDev& t, const FastTree& ft, const FastArgs& a,
-                                         int w, int lane, bool valid, int64_t me_sorted,
+                                         int w, int lane, bool valid, bool outside, int64_t me_sorted,
                                          const float* T, const float* Tl, float* acc, float* cmp,
-                                         int2 (*stack)[kStackDepth], float4 (*sh)[kWarp],
-                                         float4 (*sl)[kWarp], unsigned* cnt, bool& overflow)
+                                         int2 (*stack)[kStackDepth], LeafStage* stage,
+                                         unsigned* cnt, bool& overflow)
 {
     const unsigned FULL = 0xffffffffu;
-    const float theta_f = (float)a.theta;
     const bool soft = a.e2h >= 0x1p-126f;   // r^2 >= eps^2 is normal: no small-r test
-    const bool unit = ft.frame->unit != 0;   // every particle mass exactly 1
-    const TargetF32x2 tx = target_f32x2(T, Tl);
-    const unsigned live = __ballot_sync(FULL, valid);
-    if (lane == 0) stack[w][0] = make_int2(0, (int)live);
-    int sp = 1;
-    __syncwarp();
-    while (sp > 0) {
-        const int2 e = stack[w][--sp];
-        __syncwarp();
-        const int node = e.x;
-        const unsigned mask = (unsigned)e.y;
+    const bool unit = ft.frame->unit != 0 && !outside;   // every particle mass exactly 1
+    const float2 nT[3] = {both(-T[0]), both(-T[1]), both(-T[2])};
+    const float2 nL[3] = {both(-Tl[0]), both(-Tl[1]), both(-Tl[2])};
+    const OpenF32 opener(a.theta, a.mac);
+    // (right child straight from registers, as in the fast form's walk)
+    int node = 0, sp = 0;
+    unsigned mask = __ballot_sync(FULL, valid);
+    while (true) {
         const bool act = (mask >> lane) & 1u;
         cnt[2] += act;
         const int4 hd = ft.nhdr[node];   // (first_child, start, count, flag)
-        if (!hd.w) continue;
+        const float4 nh = ft.nh[node];
         const int fc = hd.x;
-        if (fc < 0) {
+        if (!hd.w) {
+        } else if (fc < 0) {
             const int s = hd.y, c = hd.z;
             for (int b = 0; b < c; b += kWarp) {
-                const int jj = b + lane;
-                if (jj < c) {
-                    sh[w][lane] = ft.ph[s + jj];
-                    sl[w][lane] = ft.pl[s + jj];
-                }
-                __syncwarp();
                 const int cn = min(kWarp, c - b);
+                const int np = stage_f32(stage[w], lane, ft.ph, ft.pl, s + b, cn, outside);
+                __syncwarp();
                 if (act) {
                     cnt[0] += cn - (me_sorted >= s + b && me_sorted < s + b + cn);
-                    float2 pxy = make_float2(0.f, 0.f);   // <= 32 terms, then one Kahan step
-                    float pz = 0.f;
-                    if (soft && unit) {
-#pragma unroll (kF32Unroll)
-                        for (int q = 0; q < cn; q++)
-                            pair_f32_partial2<DIM, false, true>(tx, sh[w][q], sl[w][q], a.e2h,
-                                                                pxy, pz);
-                    } else if (soft) {
-#pragma unroll (kF32Unroll)
-                        for (int q = 0; q < cn; q++)
-                            pair_f32_partial2<DIM, false, false>(tx, sh[w][q], sl[w][q], a.e2h,
-                                                                 pxy, pz);
-                    } else {
-#pragma unroll (kF32Unroll)
-                        for (int q = 0; q < cn; q++)
-                            pair_f32_partial2<DIM, true, false>(tx, sh[w][q], sl[w][q], a.e2h,
-                                                                pxy, pz);
-                    }
-                    const float part[3] = {pxy.x, pxy.y, pz};
+                    float part[3] = {0.f, 0.f, 0.f};   // <= 32 terms, then one Kahan step
+                    if (soft && unit)
+                        rows_f32<DIM, false, true>(stage[w], np, nT, nL, a.e2h, part);
+                    else if (soft)
+                        rows_f32<DIM, false, false>(stage[w], np, nT, nL, a.e2h, part);
+                    else
+                        rows_f32<DIM, true, false>(stage[w], np, nT, nL, a.e2h, part);
                     kahan_add_f32<DIM>(part, acc, cmp);
                 }
                 __syncwarp();
             }
         } else {
-            bool open = false;
-            float4 nh = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (act) {
-                // opening test on the hi coordinates (exact differences on
-                // the 2^-23 grid): the FP32 form's criterion is a heuristic,
-                // so a decision at the margin may go either way
-                nh = ft.nh[node];
-                float d2 = 0.0f;
+            float d2 = 0.0f;
 #pragma unroll
-                for (int k = 0; k < DIM; k++) {
-                    const float d = __fsub_rn(comp(nh, k), T[k]);
-                    d2 = fmaf(d, d, d2);
-                }
-                const float dist = d2 > 0.0f ? d2 * rsqrtf(d2) : 0.0f;
-                const float size_f = __int_as_float(hd.y);
-                if (a.mac == 1) {
-                    // offset criterion: open when d < size/theta + |com - centre|
-                    open = size_f >= theta_f * (dist - __int_as_float(hd.z));
-                } else {
-                    open = dist == 0.0f || size_f >= theta_f * dist;
-                }
+            for (int k = 0; k < DIM; k++) {
+                const float d = __fsub_rn(comp(nh, k), T[k]);
+                d2 = fmaf(d, d, d2);
             }
+            const bool open = opener(d2, __int_as_float(hd.y), __int_as_float(hd.z), act);
             const unsigned omask = __ballot_sync(FULL, act && open);
             if (act && !open) {
                 if (ft.nq0)
@@ -653,23 +618,34 @@ __device__ __forceinline__ void walk_f32(const TreeDev& t, const FastTree& ft, c
             }
             if (omask) {
                 if (sp + 2 > kStackDepth) { overflow = true; break; }
-                if (lane == 0) {
-                    stack[w][sp] = make_int2(fc, (int)omask);
-                    stack[w][sp + 1] = make_int2(fc + 1, (int)omask);
-                }
-                sp += 2;
-                __syncwarp();
+                if (lane == 0) stack[w][sp] = make_int2(fc, (int)omask);
+                sp++;
+                node = fc + 1;
+                mask = omask;
+                continue;
             }
         }
+        if (sp == 0) break;
+        __syncwarp();
+        const int2 e = stack[w][--sp];
+        __syncwarp();
+        node = e.x;
+        mask = (unsigned)e.y;
     }
 }
 
+// Resident blocks per SM: the walk waits for loads (7 / 8 / 9 / 10 blocks at
+// 2M galaxy, theta 0.7, leaf 16: 116.9 / 111.3 / 110.0 / 110.3 ms; at 8 to 10
+// the kernel issues on about 78 % of the clocks).
+#ifndef BHUT_F32_BLOCKS
+#define BHUT_F32_BLOCKS 9
+#endif
 template <int DIM>
-__global__ void __launch_bounds__(kFastThreads)
+__global__ void __launch_bounds__(kFastThreads, BHUT_F32_BLOCKS)
 k_traverse_fp32(TreeDev t, FastTree ft, FastArgs a)
 {
     __shared__ int2 stack[kFastWarps][kStackDepth];
-    __shared__ float4 sh[kFastWarps][kWarp], sl[kFastWarps][kWarp];
+    __shared__ LeafStage stage[kFastWarps];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned FULL = 0xffffffffu;
     const double conv = __dmul_rn(ft.frame->conv, a.G);
@@ -678,17 +654,20 @@ k_traverse_fp32(TreeDev t, FastTree ft, FastArgs a)
         const int64_t i = base + lane;
         const bool valid = i < a.nt;
         float T[3] = {0.f, 0.f, 0.f}, Tl[3] = {0.f, 0.f, 0.f};
+        bool outside = false;
         if (valid) {
             const float4 h = a.th ? a.th[i] : ft.ph[i];
             const float4 l = a.th ? a.tl[i] : ft.pl[i];
             T[0] = h.x; T[1] = h.y; T[2] = h.z;
             Tl[0] = l.x; Tl[1] = l.y; Tl[2] = l.z;
+            outside = a.th && h.w != 0.0f;
         }
+        outside = __any_sync(FULL, outside);
         float acc[3] = {0.f, 0.f, 0.f}, cmp[3] = {0.f, 0.f, 0.f};
         unsigned cnt[5] = {0, 0, 0, 0, 0};
         const int64_t me_sorted = (valid && a.th == nullptr) ? i : -1;
         bool overflow = false;
-        walk_f32<DIM>(t, ft, a, w, lane, valid, me_sorted, T, Tl, acc, cmp, stack, sh, sl, cnt,
+        walk_f32<DIM>(t, ft, a, w, lane, valid, outside, me_sorted, T, Tl, acc, cmp, stack, stage, cnt,
                       overflow);
         if (overflow && lane == 0) atomicOr(a.err, kErrStackOverflow);
         if (a.stats) {
