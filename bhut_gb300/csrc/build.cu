@@ -100,7 +100,7 @@ k_bbox(const double* __restrict__ pos, const double* __restrict__ mass, int64_t 
             }
         }
     }
-    if (__any_sync(0xffffffffu, bad) && (tid & 31) == 0) atomicOr(err, kErrNonFinite);
+    if (err && __any_sync(0xffffffffu, bad) && (tid & 31) == 0) atomicOr(err, kErrNonFinite);
     __shared__ uint64_t s_lo[kBoxThreads], s_hi[kBoxThreads], s_m[kBoxThreads];
     __shared__ bool s_last;
     __shared__ unsigned s_nan;   // bit d: axis d holds a NaN
@@ -111,6 +111,7 @@ k_bbox(const double* __restrict__ pos, const double* __restrict__ mass, int64_t 
     __syncthreads();
     if (nan) atomicOr(&s_nan, 1u << axis);
     if (mdiff) atomicOr(&s_nan, 8u);   // bit 3: masses not all equal
+    if (bad) atomicOr(&s_nan, 16u);    // bit 4: a value is not finite
     // thread d < dim reduces its axis (the threads with tid = d (mod dim):
     // the block's first index is a multiple of 6); thread 3 the masses
     if (tid < dim) {
@@ -128,7 +129,7 @@ k_bbox(const double* __restrict__ pos, const double* __restrict__ mass, int64_t 
     }
     __syncthreads();
     if (tid == 0) {
-        partial[blockIdx.x * 8 + 7] = (double)s_nan;
+        partial[blockIdx.x * 8 + 7] = (double)(s_nan & 31u);
         __threadfence();
         const unsigned ticket = atomicAdd(done_counter, 1u);
         s_last = (ticket == gridDim.x - 1);
@@ -160,7 +161,8 @@ k_bbox(const double* __restrict__ pos, const double* __restrict__ mass, int64_t 
         }
         if ((tid & 31) == 0) s_red[k][tid >> 5] = a[k];
     }
-    if (nanmask) atomicOr(&s_nan, nanmask << 4);   // bits 4..6: the grid's NaN axes, 7: masses differ
+    // bits 8..10: the grid's NaN axes, 11: masses differ, 12: not finite
+    if (nanmask) atomicOr(&s_nan, nanmask << 8);
     __syncthreads();
     if (tid < 7) {
         uint64_t acc = s_red[tid][0];
@@ -193,15 +195,16 @@ k_bbox(const double* __restrict__ pos, const double* __restrict__ mass, int64_t 
             box[8 + d] = r;
         }
         box[11] = degenerate ? 1.0 : 0.0;
-        for (int d = 0; d < 3; d++) box[12 + d] = (s_nan >> (4 + d)) & 1u ? 1.0 : 0.0;
+        for (int d = 0; d < 3; d++) box[12 + d] = (s_nan >> (8 + d)) & 1u ? 1.0 : 0.0;
         // box[15]: every particle has the same positive, finite mass (the
         // float-float traversal then measures masses in units of it)
         bool unit = false;
-        if (mass && !((s_nan >> 7) & 1u)) {
+        if (mass && !((s_nan >> 11) & 1u)) {
             const double m0 = mass[0];
             unit = m0 > 0.0 && finite_bits((uint64_t)__double_as_longlong(m0));
         }
         box[15] = unit ? 1.0 : 0.0;
+        box[16] = (s_nan >> 12) & 1u ? 1.0 : 0.0;
         *done_counter = 0;
     }
 }

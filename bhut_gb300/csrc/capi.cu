@@ -5,9 +5,11 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
-
 #include <utility>
+#include <vector>
+
 #include "../../include/bhut_gb300.h"
 #include "tree.cuh"
 
@@ -36,6 +38,9 @@ int cuda_status(cudaError_t e, const char* what)
     return e == cudaErrorMemoryAllocation ? kNoMemory : kCuda;
 }
 
+// Destroys the idle trees kept for reuse (bhut_tree_destroy); false: none.
+bool release_idle_trees();
+
 // ---- device buffers -----------------------------------------------------------
 struct DevBuf {
     void* p = nullptr;
@@ -50,6 +55,10 @@ struct DevBuf {
         }
         size_t want = need < 256 ? 256 : need;
         cudaError_t e = cudaMallocAsync(&p, want, s);
+        if (e == cudaErrorMemoryAllocation && release_idle_trees()) {
+            cudaGetLastError();
+            e = cudaMallocAsync(&p, want, s);
+        }
         if (e != cudaSuccess) {
             p = nullptr;
             return cuda_status(e, "cudaMallocAsync");
@@ -107,12 +116,19 @@ struct BuildGraph {
     }
 };
 
+constexpr size_t kStatsOffset = 16, kStatsCount = 5, kStatusBytes = 128;
+static_assert(kStatsOffset + sizeof(unsigned long long) * kStatsCount <= kStatusBytes, "status");
+
 struct bhut_tree {
     int dim = 3;
     int leaf = 32;
     int form = BHUT_FORM_EXACT;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
+    int device = -1;
+    // Pinned host memory for what the host waits for: the input's box
+    // (kBoxDoubles), then the error word and the traversal counters.
+    double* pin = nullptr;
     bool built = false;
     int64_t n = 0;
     int64_t m = 0;
@@ -124,10 +140,12 @@ struct bhut_tree {
     // nodes
     DevBuf cm, size, center, half, lo, hi, first_child, start, count, parent, leaf_list, arrive;
     // scratch
-    DevBuf sort_scratch, box_partial, box, counters, err, stats;
+    DevBuf sort_scratch, box_partial, box, counters;
+    DevBuf err;               // error word; from kStatsOffset on the traversal counters
     DevBuf frontier;          // bottom-up scratch: one entry per leaf
     DevBuf box_in;            // bounding box of pos_in, computed while staging
     bool box_in_valid = false;
+    double hbox[kBoxDoubles] = {}, hbox_in[kBoxDoubles] = {};   // host copies of box, box_in
     BuildGraph graphs[2];     // captured builds (see do_build)
     int graph_next = 0;
     bool graph_unsupported = false;
@@ -135,12 +153,28 @@ struct bhut_tree {
     // traversal targets
     DevBuf tpos, tkeys, tperm, tx, ty, tz, tbox, out, split_partial;
     // float-float copies for the fast form
-    DevBuf frame, ph, pl, nh, nl, nsize, ndelta, th, tl, quad, nq0, nq1, nhdr;
+    FastFrame frame{};        // from hbox
+    DevBuf ph, pl, nh, nl, nsize, ndelta, th, tl, quad, nq0, nq1, nhdr;
     bool ff_valid = false;
     bool ff_quad = false;
     bool ff_fine = false;     // lo parts of form "fast"
     int mac = 0;
     int multipole = BHUT_MULTIPOLE_MONO;
+
+    std::vector<DevBuf*> buffers()
+    {
+        return {&pos, &mass, &keys, &perm, &sx, &sy, &sz, &sm, &cm, &size, &center, &half, &lo, &hi,
+                &first_child, &start, &count, &parent, &leaf_list, &arrive, &sort_scratch,
+                &box_partial, &box, &counters, &err, &tpos, &tkeys, &tperm, &tx, &ty, &tz, &tbox,
+                &out, &split_partial, &ph, &pl, &nh, &nl, &nsize, &ndelta, &th, &tl, &quad, &nq0,
+                &nq1, &nhdr, &pos_in, &mass_in, &box_in, &frontier};
+    }
+    unsigned long long* stats() const
+    {
+        return reinterpret_cast<unsigned long long*>(err.as<char>() + kStatsOffset);
+    }
+    double* pin_box() const { return pin; }
+    unsigned char* pin_status() const { return reinterpret_cast<unsigned char*>(pin + kBoxDoubles); }
 
     TreeDev dev() const
     {
@@ -170,11 +204,17 @@ struct bhut_tree {
 
 namespace {
 
-int check_err_word(bhut_tree* t, const char* what)
+// Waits for the stream and turns the error word into a status; `stats`: the
+// traversal counters come with it.
+int check_err_word(bhut_tree* t, const char* what, bool stats = false)
 {
-    unsigned e = 0;
-    BHUT_CUDA(cudaMemcpyAsync(&e, t->err.p, sizeof(unsigned), cudaMemcpyDeviceToHost, t->stream));
+    const size_t bytes = stats ? kStatsOffset + sizeof(unsigned long long) * kStatsCount
+                               : sizeof(unsigned);
+    BHUT_CUDA(cudaMemcpyAsync(t->pin_status(), t->err.p, bytes, cudaMemcpyDeviceToHost, t->stream));
     BHUT_CUDA(cudaStreamSynchronize(t->stream));
+    unsigned e;
+    memcpy(&e, t->pin_status(), sizeof(e));
+    if (stats) memcpy(t->last_stats, t->pin_status() + kStatsOffset, sizeof(t->last_stats));
     if (e == 0) return kOk;
     BHUT_CUDA(cudaMemsetAsync(t->err.p, 0, sizeof(unsigned), t->stream));
     if (e & kErrNonFinite) {
@@ -183,6 +223,16 @@ int check_err_word(bhut_tree* t, const char* what)
     }
     set_error("device error word 0x%x in %s", e, what);
     return kDeviceFlag;
+}
+
+// Host copy of a device bounding box; waits for the stream.
+int read_box(bhut_tree* t, const DevBuf& box, double* host)
+{
+    BHUT_CUDA(cudaMemcpyAsync(t->pin_box(), box.p, sizeof(double) * kBoxDoubles,
+                              cudaMemcpyDeviceToHost, t->stream));
+    BHUT_CUDA(cudaStreamSynchronize(t->stream));
+    memcpy(host, t->pin_box(), sizeof(double) * kBoxDoubles);
+    return kOk;
 }
 
 // Morton keys + stable sort of `n` AoS points into keys/perm (perm is the
@@ -281,10 +331,12 @@ int do_build(bhut_tree* t, int64_t n)
     // the box of these positions was computed while they were staged
     if (t->box_in_valid) {
         std::swap(t->box, t->box_in);
+        std::copy(t->hbox_in, t->hbox_in + kBoxDoubles, t->hbox);
     } else {
         BHUT_TRY(launch_bbox(t->pos.as<double>(), t->mass.as<double>(), n, dim,
                              t->box_partial.as<double>(), t->counters.as<unsigned>(),
                              t->box.as<double>(), t->err.as<unsigned>(), s));
+        BHUT_TRY(read_box(t, t->box, t->hbox));
     }
     t->box_in_valid = false;
     // replay a captured graph of this exact buffer set; capture one when the
@@ -392,16 +444,13 @@ int load_particles(bhut_tree* t, const double* positions, const double* masses, 
                                       cudaMemcpyHostToDevice, s));
         }
     }
-    unsigned* flag = t->counters.as<unsigned>() + 4;
-    BHUT_CUDA(cudaMemsetAsync(flag, 0, sizeof(unsigned), s));
     BHUT_TRY(t->box_in.ensure(sizeof(double) * kBoxDoubles, s));
     BHUT_TRY(t->box_partial.ensure(sizeof(double) * kBoxPartialDoubles, s));
+    t->box_in_valid = false;
     BHUT_TRY(launch_stage_bbox(psrc, msrc, n, t->dim, pcopy, mcopy, t->box_partial.as<double>(),
-                               t->counters.as<unsigned>(), t->box_in.as<double>(), flag, s));
-    unsigned bad = 0;
-    BHUT_CUDA(cudaMemcpyAsync(&bad, flag, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-    BHUT_CUDA(cudaStreamSynchronize(s));
-    if (bad) {
+                               t->counters.as<unsigned>(), t->box_in.as<double>(), nullptr, s));
+    BHUT_TRY(read_box(t, t->box_in, t->hbox_in));
+    if (t->hbox_in[16] != 0.0) {
         set_error("positions must be finite (NaN or Inf found)");
         return kInvalid;
     }
@@ -431,11 +480,11 @@ int out_target(bhut_tree* t, double* out, size_t bytes, OutTarget* o)
     return kOk;
 }
 
-int finish_out(bhut_tree* t, const OutTarget& o, size_t bytes, const char* what)
+int finish_out(bhut_tree* t, const OutTarget& o, size_t bytes, const char* what, bool stats)
 {
     if (o.host && bytes)
         BHUT_CUDA(cudaMemcpyAsync(o.host, o.dev, bytes, cudaMemcpyDeviceToHost, t->stream));
-    return check_err_word(t, what);
+    return check_err_word(t, what, stats);
 }
 
 // Float-float copies of particles and nodes for the fast form (built once
@@ -446,7 +495,7 @@ int prepare_fast(bhut_tree* t)
     const bool fine = t->form == BHUT_FORM_FAST;
     if (t->ff_valid && t->ff_quad == want_quad && t->ff_fine == fine) return kOk;
     cudaStream_t s = t->stream;
-    BHUT_TRY(t->frame.ensure(sizeof(FastFrame), s));
+    t->frame = frame_of_box(t->hbox, t->dim);
     BHUT_TRY(t->ph.ensure(sizeof(float4) * t->n, s));
     BHUT_TRY(t->pl.ensure(sizeof(float4) * t->n, s));
     BHUT_TRY(t->nh.ensure(sizeof(float4) * t->m, s));
@@ -466,7 +515,7 @@ int prepare_fast(bhut_tree* t)
                                     t->frontier.as<int32_t>(), t->counters.as<unsigned>() + 6,
                                     t->err.as<unsigned>(), s));
     }
-    BHUT_TRY(launch_fast_prepare(t->box.as<double>(), t->dim, fine, t->frame.as<FastFrame>(), t->dev(),
+    BHUT_TRY(launch_fast_prepare(t->frame, fine, t->dev(),
                                  t->center.as<double>(), t->ph.as<float4>(), t->pl.as<float4>(),
                                  t->nh.as<float4>(), t->nl.as<float4>(), t->nsize.as<float>(),
                                  t->ndelta.as<float>(), quad ? t->quad.as<double>() : nullptr,
@@ -480,21 +529,10 @@ int prepare_fast(bhut_tree* t)
 
 FastTree fast_tree(const bhut_tree* t)
 {
-    return FastTree{t->frame.as<FastFrame>(), t->ph.as<float4>(), t->pl.as<float4>(),
+    return FastTree{t->frame, t->ph.as<float4>(), t->pl.as<float4>(),
                     t->nh.as<float4>(), t->nl.as<float4>(), t->nsize.as<float>(),
                     t->ndelta.as<float>(), t->ff_quad ? t->nq0.as<float4>() : nullptr,
                     t->ff_quad ? t->nq1.as<float2>() : nullptr, t->nhdr.as<int4>()};
-}
-
-// Scale of the fast form's normalised coordinates (the frame's s), read
-// back once per traversal to scale the softening.
-int frame_scale(bhut_tree* t, double* s_out)
-{
-    FastFrame f;
-    BHUT_CUDA(cudaMemcpyAsync(&f, t->frame.p, sizeof(FastFrame), cudaMemcpyDeviceToHost, t->stream));
-    BHUT_CUDA(cudaStreamSynchronize(t->stream));
-    *s_out = f.s;
-    return kOk;
 }
 
 int traverse(bhut_tree* t, const double* tx, const double* ty, const double* tz,
@@ -502,9 +540,8 @@ int traverse(bhut_tree* t, const double* tx, const double* ty, const double* tz,
              double G, double* out, bool self_targets)
 {
     TreeDev d = t->dev();
-    BHUT_TRY(t->stats.ensure(sizeof(unsigned long long) * 8, t->stream));
-    BHUT_CUDA(cudaMemsetAsync(t->stats.p, 0, sizeof(unsigned long long) * 8, t->stream));
-    unsigned long long* st = t->stats.as<unsigned long long>();
+    unsigned long long* st = t->stats();
+    BHUT_CUDA(cudaMemsetAsync(st, 0, sizeof(unsigned long long) * kStatsCount, t->stream));
     // (form fp32 keeps one order of its sums)
     const int levels = t->form == BHUT_FORM_FP32
                            ? 0
@@ -515,19 +552,17 @@ int traverse(bhut_tree* t, const double* tx, const double* ty, const double* tz,
     case BHUT_FORM_FAST:
     case BHUT_FORM_FP32: {
         BHUT_TRY(prepare_fast(t));
-        double sc = 1.0;
-        BHUT_TRY(frame_scale(t, &sc));
         const float4* th = nullptr;
         const float4* tl = nullptr;
         if (!self_targets) {
             BHUT_TRY(t->th.ensure(sizeof(float4) * nt, t->stream));
             BHUT_TRY(t->tl.ensure(sizeof(float4) * nt, t->stream));
-            BHUT_TRY(launch_fast_targets(tx, ty, tz, nt, t->dim, t->ff_fine, t->frame.as<FastFrame>(),
+            BHUT_TRY(launch_fast_targets(tx, ty, tz, nt, t->dim, t->ff_fine, t->frame,
                                          t->th.as<float4>(), t->tl.as<float4>(), t->stream));
             th = t->th.as<float4>();
             tl = t->tl.as<float4>();
         }
-        const double es = eps * sc;
+        const double es = eps * t->frame.s;
         BHUT_TRY(launch_traverse_fast(d, fast_tree(t), th, tl, tx, ty, tz, self_id, out_idx, nt,
                                       theta, eps, G, es * es, out, t->err.as<unsigned>(), st,
                                       t->stream, t->form == BHUT_FORM_FP32,
@@ -541,12 +576,100 @@ int traverse(bhut_tree* t, const double* tx, const double* ty, const double* tz,
                                        t->err.as<unsigned>(), st, t->stream, levels,
                                        t->split_partial.as<double>()));
     }
-    BHUT_CUDA(cudaMemcpyAsync(t->last_stats, st, sizeof(unsigned long long) * 5,
-                              cudaMemcpyDeviceToHost, t->stream));
     return kOk;
 }
 
+// Small trees on streams of their own are kept for the next bhut_tree_create
+// instead of being destroyed: a one-shot solve of a few thousand particles
+// spends more on creating a stream and some forty buffers, and on giving them
+// back, than on its kernels (1,000 particles: 195 of 690 us).  Bounded to
+// kIdleTrees of kIdleBytes each; given back when an allocation of the library
+// fails.  A tree in the pool holds no results: everything but stream, buffers
+// and pinned memory is reset.
+constexpr size_t kIdleTrees = 4, kIdleBytes = 32u << 20;
+
+struct IdleTrees {
+    std::mutex m;
+    std::vector<bhut_tree*> trees;
+};
+
+IdleTrees& idle_trees()
+{
+    static IdleTrees* p = new IdleTrees;   // never destroyed: CUDA is gone at exit
+    return *p;
+}
+
+bhut_tree* take_idle_tree(int dim, int leaf_size)
+{
+    int device = -1;
+    if (cudaGetDevice(&device) != cudaSuccess) return nullptr;
+    IdleTrees& pool = idle_trees();
+    std::lock_guard<std::mutex> lock(pool.m);
+    for (size_t k = pool.trees.size(); k-- > 0;) {
+        bhut_tree* t = pool.trees[k];
+        if (t->device != device) continue;
+        pool.trees.erase(pool.trees.begin() + (std::ptrdiff_t)k);
+        t->dim = dim;
+        t->leaf = leaf_size;
+        return t;
+    }
+    return nullptr;
+}
+
+// Takes a tree whose stream is idle and without error; false: not kept.
+bool keep_idle_tree(bhut_tree* t)
+{
+    if (!t->own_stream || t->device < 0 || !t->pin) return false;
+    size_t bytes = 0;
+    for (const DevBuf* b : t->buffers()) bytes += b->bytes;
+    if (bytes > kIdleBytes) return false;
+    if (cudaMemsetAsync(t->counters.p, 0, sizeof(unsigned) * 8, t->stream) != cudaSuccess ||
+        cudaMemsetAsync(t->err.p, 0, kStatusBytes, t->stream) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    for (BuildGraph& g : t->graphs) {
+        g.reset();
+        g = BuildGraph{};
+    }
+    t->form = BHUT_FORM_EXACT;
+    t->mac = 0;
+    t->multipole = BHUT_MULTIPOLE_MONO;
+    t->built = t->topo_valid = t->ff_valid = t->box_in_valid = t->graph_unsupported = false;
+    t->n = t->m = 0;
+    t->tt = TopoTables{};
+    t->graph_next = 0;
+    std::fill(std::begin(t->last_stats), std::end(t->last_stats), 0ull);
+    IdleTrees& pool = idle_trees();
+    std::lock_guard<std::mutex> lock(pool.m);
+    if (pool.trees.size() >= kIdleTrees) return false;
+    pool.trees.push_back(t);
+    return true;
+}
+
+void free_tree(bhut_tree* t)
+{
+    for (DevBuf* b : t->buffers()) b->release(t->stream);
+    cudaStreamSynchronize(t->stream);
+    for (BuildGraph& g : t->graphs) g.reset();
+    if (t->pin) cudaFreeHost(t->pin);
+    if (t->own_stream) cudaStreamDestroy(t->stream);
+    delete t;
+}
+
 }  // namespace
+
+bool bhut::release_idle_trees()
+{
+    std::vector<bhut_tree*> trees;
+    {
+        IdleTrees& pool = idle_trees();
+        std::lock_guard<std::mutex> lock(pool.m);
+        trees.swap(pool.trees);
+    }
+    for (bhut_tree* t : trees) free_tree(t);
+    return !trees.empty();
+}
 
 extern "C" {
 
@@ -568,6 +691,7 @@ int bhut_tree_create(int dim, int leaf_size, void* stream, bhut_tree** out)
     *out = nullptr;
     if (dim != 2 && dim != 3) { set_error("dim must be 2 or 3, got %d", dim); return kInvalid; }
     if (leaf_size <= 0) { set_error("leaf_size must be positive, got %d", leaf_size); return kInvalid; }
+    if (!stream && (*out = take_idle_tree(dim, leaf_size)) != nullptr) return kOk;
     bhut_tree* t = new bhut_tree();
     t->dim = dim;
     t->leaf = leaf_size;
@@ -577,13 +701,16 @@ int bhut_tree_create(int dim, int leaf_size, void* stream, bhut_tree** out)
         cudaError_t e = cudaStreamCreateWithFlags(&t->stream, cudaStreamNonBlocking);
         if (e != cudaSuccess) { delete t; return cuda_status(e, "cudaStreamCreate"); }
         t->own_stream = true;
+        if (cudaGetDevice(&t->device) != cudaSuccess) t->device = -1;
     }
     int st = t->counters.ensure(sizeof(unsigned) * 8, t->stream);
-    if (st == kOk) st = t->err.ensure(sizeof(unsigned), t->stream);
+    if (st == kOk) st = t->err.ensure(kStatusBytes, t->stream);
     if (st == kOk) {
-        cudaError_t e = cudaMemsetAsync(t->counters.p, 0, sizeof(unsigned) * 8, t->stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(t->err.p, 0, sizeof(unsigned), t->stream);
-        if (e != cudaSuccess) st = cuda_status(e, "cudaMemsetAsync");
+        cudaError_t e = cudaMallocHost(&t->pin, sizeof(double) * kBoxDoubles + kStatusBytes);
+        if (e == cudaSuccess)
+            e = cudaMemsetAsync(t->counters.p, 0, sizeof(unsigned) * 8, t->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(t->err.p, 0, kStatusBytes, t->stream);
+        if (e != cudaSuccess) st = cuda_status(e, "tree status");
     }
     if (st != kOk) { bhut_tree_destroy(t); return st; }
     *out = t;
@@ -721,7 +848,7 @@ int bhut_tree_accel_self(bhut_tree* t, double theta, double softening, double G,
     BHUT_TRY(traverse(t, t->sx.as<double>(), t->sy.as<double>(), t->sz.as<double>(),
                       t->perm.as<int32_t>(), t->perm.as<int32_t>(), t->n, theta, softening, G,
                       o.dev, true));
-    return finish_out(t, o, bytes, "accelerations");
+    return finish_out(t, o, bytes, "accelerations", true);
 }
 
 int bhut_tree_accel_targets(bhut_tree* t, const double* targets, int64_t mt, double theta,
@@ -750,7 +877,7 @@ int bhut_tree_accel_targets(bhut_tree* t, const double* targets, int64_t mt, dou
     BHUT_TRY(out_target(t, out, bytes, &o));
     BHUT_TRY(traverse(t, t->tx.as<double>(), t->ty.as<double>(), t->tz.as<double>(), nullptr,
                       t->tperm.as<int32_t>(), mt, theta, softening, G, o.dev, false));
-    return finish_out(t, o, bytes, "accelerations at targets");
+    return finish_out(t, o, bytes, "accelerations at targets", true);
 }
 
 int bhut_tree_stats(const bhut_tree* t, int64_t* p2p, int64_t* m2p, int64_t* visits)
@@ -830,21 +957,8 @@ int bhut_tree_export(const bhut_tree* t, double* center, double* half_size, doub
 void bhut_tree_destroy(bhut_tree* t)
 {
     if (!t) return;
-    cudaStream_t s = t->stream;
-    DevBuf* all[] = {&t->pos, &t->mass, &t->keys, &t->perm, &t->sx, &t->sy, &t->sz, &t->sm,
-                     &t->cm, &t->size, &t->center, &t->half, &t->lo, &t->hi, &t->first_child,
-                     &t->start, &t->count, &t->parent, &t->leaf_list, &t->arrive,
-                     &t->sort_scratch, &t->box_partial, &t->box, &t->counters, &t->err, &t->stats,
-                     &t->tpos, &t->tkeys, &t->tperm, &t->tx, &t->ty, &t->tz, &t->tbox, &t->out,
-                     &t->split_partial,
-                     &t->frame, &t->ph, &t->pl, &t->nh, &t->nl, &t->nsize, &t->ndelta, &t->th,
-                     &t->tl, &t->quad, &t->nq0, &t->nq1, &t->nhdr, &t->pos_in, &t->mass_in,
-                     &t->box_in, &t->frontier};
-    for (DevBuf* b : all) b->release(s);
-    cudaStreamSynchronize(s);
-    for (BuildGraph& g : t->graphs) g.reset();
-    if (t->own_stream) cudaStreamDestroy(s);
-    delete t;
+    if (cudaStreamSynchronize(t->stream) == cudaSuccess && keep_idle_tree(t)) return;
+    free_tree(t);
 }
 
 int bhut_morton_keys(const double* positions, int64_t n, int dim, uint64_t* keys, void* stream)
@@ -946,7 +1060,7 @@ int bhut_direct_accelerations(const double* positions, const double* masses, int
                                       targets ? t->tpos.as<double>() : nullptr,
                                       targets ? nullptr : self_idx.as<int64_t>(), mt, softening, G,
                                       o.dev, partial.as<double>(), chunks, s);
-    if (rc == kOk) rc = finish_out(t, o, bytes, "direct sum");
+    if (rc == kOk) rc = finish_out(t, o, bytes, "direct sum", false);
     self_idx.release(s);
     partial.release(s);
     bhut_tree_destroy(t);
@@ -1013,7 +1127,7 @@ int bhut_normalize_to_unit(const double* points, int64_t n, int dim, const doubl
     if (rc == kOk) rc = out_target(t, out, bytes, &o);
     if (rc == kOk) rc = launch_normalize(t->pos.as<double>(), n, dim, lim.as<double>(),
                                          lim.as<double>() + 3, 1.0 - eps, o.dev, s);
-    if (rc == kOk) rc = finish_out(t, o, bytes, "normalize_to_unit");
+    if (rc == kOk) rc = finish_out(t, o, bytes, "normalize_to_unit", false);
     lim.release(s);
     bhut_tree_destroy(t);
     return rc;
@@ -1232,6 +1346,7 @@ int bhut_tree_import(bhut_tree* t, const double* positions, const double* masses
     if (rc == kOk) rc = launch_bbox(t->pos.as<double>(), t->mass.as<double>(), n, dim,
                                     t->box_partial.as<double>(), t->counters.as<unsigned>(),
                                     t->box.as<double>(), t->err.as<unsigned>(), s);
+    if (rc == kOk) rc = read_box(t, t->box, t->hbox);
     unsigned nleaves = 0;
     if (rc == kOk) {
         cudaError_t e = cudaMemcpyAsync(&nleaves, leaves, sizeof(unsigned), cudaMemcpyDeviceToHost, s);

@@ -33,13 +33,14 @@ constexpr float kHugeR = 0x1p+100f;    // r^2 above this -> FP64 pair
 constexpr float kBandRel = 0x1p-18f;   // opening-test error band, relative part
 constexpr float kBandAbs = 0x1p-40f;   // ... absolute part per unit of (1 + |target|)
 
-static __device__ void frame_from_box(const double* box, int dim, FastFrame* f)
+// (Only single roundings and powers of two: host and device agree bit for bit.)
+static __host__ __device__ inline void frame_from_box(const double* box, int dim, FastFrame* f)
 {
     double h = 0.0;
     for (int d = 0; d < 3; d++) f->c[d] = 0.0;
     for (int d = 0; d < dim; d++) {
-        f->c[d] = __dmul_rn(__dadd_rn(box[d], box[3 + d]), 0.5);
-        double e = __dmul_rn(__dsub_rn(box[3 + d], box[d]), 0.5);
+        f->c[d] = (box[d] + box[3 + d]) * 0.5;
+        double e = (box[3 + d] - box[d]) * 0.5;
         h = e > h ? e : h;
     }
     if (!(h > 0.0)) h = 1.0;
@@ -61,11 +62,11 @@ static __device__ void frame_from_box(const double* box, int dim, FastFrame* f)
 // bounding-box kernel): masses are measured in units of m0, so a particle's
 // normalised mass is exactly 1 and a node's is M / m0 (FP64, then split hi +
 // lo).
-static __device__ void frame_unit_mass(double m0, bool uniform, FastFrame* f)
+static __host__ __device__ inline void frame_unit_mass(double m0, bool uniform, FastFrame* f)
 {
     if (!uniform || !(m0 > 0x1p-1000 && m0 < 0x1p+1000)) return;
-    f->ms = __drcp_rn(m0);
-    f->conv = __dmul_rn(__dmul_rn(m0, f->s), f->s);   // s a power of two: exact
+    f->ms = 1.0 / m0;
+    f->conv = m0 * f->s * f->s;   // s a power of two: exact
     f->unit = 1;
 }
 

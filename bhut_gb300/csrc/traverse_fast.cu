@@ -82,20 +82,19 @@ constexpr int kFastBlocksPerSM = BHUT_FAST_BLOCKS;
 // ---------------------------------------------------------------------------
 // frame (normalisation) derived from the tree's bounding box
 // ---------------------------------------------------------------------------
-__global__ void k_frame(const double* __restrict__ box, int dim, FastFrame* __restrict__ f)
+FastFrame frame_of_box(const double* box, int dim)
 {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        frame_from_box(box, dim, f);
-        frame_unit_mass(box[6], box[15] != 0.0, f);
-    }
+    FastFrame f;
+    frame_from_box(box, dim, &f);
+    frame_unit_mass(box[6], box[15] != 0.0, &f);
+    return f;
 }
 
 __global__ void k_ff_particles(const double* __restrict__ sx, const double* __restrict__ sy,
                                const double* __restrict__ sz, const double* __restrict__ sm,
-                               int64_t n, int dim, bool fine, const FastFrame* __restrict__ fr,
+                               int64_t n, int dim, bool fine, FastFrame f,
                                float4* __restrict__ ph, float4* __restrict__ pl)
 {
-    const FastFrame f = *fr;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
         float4 h, l;
@@ -111,13 +110,12 @@ __global__ void k_ff_particles(const double* __restrict__ sx, const double* __re
 }
 
 __global__ void k_ff_nodes(TreeDev t, bool fine, const double* __restrict__ center,
-                           const FastFrame* __restrict__ fr, float4* __restrict__ nh,
+                           FastFrame f, float4* __restrict__ nh,
                            float4* __restrict__ nl, float* __restrict__ nsize,
                            float* __restrict__ ndelta, const double* __restrict__ quad,
                            float4* __restrict__ nq0, float2* __restrict__ nq1,
                            int4* __restrict__ nhdr, const float4* __restrict__ ph)
 {
-    const FastFrame f = *fr;
     const int dim = t.dim;
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < t.m;
          k += (int64_t)gridDim.x * blockDim.x) {
@@ -161,10 +159,9 @@ __global__ void k_ff_nodes(TreeDev t, bool fine, const double* __restrict__ cent
 // th.w = 1 marks a target outside the box, tl.w = max |u|.
 __global__ void k_ff_targets(const double* __restrict__ tx, const double* __restrict__ ty,
                              const double* __restrict__ tz, int64_t nt, int dim, bool fine,
-                             const FastFrame* __restrict__ fr, float4* __restrict__ th,
+                             FastFrame f, float4* __restrict__ th,
                              float4* __restrict__ tl)
 {
-    const FastFrame f = *fr;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nt;
          i += (int64_t)gridDim.x * blockDim.x) {
         double u[3] = {__dmul_rn(__dsub_rn(tx[i], f.c[0]), f.s),
@@ -400,7 +397,7 @@ __device__ __forceinline__ void walk(const TreeDev& t, const FastTree& ft, const
 #pragma unroll
                     for (int k = 0; k < DIM; k++) {
                         float h, l;
-                        split_plain(__ddiv_rn(f[k], ft.frame->conv), h, l);
+                        split_plain(__ddiv_rn(f[k], ft.frame.conv), h, l);
                         ff_add(ah[k], al[k], h, l);
                     }
                     cnt[4]++;
@@ -458,7 +455,7 @@ k_traverse_fast(TreeDev t, FastTree ft, FastArgs a, int levels, double* __restri
     __shared__ double sum[SPLIT ? kFastWarps : 1][SPLIT ? DIM : 1][kWarp];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned FULL = 0xffffffffu;
-    const FastFrame fr = *ft.frame;
+    const FastFrame& fr = ft.frame;
     const double conv = __dmul_rn(fr.conv, a.G);
     const int shares = SPLIT ? (1 << levels) / kFastWarps : 1;   // blocks per group
     const int64_t step = SPLIT ? gridDim.x / shares : (int64_t)gridDim.x * kFastWarps;
@@ -566,7 +563,7 @@ __device__ __forceinline__ void walk_f32(const TreeDev& t, const FastTree& ft, c
 {
     const unsigned FULL = 0xffffffffu;
     const bool soft = a.e2h >= 0x1p-126f;   // r^2 >= eps^2 is normal: no small-r test
-    const bool unit = ft.frame->unit != 0 && !outside;   // every particle mass exactly 1
+    const bool unit = ft.frame.unit != 0 && !outside;   // every particle mass exactly 1
     const float2 nT[3] = {both(-T[0]), both(-T[1]), both(-T[2])};
     const float2 nL[3] = {both(-Tl[0]), both(-Tl[1]), both(-Tl[2])};
     const OpenF32 opener(a.theta, a.mac);
@@ -648,7 +645,7 @@ k_traverse_fp32(TreeDev t, FastTree ft, FastArgs a)
     __shared__ LeafStage stage[kFastWarps];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned FULL = 0xffffffffu;
-    const double conv = __dmul_rn(ft.frame->conv, a.G);
+    const double conv = __dmul_rn(ft.frame.conv, a.G);
     for (int64_t base = ((int64_t)blockIdx.x * kFastWarps + w) * kWarp; base < a.nt;
          base += (int64_t)gridDim.x * kFastWarps * kWarp) {
         const int64_t i = base + lane;
@@ -690,24 +687,23 @@ k_traverse_fp32(TreeDev t, FastTree ft, FastArgs a)
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-int launch_fast_prepare(const double* box, int dim, bool fine, FastFrame* frame, const TreeDev& t,
+int launch_fast_prepare(const FastFrame& frame, bool fine, const TreeDev& t,
                         const double* center, float4* ph, float4* pl, float4* nh, float4* nl,
                         float* nsize, float* ndelta, const double* quad, float4* nq0,
                         float2* nq1, int4* nhdr, cudaStream_t s)
 {
-    k_frame<<<1, 32, 0, s>>>(box, dim, frame);
-    k_ff_particles<<<grid_for(t.n, 256), 256, 0, s>>>(t.sx, t.sy, t.sz, t.sm, t.n, dim, fine, frame,
+    k_ff_particles<<<grid_for(t.n, 256), 256, 0, s>>>(t.sx, t.sy, t.sz, t.sm, t.n, t.dim, fine, frame,
                                                       ph,
                                                       pl);
     k_ff_nodes<<<grid_for(t.m, 256), 256, 0, s>>>(t, fine, center, frame, nh, nl, nsize, ndelta, quad,
                                                   nq0, nq1, nhdr, ph);
     BHUT_CUDA(cudaGetLastError());
-    note_launches(3);
+    note_launches(2);
     return kOk;
 }
 
 int launch_fast_targets(const double* tx, const double* ty, const double* tz, int64_t nt, int dim,
-                        bool fine, const FastFrame* frame, float4* th, float4* tl, cudaStream_t s)
+                        bool fine, const FastFrame& frame, float4* th, float4* tl, cudaStream_t s)
 {
     k_ff_targets<<<grid_for(nt, 256), 256, 0, s>>>(tx, ty, tz, nt, dim, fine, frame, th, tl);
     BHUT_CUDA(cudaGetLastError());

@@ -70,7 +70,7 @@ struct FastFrame {
 
 // Float-float copies of the particles (Morton order) and nodes.
 struct FastTree {
-    const FastFrame* frame;
+    FastFrame frame;
     const float4* ph;   // (x, y, z, m) hi
     const float4* pl;   // (x, y, z, m) lo
     const float4* nh;   // (com, mass) hi per internal node, LeafBox::c per leaf
@@ -193,15 +193,17 @@ struct NodeOut {
 // Bounding box: box[0..2] = min, box[3..5] = max, box[6] = max |mass| (0
 // without masses), box[8..10] = RN(1 / (max - min)) per axis (1 for a zero
 // extent), box[11] = 1 if an axis has zero extent, box[12..14] = 1 if the
-// axis holds a NaN, box[15] = 1 if every mass equals mass[0] > 0 (finite).
+// axis holds a NaN, box[15] = 1 if every mass equals mass[0] > 0 (finite),
+// box[16] = 1 if a position or mass is not finite.
 // `partial` holds kBoxPartialDoubles doubles.
 constexpr unsigned kBoxMaxBlocks = 152u * 4u;
 constexpr int kBoxPartialDoubles = 8 * (int)kBoxMaxBlocks;
-constexpr int kBoxDoubles = 16;
+constexpr int kBoxDoubles = 17;
 int launch_bbox(const double* pos, const double* mass, int64_t n, int dim, double* partial,
                 unsigned* counter, double* box, unsigned* err, cudaStream_t s);
 // The same box while copying positions and masses to pos_copy / mass_copy
-// (either may be NULL); a non-finite value sets kErrNonFinite in *err.
+// (either may be NULL); a non-finite value sets kErrNonFinite in *err (may be
+// NULL).
 int launch_stage_bbox(const double* pos, const double* mass, int64_t n, int dim, double* pos_copy,
                       double* mass_copy, double* partial, unsigned* counter, double* box,
                       unsigned* err, cudaStream_t s);
@@ -231,12 +233,13 @@ int launch_traverse_exact(const TreeDev& t, const double* tx, const double* ty, 
                           double eps, double G, double* out, unsigned* err,
                           unsigned long long* stats, cudaStream_t s, int levels, double* partial);
 // `fine`: the lo parts of form "fast" (split_grid), else those of "fp32".
-int launch_fast_prepare(const double* box, int dim, bool fine, FastFrame* frame, const TreeDev& t,
+FastFrame frame_of_box(const double* box, int dim);   // box on the host
+int launch_fast_prepare(const FastFrame& frame, bool fine, const TreeDev& t,
                         const double* center, float4* ph, float4* pl, float4* nh, float4* nl,
                         float* nsize, float* ndelta, const double* quad, float4* nq0,
                         float2* nq1, int4* nhdr, cudaStream_t s);
 int launch_fast_targets(const double* tx, const double* ty, const double* tz, int64_t nt, int dim,
-                        bool fine, const FastFrame* frame, float4* th, float4* tl, cudaStream_t s);
+                        bool fine, const FastFrame& frame, float4* th, float4* tl, cudaStream_t s);
 int launch_traverse_fast(const TreeDev& t, const FastTree& ft, const float4* th, const float4* tl,
                          const double* tx, const double* ty, const double* tz,
                          const int32_t* self_id, const int32_t* out_idx, int64_t nt, double theta,
