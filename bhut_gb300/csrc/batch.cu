@@ -1179,9 +1179,9 @@ int enqueue_solve(bhut_batch* b, double theta, double eps, double G, double* out
     BHUT_TRY(launch_bottom_up(b->dev(), b->leaf_list.as<int32_t>(), b->ltot,
                               b->first_child.as<int32_t>(), b->start.as<int32_t>(),
                               b->count.as<int32_t>(), b->parent.as<int32_t>(),
-                              b->arrive.as<unsigned>(), o, false, nullptr, nullptr,
+                              b->arrive.as<unsigned>(), o, false,
                               b->frontier.as<int32_t>(), b->counter.as<unsigned>() + 2,
-                              b->err.as<unsigned>(), s));
+                              b->err.as<unsigned>(), true, s));
     if (b->refit_rule) {
         k_seg_roots_update<<<grid_for(ns, 128), 128, 0, s>>>(
             b->d_node_off.as<int64_t>(), b->center.as<double>(), b->half.as<double>(), dim, ns,
@@ -1196,7 +1196,7 @@ int enqueue_solve(bhut_batch* b, double theta, double eps, double G, double* out
                                     b->count.as<int32_t>(), b->parent.as<int32_t>(),
                                     b->arrive.as<unsigned>(), b->quad.as<double>(),
                                     b->frontier.as<int32_t>(), b->counter.as<unsigned>() + 2,
-                                    b->err.as<unsigned>(), s));
+                                    b->err.as<unsigned>(), true, s));
     const bool fine = b->form == BHUT_FORM_FAST;
     k_seg_ff_particles<<<grid_for(n, 256), 256, 0, s>>>(b->dev(), fine, b->sys_of.as<int32_t>(),
                                                         b->frames.as<FastFrame>(),

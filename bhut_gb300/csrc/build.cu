@@ -217,36 +217,10 @@ __global__ void k_morton(const double* __restrict__ pos, int64_t n,
                          const double* __restrict__ box, uint64_t* __restrict__ keys,
                          int32_t* __restrict__ idx)
 {
-    double pmin[3], ext[3], off[3], rcp[3];
-    for (int d = 0; d < dim; d++) {
-        pmin[d] = box[d];
-        double e = __dsub_rn(box[3 + d], box[d]);
-        ext[d] = e <= 0 ? 1.0 : e;
-        off[d] = e <= 0 ? 0.5 : 0.0;
-        rcp[d] = box[8 + d];   // RN(1 / extent), from the bounding-box kernel
-    }
-    const bool degenerate = box[11] != 0.0;
+    const MortonBox<dim> mb(box);
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
-        uint64_t key;
-        if (degenerate) {   // an axis of zero extent (uniform branch)
-            if (dim == 3) {
-                key = morton3(quantise(pos[3 * i], pmin[0], ext[0], off[0]),
-                              quantise(pos[3 * i + 1], pmin[1], ext[1], off[1]),
-                              quantise(pos[3 * i + 2], pmin[2], ext[2], off[2]));
-            } else {
-                key = morton2(quantise(pos[2 * i], pmin[0], ext[0], off[0]),
-                              quantise(pos[2 * i + 1], pmin[1], ext[1], off[1]));
-            }
-        } else if (dim == 3) {
-            key = morton3(quantise_rcp(pos[3 * i], pmin[0], ext[0], rcp[0]),
-                          quantise_rcp(pos[3 * i + 1], pmin[1], ext[1], rcp[1]),
-                          quantise_rcp(pos[3 * i + 2], pmin[2], ext[2], rcp[2]));
-        } else {
-            key = morton2(quantise_rcp(pos[2 * i], pmin[0], ext[0], rcp[0]),
-                          quantise_rcp(pos[2 * i + 1], pmin[1], ext[1], rcp[1]));
-        }
-        keys[i] = key;
+        keys[i] = mb.key(pos, i);
         if (idx) idx[i] = (int32_t)i;
     }
 }
@@ -384,135 +358,131 @@ __device__ double pairwise_sum(F load, int64_t n)
     return ret;
 }
 
-// One leaf: tight AABB (build only), pairwise mass, row-order weighted sum.
-// In refit mode positions come from the caller's original-order arrays via
-// perm (refit.py:133-149); in build mode from the sorted SoA.
-// DIM is a template parameter so that the per-axis accumulators stay in
-// registers (a runtime axis index would place them in local memory).
+// Four lanes work on a node: lane q < DIM on axis q, lane 3 on the mass (each
+// sum keeps the reference's order, so a node's chain of dependent FP64
+// additions cannot be shortened, but its axes run beside each other and a
+// level's divisions take one instruction instead of three).  `quad` is the
+// lanes' mask, `lead` the first of them.
+struct Quad {
+    unsigned mask;
+    int lead, q;
+    __device__ __forceinline__ Quad()
+        : mask(0xfu << (threadIdx.x & 28)), lead(threadIdx.x & 28), q(threadIdx.x & 3) {}
+    __device__ __forceinline__ double from(double v, int lane) const
+    {
+        return __shfl_sync(mask, v, lead + lane);
+    }
+};
+
+// The node's box on the quad's axes: bounds, centre, half-size, size.
 template <int DIM>
-__device__ void leaf_node(int32_t id, bool refit, const TreeDev& t,
-                          const double* __restrict__ opos, const double* __restrict__ omass,
+__device__ __forceinline__ void put_box(const Quad& w, int32_t id, uint64_t klo, uint64_t khi,
+                                        const NodeOut& o)
+{
+    double e = 0.0;
+    if (w.q < DIM) {
+        const double lo = __longlong_as_double((long long)ord_inv(klo));
+        const double hi = __longlong_as_double((long long)ord_inv(khi));
+        o.lo[3 * id + w.q] = lo;
+        o.hi[3 * id + w.q] = hi;
+        o.center[DIM * id + w.q] = __dmul_rn(__dadd_rn(lo, hi), 0.5);
+        e = __dsub_rn(hi, lo);
+    }
+    double ext = w.from(e, 0);   // extents order as integers (not negative)
+    for (int d = 1; d < DIM; d++) {
+        const double x = w.from(e, d);
+        if (__double_as_longlong(x) > __double_as_longlong(ext)) ext = x;
+    }
+    if (w.q == 0) {
+        const double half = __dmul_rn(ext, 0.5);
+        o.half[id] = half;
+        o.size[id] = __dmul_rn(2.0, half);
+    }
+}
+
+// Centre of mass (weighted sums acc per axis; the box centre without mass)
+// and mass of the node.
+template <int DIM>
+__device__ __forceinline__ void put_moments(const Quad& w, int32_t id, double acc, double total,
+                                            const NodeOut& o)
+{
+    double v = 0.0;
+    if (w.q < DIM) v = total > 0 ? __ddiv_rn(acc, total) : o.center[DIM * id + w.q];
+    else if (w.q == 3) v = total;
+    reinterpret_cast<double*>(&o.cm[id])[w.q] = v;
+}
+
+// One leaf: tight AABB (build only), pairwise mass, row-order weighted sum
+// (of the Morton-ordered copies, which a refit renews through the frozen
+// permutation, refit.py:133-149).
+template <int DIM>
+__device__ void leaf_node(const Quad& w, int32_t id, bool refit, const TreeDev& t,
                           const int32_t* __restrict__ start, const int32_t* __restrict__ count,
-                          NodeOut o)
+                          const NodeOut& o)
 {
     const int64_t s = start[id], c = count[id];
-    double total;
-    double acc[3] = {0.0, 0.0, 0.0};
-    if (!refit) {
+    double total = 0.0, acc = 0.0;
+    // AABB on order-preserving integer images (same values as FP64
+    // comparisons; the FP64 pipe is the scarce one); loads run ahead of the
+    // row-order sums
+    uint64_t klo = ~0ull, khi = 0ull;
+    if (w.q < DIM) {
+        const double* __restrict__ axis = w.q == 0 ? t.sx : (w.q == 1 ? t.sy : t.sz);
+#pragma unroll 4
+        for (int64_t i = s; i < s + c; i++) {
+            const double v = axis[i];
+            const uint64_t k = ord_key((uint64_t)__double_as_longlong(v));
+            klo = k < klo ? k : klo;
+            khi = k > khi ? k : khi;
+            acc = __dadd_rn(acc, __dmul_rn(t.sm[i], v));
+        }
+    } else if (w.q == 3) {
         auto ld = [&](int64_t i) { return t.sm[s + i]; };
         total = __dadd_rn(0.0, pairwise_sum(ld, c));
-        // AABB on order-preserving integer images (same values as FP64
-        // comparisons; the FP64 pipe is the scarce one); loads run ahead of
-        // the row-order sums
-        uint64_t klo[3] = {~0ull, ~0ull, ~0ull}, khi[3] = {0ull, 0ull, 0ull};
-        const double* axes[3] = {t.sx, t.sy, t.sz};
-#pragma unroll 4
-        for (int64_t i = 0; i < c; i++) {
-            const double mi = t.sm[s + i];
-            for (int d = 0; d < DIM; d++) {
-                const double v = axes[d][s + i];
-                const uint64_t k = ord_key((uint64_t)__double_as_longlong(v));
-                klo[d] = k < klo[d] ? k : klo[d];
-                khi[d] = k > khi[d] ? k : khi[d];
-                acc[d] = __dadd_rn(acc[d], __dmul_rn(mi, v));
-            }
-        }
-        double lo[3], hi[3];
-        for (int d = 0; d < DIM; d++) {
-            lo[d] = __longlong_as_double((long long)ord_inv(klo[d]));
-            hi[d] = __longlong_as_double((long long)ord_inv(khi[d]));
-        }
-        double ext = 0.0;
-        for (int d = 0; d < DIM; d++) {
-            o.lo[3 * id + d] = lo[d];
-            o.hi[3 * id + d] = hi[d];
-            o.center[DIM * id + d] = __dmul_rn(__dadd_rn(lo[d], hi[d]), 0.5);
-            double e = __dsub_rn(hi[d], lo[d]);
-            ext = (d == 0 || e > ext) ? e : ext;
-        }
-        o.half[id] = __dmul_rn(ext, 0.5);
-        o.size[id] = __dmul_rn(2.0, o.half[id]);
-    } else {
-        auto ld = [&](int64_t i) { return omass[t.perm[s + i]]; };
-        total = __dadd_rn(0.0, pairwise_sum(ld, c));
-#pragma unroll 4
-        for (int64_t i = 0; i < c; i++) {
-            int64_t p = t.perm[s + i];
-            double mi = omass[p];
-            for (int d = 0; d < DIM; d++)
-                acc[d] = __dadd_rn(acc[d], __dmul_rn(mi, opos[p * DIM + d]));
-        }
     }
-    NodeCM cm;
-    double com[3];
-    for (int d = 0; d < 3; d++) com[d] = 0.0;
-    if (total > 0) {
-        for (int d = 0; d < DIM; d++) com[d] = __ddiv_rn(acc[d], total);
-    } else {
-        for (int d = 0; d < DIM; d++) com[d] = o.center[DIM * id + d];
-    }
-    cm.x = com[0]; cm.y = com[1]; cm.z = com[2]; cm.w = total;
-    o.cm[id] = cm;
+    __syncwarp(w.mask);
+    total = w.from(total, 3);
+    if (!refit) put_box<DIM>(w, id, klo, khi, o);
+    put_moments<DIM>(w, id, acc, total, o);
 }
 
 // Internal node from its two children (build.py:276-292 in build mode,
-// refit.py:173-192 in refit mode).
-// Reads a node record written by another thread of this kernel (L2, not L1).
-__device__ __forceinline__ NodeCM load_cm_cg(const NodeCM* p)
-{
-    double2 u = __ldcg(reinterpret_cast<const double2*>(p));
-    double2 v = __ldcg(reinterpret_cast<const double2*>(p) + 1);
-    return NodeCM{u.x, u.y, v.x, v.y};
-}
-
+// refit.py:173-192 in refit mode), written by other threads (L2, not L1).
 template <int DIM>
-__device__ void internal_node(int32_t id, int32_t fc, bool refit, NodeOut o)
+__device__ void internal_node(const Quad& w, int32_t id, int32_t fc, bool refit, const NodeOut& o)
 {
-    NodeCM a = load_cm_cg(&o.cm[fc]);
-    NodeCM b = load_cm_cg(&o.cm[fc + 1]);
+    const double ca = __ldcg(reinterpret_cast<const double*>(&o.cm[fc]) + w.q);
+    const double cb = __ldcg(reinterpret_cast<const double*>(&o.cm[fc + 1]) + w.q);
+    const double ma = w.from(ca, 3), mb = w.from(cb, 3);
     if (!refit) {
-        double ext = 0.0;
-        for (int d = 0; d < DIM; d++) {
-            const uint64_t l0 = ord_key((uint64_t)__double_as_longlong(__ldcg(&o.lo[3 * fc + d])));
-            const uint64_t l1 = ord_key((uint64_t)__double_as_longlong(__ldcg(&o.lo[3 * (fc + 1) + d])));
-            const uint64_t h0 = ord_key((uint64_t)__double_as_longlong(__ldcg(&o.hi[3 * fc + d])));
-            const uint64_t h1 = ord_key((uint64_t)__double_as_longlong(__ldcg(&o.hi[3 * (fc + 1) + d])));
-            const double lo = __longlong_as_double((long long)ord_inv(l1 < l0 ? l1 : l0));
-            const double hi = __longlong_as_double((long long)ord_inv(h1 > h0 ? h1 : h0));
-            o.lo[3 * id + d] = lo;
-            o.hi[3 * id + d] = hi;
-            o.center[DIM * id + d] = __dmul_rn(__dadd_rn(lo, hi), 0.5);
-            double e = __dsub_rn(hi, lo);
-            ext = (d == 0 || e > ext) ? e : ext;
+        uint64_t klo = 0, khi = 0;
+        if (w.q < DIM) {
+            const uint64_t l0 = ord_key((uint64_t)__double_as_longlong(__ldcg(&o.lo[3 * fc + w.q])));
+            const uint64_t l1 = ord_key((uint64_t)__double_as_longlong(__ldcg(&o.lo[3 * (fc + 1) + w.q])));
+            const uint64_t h0 = ord_key((uint64_t)__double_as_longlong(__ldcg(&o.hi[3 * fc + w.q])));
+            const uint64_t h1 = ord_key((uint64_t)__double_as_longlong(__ldcg(&o.hi[3 * (fc + 1) + w.q])));
+            klo = l1 < l0 ? l1 : l0;
+            khi = h1 > h0 ? h1 : h0;
         }
-        o.half[id] = __dmul_rn(ext, 0.5);
-        o.size[id] = __dmul_rn(2.0, o.half[id]);
+        put_box<DIM>(w, id, klo, khi, o);
     }
-    double ma = a.w, mb = b.w;
-    double ca[3] = {a.x, a.y, a.z}, cb[3] = {b.x, b.y, b.z};
-    double total, w[3] = {0.0, 0.0, 0.0};
+    double total, acc = 0.0;
     if (!refit) {
-        total = __dadd_rn(0.0, __dadd_rn(__dadd_rn(-0.0, ma), mb));
-        for (int d = 0; d < DIM; d++)
-            w[d] = __dadd_rn(__dadd_rn(w[d], __dmul_rn(ma, ca[d])), __dmul_rn(mb, cb[d]));
+        total = __dadd_rn(0.0, __dadd_rn(ma, mb));
+        acc = __dadd_rn(__dadd_rn(acc, __dmul_rn(ma, ca)), __dmul_rn(mb, cb));
     } else {
         total = 0.0;
         if (ma > 0) {
             total = __dadd_rn(total, ma);
-            for (int d = 0; d < DIM; d++) w[d] = __dadd_rn(w[d], __dmul_rn(ma, ca[d]));
+            acc = __dadd_rn(acc, __dmul_rn(ma, ca));
         }
         if (mb > 0) {
             total = __dadd_rn(total, mb);
-            for (int d = 0; d < DIM; d++) w[d] = __dadd_rn(w[d], __dmul_rn(mb, cb[d]));
+            acc = __dadd_rn(acc, __dmul_rn(mb, cb));
         }
     }
-    double com[3] = {0.0, 0.0, 0.0};
-    if (total > 0) {
-        for (int d = 0; d < DIM; d++) com[d] = __ddiv_rn(w[d], total);
-    } else {
-        for (int d = 0; d < DIM; d++) com[d] = o.center[DIM * id + d];
-    }
-    o.cm[id] = NodeCM{com[0], com[1], com[2], total};
+    __syncwarp(w.mask);   // (o.center of this node, read below, is the lane's own)
+    put_moments<DIM>(w, id, acc, total, o);
 }
 
 // The leaf list is taken in groups of kBuThreads consecutive entries (one
@@ -555,23 +525,22 @@ __device__ __forceinline__ void hand_over(int32_t node, int32_t* frontier, unsig
     else atomicOr(err, kErrBadNode);
 }
 
-// Node operations of a bottom-up pass: the moments (build and refit modes)
-// or the quadrupoles.
+// Node operations of a bottom-up pass: the moments (build and refit modes;
+// four lanes to a node) or the quadrupoles (one).
 template <int DIM>
 struct MomentOps {
+    static constexpr int kLanes = 4;
     TreeDev t;
     NodeOut o;
     bool refit;
-    const double* opos;
-    const double* omass;
     const int32_t* start;
     const int32_t* count;
-    __device__ void leaf(int32_t id) const { leaf_node<DIM>(id, refit, t, opos, omass, start, count, o); }
-    __device__ void internal(int32_t p, int32_t fc) const { internal_node<DIM>(p, fc, refit, o); }
+    __device__ void leaf(int32_t id) const { leaf_node<DIM>(Quad(), id, refit, t, start, count, o); }
+    __device__ void internal(int32_t p, int32_t fc) const { internal_node<DIM>(Quad(), p, fc, refit, o); }
 };
 
 template <class Ops>
-__global__ void __launch_bounds__(kBuThreads)
+__global__ void __launch_bounds__(kBuThreads * Ops::kLanes)
 k_bottom_up(Ops ops, TreeDev t, const int32_t* __restrict__ leaf_list, int64_t entries,
             const int32_t* __restrict__ first_child, const int32_t* __restrict__ start,
             const int32_t* __restrict__ count, const int32_t* __restrict__ parent,
@@ -579,18 +548,19 @@ k_bottom_up(Ops ops, TreeDev t, const int32_t* __restrict__ leaf_list, int64_t e
             unsigned* __restrict__ err)
 {
     __shared__ int32_t s_node[kBuThreads];
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x / Ops::kLanes;          // entry, then pair
+    const bool lead = threadIdx.x % Ops::kLanes == 0;   // reports and lists for its lanes
     for (int64_t base = (int64_t)blockIdx.x * kBuThreads; base < entries;
          base += (int64_t)gridDim.x * kBuThreads) {
         const int64_t li = base + tid;
         int32_t id = li < entries ? leaf_list[li] : kHole;
         if (id != kHole && (id < 0 || id >= t.m || start[id] < 0 || count[id] < 1 ||
                             (int64_t)start[id] + count[id] > t.n)) {
-            atomicOr(err, kErrBadNode);
+            if (lead) atomicOr(err, kErrBadNode);
             id = kGone;
         }
         if (id >= 0) ops.leaf(id);
-        s_node[tid] = id;
+        if (lead) s_node[tid] = id;
         __syncthreads();
         for (int j = 0, slots = kBuThreads; j < kBuLevels; j++, slots >>= 1) {
             int32_t out = kHole;
@@ -602,27 +572,27 @@ k_bottom_up(Ops ops, TreeDev t, const int32_t* __restrict__ leaf_list, int64_t e
                     int32_t pa = -1, pb = -1;
                     if (a >= 0) {
                         pa = parent[a];
-                        if (bad_parent(t, first_child, pa)) { atomicOr(err, kErrBadNode); pa = -2; }
+                        if (bad_parent(t, first_child, pa)) { if (lead) atomicOr(err, kErrBadNode); pa = -2; }
                     }
                     if (b >= 0) {
                         pb = parent[b];
-                        if (bad_parent(t, first_child, pb)) { atomicOr(err, kErrBadNode); pb = -2; }
+                        if (bad_parent(t, first_child, pb)) { if (lead) atomicOr(err, kErrBadNode); pb = -2; }
                     }
                     if (pa >= 0 && pa == pb) {
                         ops.internal(pa, first_child[pa]);
                         out = pa;
                     } else {   // parents completed elsewhere (or roots: nothing to do)
-                        if (pa >= 0) hand_over(a, frontier, frontier_count, entries, err);
-                        if (pb >= 0) hand_over(b, frontier, frontier_count, entries, err);
+                        if (lead && pa >= 0) hand_over(a, frontier, frontier_count, entries, err);
+                        if (lead && pb >= 0) hand_over(b, frontier, frontier_count, entries, err);
                         out = kGone;
                     }
                 }
             }
             __syncthreads();
-            if (tid < slots / 2) s_node[tid] = out;
+            if (lead && tid < slots / 2) s_node[tid] = out;
             __syncthreads();
         }
-        if (tid == 0 && s_node[0] >= 0) {
+        if (threadIdx.x == 0 && s_node[0] >= 0) {
             const int32_t p = parent[s_node[0]];
             if (bad_parent(t, first_child, p)) atomicOr(err, kErrBadNode);
             else if (p >= 0) hand_over(s_node[0], frontier, frontier_count, entries, err);
@@ -660,16 +630,27 @@ k_bottom_up_top(Ops ops, TreeDev t, const int32_t* __restrict__ first_child,
         s_cnt[i] = 0;
     }
     __syncthreads();
-    for (unsigned f = threadIdx.x; f < nf; f += blockDim.x) {
+    // the lanes of a node climb together, the first of them at the counters
+    constexpr int L = Ops::kLanes;
+    const unsigned lanes = (L == 1 ? 1u : 0xfu) << (threadIdx.x & 31 & ~(L - 1));
+    const bool lead = threadIdx.x % L == 0;
+    for (unsigned f = threadIdx.x / L; f < nf; f += blockDim.x / L) {
         int32_t node = frontier[f];
         for (int step = 0;; step++) {
-            if (step >= kMaxClimb || node < 0 || node >= t.m) { atomicOr(err, kErrBadNode); break; }
+            if (step >= kMaxClimb || node < 0 || node >= t.m) {
+                if (lead) atomicOr(err, kErrBadNode);
+                break;
+            }
             const int32_t p = parent[node];
             if (p < 0) break;
-            if (bad_parent(t, first_child, p)) { atomicOr(err, kErrBadNode); break; }
+            if (bad_parent(t, first_child, p)) {
+                if (lead) atomicOr(err, kErrBadNode);
+                break;
+            }
             __threadfence_block();
-            unsigned prev;
-            if (shared_counters) {
+            __syncwarp(lanes);
+            unsigned prev = 0;
+            if (lead && shared_counters) {
                 // linear probing from a multiplicative hash; at most f - 1
                 // keys in 2f slots, so a free or matching slot is found
                 unsigned h = ((unsigned)p * 2654435761u) >> 20;   // 12 bits
@@ -679,11 +660,12 @@ k_bottom_up_top(Ops ops, TreeDev t, const int32_t* __restrict__ first_child,
                     if (k == -1 || k == p) break;
                     if (++probes >= kBuTopHash) break;
                 }
-                if (probes >= kBuTopHash) { atomicOr(err, kErrBadNode); break; }
-                prev = atomicAdd(&s_cnt[h], 1u);
-            } else {
+                if (probes >= kBuTopHash) atomicOr(err, kErrBadNode);
+                else prev = atomicAdd(&s_cnt[h], 1u);
+            } else if (lead) {
                 prev = atomicAdd_block(&arrive[p], 1u);
             }
+            if (L > 1) prev = __shfl_sync(lanes, prev, threadIdx.x & 31 & ~(L - 1));
             if (prev == 0) break;
             __threadfence_block();
             ops.internal(p, first_child[p]);
@@ -696,18 +678,22 @@ template <class Ops>
 int launch_climb(const Ops& ops, const TreeDev& t, const int32_t* leaf_list, int64_t entries,
                  const int32_t* first_child, const int32_t* start, const int32_t* count,
                  const int32_t* parent, unsigned* arrive, int32_t* frontier,
-                 unsigned* frontier_count, unsigned* err, cudaStream_t s)
+                 unsigned* frontier_count, unsigned* err, bool ordered, cudaStream_t s)
 {
-    BHUT_CUDA(cudaMemsetAsync(arrive, 0, sizeof(unsigned) * (size_t)t.m, s));
-    BHUT_CUDA(cudaMemsetAsync(frontier_count, 0, sizeof(unsigned), s));
+    const bool one = ordered && entries <= kBuThreads;   // no frontier: one group
+    if (!one) {
+        BHUT_CUDA(cudaMemsetAsync(arrive, 0, sizeof(unsigned) * (size_t)t.m, s));
+        BHUT_CUDA(cudaMemsetAsync(frontier_count, 0, sizeof(unsigned), s));
+    }
     const unsigned groups = (unsigned)((entries + kBuThreads - 1) / kBuThreads);
-    k_bottom_up<Ops><<<groups < 152u * 8u ? groups : 152u * 8u, kBuThreads, 0, s>>>(
+    k_bottom_up<Ops><<<groups < 152u * 8u ? groups : 152u * 8u, kBuThreads * Ops::kLanes, 0, s>>>(
         ops, t, leaf_list, entries, first_child, start, count, parent, frontier,
         frontier_count, err);
-    k_bottom_up_top<Ops><<<1, kBuTopThreads, 0, s>>>(ops, t, first_child, parent, arrive,
-                                                     frontier, frontier_count, entries, err);
+    if (!one)
+        k_bottom_up_top<Ops><<<1, kBuTopThreads, 0, s>>>(ops, t, first_child, parent, arrive,
+                                                         frontier, frontier_count, entries, err);
     BHUT_CUDA(cudaGetLastError());
-    note_launches(2);
+    note_launches(one ? 1 : 2);
     return kOk;
 }
 
@@ -729,6 +715,7 @@ __device__ __forceinline__ void quad_add(double* q, double m, double dx, double 
 }
 
 struct QuadOps {
+    static constexpr int kLanes = 1;
     TreeDev t;
     double* quad;
     const int32_t* start;
@@ -760,10 +747,10 @@ struct QuadOps {
 int launch_quadrupoles(const TreeDev& t, const int32_t* leaf_list, int64_t entries,
                        const int32_t* first_child, const int32_t* start, const int32_t* count,
                        const int32_t* parent, unsigned* arrive, double* quad, int32_t* frontier,
-                       unsigned* frontier_count, unsigned* err, cudaStream_t s)
+                       unsigned* frontier_count, unsigned* err, bool ordered, cudaStream_t s)
 {
     return launch_climb(QuadOps{t, quad, start, count}, t, leaf_list, entries, first_child,
-                        start, count, parent, arrive, frontier, frontier_count, err, s);
+                        start, count, parent, arrive, frontier, frontier_count, err, ordered, s);
 }
 
 // Refit-vs-rebuild test of refit.py:236-249: any particle with
@@ -873,16 +860,16 @@ int launch_topology(const TopoTables& tt, int32_t* first_child, int32_t* start, 
 int launch_bottom_up(const TreeDev& t, const int32_t* leaf_list, int64_t entries,
                      const int32_t* first_child, const int32_t* start, const int32_t* count,
                      const int32_t* parent, unsigned* arrive, NodeOut o, bool refit,
-                     const double* opos, const double* omass, int32_t* frontier,
-                     unsigned* frontier_count, unsigned* err, cudaStream_t s)
+                     int32_t* frontier, unsigned* frontier_count, unsigned* err, bool ordered,
+                     cudaStream_t s)
 {
     if (t.dim == 3)
-        return launch_climb(MomentOps<3>{t, o, refit, opos, omass, start, count}, t, leaf_list,
+        return launch_climb(MomentOps<3>{t, o, refit, start, count}, t, leaf_list,
                             entries, first_child, start, count, parent, arrive, frontier,
-                            frontier_count, err, s);
-    return launch_climb(MomentOps<2>{t, o, refit, opos, omass, start, count}, t, leaf_list,
+                            frontier_count, err, ordered, s);
+    return launch_climb(MomentOps<2>{t, o, refit, start, count}, t, leaf_list,
                         entries, first_child, start, count, parent, arrive, frontier,
-                        frontier_count, err, s);
+                        frontier_count, err, ordered, s);
 }
 
 int launch_outside_root(const double* pos, int64_t n, int dim, const double* center0,

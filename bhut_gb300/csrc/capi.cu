@@ -2,6 +2,7 @@
 // pointer staging, and the build / refit / traversal pipelines.
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -173,6 +174,7 @@ struct bhut_tree {
     {
         return reinterpret_cast<unsigned long long*>(err.as<char>() + kStatsOffset);
     }
+    bool imported() const { return tt.n < 0; }   // bhut_tree_import
     double* pin_box() const { return pin; }
     unsigned char* pin_status() const { return reinterpret_cast<unsigned char*>(pin + kBoxDoubles); }
 
@@ -236,23 +238,21 @@ int read_box(bhut_tree* t, const DevBuf& box, double* host)
 }
 
 // Morton keys + stable sort of `n` AoS points into keys/perm (perm is the
-// sort payload, original index).  Uses the handle's scratch.
-int sort_points(bhut_tree* t, const double* dpos, const double* dmass, int64_t n, DevBuf& keys,
-                DevBuf& perm, DevBuf& box)
+// sort payload, original index) and, with tx, their Morton-ordered copies.
+// Uses the handle's scratch.
+int sort_points(bhut_tree* t, const double* dpos, int64_t n, DevBuf& keys, DevBuf& perm,
+                DevBuf& box, double* tx, double* ty, double* tz)
 {
     cudaStream_t s = t->stream;
     BHUT_TRY(keys.ensure(sizeof(uint64_t) * n, s));
     BHUT_TRY(perm.ensure(sizeof(int32_t) * n, s));
     BHUT_TRY(box.ensure(sizeof(double) * kBoxDoubles, s));
     BHUT_TRY(t->box_partial.ensure(sizeof(double) * kBoxPartialDoubles, s));
-    BHUT_TRY(launch_bbox(dpos, dmass, n, t->dim, t->box_partial.as<double>(),
-                         t->counters.as<unsigned>(), box.as<double>(), t->err.as<unsigned>(), s));
-    BHUT_TRY(launch_morton(dpos, n, t->dim, box.as<double>(), keys.as<uint64_t>(),
-                           perm.as<int32_t>(), s));
     BHUT_TRY(t->sort_scratch.ensure(sort_scratch_bytes(n), s));
-    BHUT_TRY(radix_sort_pairs(keys.as<uint64_t>(), perm.as<int32_t>(), n, t->dim == 3 ? 63 : 42,
-                              t->sort_scratch.p, s));
-    return kOk;
+    BHUT_TRY(launch_bbox(dpos, nullptr, n, t->dim, t->box_partial.as<double>(),
+                         t->counters.as<unsigned>(), box.as<double>(), t->err.as<unsigned>(), s));
+    return launch_order(dpos, nullptr, n, t->dim, box.as<double>(), keys.as<uint64_t>(),
+                        perm.as<int32_t>(), tx, ty, tz, nullptr, t->sort_scratch.p, s);
 }
 
 // Kernels of one build after its buffers exist: Morton keys, radix sort,
@@ -262,19 +262,16 @@ int enqueue_build(bhut_tree* t, int64_t n)
 {
     cudaStream_t s = t->stream;
     const int dim = t->dim;
-    BHUT_TRY(launch_morton(t->pos.as<double>(), n, dim, t->box.as<double>(),
-                           t->keys.as<uint64_t>(), t->perm.as<int32_t>(), s));
-    BHUT_TRY(radix_sort_pairs(t->keys.as<uint64_t>(), t->perm.as<int32_t>(), n,
-                              dim == 3 ? 63 : 42, t->sort_scratch.p, s));
-    BHUT_TRY(launch_gather(t->pos.as<double>(), t->mass.as<double>(), t->perm.as<int32_t>(), n, dim,
-                           t->sx.as<double>(), t->sy.as<double>(), t->sz.as<double>(),
-                           t->sm.as<double>(), s));
+    BHUT_TRY(launch_order(t->pos.as<double>(), t->mass.as<double>(), n, dim, t->box.as<double>(),
+                          t->keys.as<uint64_t>(), t->perm.as<int32_t>(), t->sx.as<double>(),
+                          t->sy.as<double>(), t->sz.as<double>(), t->sm.as<double>(),
+                          t->sort_scratch.p, s));
     BHUT_TRY(launch_bottom_up(t->dev(), t->leaf_list.as<int32_t>(), t->tt.leaf_slots,
                               t->first_child.as<int32_t>(), t->start.as<int32_t>(),
                               t->count.as<int32_t>(), t->parent.as<int32_t>(),
-                              t->arrive.as<unsigned>(), t->nodes(), false, nullptr, nullptr,
+                              t->arrive.as<unsigned>(), t->nodes(), false,
                               t->frontier.as<int32_t>(), t->counters.as<unsigned>() + 6,
-                              t->err.as<unsigned>(), s));
+                              t->err.as<unsigned>(), true, s));
     return kOk;
 }
 
@@ -460,6 +457,21 @@ int load_particles(bhut_tree* t, const double* positions, const double* masses, 
     return kOk;
 }
 
+// k_outside_root from the bounding boxes alone: the root's centre and
+// half-size follow from the box of its build as in k_bottom_up, and
+// |x - centre|, rounded, is largest at an end of the new box.
+bool outside_root(const double* root, const double* box, int dim)
+{
+    double half = 0.0, most = 0.0;
+    for (int d = 0; d < dim; d++) half = std::max(half, root[3 + d] - root[d]);
+    half *= 0.5;
+    for (int d = 0; d < dim; d++) {
+        const double c = (root[d] + root[3 + d]) * 0.5;
+        most = std::max(most, std::max(std::fabs(box[d] - c), std::fabs(box[3 + d] - c)));
+    }
+    return most > 1.1 * half;
+}
+
 // Writes a device result either straight into a device out pointer or via a
 // device buffer and a copy to host memory.
 struct OutTarget {
@@ -513,7 +525,7 @@ int prepare_fast(bhut_tree* t)
                                     t->count.as<int32_t>(), t->parent.as<int32_t>(),
                                     t->arrive.as<unsigned>(), t->quad.as<double>(),
                                     t->frontier.as<int32_t>(), t->counters.as<unsigned>() + 6,
-                                    t->err.as<unsigned>(), s));
+                                    t->err.as<unsigned>(), !t->imported(), s));
     }
     BHUT_TRY(launch_fast_prepare(t->frame, fine, t->dev(),
                                  t->center.as<double>(), t->ph.as<float4>(), t->pl.as<float4>(),
@@ -749,13 +761,19 @@ int bhut_tree_refit(bhut_tree* t, const double* positions, const double* masses,
     }
     cudaStream_t s = t->stream;
     BHUT_TRY(load_particles(t, positions, masses, n));
-    unsigned* flag = t->counters.as<unsigned>() + 2;
-    BHUT_CUDA(cudaMemsetAsync(flag, 0, sizeof(unsigned), s));
-    BHUT_TRY(launch_outside_root(t->pos.as<double>(), n, t->dim, t->center.as<double>(),
-                                 t->half.as<double>(), flag, s));
-    unsigned outside = 0;
-    BHUT_CUDA(cudaMemcpyAsync(&outside, flag, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-    BHUT_CUDA(cudaStreamSynchronize(s));
+    bool outside = false;
+    if (!t->imported()) {
+        outside = outside_root(t->hbox, t->hbox_in, t->dim);
+    } else {   // the root's box is the caller's
+        unsigned* flag = t->counters.as<unsigned>() + 2;
+        BHUT_CUDA(cudaMemsetAsync(flag, 0, sizeof(unsigned), s));
+        BHUT_TRY(launch_outside_root(t->pos.as<double>(), n, t->dim, t->center.as<double>(),
+                                     t->half.as<double>(), flag, s));
+        unsigned found = 0;
+        BHUT_CUDA(cudaMemcpyAsync(&found, flag, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+        BHUT_CUDA(cudaStreamSynchronize(s));
+        outside = found != 0;
+    }
     if (outside) {
         if (rebuilt) *rebuilt = 1;
         t->built = false;
@@ -768,9 +786,10 @@ int bhut_tree_refit(bhut_tree* t, const double* positions, const double* masses,
     BHUT_TRY(launch_bottom_up(t->dev(), t->leaf_list.as<int32_t>(), t->tt.leaf_slots,
                               t->first_child.as<int32_t>(), t->start.as<int32_t>(),
                               t->count.as<int32_t>(), t->parent.as<int32_t>(),
-                              t->arrive.as<unsigned>(), t->nodes(), true, t->pos.as<double>(),
-                              t->mass.as<double>(), t->frontier.as<int32_t>(),
-                              t->counters.as<unsigned>() + 6, t->err.as<unsigned>(), s));
+                              t->arrive.as<unsigned>(), t->nodes(), true,
+                              t->frontier.as<int32_t>(),
+                              t->counters.as<unsigned>() + 6, t->err.as<unsigned>(),
+                              !t->imported(), s));
     t->ff_valid = false;
     return check_err_word(t, "refit");
 }
@@ -795,9 +814,10 @@ int bhut_tree_refit_only(bhut_tree* t, const double* positions, const double* ma
     BHUT_TRY(launch_bottom_up(t->dev(), t->leaf_list.as<int32_t>(), t->tt.leaf_slots,
                               t->first_child.as<int32_t>(), t->start.as<int32_t>(),
                               t->count.as<int32_t>(), t->parent.as<int32_t>(),
-                              t->arrive.as<unsigned>(), t->nodes(), true, t->pos.as<double>(),
-                              t->mass.as<double>(), t->frontier.as<int32_t>(),
-                              t->counters.as<unsigned>() + 6, t->err.as<unsigned>(), s));
+                              t->arrive.as<unsigned>(), t->nodes(), true,
+                              t->frontier.as<int32_t>(),
+                              t->counters.as<unsigned>() + 6, t->err.as<unsigned>(),
+                              !t->imported(), s));
     t->ff_valid = false;
     return check_err_word(t, "refit");
 }
@@ -867,10 +887,9 @@ int bhut_tree_accel_targets(bhut_tree* t, const double* targets, int64_t mt, dou
     BHUT_TRY(stage_in(t->tpos, targets, bytes, s));
     // Morton-order the targets (their own box) so each warp's 32 targets are
     // close together; results are scattered back to input order.
-    BHUT_TRY(sort_points(t, t->tpos.as<double>(), nullptr, mt, t->tkeys, t->tperm, t->tbox));
     for (DevBuf* b : {&t->tx, &t->ty, &t->tz}) BHUT_TRY(b->ensure(sizeof(double) * mt, s));
-    BHUT_TRY(launch_gather(t->tpos.as<double>(), nullptr, t->tperm.as<int32_t>(), mt, dim,
-                           t->tx.as<double>(), t->ty.as<double>(), t->tz.as<double>(), nullptr, s));
+    BHUT_TRY(sort_points(t, t->tpos.as<double>(), mt, t->tkeys, t->tperm, t->tbox,
+                         t->tx.as<double>(), t->ty.as<double>(), t->tz.as<double>()));
     int st = check_err_word(t, "targets");
     if (st != kOk) return st;
     OutTarget o;
@@ -994,7 +1013,8 @@ int bhut_morton_argsort(const double* positions, int64_t n, int dim, uint64_t* s
     bhut_tree* t = nullptr;
     BHUT_TRY(bhut_tree_create(dim, 1, stream, &t));
     int rc = stage_in(t->pos, positions, sizeof(double) * n * dim, t->stream);
-    if (rc == kOk) rc = sort_points(t, t->pos.as<double>(), nullptr, n, t->keys, t->perm, t->box);
+    if (rc == kOk) rc = sort_points(t, t->pos.as<double>(), n, t->keys, t->perm, t->box, nullptr,
+                                    nullptr, nullptr);
     int32_t* p32 = nullptr;
     if (rc == kOk && sorted_keys) {
         cudaError_t e = cudaMemcpyAsync(sorted_keys, t->keys.p, sizeof(uint64_t) * n,

@@ -27,7 +27,14 @@
 // dependencies are between launches.  Two launches per pass.
 #include <atomic>
 
-#include "common.cuh"
+#include "tree.cuh"
+
+// Points that one block orders (launch_order).  Whole rebuilds, us, by one
+// block / by passes: 1,000 points 126 / 177, 4,000 168 / 228, 8,000 237 / 248,
+// 12,000 282 / 246.
+#ifndef BHUT_ORDER_SMALL
+#define BHUT_ORDER_SMALL 8192
+#endif
 
 namespace bhut {
 
@@ -270,6 +277,187 @@ SortLayout carve(void* scratch, int64_t n)
 }
 
 }  // namespace
+
+// ---------------------------------------------------------------------------
+// Small inputs: Morton keys, stable sort and Morton-ordered copies by one block.
+//
+// Up to a few thousand points the passes above take as long as their launches
+// (two a pass, 18 with the keys and the gather).  One block holds the keys in
+// registers and ranks, scatters and reads them back through shared memory,
+// eight bits at a time as above; places past the last point carry the largest
+// key and stay behind all others.
+// ---------------------------------------------------------------------------
+namespace {
+
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallWarps = kSmallThreads / kWarp;
+
+template <int ITEMS>
+struct SmallSmem {
+    uint64_t keys[kSmallThreads * ITEMS];
+    uint16_t idx[kSmallThreads * ITEMS];
+    uint32_t counts[kSmallWarps][256];
+    uint32_t offset[256];
+    uint32_t sums[8];
+};
+
+template <int DIM, int ITEMS>
+__global__ void __launch_bounds__(kSmallThreads)
+k_order_small(const double* __restrict__ pos, const double* __restrict__ mass, int n,
+              const double* __restrict__ box, uint64_t* __restrict__ keys,
+              int32_t* __restrict__ perm, double* __restrict__ sx, double* __restrict__ sy,
+              double* __restrict__ sz, double* __restrict__ sm)
+{
+    static_assert(kSmallThreads * ITEMS <= 65536, "16-bit indices");
+    extern __shared__ __align__(16) unsigned char small_raw[];
+    SmallSmem<ITEMS>& S = *reinterpret_cast<SmallSmem<ITEMS>*>(small_raw);
+    const unsigned FULL = 0xffffffffu;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    const MortonBox<DIM> mb(box);
+    uint64_t k[ITEMS];
+    uint32_t id[ITEMS], rank[ITEMS];
+#pragma unroll
+    for (int i = 0; i < ITEMS; i++) {
+        const int p = (warp * ITEMS + i) * kWarp + lane;
+        k[i] = p < n ? mb.key(pos, p) : ~0ull;
+        id[i] = (uint32_t)p;
+    }
+    constexpr int kPasses = DIM == 3 ? 8 : 6;   // 63 and 42 key bits
+    for (int pass = 0; pass < kPasses; pass++) {
+        const int shift = 8 * pass;
+        for (int j = tid; j < kSmallWarps * 256; j += kSmallThreads) (&S.counts[0][0])[j] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ITEMS; i++) {
+            const unsigned d = (unsigned)(k[i] >> shift) & 0xffu;
+            unsigned peers = FULL;
+#pragma unroll
+            for (int b = 0; b < 8; b++) {
+                const bool bit = (d >> b) & 1u;
+                const unsigned bal = __ballot_sync(FULL, bit);
+                peers &= bit ? bal : ~bal;
+            }
+            const uint32_t before = S.counts[warp][d];
+            rank[i] = before + __popc(peers & below);
+            __syncwarp();
+            if ((peers & below) == 0) S.counts[warp][d] = before + __popc(peers);
+            __syncwarp();
+        }
+        __syncthreads();
+        // four threads per digit: prefix over the warps, eight warps each
+        const int digit = tid >> 2, part = tid & 3;
+        uint32_t c[8], run = 0;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            c[j] = run;
+            run += S.counts[8 * part + j][digit];
+        }
+        uint32_t x = run;
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, x, o);
+            if (part >= o) x += y;
+        }
+        const uint32_t first = x - run;
+#pragma unroll
+        for (int j = 0; j < 8; j++) S.counts[8 * part + j][digit] = first + c[j];
+        if (part == 3) S.offset[digit] = x;
+        __syncthreads();
+        uint32_t v = 0, inc = 0;
+        if (tid < 256) {   // exclusive scan over the digits
+            v = inc = S.offset[tid];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(FULL, inc, o);
+                if (lane >= o) inc += y;
+            }
+            if (lane == 31) S.sums[warp] = inc;
+        }
+        __syncthreads();
+        if (tid < 256) {
+            uint32_t base = 0;
+            for (int w = 0; w < warp; w++) base += S.sums[w];
+            S.offset[tid] = base + inc - v;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ITEMS; i++) {
+            const unsigned d = (unsigned)(k[i] >> shift) & 0xffu;
+            const uint32_t at = S.offset[d] + S.counts[warp][d] + rank[i];
+            S.keys[at] = k[i];
+            S.idx[at] = (uint16_t)id[i];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ITEMS; i++) {
+            const int p = (warp * ITEMS + i) * kWarp + lane;
+            k[i] = S.keys[p];
+            id[i] = S.idx[p];
+        }
+        // (the next pass writes keys only after its barriers)
+    }
+#pragma unroll
+    for (int i = 0; i < ITEMS; i++) {
+        const int p = (warp * ITEMS + i) * kWarp + lane;
+        if (p >= n) continue;
+        const int64_t q = id[i];
+        keys[p] = k[i];
+        perm[p] = (int32_t)q;
+        if (sx) {
+            sx[p] = pos[q * DIM];
+            sy[p] = pos[q * DIM + 1];
+            sz[p] = DIM == 3 ? pos[q * DIM + 2] : 0.0;
+            if (mass) sm[p] = mass[q];
+        }
+    }
+}
+
+template <int DIM, int ITEMS>
+int run_order_small(const double* pos, const double* mass, int n, const double* box,
+                    uint64_t* keys, int32_t* perm, double* sx, double* sy, double* sz, double* sm,
+                    cudaStream_t stream)
+{
+    static std::atomic<bool> smem_set[64];
+    int dev = 0;
+    BHUT_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !smem_set[dev].load(std::memory_order_acquire)) {
+        BHUT_CUDA(cudaFuncSetAttribute(k_order_small<DIM, ITEMS>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)sizeof(SmallSmem<ITEMS>)));
+        if (dev >= 0 && dev < 64) smem_set[dev].store(true, std::memory_order_release);
+    }
+    k_order_small<DIM, ITEMS><<<1, kSmallThreads, sizeof(SmallSmem<ITEMS>), stream>>>(
+        pos, mass, n, box, keys, perm, sx, sy, sz, sm);
+    BHUT_CUDA(cudaGetLastError());
+    note_launches(1);
+    return kOk;
+}
+
+template <int DIM>
+int order_small(const double* pos, const double* mass, int n, const double* box, uint64_t* keys,
+                int32_t* perm, double* sx, double* sy, double* sz, double* sm, cudaStream_t s)
+{
+    if (n <= 1024) return run_order_small<DIM, 1>(pos, mass, n, box, keys, perm, sx, sy, sz, sm, s);
+    if (n <= 2048) return run_order_small<DIM, 2>(pos, mass, n, box, keys, perm, sx, sy, sz, sm, s);
+    if (n <= 4096) return run_order_small<DIM, 4>(pos, mass, n, box, keys, perm, sx, sy, sz, sm, s);
+    return run_order_small<DIM, 8>(pos, mass, n, box, keys, perm, sx, sy, sz, sm, s);
+}
+
+}  // namespace
+
+int launch_order(const double* pos, const double* mass, int64_t n, int dim, const double* box,
+                 uint64_t* keys, int32_t* perm, double* sx, double* sy, double* sz, double* sm,
+                 void* scratch, cudaStream_t s)
+{
+    static_assert(BHUT_ORDER_SMALL <= kSmallThreads * 8, "the largest block");
+    if (n <= BHUT_ORDER_SMALL)
+        return dim == 3 ? order_small<3>(pos, mass, (int)n, box, keys, perm, sx, sy, sz, sm, s)
+                        : order_small<2>(pos, mass, (int)n, box, keys, perm, sx, sy, sz, sm, s);
+    BHUT_TRY(launch_morton(pos, n, dim, box, keys, perm, s));
+    BHUT_TRY(radix_sort_pairs(keys, perm, n, dim == 3 ? 63 : 42, scratch, s));
+    return sx ? launch_gather(pos, mass, perm, n, dim, sx, sy, sz, sm, s) : kOk;
+}
 
 int radix_sort_pairs(uint64_t* keys, int32_t* vals, int64_t n, int bits, void* scratch,
                      cudaStream_t stream)

@@ -179,6 +179,38 @@ static __device__ __forceinline__ uint64_t morton2(uint64_t cx, uint64_t cy)
     return expand2(cx) | (expand2(cy) << 1);
 }
 
+// Morton keys of points in a tree's box (the data of launch_bbox).
+template <int DIM>
+struct MortonBox {
+    double pmin[3], ext[3], off[3], rcp[3];
+    bool degenerate;
+    __device__ __forceinline__ explicit MortonBox(const double* __restrict__ box)
+    {
+#pragma unroll
+        for (int d = 0; d < DIM; d++) {
+            pmin[d] = box[d];
+            const double e = __dsub_rn(box[3 + d], box[d]);
+            ext[d] = e <= 0 ? 1.0 : e;
+            off[d] = e <= 0 ? 0.5 : 0.0;
+            rcp[d] = box[8 + d];   // RN(1 / extent), from the bounding-box kernel
+        }
+        degenerate = box[11] != 0.0;
+    }
+    __device__ __forceinline__ uint64_t key(const double* __restrict__ pos, int64_t i) const
+    {
+        uint64_t c[3] = {0, 0, 0};
+        if (degenerate) {   // an axis of zero extent (uniform branch)
+#pragma unroll
+            for (int d = 0; d < DIM; d++) c[d] = quantise(pos[DIM * i + d], pmin[d], ext[d], off[d]);
+        } else {
+#pragma unroll
+            for (int d = 0; d < DIM; d++)
+                c[d] = quantise_rcp(pos[DIM * i + d], pmin[d], ext[d], rcp[d]);
+        }
+        return DIM == 3 ? morton3(c[0], c[1], c[2]) : morton2(c[0], c[1]);
+    }
+};
+
 // Node arrays written by the bottom-up pass.
 struct NodeOut {
     NodeCM* cm;        // (com, mass)
@@ -209,23 +241,29 @@ int launch_stage_bbox(const double* pos, const double* mass, int64_t n, int dim,
                       unsigned* err, cudaStream_t s);
 int launch_morton(const double* pos, int64_t n, int dim, const double* box, uint64_t* keys,
                   int32_t* idx, cudaStream_t s);
+// Morton keys in ascending order, the stable permutation and (sx not NULL) the
+// Morton-ordered copies; the scratch sort_scratch_bytes(n) (sort.cu).
+int launch_order(const double* pos, const double* mass, int64_t n, int dim, const double* box,
+                 uint64_t* keys, int32_t* perm, double* sx, double* sy, double* sz, double* sm,
+                 void* scratch, cudaStream_t s);
 int launch_gather(const double* pos, const double* mass, const int32_t* perm, int64_t n, int dim,
                   double* sx, double* sy, double* sz, double* sm, cudaStream_t s);
 int launch_topology(const TopoTables& tt, int32_t* first_child, int32_t* start, int32_t* count,
                     int32_t* parent, int32_t* leaf_list, unsigned* err, cudaStream_t s);
-// Node boxes and moments from the leaves up (build, or refit with opos /
-// omass in input order); quadrupoles the same way.  The leaf list holds
+// Node boxes and moments from the leaves up (in a refit the moments only);
+// quadrupoles the same way.  `ordered`: the list is in slot order (k_topology),
+// not that of an imported tree.  The leaf list holds
 // `entries` leaves and holes (-1); `frontier` holds as many entries of
 // scratch, `frontier_count` one counter.
 int launch_bottom_up(const TreeDev& t, const int32_t* leaf_list, int64_t entries,
                      const int32_t* first_child, const int32_t* start, const int32_t* count,
                      const int32_t* parent, unsigned* arrive, NodeOut o, bool refit,
-                     const double* opos, const double* omass, int32_t* frontier,
-                     unsigned* frontier_count, unsigned* err, cudaStream_t s);
+                     int32_t* frontier, unsigned* frontier_count, unsigned* err, bool ordered,
+                     cudaStream_t s);
 int launch_quadrupoles(const TreeDev& t, const int32_t* leaf_list, int64_t entries,
                        const int32_t* first_child, const int32_t* start, const int32_t* count,
                        const int32_t* parent, unsigned* arrive, double* quad, int32_t* frontier,
-                       unsigned* frontier_count, unsigned* err, cudaStream_t s);
+                       unsigned* frontier_count, unsigned* err, bool ordered, cudaStream_t s);
 int launch_outside_root(const double* pos, int64_t n, int dim, const double* center0,
                         const double* half0, unsigned* flag, cudaStream_t s);
 int launch_traverse_exact(const TreeDev& t, const double* tx, const double* ty, const double* tz,
