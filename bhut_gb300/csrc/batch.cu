@@ -427,48 +427,12 @@ __global__ void k_seg_ff_particles(TreeDev t, bool fine, const int32_t* __restri
 
 __global__ void k_seg_ff_nodes(TreeDev t, bool fine, const int32_t* __restrict__ node_sys,
                                const FastFrame* __restrict__ frames,
-                               const double* __restrict__ center, float4* __restrict__ nh,
-                               float4* __restrict__ nl, float* __restrict__ nsize,
-                               float* __restrict__ ndelta, const double* __restrict__ quad,
-                               float4* __restrict__ nq0, float2* __restrict__ nq1,
-                               int4* __restrict__ nhdr, const float4* __restrict__ ph)
+                               const double* __restrict__ center, const double* __restrict__ quad,
+                               const float4* __restrict__ ph, NodeCopies o)
 {
-    const int dim = t.dim;
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < t.m;
-         k += (int64_t)gridDim.x * blockDim.x) {
-        const FastFrame& f = frames[node_sys[k]];
-        const NodeCM c = t.cm[k];
-        float4 h, l;
-        split_grid(__dmul_rn(__dsub_rn(c.x, f.c[0]), f.s), fine, h.x, l.x);
-        split_grid(__dmul_rn(__dsub_rn(c.y, f.c[1]), f.s), fine, h.y, l.y);
-        if (dim == 3) split_grid(__dmul_rn(__dsub_rn(c.z, f.c[2]), f.s), fine, h.z, l.z);
-        else h.z = l.z = 0.0f;
-        const int fc = t.first_child[k];
-        split_plain(__dmul_rn(c.w, f.ms), h.w, l.w);
-        if (fc < 0) leaf_box(ph, t.start[k], t.count[k], h, l);   // (LeafBox in a leaf's place)
-        nh[k] = h;
-        nl[k] = l;
-        nsize[k] = __double2float_rn(__dmul_rn(t.size[k], f.s));
-        double dd = 0.0;
-        for (int d = 0; d < dim; d++) {
-            const double cc = d == 0 ? c.x : (d == 1 ? c.y : c.z);
-            const double v = cc - center[k * dim + d];
-            dd += v * v;
-        }
-        ndelta[k] = __double2float_ru(sqrt(dd) * f.s);
-        // header: leaf (-1, start, count, flag); internal (first child, size,
-        // |com - centre| as float bits, flag)
-        nhdr[k] = fc < 0 ? make_int4(fc, t.start[k], t.count[k], c.w != 0.0)
-                         : make_int4(fc, __float_as_int(nsize[k]), __float_as_int(ndelta[k]),
-                                     node_flag(c, h));
-        if (quad) {   // mass x length^2: scale by ms s^2
-            const double qs = f.ms * f.s * f.s;
-            const double* q = quad + 6 * k;
-            nq0[k] = make_float4((float)(q[0] * qs), (float)(q[1] * qs), (float)(q[2] * qs),
-                                 (float)(q[3] * qs));
-            nq1[k] = make_float2((float)(q[4] * qs), (float)(q[5] * qs));
-        }
-    }
+         k += (int64_t)gridDim.x * blockDim.x)
+        put_node(t, k, frames[node_sys[k]], fine, center, quad, ph, o);
 }
 
 // ---------------------------------------------------------------------------
@@ -483,8 +447,7 @@ struct BatchDev {
     const float4* pl;
     const float4* nh;
     const float4* nl;
-    const float* nsize;
-    const float* ndelta;
+    const LeafBox* twig;
     const float4* nq0;            // quadrupoles (FP32 form); NULL: monopoles
     const float2* nq1;
     const int4* nhdr;             // (first_child, start, count, flag)
@@ -639,50 +602,141 @@ k_batch_traverse(BatchDev b, BatchArgs a)
             const int4 hd = b.nhdr[node];   // (first_child, start, count, flag)
             const float4 nhv = b.nh[node];
             const int fc = hd.x;
+            const bool staged = kStaged && (FP32 || soft);
+            LeafBox box;
+            // runs of particles to take, as in the single-tree walks: with
+            // FP32 rows a leaf, or a twig's right and left leaf; else one run
+            unsigned lmask = 0;
+            int s0 = hd.y, c0 = 0, s1 = 0, c1 = 0;
             if (!hd.w) {
             } else if (fc < 0) {
-                const int s0 = hd.y, c = hd.z;
-                LeafBox box;
+                lmask = mask;
+                c0 = hd.z;
                 if (kStaged && soft) {
                     box.c = nhv;
                     box.h = b.nl[node];
                 }
-                for (int bb = 0; bb < c; bb += kWarp) {
-                    const int jj = bb + lane;
-                    const int cn = min(kWarp, c - bb);
-                    const bool staged = kStaged && (FP32 || soft);
-                    int np = 0;
-                    if (FP32 && kStaged) {
-                        np = stage_f32(stage[kStaged ? w : 0], lane, b.ph, b.pl, s0 + bb, cn, false);
-                    } else if (jj < c) {
-                        const float4 h = b.ph[s0 + jj], l = b.pl[s0 + jj];
-                        if (staged) {
-                            stage[kStaged ? w : 0].put(lane, h, l);
-                        } else {
-                            sh[lane] = h;
-                            sl[lane] = l;
+            } else {
+                bool open = false;
+                float4 nlv = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (FP32) {   // hi coordinates only, as the single-tree walk
+                    float d2 = 0.0f;
+#pragma unroll
+                    for (int k = 0; k < DIM; k++) {
+                        const float d = __fsub_rn(comp(nhv, k), Th[k]);
+                        d2 = fmaf(d, d, d2);
+                    }
+                    open = opener(d2, __int_as_float(hd.y), __int_as_float(hd.z), act);
+                } else if (act) {
+                    nlv = b.nl[node];
+                    float d2 = 0.0f;
+#pragma unroll
+                    for (int k = 0; k < DIM; k++) {
+                        const float d = __fadd_rn(__fsub_rn(comp(nhv, k), Th[k]),
+                                                  __fsub_rn(comp(nlv, k), Tl[k]));
+                        d2 = fmaf(d, d, d2);
+                    }
+                    const float dist = d2 > 0.0f ? d2 * rsqrtf(d2) : 0.0f;
+                    const float size_f = __int_as_float(hd.y);
+                    const float td = theta_f * dist;
+                    const float band = theta_f * fmaf(kBandRel, dist, 2.0f * kBandAbs);
+                    if (size_f >= td + band) open = true;
+                    else if (size_f < td - band) open = false;
+                    else {
+                        open = open_exact64<DIM>(x, y, z, t.cm[node], t.size[node], a.theta);
+                        cnt[3]++;
+                    }
+                }
+                const unsigned omask = __ballot_sync(FULL, act && open);
+                if (act && !open && sub == 0) {
+                    if (FP32) {
+                        nlv = b.nl[node];
+                        if (b.nq0)
+                            node_quad_f32<DIM>(Th, Tl, nhv, nlv, b.nq0[node], b.nq1[node], e2h,
+                                               ah, al);
+                        else
+                            pair_f32<DIM>(Th, Tl, nhv, nlv, e2h, ah, al);
+                    } else if (soft && !(hd.w & kNodeOutside)) {
+                        pair_ff_soft<DIM, false>(Th, Tl, nhv, nlv, e2h, e2l, ah, al);
+                    } else if ((hd.w & kNodeOutside) || !pair_ff<DIM, false>(Th, Tl, nhv, nlv, e2h, e2l, ah, al)) {
+                        const NodeCM cm = t.cm[node];
+                        pair_fp64<DIM>(x, y, z, cm.x, cm.y, cm.z, cm.w, eps2, a64);
+                        cnt[4]++;
+                    }
+                    cnt[1]++;
+                }
+                if (staged && omask && (hd.w & kTwig)) {
+                    lmask = omask;
+                    if (FP32) {
+                        s1 = b.nhdr[fc].y;
+                        c1 = twig_left(hd.w);
+                        s0 = s1 + c1;
+                        c0 = twig_right(hd.w);
+                    } else {
+                        box = b.twig[node];
+                        s0 = __float_as_int(box.h.w);
+                        c0 = twig_left(hd.w) + twig_right(hd.w);
+                    }
+                    cnt[2] += act && open ? 2 : 0;
+                } else if (omask) {
+                    if (!st.push(fc, omask)) {
+                        overflow = true;
+                        break;
+                    }
+                    node = fc + 1;
+                    mask = omask;
+                    continue;
+                }
+            }
+            const bool lact = (lmask >> lane) & 1u;
+            if (kStaged && FP32) {
+                LeafStage& sg = stage[kStaged ? w : 0];
+                for (; c0 > 0; s0 += kWarp, c0 -= kWarp) {
+                    const int cn = min(kWarp, c0);
+                    stage_f32(sg, lane, b.ph, b.pl, s0, cn, s1, c1, false);
+                    __syncwarp();
+                    if (lact) {   // per run <= 32 terms in FP32, then one Kahan step
+                        for (int run = 0, first = 0; run < 2; run++) {
+                            const int at = run ? s1 : s0, k = run ? c1 : cn, np = rows_for(k);
+                            if (k == 0) break;
+                            cnt[0] += k - (i >= at && i < at + k);
+                            float part[3] = {0.f, 0.f, 0.f};
+                            if (soft && unit)
+                                rows_f32<DIM, false, true>(sg, first, np, nT, nL, e2h, part);
+                            else if (soft)
+                                rows_f32<DIM, false, false>(sg, first, np, nT, nL, e2h, part);
+                            else
+                                rows_f32<DIM, true, false>(sg, first, np, nT, nL, e2h, part);
+                            kahan_add_f32<DIM>(part, ah, al);
+                            first += np;
                         }
                     }
                     __syncwarp();
-                    if (act && sub == 0) cnt[0] += cn - (i >= s0 + bb && i < s0 + bb + cn);
-                    if (FP32 && kStaged) {   // <= 32 terms in FP32, then one Kahan step
-                        if (act) {
-                            const LeafStage& sg = stage[kStaged ? w : 0];
-                            float part[3] = {0.f, 0.f, 0.f};
-                            if (soft && unit) rows_f32<DIM, false, true>(sg, np, nT, nL, e2h, part);
-                            else if (soft) rows_f32<DIM, false, false>(sg, np, nT, nL, e2h, part);
-                            else rows_f32<DIM, true, false>(sg, np, nT, nL, e2h, part);
-                            kahan_add_f32<DIM>(part, ah, al);
+                }
+            } else if (c0) {
+                const int block = staged ? kStage : kWarp;
+                for (int bb = 0; bb < c0; bb += block) {
+                    const int cn = min(block, c0 - bb);
+                    for (int jj = lane; jj < cn; jj += kWarp) {
+                        const float4 h = b.ph[s0 + bb + jj], l = b.pl[s0 + bb + jj];
+                        if (staged) {
+                            stage[kStaged ? w : 0].put(jj, h, l);
+                        } else {
+                            sh[jj] = h;
+                            sl[jj] = l;
                         }
-                    } else if (staged) {   // as the single-tree walk
+                    }
+                    __syncwarp();
+                    if (lact && sub == 0) cnt[0] += cn - (i >= s0 + bb && i < s0 + bb + cn);
+                    if (staged) {   // as the single-tree walk
                         const LeafStage& sg = stage[kStaged ? w : 0];
                         if (unit)
-                            leaf_block_soft<DIM, true>(mask, lane, Th, Tl, sg, cn, box,
+                            leaf_block_soft<DIM, true>(lmask, lane, Th, Tl, sg, cn, box,
                                                        e2h, e2l, ah, al);
                         else
-                            leaf_block_soft<DIM, false>(mask, lane, Th, Tl, sg, cn, box,
+                            leaf_block_soft<DIM, false>(lmask, lane, Th, Tl, sg, cn, box,
                                                         e2h, e2l, ah, al);
-                    } else if (act) {
+                    } else if (lact) {
                         if (FP32) {   // <= 32 terms in FP32, then one Kahan step
                             float2 pxy = make_float2(0.f, 0.f);
                             float pz = 0.f;
@@ -728,71 +782,13 @@ k_batch_traverse(BatchDev b, BatchArgs a)
                     }
                     __syncwarp();
                 }
-                if (!FP32 && act) {
+                if (!FP32 && lact) {
 #pragma unroll
                     for (int k = 0; k < DIM; k++) {
                         const float hs = __fadd_rn(ah[k], al[k]);
                         al[k] = __fsub_rn(al[k], __fsub_rn(hs, ah[k]));
                         ah[k] = hs;
                     }
-                }
-            } else {
-                bool open = false;
-                float4 nlv = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (FP32) {   // hi coordinates only, as the single-tree walk
-                    float d2 = 0.0f;
-#pragma unroll
-                    for (int k = 0; k < DIM; k++) {
-                        const float d = __fsub_rn(comp(nhv, k), Th[k]);
-                        d2 = fmaf(d, d, d2);
-                    }
-                    open = opener(d2, __int_as_float(hd.y), __int_as_float(hd.z), act);
-                } else if (act) {
-                    nlv = b.nl[node];
-                    float d2 = 0.0f;
-#pragma unroll
-                    for (int k = 0; k < DIM; k++) {
-                        const float d = __fadd_rn(__fsub_rn(comp(nhv, k), Th[k]),
-                                                  __fsub_rn(comp(nlv, k), Tl[k]));
-                        d2 = fmaf(d, d, d2);
-                    }
-                    const float dist = d2 > 0.0f ? d2 * rsqrtf(d2) : 0.0f;
-                    const float size_f = __int_as_float(hd.y);
-                    const float td = theta_f * dist;
-                    const float band = theta_f * fmaf(kBandRel, dist, 2.0f * kBandAbs);
-                    if (size_f >= td + band) open = true;
-                    else if (size_f < td - band) open = false;
-                    else {
-                        open = open_exact64<DIM>(x, y, z, t.cm[node], t.size[node], a.theta);
-                        cnt[3]++;
-                    }
-                }
-                const unsigned omask = __ballot_sync(FULL, act && open);
-                if (act && !open && sub == 0) {
-                    if (FP32) {
-                        nlv = b.nl[node];
-                        if (b.nq0)
-                            node_quad_f32<DIM>(Th, Tl, nhv, nlv, b.nq0[node], b.nq1[node], e2h,
-                                               ah, al);
-                        else
-                            pair_f32<DIM>(Th, Tl, nhv, nlv, e2h, ah, al);
-                    } else if (soft && hd.w == 1) {
-                        pair_ff_soft<DIM, false>(Th, Tl, nhv, nlv, e2h, e2l, ah, al);
-                    } else if (hd.w == 2 || !pair_ff<DIM, false>(Th, Tl, nhv, nlv, e2h, e2l, ah, al)) {
-                        const NodeCM cm = t.cm[node];
-                        pair_fp64<DIM>(x, y, z, cm.x, cm.y, cm.z, cm.w, eps2, a64);
-                        cnt[4]++;
-                    }
-                    cnt[1]++;
-                }
-                if (omask) {
-                    if (!st.push(fc, omask)) {
-                        overflow = true;
-                        break;
-                    }
-                    node = fc + 1;
-                    mask = omask;
-                    continue;
                 }
             }
             if (st.empty()) break;
@@ -918,7 +914,7 @@ struct bhut_batch {
     bool layout_valid = false, built = false, topo_valid = false;
     BufB pos, mass, d_part_off, d_node_off, d_leaf_off, d_tasks, keys, perm, sys_of, key2,
         sx, sy, sz, sm, cm, size, center, half, lo, hi, first_child, start, count, parent,
-        leaf_list, arrive, sort_scratch, box, frames, ph, pl, nh, nl, nsize, ndelta, counter,
+        leaf_list, arrive, sort_scratch, box, frames, ph, pl, nh, nl, twig, counter,
         err, stats, out, keep, perm_in, quad, nq0, nq1, nhdr, roots, forced, frontier,
         node_sys, acc, d_chunks;
     int64_t nchunks = 0;
@@ -935,7 +931,7 @@ struct bhut_batch {
         for (BufB* x : {&pos, &mass, &d_part_off, &d_node_off, &d_leaf_off, &d_tasks, &keys, &perm,
                         &sys_of, &key2, &sx, &sy, &sz, &sm, &cm, &size, &center, &half, &lo, &hi,
                         &first_child, &start, &count, &parent, &leaf_list, &arrive,
-                        &sort_scratch, &box, &frames, &ph, &pl, &nh, &nl, &nsize, &ndelta,
+                        &sort_scratch, &box, &frames, &ph, &pl, &nh, &nl, &twig,
                         &counter, &err, &stats, &out, &keep, &perm_in, &quad, &nq0, &nq1, &nhdr,
                         &roots, &forced, &frontier, &node_sys, &acc, &d_chunks})
             x->release(stream);
@@ -1044,8 +1040,7 @@ int plan_layout(bhut_batch* b, const int64_t* offsets, int64_t nsys)
     BHUT_TRY(b->frontier.ensure(sizeof(int32_t) * b->ltot, s));
     BHUT_TRY(b->nh.ensure(sizeof(float4) * mtot, s));
     BHUT_TRY(b->nl.ensure(sizeof(float4) * mtot, s));
-    BHUT_TRY(b->nsize.ensure(sizeof(float) * mtot, s));
-    BHUT_TRY(b->ndelta.ensure(sizeof(float) * mtot, s));
+    BHUT_TRY(b->twig.ensure(sizeof(LeafBox) * (b->form == BHUT_FORM_FAST ? mtot : 1), s));
     BHUT_TRY(b->quad.ensure(sizeof(double) * 6 * mtot, s));
     BHUT_TRY(b->nq0.ensure(sizeof(float4) * mtot, s));
     BHUT_TRY(b->nq1.ensure(sizeof(float2) * mtot, s));
@@ -1201,11 +1196,12 @@ int enqueue_solve(bhut_batch* b, double theta, double eps, double G, double* out
     k_seg_ff_particles<<<grid_for(n, 256), 256, 0, s>>>(b->dev(), fine, b->sys_of.as<int32_t>(),
                                                         b->frames.as<FastFrame>(),
                                                         b->ph.as<float4>(), b->pl.as<float4>());
+    const NodeCopies copies{b->nh.as<float4>(), b->nl.as<float4>(),
+                            fine ? b->twig.as<LeafBox>() : nullptr, b->nq0.as<float4>(),
+                            b->nq1.as<float2>(), b->nhdr.as<int4>()};
     k_seg_ff_nodes<<<grid_for(b->mtot, 256), 256, 0, s>>>(
-        b->dev(), fine, b->node_sys.as<int32_t>(), b->frames.as<FastFrame>(), b->center.as<double>(),
-        b->nh.as<float4>(), b->nl.as<float4>(), b->nsize.as<float>(), b->ndelta.as<float>(),
-        quad ? b->quad.as<double>() : nullptr, b->nq0.as<float4>(), b->nq1.as<float2>(),
-        b->nhdr.as<int4>(), b->ph.as<float4>());
+        b->dev(), fine, b->node_sys.as<int32_t>(), b->frames.as<FastFrame>(),
+        b->center.as<double>(), quad ? b->quad.as<double>() : nullptr, b->ph.as<float4>(), copies);
     BHUT_CUDA(cudaGetLastError());
     note_launches(2);
     // traversal
@@ -1213,8 +1209,7 @@ int enqueue_solve(bhut_batch* b, double theta, double eps, double G, double* out
     BHUT_CUDA(cudaMemsetAsync(b->stats.p, 0, sizeof(unsigned long long) * 8, s));
     BatchDev bd{b->dev(), b->d_part_off.as<int64_t>(), b->d_node_off.as<int64_t>(),
                 b->frames.as<FastFrame>(), b->ph.as<float4>(), b->pl.as<float4>(),
-                b->nh.as<float4>(), b->nl.as<float4>(), b->nsize.as<float>(),
-                b->ndelta.as<float>(), quad ? b->nq0.as<float4>() : nullptr,
+                b->nh.as<float4>(), b->nl.as<float4>(), b->twig.as<LeafBox>(), quad ? b->nq0.as<float4>() : nullptr,
                 quad ? b->nq1.as<float2>() : nullptr, b->nhdr.as<int4>()};
     BatchArgs a{b->d_tasks.as<int2>(), (int)b->tasks.size(), b->counter.as<unsigned>(), theta,
                 eps, G, b->mac, out, b->err.as<unsigned>(), b->stats.as<unsigned long long>()};

@@ -155,7 +155,7 @@ struct bhut_tree {
     DevBuf tpos, tkeys, tperm, tx, ty, tz, tbox, out, split_partial;
     // float-float copies for the fast form
     FastFrame frame{};        // from hbox
-    DevBuf ph, pl, nh, nl, nsize, ndelta, th, tl, quad, nq0, nq1, nhdr;
+    DevBuf ph, pl, nh, nl, twig, th, tl, quad, nq0, nq1, nhdr;
     bool ff_valid = false;
     bool ff_quad = false;
     bool ff_fine = false;     // lo parts of form "fast"
@@ -167,7 +167,7 @@ struct bhut_tree {
         return {&pos, &mass, &keys, &perm, &sx, &sy, &sz, &sm, &cm, &size, &center, &half, &lo, &hi,
                 &first_child, &start, &count, &parent, &leaf_list, &arrive, &sort_scratch,
                 &box_partial, &box, &counters, &err, &tpos, &tkeys, &tperm, &tx, &ty, &tz, &tbox,
-                &out, &split_partial, &ph, &pl, &nh, &nl, &nsize, &ndelta, &th, &tl, &quad, &nq0,
+                &out, &split_partial, &ph, &pl, &nh, &nl, &twig, &th, &tl, &quad, &nq0,
                 &nq1, &nhdr, &pos_in, &mass_in, &box_in, &frontier};
     }
     unsigned long long* stats() const
@@ -512,8 +512,7 @@ int prepare_fast(bhut_tree* t)
     BHUT_TRY(t->pl.ensure(sizeof(float4) * t->n, s));
     BHUT_TRY(t->nh.ensure(sizeof(float4) * t->m, s));
     BHUT_TRY(t->nl.ensure(sizeof(float4) * t->m, s));
-    BHUT_TRY(t->nsize.ensure(sizeof(float) * t->m, s));
-    BHUT_TRY(t->ndelta.ensure(sizeof(float) * t->m, s));
+    if (fine) BHUT_TRY(t->twig.ensure(sizeof(LeafBox) * t->m, s));
     BHUT_TRY(t->nhdr.ensure(sizeof(int4) * t->m, s));
     const bool quad = t->multipole == BHUT_MULTIPOLE_QUAD && t->form == BHUT_FORM_FP32;
     if (quad) {
@@ -527,12 +526,11 @@ int prepare_fast(bhut_tree* t)
                                     t->frontier.as<int32_t>(), t->counters.as<unsigned>() + 6,
                                     t->err.as<unsigned>(), !t->imported(), s));
     }
-    BHUT_TRY(launch_fast_prepare(t->frame, fine, t->dev(),
-                                 t->center.as<double>(), t->ph.as<float4>(), t->pl.as<float4>(),
-                                 t->nh.as<float4>(), t->nl.as<float4>(), t->nsize.as<float>(),
-                                 t->ndelta.as<float>(), quad ? t->quad.as<double>() : nullptr,
-                                 t->nq0.as<float4>(), t->nq1.as<float2>(), t->nhdr.as<int4>(),
-                                 s));
+    const NodeCopies o{t->nh.as<float4>(), t->nl.as<float4>(), fine ? t->twig.as<LeafBox>() : nullptr,
+                       t->nq0.as<float4>(), t->nq1.as<float2>(), t->nhdr.as<int4>()};
+    BHUT_TRY(launch_fast_prepare(t->frame, fine, t->dev(), t->center.as<double>(),
+                                 quad ? t->quad.as<double>() : nullptr, t->ph.as<float4>(),
+                                 t->pl.as<float4>(), o, s));
     t->ff_quad = quad;
     t->ff_fine = fine;
     t->ff_valid = true;
@@ -542,8 +540,7 @@ int prepare_fast(bhut_tree* t)
 FastTree fast_tree(const bhut_tree* t)
 {
     return FastTree{t->frame, t->ph.as<float4>(), t->pl.as<float4>(),
-                    t->nh.as<float4>(), t->nl.as<float4>(), t->nsize.as<float>(),
-                    t->ndelta.as<float>(), t->ff_quad ? t->nq0.as<float4>() : nullptr,
+                    t->nh.as<float4>(), t->nl.as<float4>(), t->twig.as<LeafBox>(), t->ff_quad ? t->nq0.as<float4>() : nullptr,
                     t->ff_quad ? t->nq1.as<float2>() : nullptr, t->nhdr.as<int4>()};
 }
 

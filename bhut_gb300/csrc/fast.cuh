@@ -90,13 +90,13 @@ static __device__ __forceinline__ void split_grid(double u, bool fine, float& h,
     l = __double2float_rn(r);
 }
 
-// A node's header flag: 0 without mass (skipped), 1, or 2 when its centre of
+// A node's header flag: 0 without mass (skipped), 1, or 3 when its centre of
 // mass lies outside the box (masses of both signs): its coordinates are not
 // on the grid and its monopole is taken in FP64.
 static __device__ __forceinline__ int node_flag(const NodeCM& c, const float4& h)
 {
     const bool out = !(fabsf(h.x) <= 1.0f && fabsf(h.y) <= 1.0f && fabsf(h.z) <= 1.0f);
-    return c.w == 0.0 ? 0 : (out ? 2 : 1);
+    return c.w == 0.0 ? 0 : (out ? 3 : 1);
 }
 
 static __device__ __forceinline__ void split_plain(double u, float& h, float& l)
@@ -345,24 +345,27 @@ static __device__ __forceinline__ int nth_set_bit(unsigned m, int r)
 constexpr float kFarScale = 0.54433105395181735517;   // (2/3)^(3/2), float-float
 constexpr float kFarScaleLo = 0.54433105395181735517 - (double)kFarScale;
 
-//
 // Two sources go through each operation together (f32x2: FADD2 / FFMA2, the
 // same IEEE operations; a difference is an FFMA2 by -1): half the issue slots
 // and two independent chains per lane.
-constexpr float kFarRatio = 16.0f;
+// kFarRatio 16 / 32 / 64 / 256: 1M Plummer 137.0 / 134.8 / 133.6 / 132.4 ms;
+// error against FP64 sums in 2-D, 60k, 1.3e-12 / 1.3e-12 / 2.2e-12 / 6.9e-12
+// (FP64 monopoles and pair_ff_soft alone give 2.2e-12).
+constexpr float kFarRatio = 32.0f;
 struct FarLeaf {
     float s0;      // bias of r^2, at least max R
     float si, li;  // s0 + eps^2 as si + li
     float b[3];    // bias of the force sums
 };
 
-// One leaf block staged for a warp, two sources to a row: source 2p in the
-// even and 2p + 1 in the odd components.
+// Up to kStage sources staged for a warp, two to a row: source 2p in the even
+// and 2p + 1 in the odd components.
+constexpr int kStage = 2 * kWarp;
 struct LeafStage {
-    float4 a[kWarp / 2];   // (x hi, x hi', y hi, y hi')
-    float4 b[kWarp / 2];   // (x lo, x lo', y lo, y lo')
-    float4 c[kWarp / 2];   // (z hi, z hi', z lo, z lo')
-    float4 d[kWarp / 2];   // (m hi, m hi', m lo, m lo')
+    float4 a[kStage / 2];   // (x hi, x hi', y hi, y hi')
+    float4 b[kStage / 2];   // (x lo, x lo', y lo, y lo')
+    float4 c[kStage / 2];   // (z hi, z hi', z lo, z lo')
+    float4 d[kStage / 2];   // (m hi, m hi', m lo, m lo')
     __device__ __forceinline__ void put(int q, float4 h, float4 l)
     {
         const int p = q >> 1, o = q & 1;
@@ -380,14 +383,6 @@ struct LeafStage {
         h = odd ? make_float4(A.y, A.w, C.y, D.y) : make_float4(A.x, A.z, C.x, D.x);
         l = odd ? make_float4(B.y, B.w, C.w, D.w) : make_float4(B.x, B.z, C.z, D.z);
     }
-};
-
-// A leaf's bounding box (c, h: centre and half extents, with a margin of
-// 2^-21 for the lo parts of particles and targets and for rounding) and its
-// largest |mass| (negative when some mass is).
-struct LeafBox {
-    float4 c;   // w: mass
-    float4 h;
 };
 
 // For sums of at most np terms.  False: the leaf is not distant (max R over
@@ -601,7 +596,7 @@ __device__ __forceinline__ void split_target(const LaneSplit& sp, const float* T
     }
 }
 
-// One staged block of cn <= 32 leaf particles for the targets of the lanes in
+// One staged block of cn <= kStage leaf particles for the targets of the lanes in
 // `mask` (those that opened the leaf's parent), float-float soft path
 // (far_pairs when the leaf is distant for every working lane, else
 // pair_ff_soft).  Called by all 32 lanes.
@@ -664,6 +659,72 @@ static __device__ __forceinline__ void leaf_box(const float4* __restrict__ ph, i
     const float s = 1.0f + 0x1p-20f, o = 0x1p-21f;
     h = make_float4(fmaf(0.5f * (hi[0] - lo[0]), s, o), fmaf(0.5f * (hi[1] - lo[1]), s, o),
                     fmaf(0.5f * (hi[2] - lo[2]), s, o), 0.0f);
+}
+
+// Header of a node, one load per visit: leaf (-1, start, count, flag); internal
+// (first child, size, |com - box centre| as float bits, flag).  Flags: see
+// node_flag; kTwig and the counts at bits 8 and 16 for a twig, an internal
+// node whose children are leaves of neighbouring particles (at most 32 each,
+// with mass): a target that opens it takes both leaves, which need no visit of
+// their own.
+constexpr int kNodeMass = 1, kNodeOutside = 2, kTwig = 4;
+static __device__ __forceinline__ int twig_left(int w) { return (w >> 8) & 0xff; }
+static __device__ __forceinline__ int twig_right(int w) { return (w >> 16) & 0xff; }
+
+// What the traversals read of node k (FP32 copies in frame f), from the tree
+// and the particles' copies ph.
+static __device__ __forceinline__ void put_node(const TreeDev& t, int64_t k, const FastFrame& f,
+                                                bool fine, const double* __restrict__ center,
+                                                const double* __restrict__ quad,
+                                                const float4* __restrict__ ph, const NodeCopies& o)
+{
+    const NodeCM c = t.cm[k];
+    const int dim = t.dim, fc = t.first_child[k];
+    float4 h, l;
+    split_grid(__dmul_rn(__dsub_rn(c.x, f.c[0]), f.s), fine, h.x, l.x);
+    split_grid(__dmul_rn(__dsub_rn(c.y, f.c[1]), f.s), fine, h.y, l.y);
+    if (dim == 3) split_grid(__dmul_rn(__dsub_rn(c.z, f.c[2]), f.s), fine, h.z, l.z);
+    else h.z = l.z = 0.0f;
+    split_plain(__dmul_rn(c.w, f.ms), h.w, l.w);
+    int4 hd;
+    if (fc < 0) {
+        leaf_box(ph, t.start[k], t.count[k], h, l);   // (LeafBox in a leaf's place)
+        hd = make_int4(fc, t.start[k], t.count[k], c.w != 0.0 ? kNodeMass : 0);
+    } else {
+        // distance between the centre of mass and the AABB centre (offset MAC)
+        double dd = 0.0;
+        for (int d = 0; d < dim; d++) {
+            const double cc = d == 0 ? c.x : (d == 1 ? c.y : c.z);
+            const double v = cc - center[k * dim + d];
+            dd += v * v;
+        }
+        int flag = node_flag(c, h);
+        if (flag && t.first_child[fc] < 0 && t.first_child[fc + 1] < 0) {
+            const int s = t.start[fc], n0 = t.count[fc], n1 = t.count[fc + 1];
+            if (n0 >= 1 && n1 >= 1 && n0 <= kWarp && n1 <= kWarp && t.start[fc + 1] == s + n0 &&
+                t.cm[fc].w != 0.0 && t.cm[fc + 1].w != 0.0) {
+                flag |= kTwig | n0 << 8 | n1 << 16;
+                if (o.twig) {
+                    LeafBox b;
+                    leaf_box(ph, s, n0 + n1, b.c, b.h);
+                    b.h.w = __int_as_float(s);
+                    o.twig[k] = b;
+                }
+            }
+        }
+        hd = make_int4(fc, __float_as_int(__double2float_rn(__dmul_rn(t.size[k], f.s))),
+                       __float_as_int(__double2float_ru(sqrt(dd) * f.s)), flag);
+    }
+    o.nh[k] = h;
+    o.nl[k] = l;
+    o.nhdr[k] = hd;
+    if (quad) {   // mass x length^2: scale by ms s^2
+        const double qs = f.ms * f.s * f.s;
+        const double* q = quad + 6 * k;
+        o.nq0[k] = make_float4((float)(q[0] * qs), (float)(q[1] * qs), (float)(q[2] * qs),
+                               (float)(q[3] * qs));
+        o.nq1[k] = make_float2((float)(q[4] * qs), (float)(q[5] * qs));
+    }
 }
 
 // FP64 pair in physical units, G-less (the Numba loop arithmetic).
@@ -797,7 +858,7 @@ __device__ __forceinline__ void pair_f32_partial2(const TargetF32x2& t, float4 s
     if (DIM == 3) pz = fmaf(f, dz, pz);
 }
 
-// Rows 0 .. np - 1 of a staged leaf block (two sources to a row) for a target
+// Rows first .. first + np - 1 of a staged block (two sources to a row) for a target
 // with negated coordinates (nT, nL): displacements, r^2 and w = r^-3 of both
 // sources in f32x2 instructions, the forces added to the partial sum p one
 // source after the other.  Every operation and its order are those of
@@ -806,10 +867,10 @@ __device__ __forceinline__ void pair_f32_partial2(const TargetF32x2& t, float4 s
 // exactly.  np is a multiple of four; places past the last source hold
 // stand-ins that add exactly zero.
 template <int DIM, bool CHECK, bool UNIT>
-__device__ __forceinline__ void rows_f32(const LeafStage& st, int np, const float2* nT,
+__device__ __forceinline__ void rows_f32(const LeafStage& st, int first, int np, const float2* nT,
                                          const float2* nL, float e2, float* p)
 {
-    for (int r0 = 0; r0 < np; r0 += 4)
+    for (int r0 = first; r0 < first + np; r0 += 4)
 #pragma unroll
     for (int r = r0; r < r0 + 4; r++) {
         const float4 A = st.a[r], B = st.b[r];
@@ -841,23 +902,31 @@ __device__ __forceinline__ void rows_f32(const LeafStage& st, int np, const floa
     }
 }
 
-// Stages sources [first, first + cn) of a leaf, cn <= 32, for rows_f32 and
-// returns the rows.  Stand-ins: for targets in the box (|T| <= 1) far away, so
-// that r^2 is about 3e36 and r^-3 rounds to zero; when some target lies
-// outside, without mass (the masses must then be used), at a point off every
-// grid.
-static __device__ __forceinline__ int stage_f32(LeafStage& st, int lane, const float4* ph,
-                                                const float4* pl, int first, int cn, bool outside)
+
+// Rows that rows_f32 takes for c sources.
+static __device__ __forceinline__ int rows_for(int c) { return ((c + 7) >> 3) << 2; }
+
+// Stages two runs of at most 32 sources for rows_f32, the second (which may be
+// empty) in the rows after the first's.  Stand-ins fill the rows: for targets
+// in the box (|T| <= 1) far away, so that r^2 is about 3e36 and r^-3 rounds to
+// zero; when some target lies outside, without mass (the masses must then be
+// used), at a point off every grid.
+static __device__ __forceinline__ void stage_f32(LeafStage& st, int lane, const float4* ph,
+                                                 const float4* pl, int s0, int c0, int s1, int c1,
+                                                 bool outside)
 {
-    const int np = ((cn + 7) >> 3) << 2;
+    const int n0 = 2 * rows_for(c0), n = n0 + 2 * rows_for(c1);
     const float v = outside ? 3.14159265f : 1e18f;
-    float4 h = make_float4(v, v * 1.25f, v * 1.5f, 0.0f), l = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (lane < cn) {
-        h = ph[first + lane];
-        l = pl[first + lane];
+    for (int j = lane; j < n; j += kWarp) {
+        const int q = j < n0 ? j : j - n0;
+        float4 h = make_float4(v, v * 1.25f, v * 1.5f, 0.0f), l = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (q < (j < n0 ? c0 : c1)) {
+            const int at = (j < n0 ? s0 : s1) + q;
+            h = ph[at];
+            l = pl[at];
+        }
+        st.put(j, h, l);
     }
-    if (lane < 2 * np) st.put(lane, h, l);
-    return np;
 }
 
 template <int DIM>

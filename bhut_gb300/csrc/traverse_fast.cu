@@ -38,12 +38,20 @@ namespace bhut {
 constexpr int kFastWarps = 4;
 constexpr int kFastThreads = kFastWarps * kWarp;
 constexpr int kSplitMaxLevels = 10;
-// Tuning (overridable at build time): resident blocks per SM for the fast
-// form (5: 20 warps per SM, registers capped at 96; 4 / 5 / 6 blocks at 1M
-// Plummer 142.4 / 140.5 / 139.1 ms, at 200k 22.5 / 23.0 / 23.8 ms, without
-// softening at 200k 11.0 / 10.6 / 11.3 ms).
+// Tuning (overridable at build time): resident blocks per SM of the fast form
+// (4 / 5 / 6 cap the registers at 128 / 96 / 80).  Self solves with softening,
+// 5 / 6 / 7 blocks: 1M Plummer 134.6 / 131.1 / 135.6 ms, 200k 21.8 / 22.0 /
+// 23.4 ms, but 100k, about one wave, 9.8 / 9.9 / 10.3 and a 100k uniform cube
+// 4.31 / 4.67 / 4.95 ms: so 6 from a few waves on and 5 below.  Without
+// softening (the checks cost registers) 3 / 4 / 5 / 6: 250k 32.3 / 30.4 / 31.0
+// / 32.4 ms, 100k cube 5.2 / 5.0 / 4.6 / - ms.  Split, 4 / 5 / 6: 250k targets
+// of 1M 28.7 / 27.1 / 26.0 ms, 2-D 60k self 1.28 / 1.18 / 1.09; without
+// softening 30k cube 1.12 / 1.07 / 1.10.
 #ifndef BHUT_FAST_BLOCKS
 #define BHUT_FAST_BLOCKS 5
+#endif
+#ifndef BHUT_FAST_BLOCKS_MORE
+#define BHUT_FAST_BLOCKS_MORE 6
 #endif
 // Split traversals (split_levels): split while fewer warps than this walk
 // and their subtrees hold more nodes than that.  Swept on GB300:
@@ -73,12 +81,10 @@ constexpr int kSplitMaxLevels = 10;
 #ifndef BHUT_SPLIT_WARPS_EXACT
 #define BHUT_SPLIT_WARPS_EXACT 25000
 #endif
-constexpr int64_t kWaveWarps = 152 * 4 * 5;   // resident warps of the traversals
+constexpr int64_t kWaveWarps = 152 * kFastWarps * BHUT_FAST_BLOCKS;   // resident warps
 #ifndef BHUT_SPLIT_NODES
 #define BHUT_SPLIT_NODES 16
 #endif
-constexpr int kFastBlocksPerSM = BHUT_FAST_BLOCKS;
-
 // ---------------------------------------------------------------------------
 // frame (normalisation) derived from the tree's bounding box
 // ---------------------------------------------------------------------------
@@ -110,49 +116,12 @@ __global__ void k_ff_particles(const double* __restrict__ sx, const double* __re
 }
 
 __global__ void k_ff_nodes(TreeDev t, bool fine, const double* __restrict__ center,
-                           FastFrame f, float4* __restrict__ nh,
-                           float4* __restrict__ nl, float* __restrict__ nsize,
-                           float* __restrict__ ndelta, const double* __restrict__ quad,
-                           float4* __restrict__ nq0, float2* __restrict__ nq1,
-                           int4* __restrict__ nhdr, const float4* __restrict__ ph)
+                           const double* __restrict__ quad, FastFrame f,
+                           const float4* __restrict__ ph, NodeCopies o)
 {
-    const int dim = t.dim;
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < t.m;
-         k += (int64_t)gridDim.x * blockDim.x) {
-        NodeCM c = t.cm[k];
-
-        float4 h, l;
-        split_grid(__dmul_rn(__dsub_rn(c.x, f.c[0]), f.s), fine, h.x, l.x);
-        split_grid(__dmul_rn(__dsub_rn(c.y, f.c[1]), f.s), fine, h.y, l.y);
-        if (dim == 3) split_grid(__dmul_rn(__dsub_rn(c.z, f.c[2]), f.s), fine, h.z, l.z);
-        else h.z = l.z = 0.0f;
-        const int fc = t.first_child[k];
-        split_plain(__dmul_rn(c.w, f.ms), h.w, l.w);
-        if (fc < 0) leaf_box(ph, t.start[k], t.count[k], h, l);   // (LeafBox in a leaf's place)
-        nh[k] = h;
-        nl[k] = l;
-        nsize[k] = __double2float_rn(__dmul_rn(t.size[k], f.s));
-        // distance between the centre of mass and the AABB centre (offset MAC)
-        double dd = 0.0;
-        for (int d = 0; d < dim; d++) {
-            const double cc = d == 0 ? c.x : (d == 1 ? c.y : c.z);
-            const double v = cc - center[k * dim + d];
-            dd += v * v;
-        }
-        ndelta[k] = __double2float_ru(sqrt(dd) * f.s);
-        // header: leaf (-1, start, count, flag); internal (first child, size,
-        // |com - centre| as float bits, flag)
-        nhdr[k] = fc < 0 ? make_int4(fc, t.start[k], t.count[k], c.w != 0.0)
-                         : make_int4(fc, __float_as_int(nsize[k]), __float_as_int(ndelta[k]),
-                                     node_flag(c, h));
-        if (quad) {   // mass x length^2: scale by ms s^2
-            const double qs = f.ms * f.s * f.s;
-            const double* q = quad + 6 * k;
-            nq0[k] = make_float4((float)(q[0] * qs), (float)(q[1] * qs), (float)(q[2] * qs),
-                                 (float)(q[3] * qs));
-            nq1[k] = make_float2((float)(q[4] * qs), (float)(q[5] * qs));
-        }
-    }
+         k += (int64_t)gridDim.x * blockDim.x)
+        put_node(t, k, f, fine, center, quad, ph, o);
 }
 
 // Targets: grid split when inside the box (|u| <= 1), plain split otherwise;
@@ -227,7 +196,7 @@ __device__ __forceinline__ void leaf_block_check(unsigned mask, int lane, const 
         split_add<DIM>(sp, mine, ph, pl, ah, al);
         return;
     }
-    unsigned fb = 0;
+    unsigned long long fb = 0;
     if (sp.work) {
 #pragma unroll 1
         for (int p = sp.sub; 2 * p < cn; p += sp.f) {
@@ -237,7 +206,8 @@ __device__ __forceinline__ void leaf_block_check(unsigned mask, int lane, const 
                 if (q >= cn) break;
                 float4 h, l;
                 st.get(p, o, h, l);
-                fb |= (unsigned)!pair_ff<DIM, false, true>(T, L, h, l, a.e2h, a.e2l, ph, pl) << q;
+                fb |= (unsigned long long)!pair_ff<DIM, false, true>(T, L, h, l, a.e2h, a.e2l, ph,
+                                                                     pl) << q;
             }
         }
     }
@@ -248,7 +218,7 @@ __device__ __forceinline__ void leaf_block_check(unsigned mask, int lane, const 
         const int64_t i = base + sp.owner;
         const double X = a.tx[i], Y = a.ty[i], Z = DIM == 3 ? a.tz[i] : 0.0;
         while (fb) {
-            const int gi = first + __ffs(fb) - 1;
+            const int gi = first + __ffsll((long long)fb) - 1;
             fb &= fb - 1;
             pair_fp64<DIM>(X, Y, Z, t.sx[gi], t.sy[gi], DIM == 3 ? t.sz[gi] : 0.0, t.sm[gi],
                            eps2, p64);
@@ -273,6 +243,11 @@ __device__ __forceinline__ void leaf_block_check(unsigned mask, int lane, const 
 // (highest first) through the top `levels` levels and walks the subtree it
 // reaches.  A node of those levels is worked on (leaf, monopoles, counts) by
 // the warp whose remaining bits are zero.
+// A twig (put_node) that some lane opens is worked on like a leaf: its two
+// leaves, always visited by the same lanes, cost one visit, one staging and
+// one set of bounds instead of two (1M Plummer 142.7 ms without, 137.0 with,
+// 2-D 60k in leaves of 16 1.49 and 1.35).  A box of two leaves is distant less
+// often: the larger kFarRatio makes up for it.
 template <int DIM, bool FAR, bool CHECK, bool UNIT, bool SPLIT>
 __device__ __forceinline__ void walk(const TreeDev& t, const FastTree& ft, const FastArgs& a,
                                      int w, int lane, bool valid, int64_t base, int64_t me_sorted,
@@ -298,56 +273,13 @@ __device__ __forceinline__ void walk(const TreeDev& t, const FastTree& ft, const
         const int4 hd = ft.nhdr[node];   // (first_child, start, count, flag)
         const float4 nh = ft.nh[node], nl = ft.nl[node];
         const int fc = hd.x;
+        LeafBox box{nh, nl};
+        unsigned lmask = 0;               // lanes that take the particles [s, s + c)
+        int s = hd.y, c = 0;
         if (!hd.w) {                      // mass == 0 skip (bh.py:514)
         } else if (fc < 0) {
-            const int s = hd.y, c = own ? hd.z : 0;
-            LeafBox box{nh, nl};
-            if (UNIT) box.c.w = 1.0f;
-            for (int b = 0; b < c; b += kWarp) {
-                const int jj = b + lane;
-                if (jj < c) stage[w].put(lane, ft.ph[s + jj], ft.pl[s + jj]);
-                __syncwarp();
-                const int cn = min(kWarp, c - b);
-                if (act) {
-                    // The target itself (self mode: sorted index `me_sorted`)
-                    // sits at zero displacement and adds exactly zero, so it
-                    // is not skipped; it is only left out of the pair count
-                    // (bh.py:254).
-                    cnt[0] += cn - (me_sorted >= s + b && me_sorted < s + b + cn);
-                }
-                if (!FAR && !CHECK) {
-                    leaf_block_soft<DIM, UNIT>(mask, lane, Th, Tl, stage[w], cn, box, a.e2h, a.e2l,
-                                               ah, al);
-                } else if (!FAR) {
-                    leaf_block_check<DIM, UNIT>(mask, lane, Th, Tl, a, base, stage[w], cn, s + b, t,
-                                                box, eps2, ah, al, a64, cnt[4]);
-                } else if (act) {
-                    unsigned fb = 0;   // pairs left to FP64 (rare), taken after the loop
-#pragma unroll 1
-                    for (int q = 0; q < cn; q++) {
-                        float4 h, l;
-                        stage[w].get(q >> 1, q & 1, h, l);
-                        fb |= (unsigned)!pair_ff<DIM, FAR, CHECK>(Th, Tl, h, l, a.e2h, a.e2l, ah,
-                                                                  al) << q;
-                    }
-                    while (fb) {
-                        const int gi = s + b + __ffs(fb) - 1;
-                        fb &= fb - 1;
-                        pair_fp64<DIM>(a.tx[me], a.ty[me], DIM == 3 ? a.tz[me] : 0.0, t.sx[gi],
-                                       t.sy[gi], DIM == 3 ? t.sz[gi] : 0.0, t.sm[gi], eps2, a64);
-                        cnt[4]++;
-                    }
-                }
-                __syncwarp();
-            }
-            if (FAR && act) {   // renormalise once per leaf (ff_add did)
-#pragma unroll
-                for (int k = 0; k < DIM; k++) {
-                    float hsum = __fadd_rn(ah[k], al[k]);
-                    al[k] = __fsub_rn(al[k], __fsub_rn(hsum, ah[k]));
-                    ah[k] = hsum;
-                }
-            }
+            lmask = mask;
+            c = own ? hd.z : 0;
         } else {
             // The hi parts alone decide outside a band of 2^-14 of d^2 plus
             // 2^-28 (the lo parts move d by delta <= 2^-22, and 2 d delta <=
@@ -387,7 +319,7 @@ __device__ __forceinline__ void walk(const TreeDev& t, const FastTree& ft, const
             }
             const unsigned omask = __ballot_sync(FULL, act && open);
             if (act && !open && own) {
-                if (!FAR && !CHECK && hd.w == 1) {
+                if (!FAR && !CHECK && !(hd.w & kNodeOutside)) {
                     pair_ff_soft<DIM, false>(Th, Tl, nh, nl, a.e2h, a.e2l, ah, al);
                 } else if (!FAR && !CHECK) {   // (into the sums: the soft path has no a64)
                     const NodeCM cm = t.cm[node];
@@ -401,7 +333,8 @@ __device__ __forceinline__ void walk(const TreeDev& t, const FastTree& ft, const
                         ff_add(ah[k], al[k], h, l);
                     }
                     cnt[4]++;
-                } else if (hd.w == 2 || !pair_ff<DIM, FAR, CHECK>(Th, Tl, nh, nl, a.e2h, a.e2l, ah, al)) {
+                } else if ((hd.w & kNodeOutside) ||
+                           !pair_ff<DIM, FAR, CHECK>(Th, Tl, nh, nl, a.e2h, a.e2l, ah, al)) {
                     const NodeCM cm = t.cm[node];
                     pair_fp64<DIM>(a.tx[me], a.ty[me], DIM == 3 ? a.tz[me] : 0.0, cm.x, cm.y,
                                    cm.z, cm.w, eps2, a64);
@@ -416,13 +349,68 @@ __device__ __forceinline__ void walk(const TreeDev& t, const FastTree& ft, const
                 mask = omask;
                 continue;
             }
-            if (omask) {
+                        if (!FAR && omask && (hd.w & kTwig)) {   // both leaves here
+                box = ft.twig[node];
+                lmask = omask;
+                s = __float_as_int(box.h.w);
+                c = twig_left(hd.w) + twig_right(hd.w);
+                cnt[2] += open ? 2 : 0;
+            } else if (omask) {
                 if (sp + 2 > kStackDepth) { overflow = true; break; }
                 if (lane == 0) stack[w][sp] = make_int2(fc, (int)omask);
                 sp++;
                 node = fc + 1;
                 mask = omask;
                 continue;
+            }
+        }
+        if (c) {
+            const bool lact = (lmask >> lane) & 1u;
+            if (UNIT) box.c.w = 1.0f;
+            for (int b = 0; b < c; b += kStage) {
+                const int cn = min(kStage, c - b);
+                for (int j = lane; j < cn; j += kWarp)
+                    stage[w].put(j, ft.ph[s + b + j], ft.pl[s + b + j]);
+                __syncwarp();
+                if (lact) {
+                    // The target itself (self mode: sorted index `me_sorted`)
+                    // sits at zero displacement and adds exactly zero, so it
+                    // is not skipped; it is only left out of the pair count
+                    // (bh.py:254).
+                    cnt[0] += cn - (me_sorted >= s + b && me_sorted < s + b + cn);
+                }
+                if (!FAR && !CHECK) {
+                    leaf_block_soft<DIM, UNIT>(lmask, lane, Th, Tl, stage[w], cn, box, a.e2h, a.e2l,
+                                               ah, al);
+                } else if (!FAR) {
+                    leaf_block_check<DIM, UNIT>(lmask, lane, Th, Tl, a, base, stage[w], cn, s + b, t,
+                                                box, eps2, ah, al, a64, cnt[4]);
+                } else if (lact) {
+                    unsigned long long fb = 0;   // pairs left to FP64 (rare), taken after the loop
+#pragma unroll 1
+                    for (int q = 0; q < cn; q++) {
+                        float4 h, l;
+                        stage[w].get(q >> 1, q & 1, h, l);
+                        fb |= (unsigned long long)!pair_ff<DIM, FAR, CHECK>(Th, Tl, h, l, a.e2h, a.e2l,
+                                                                            ah, al) << q;
+                    }
+                    while (fb) {
+                        const int gi = s + b + __ffsll((long long)fb) - 1;
+                        fb &= fb - 1;
+                        pair_fp64<DIM>(a.tx[me], a.ty[me], DIM == 3 ? a.tz[me] : 0.0, t.sx[gi],
+                                       t.sy[gi], DIM == 3 ? t.sz[gi] : 0.0, t.sm[gi], eps2, a64);
+                        cnt[4]++;
+                    }
+                }
+                __syncwarp();
+            }
+            if (FAR && lact) {   // renormalise once per leaf (ff_add did)
+#pragma unroll
+                for (int k = 0; k < DIM; k++) {
+                    float hsum = __fadd_rn(ah[k], al[k]);
+                    al[k] = __fsub_rn(al[k], __fsub_rn(hsum, ah[k]));
+                    ah[k] = hsum;
+                }
             }
         }
         if (sp == 0) break;
@@ -446,8 +434,8 @@ __device__ __forceinline__ void walk(const TreeDev& t, const FastTree& ft, const
 // group's warps in different blocks, lose the nodes that they share in L1.
 // A block adds its four sums in FP64; with more than four warps per group the blocks' sums go to `partial`
 // and k_split_sum adds them (fixed order, no atomics).
-template <int DIM, bool SOFT, bool SPLIT>
-__global__ void __launch_bounds__(kFastThreads, kFastBlocksPerSM)
+template <int DIM, bool SOFT, bool SPLIT, int BLOCKS>
+__global__ void __launch_bounds__(kFastThreads, BLOCKS)
 k_traverse_fast(TreeDev t, FastTree ft, FastArgs a, int levels, double* __restrict__ partial)
 {
     __shared__ int2 stack[kFastWarps][kStackDepth];
@@ -576,26 +564,14 @@ __device__ __forceinline__ void walk_f32(const TreeDev& t, const FastTree& ft, c
         const int4 hd = ft.nhdr[node];   // (first_child, start, count, flag)
         const float4 nh = ft.nh[node];
         const int fc = hd.x;
+        // runs of particles to take: a leaf's blocks of 32, or a twig's right
+        // and left leaf (the order in which the leaves would be visited)
+        unsigned lmask = 0;
+        int s0 = hd.y, c0 = 0, s1 = 0, c1 = 0;
         if (!hd.w) {
         } else if (fc < 0) {
-            const int s = hd.y, c = hd.z;
-            for (int b = 0; b < c; b += kWarp) {
-                const int cn = min(kWarp, c - b);
-                const int np = stage_f32(stage[w], lane, ft.ph, ft.pl, s + b, cn, outside);
-                __syncwarp();
-                if (act) {
-                    cnt[0] += cn - (me_sorted >= s + b && me_sorted < s + b + cn);
-                    float part[3] = {0.f, 0.f, 0.f};   // <= 32 terms, then one Kahan step
-                    if (soft && unit)
-                        rows_f32<DIM, false, true>(stage[w], np, nT, nL, a.e2h, part);
-                    else if (soft)
-                        rows_f32<DIM, false, false>(stage[w], np, nT, nL, a.e2h, part);
-                    else
-                        rows_f32<DIM, true, false>(stage[w], np, nT, nL, a.e2h, part);
-                    kahan_add_f32<DIM>(part, acc, cmp);
-                }
-                __syncwarp();
-            }
+            lmask = mask;
+            c0 = hd.z;
         } else {
             float d2 = 0.0f;
 #pragma unroll
@@ -613,7 +589,14 @@ __device__ __forceinline__ void walk_f32(const TreeDev& t, const FastTree& ft, c
                     pair_f32<DIM>(T, Tl, nh, ft.nl[node], a.e2h, acc, cmp);
                 cnt[1]++;
             }
-            if (omask) {
+            if (omask && (hd.w & kTwig)) {
+                lmask = omask;
+                s1 = ft.nhdr[fc].y;
+                c1 = twig_left(hd.w);
+                s0 = s1 + c1;
+                c0 = twig_right(hd.w);
+                cnt[2] += act && open ? 2 : 0;
+            } else if (omask) {
                 if (sp + 2 > kStackDepth) { overflow = true; break; }
                 if (lane == 0) stack[w][sp] = make_int2(fc, (int)omask);
                 sp++;
@@ -621,6 +604,29 @@ __device__ __forceinline__ void walk_f32(const TreeDev& t, const FastTree& ft, c
                 mask = omask;
                 continue;
             }
+        }
+        for (; c0 > 0; s0 += kWarp, c0 -= kWarp) {
+            const int cn = min(kWarp, c0);
+            stage_f32(stage[w], lane, ft.ph, ft.pl, s0, cn, s1, c1, outside);
+            __syncwarp();
+            if ((lmask >> lane) & 1u) {
+                // per run <= 32 terms, then one Kahan step
+                for (int run = 0, first = 0; run < 2; run++) {
+                    const int at = run ? s1 : s0, k = run ? c1 : cn, np = rows_for(k);
+                    if (k == 0) break;
+                    cnt[0] += k - (me_sorted >= at && me_sorted < at + k);
+                    float part[3] = {0.f, 0.f, 0.f};
+                    if (soft && unit)
+                        rows_f32<DIM, false, true>(stage[w], first, np, nT, nL, a.e2h, part);
+                    else if (soft)
+                        rows_f32<DIM, false, false>(stage[w], first, np, nT, nL, a.e2h, part);
+                    else
+                        rows_f32<DIM, true, false>(stage[w], first, np, nT, nL, a.e2h, part);
+                    kahan_add_f32<DIM>(part, acc, cmp);
+                    first += np;
+                }
+            }
+            __syncwarp();
         }
         if (sp == 0) break;
         __syncwarp();
@@ -631,11 +637,12 @@ __device__ __forceinline__ void walk_f32(const TreeDev& t, const FastTree& ft, c
     }
 }
 
-// Resident blocks per SM: the walk waits for loads (7 / 8 / 9 / 10 blocks at
-// 2M galaxy, theta 0.7, leaf 16: 116.9 / 111.3 / 110.0 / 110.3 ms; at 8 to 10
-// the kernel issues on about 78 % of the clocks).
+// Resident blocks per SM: the walk waits for loads (8 / 9 / 10 / 11 blocks at
+// 2M galaxy, theta 0.7, leaf 16: 109.9 / 111.1 / 106.5 / 111.7 ms; the kernel
+// issues on about 78 % of the clocks).  Twigs taken in one visit: 108.9 ms
+// without, 106.5 with.
 #ifndef BHUT_F32_BLOCKS
-#define BHUT_F32_BLOCKS 9
+#define BHUT_F32_BLOCKS 10
 #endif
 template <int DIM>
 __global__ void __launch_bounds__(kFastThreads, BHUT_F32_BLOCKS)
@@ -687,16 +694,13 @@ k_traverse_fp32(TreeDev t, FastTree ft, FastArgs a)
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-int launch_fast_prepare(const FastFrame& frame, bool fine, const TreeDev& t,
-                        const double* center, float4* ph, float4* pl, float4* nh, float4* nl,
-                        float* nsize, float* ndelta, const double* quad, float4* nq0,
-                        float2* nq1, int4* nhdr, cudaStream_t s)
+int launch_fast_prepare(const FastFrame& frame, bool fine, const TreeDev& t, const double* center,
+                        const double* quad, float4* ph, float4* pl, const NodeCopies& o,
+                        cudaStream_t s)
 {
-    k_ff_particles<<<grid_for(t.n, 256), 256, 0, s>>>(t.sx, t.sy, t.sz, t.sm, t.n, t.dim, fine, frame,
-                                                      ph,
-                                                      pl);
-    k_ff_nodes<<<grid_for(t.m, 256), 256, 0, s>>>(t, fine, center, frame, nh, nl, nsize, ndelta, quad,
-                                                  nq0, nq1, nhdr, ph);
+    k_ff_particles<<<grid_for(t.n, 256), 256, 0, s>>>(t.sx, t.sy, t.sz, t.sm, t.n, t.dim, fine,
+                                                      frame, ph, pl);
+    k_ff_nodes<<<grid_for(t.m, 256), 256, 0, s>>>(t, fine, center, quad, frame, ph, o);
     BHUT_CUDA(cudaGetLastError());
     note_launches(2);
     return kOk;
@@ -762,24 +766,23 @@ int launch_traverse_fast(const TreeDev& t, const FastTree& ft, const float4* th,
         else k_traverse_fp32<2><<<grid, kFastThreads, 0, s>>>(t, ft, a);
     } else {
         const bool soft = a.e2h >= 2.0f * kTinyR;
-        if (levels > 0) {
-            const int shares = (1 << levels) / kFastWarps;
-            const unsigned g = (unsigned)warps * (unsigned)shares;
-            if (t.dim == 3) {
-                if (soft) k_traverse_fast<3, true, true><<<g, kFastThreads, 0, s>>>(t, ft, a, levels, partial);
-                else k_traverse_fast<3, false, true><<<g, kFastThreads, 0, s>>>(t, ft, a, levels, partial);
-            } else {
-                if (soft) k_traverse_fast<2, true, true><<<g, kFastThreads, 0, s>>>(t, ft, a, levels, partial);
-                else k_traverse_fast<2, false, true><<<g, kFastThreads, 0, s>>>(t, ft, a, levels, partial);
-            }
-            if (shares > 1) BHUT_TRY(launch_split_sum(partial, nt, t.dim, shares, out_idx, out, s));
-        } else if (t.dim == 3) {
-            if (soft) k_traverse_fast<3, true, false><<<grid, kFastThreads, 0, s>>>(t, ft, a, 0, nullptr);
-            else k_traverse_fast<3, false, false><<<grid, kFastThreads, 0, s>>>(t, ft, a, 0, nullptr);
-        } else {
-            if (soft) k_traverse_fast<2, true, false><<<grid, kFastThreads, 0, s>>>(t, ft, a, 0, nullptr);
-            else k_traverse_fast<2, false, false><<<grid, kFastThreads, 0, s>>>(t, ft, a, 0, nullptr);
-        }
+        constexpr int B = BHUT_FAST_BLOCKS, MORE = BHUT_FAST_BLOCKS_MORE;
+        const bool d3 = t.dim == 3;
+        const int shares = levels > 0 ? (1 << levels) / kFastWarps : 0;
+        const unsigned g = shares ? (unsigned)warps * (unsigned)shares : grid;
+        const auto kernel =
+            shares                     ? (soft ? (d3 ? k_traverse_fast<3, true, true, MORE>
+                                                     : k_traverse_fast<2, true, true, MORE>)
+                                               : (d3 ? k_traverse_fast<3, false, true, B>
+                                                     : k_traverse_fast<2, false, true, B>))
+            : !soft                    ? (d3 ? k_traverse_fast<3, false, false, B>
+                                             : k_traverse_fast<2, false, false, B>)
+            : warps >= 3 * kWaveWarps  ? (d3 ? k_traverse_fast<3, true, false, MORE>
+                                             : k_traverse_fast<2, true, false, MORE>)
+                                       : (d3 ? k_traverse_fast<3, true, false, B>
+                                             : k_traverse_fast<2, true, false, B>);
+        kernel<<<g, kFastThreads, 0, s>>>(t, ft, a, levels, partial);
+        if (shares > 1) BHUT_TRY(launch_split_sum(partial, nt, t.dim, shares, out_idx, out, s));
     }
     BHUT_CUDA(cudaGetLastError());
     note_launches(1);

@@ -68,6 +68,24 @@ struct FastFrame {
     int unit;
 };
 
+// A leaf's bounding box (c, h: centre and half extents, with a margin of
+// 2^-21 for the lo parts of particles and targets and for rounding) and its
+// largest |mass| (negative when some mass is).
+struct LeafBox {
+    float4 c;   // w: mass
+    float4 h;
+};
+
+// The traversals' copies of the nodes; twig may be NULL (form "fp32").
+struct NodeCopies {
+    float4* nh;
+    float4* nl;
+    LeafBox* twig;
+    float4* nq0;
+    float2* nq1;
+    int4* nhdr;
+};
+
 // Float-float copies of the particles (Morton order) and nodes.
 struct FastTree {
     FastFrame frame;
@@ -75,13 +93,10 @@ struct FastTree {
     const float4* pl;   // (x, y, z, m) lo
     const float4* nh;   // (com, mass) hi per internal node, LeafBox::c per leaf
     const float4* nl;   // (com, mass) lo per internal node, LeafBox::h per leaf
-    const float* nsize; // 2 * half_size, normalised, per node
-    const float* ndelta; // |com - AABB centre|, normalised, per node (offset criterion)
+    const LeafBox* twig; // box of a twig's particles (node_flag), h.w: its first particle
     const float4* nq0;   // quadrupole (xx, yy, zz, xy), normalised, per node; NULL: monopoles
     const float2* nq1;   // quadrupole (xz, yz)
-    const int4* nhdr;    // per node, one load per visit: leaf (-1, start, count, flag),
-                         // internal (first child, size, |com - centre| as float bits, flag);
-                         // the flag is 0 for a node without mass (node_flag)
+    const int4* nhdr;    // per node, one load per visit (put_node)
 };
 
 // Morton encoding (bhut/utils/morton.py:14-45, 183-198) and the quantisation
@@ -272,10 +287,9 @@ int launch_traverse_exact(const TreeDev& t, const double* tx, const double* ty, 
                           unsigned long long* stats, cudaStream_t s, int levels, double* partial);
 // `fine`: the lo parts of form "fast" (split_grid), else those of "fp32".
 FastFrame frame_of_box(const double* box, int dim);   // box on the host
-int launch_fast_prepare(const FastFrame& frame, bool fine, const TreeDev& t,
-                        const double* center, float4* ph, float4* pl, float4* nh, float4* nl,
-                        float* nsize, float* ndelta, const double* quad, float4* nq0,
-                        float2* nq1, int4* nhdr, cudaStream_t s);
+int launch_fast_prepare(const FastFrame& frame, bool fine, const TreeDev& t, const double* center,
+                        const double* quad, float4* ph, float4* pl, const NodeCopies& o,
+                        cudaStream_t s);
 int launch_fast_targets(const double* tx, const double* ty, const double* tz, int64_t nt, int dim,
                         bool fine, const FastFrame& frame, float4* th, float4* tl, cudaStream_t s);
 int launch_traverse_fast(const TreeDev& t, const FastTree& ft, const float4* th, const float4* tl,

@@ -56,9 +56,11 @@ from .batch import BatchedSolver
 #  batch: positions and masses copies (32), keys, second keys (16), perm and
 #    system ids (8), sorted SoA (32), float-float copies (32), sort scratch
 #    (12), kept-order and tick permutations (12);
-#  nodes: about 2 N / leaf_size of 268 B (centre of mass and mass 32, size,
-#    half, centre, AABB scratch 88, topology links 20, float-float copies and
-#    header 56, quadrupoles and their float copies 72).
+#  nodes: about 2 N / leaf_size of 260 B, 292 in form "fast" (centre of mass
+#    and mass 32, size, half, centre, AABB scratch 88, topology links 20,
+#    float-float copies and header 48, in form "fast" boxes of leaf pairs 32,
+#    quadrupoles and their float copies 72); 268 serves both, the margin below
+#    is far wider.
 STATE_BYTES = 2 * (3 * 24 + 8 + 4)
 BATCH_BYTES = 32 + 16 + 8 + 32 + 32 + 12 + 12
 NODE_BYTES = 268
