@@ -335,13 +335,16 @@ static __device__ __forceinline__ int nth_set_bit(unsigned m, int r)
 //     ALU pipe;
 //   * the displacement stays (d, l) without renormalisation: |l| <= 2^-23,
 //     and the products with l are rounded once at 2^-24 of themselves, i.e.
-//     2^-47 / D of the pair -- the error that the coordinates have anyway
-//     (r^2 alone is renormalised);
-//   * y is the rsqrt of 2 R / 3: then w = y^3 (1 - A), A = R y^2 - 3/2, has
-//     no constant left (A^2 terms below 2^-43); the leaf's sums carry the
-//     factor (3/2)^(3/2), taken off at its end.
-// 56 FP32 operations and one MUFU per pair with unit masses, against 77, 15
-// on the ALU pipe and one MUFU of pair_ff_soft.
+//     2^-47 / D of the pair -- the error that the coordinates have anyway;
+//   * neither r^2 = (R0, lo) nor y is renormalised: y is the rsqrt of 2 r^2 / 3,
+//     Y the rounded y^2 and taken as it is.  A = r^2 Y - 3/2 and b = y^2 - Y
+//     are small, and the cube of the root is Y y (1 - A) - b y / 2 with no
+//     constant left (A^2 terms below 2^-42); -y / 2 costs an ALU addition.
+//     The leaf's sums carry the factor (3/2)^(3/2), taken off at its end.
+// 53 FP32 operations and one MUFU per pair with unit masses, against 77, 15
+// on the ALU pipe and one MUFU of pair_ff_soft.  (56, with r^2 renormalised
+// and b in A: 1M Plummer 134.1 ms, 250k targets 25.8, 100k cube without
+// softening 5.07; 53: 133.1, 24.9, 4.86; errors against FP64 the same.)
 constexpr float kFarScale = 0.54433105395181735517;   // (2/3)^(3/2), float-float
 constexpr float kFarScaleLo = 0.54433105395181735517 - (double)kFarScale;
 
@@ -431,6 +434,13 @@ static __device__ __forceinline__ float2 neg2(float2 v)
                        __int_as_float(__float_as_int(v.y) ^ 0x80000000));
 }
 
+// -v / 2 of positive normal numbers above 2^-125, by one ALU addition each.
+static __device__ __forceinline__ float2 neg_half2(float2 v)
+{
+    return make_float2(__int_as_float(__float_as_int(v.x) + 0x7f800000),
+                       __int_as_float(__float_as_int(v.y) + 0x7f800000));
+}
+
 // Rows p = sub, sub + step, ... of a staged distant leaf of cn sources, as an
 // unbiased float-float sum.
 template <int DIM, bool UNIT>
@@ -469,15 +479,13 @@ __device__ __forceinline__ void far_pairs(const float* Th, const float* Tl, cons
             s = t;
         }
         const float2 R0 = __fadd2_rn(s, both(-f.s0));     // exact: s <= 2 s0
-        const float2 R = __fadd2_rn(R0, lo);              // FastTwoSum(R0, lo)
-        lo = __fadd2_rn(lo, __ffma2_rn(R, m1, R0));
-        const float2 rs = __fmul2_rn(R, both(2.0f / 3.0f));
+        const float2 rs = __ffma2_rn(lo, both(2.0f / 3.0f), __fmul2_rn(R0, both(2.0f / 3.0f)));
         const float2 y = make_float2(rsqrt_mufu(rs.x), rsqrt_mufu(rs.y));
         const float2 Y = __fmul2_rn(y, y);
         const float2 Ye = __ffma2_rn(y, y, neg2(Y));
-        const float2 A1 = __ffma2_rn(R, Ye, __ffma2_rn(lo, Y, __ffma2_rn(R, Y, both(-1.5f))));
+        const float2 A1 = __ffma2_rn(lo, Y, __ffma2_rn(R0, Y, both(-1.5f)));
         const float2 W = __fmul2_rn(Y, y), nW = neg2(W);
-        const float2 We = __ffma2_rn(Ye, y, __ffma2_rn(Y, y, nW));
+        const float2 We = __ffma2_rn(Ye, neg_half2(y), __ffma2_rn(Y, y, nW));
         float2 fh = W, fl = __ffma2_rn(nW, A1, We);
         if (!UNIT) {
             const float4 M = st.d[p];
