@@ -464,79 +464,18 @@ struct BatchArgs {
     unsigned long long* stats;
 };
 
-// The warp's traversal stack of (node, lane mask) entries (left children; the
-// right child of an opened node is visited next), two placements:
-//  STK 0: in shared memory, lane 0 writes, every lane reads (__syncwarp
-//         around each pop);
-//  STK 1: in registers, entry j held by lane j % 32 in register j / 32;
-//         a pop is two shuffles from the owning lane, a push a predicated
-//         register write; no shared memory, no __syncwarp.
-// Entries are warp-uniform, so every lane keeps the same depth `sp`.
-template <int STK> struct WarpStack;
-
-template <> struct WarpStack<0> {
-    int2* s;
-    int sp = 0, lane;
-    __device__ WarpStack(int2* s_, int lane_) : s(s_), lane(lane_) {}
-    __device__ bool empty() const { return sp == 0; }
-    __device__ int2 pop()
-    {
-        __syncwarp();
-        const int2 e = s[--sp];
-        __syncwarp();
-        return e;
-    }
-    __device__ bool push(int node, unsigned m)
-    {
-        if (sp + 2 > kStackDepth) return false;
-        if (lane == 0) s[sp] = make_int2(node, (int)m);
-        sp++;
-        return true;
-    }
-};
-
-template <> struct WarpStack<1> {
-    static_assert(kStackDepth <= 2 * kWarp, "register stack holds two entries per lane");
-    int n0 = 0, m0 = 0, n1 = 0, m1 = 0;
-    int sp = 0, lane;
-    __device__ WarpStack(int2*, int lane_) : lane(lane_) {}
-    __device__ void put(int j, int node, int mask)
-    {
-        if (lane == (j & 31)) {
-            if (j < kWarp) { n0 = node; m0 = mask; }
-            else { n1 = node; m1 = mask; }
-        }
-    }
-    __device__ bool empty() const { return sp == 0; }
-    __device__ int2 pop()
-    {
-        --sp;
-        const bool hi = sp >= kWarp;
-        const int node = __shfl_sync(0xffffffffu, hi ? n1 : n0, sp & 31);
-        const int mask = __shfl_sync(0xffffffffu, hi ? m1 : m0, sp & 31);
-        return make_int2(node, mask);
-    }
-    __device__ bool push(int node, unsigned m)
-    {
-        if (sp + 2 > kStackDepth) return false;
-        put(sp, node, (int)m);
-        sp++;
-        return true;
-    }
-};
-
-// Resident blocks per SM of the FP32 form (1 / 8 / 9 / 10 at 256 systems:
-// 61.0 / 45.9 / 46.8 / 44.8 ms; 24 systems with quadrupoles 11.3 / 8.9 / 9.0 /
-// 8.7 ms).
+// Resident blocks per SM of the FP32 form (7 / 8 / 9 / 10 at 256 systems:
+// 43.2 / 42.2 / 43.2 / 43.1 ms; 24 systems with quadrupoles 8.45 / 8.28 / 8.56
+// / 8.56 ms).
 #ifndef BHUT_BATCH_BLOCKS
-#define BHUT_BATCH_BLOCKS 10
+#define BHUT_BATCH_BLOCKS 8
 #endif
 template <int DIM, bool FP32, int TPW, int STK>
 __global__ void __launch_bounds__(kBatchThreads, FP32 ? BHUT_BATCH_BLOCKS : 1)
 k_batch_traverse(BatchDev b, BatchArgs a)
 {
     constexpr int LPT = kWarp / TPW;            // lanes per target
-    __shared__ int2 stack[STK == 0 ? kBatchWarps : 1][kStackDepth];
+    __shared__ StackEntry stack[STK == 0 ? kBatchWarps : 1][kStackDepth];
     // two-lane tasks read source by source, the others row by row (LeafStage)
     constexpr bool kStaged = TPW == 32;
     constexpr bool SCALAR = !kStaged || !FP32;   // (form fast without a large softening)
@@ -585,8 +524,6 @@ k_batch_traverse(BatchDev b, BatchArgs a)
             }
         }
         const TargetF32x2 tx = target_f32x2(Th, Tl);
-        const float2 nT[3] = {both(-Th[0]), both(-Th[1]), both(-Th[2])};
-        const float2 nL[3] = {both(-Tl[0]), both(-Tl[1]), both(-Tl[2])};
         const bool unit = fr.unit != 0;   // every particle mass of this system exactly 1
         float ah[3] = {0.f, 0.f, 0.f}, al[3] = {0.f, 0.f, 0.f};   // ff sum, or (sum, Kahan comp)
         double a64[3] = {0.0, 0.0, 0.0};
@@ -594,207 +531,180 @@ k_batch_traverse(BatchDev b, BatchArgs a)
         bool overflow = false;
 
         WarpStack<STK> st(stack[STK == 0 ? w : 0], lane);
-        int node = root;
-        unsigned mask = __ballot_sync(FULL, valid);
-        while (true) {
-            const bool act = (mask >> lane) & 1u;
-            cnt[2] += act && sub == 0;
-            const int4 hd = b.nhdr[node];   // (first_child, start, count, flag)
-            const float4 nhv = b.nh[node];
-            const int fc = hd.x;
-            const bool staged = kStaged && (FP32 || soft);
-            LeafBox box;
-            // runs of particles to take, as in the single-tree walks: with
-            // FP32 rows a leaf, or a twig's right and left leaf; else one run
-            unsigned lmask = 0;
-            int s0 = hd.y, c0 = 0, s1 = 0, c1 = 0;
-            if (!hd.w) {
-            } else if (fc < 0) {
-                lmask = mask;
-                c0 = hd.z;
-                if (kStaged && soft) {
-                    box.c = nhv;
-                    box.h = b.nl[node];
-                }
-            } else {
-                bool open = false;
-                float4 nlv = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (FP32) {   // hi coordinates only, as the single-tree walk
-                    float d2 = 0.0f;
+        if constexpr (FP32 && kStaged) {
+            walk_f32<DIM>(b, root, lane, valid, valid ? (int)i : -1, false, unit, opener, e2h, Th, Tl,
+                          ah, al, st, stage[w], cnt, overflow);
+        } else {
+            int node = root;
+            unsigned mask = __ballot_sync(FULL, valid);
+            while (true) {
+                const bool act = (mask >> lane) & 1u;
+                cnt[2] += act && sub == 0;
+                const int4 hd = b.nhdr[node];   // (first_child, start, count, flag)
+                const float4 nhv = b.nh[node];
+                const int fc = hd.x;
+                const bool staged = kStaged && soft;
+                LeafBox box;
+                unsigned lmask = 0;   // lanes that take the particles [s0, s0 + c0)
+                int s0 = hd.y, c0 = 0;
+                if (!hd.w) {
+                } else if (fc < 0) {
+                    lmask = mask;
+                    c0 = hd.z;
+                    if (staged) {
+                        box.c = nhv;
+                        box.h = b.nl[node];
+                    }
+                } else {
+                    bool open = false;
+                    float4 nlv = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (FP32) {   // hi coordinates only, as the single-tree walk
+                        float d2 = 0.0f;
 #pragma unroll
-                    for (int k = 0; k < DIM; k++) {
-                        const float d = __fsub_rn(comp(nhv, k), Th[k]);
-                        d2 = fmaf(d, d, d2);
-                    }
-                    open = opener(d2, __int_as_float(hd.y), __int_as_float(hd.z), act);
-                } else if (act) {
-                    nlv = b.nl[node];
-                    float d2 = 0.0f;
-#pragma unroll
-                    for (int k = 0; k < DIM; k++) {
-                        const float d = __fadd_rn(__fsub_rn(comp(nhv, k), Th[k]),
-                                                  __fsub_rn(comp(nlv, k), Tl[k]));
-                        d2 = fmaf(d, d, d2);
-                    }
-                    const float dist = d2 > 0.0f ? d2 * rsqrtf(d2) : 0.0f;
-                    const float size_f = __int_as_float(hd.y);
-                    const float td = theta_f * dist;
-                    const float band = theta_f * fmaf(kBandRel, dist, 2.0f * kBandAbs);
-                    if (size_f >= td + band) open = true;
-                    else if (size_f < td - band) open = false;
-                    else {
-                        open = open_exact64<DIM>(x, y, z, t.cm[node], t.size[node], a.theta);
-                        cnt[3]++;
-                    }
-                }
-                const unsigned omask = __ballot_sync(FULL, act && open);
-                if (act && !open && sub == 0) {
-                    if (FP32) {
+                        for (int k = 0; k < DIM; k++) {
+                            const float d = __fsub_rn(comp(nhv, k), Th[k]);
+                            d2 = fmaf(d, d, d2);
+                        }
+                        open = opener(d2, __int_as_float(hd.y), __int_as_float(hd.z), act);
+                    } else if (act) {
                         nlv = b.nl[node];
-                        if (b.nq0)
-                            node_quad_f32<DIM>(Th, Tl, nhv, nlv, b.nq0[node], b.nq1[node], e2h,
-                                               ah, al);
-                        else
-                            pair_f32<DIM>(Th, Tl, nhv, nlv, e2h, ah, al);
-                    } else if (soft && !(hd.w & kNodeOutside)) {
-                        pair_ff_soft<DIM, false>(Th, Tl, nhv, nlv, e2h, e2l, ah, al);
-                    } else if ((hd.w & kNodeOutside) || !pair_ff<DIM, false>(Th, Tl, nhv, nlv, e2h, e2l, ah, al)) {
-                        const NodeCM cm = t.cm[node];
-                        pair_fp64<DIM>(x, y, z, cm.x, cm.y, cm.z, cm.w, eps2, a64);
-                        cnt[4]++;
+                        float d2 = 0.0f;
+#pragma unroll
+                        for (int k = 0; k < DIM; k++) {
+                            const float d = __fadd_rn(__fsub_rn(comp(nhv, k), Th[k]),
+                                                      __fsub_rn(comp(nlv, k), Tl[k]));
+                            d2 = fmaf(d, d, d2);
+                        }
+                        const float dist = d2 > 0.0f ? d2 * rsqrtf(d2) : 0.0f;
+                        const float size_f = __int_as_float(hd.y);
+                        const float td = theta_f * dist;
+                        const float band = theta_f * fmaf(kBandRel, dist, 2.0f * kBandAbs);
+                        if (size_f >= td + band) open = true;
+                        else if (size_f < td - band) open = false;
+                        else {
+                            open = open_exact64<DIM>(x, y, z, t.cm[node], t.size[node], a.theta);
+                            cnt[3]++;
+                        }
                     }
-                    cnt[1]++;
-                }
-                if (staged && omask && (hd.w & kTwig)) {
-                    lmask = omask;
-                    if (FP32) {
-                        s1 = b.nhdr[fc].y;
-                        c1 = twig_left(hd.w);
-                        s0 = s1 + c1;
-                        c0 = twig_right(hd.w);
-                    } else {
+                    const unsigned omask = __ballot_sync(FULL, act && open);
+                    if (act && !open && sub == 0) {
+                        if (FP32) {
+                            nlv = b.nl[node];
+                            if (b.nq0)
+                                node_quad_f32<DIM>(Th, Tl, nhv, nlv, b.nq0[node], b.nq1[node], e2h,
+                                                   ah, al);
+                            else
+                                pair_f32<DIM>(Th, Tl, nhv, nlv, e2h, ah, al);
+                        } else if (soft && !(hd.w & kNodeOutside)) {
+                            pair_ff_soft<DIM, false>(Th, Tl, nhv, nlv, e2h, e2l, ah, al);
+                        } else if ((hd.w & kNodeOutside) || !pair_ff<DIM, false>(Th, Tl, nhv, nlv, e2h, e2l, ah, al)) {
+                            const NodeCM cm = t.cm[node];
+                            pair_fp64<DIM>(x, y, z, cm.x, cm.y, cm.z, cm.w, eps2, a64);
+                            cnt[4]++;
+                        }
+                        cnt[1]++;
+                    }
+                    if (staged && omask && (hd.w & kTwig)) {
+                        lmask = omask;
                         box = b.twig[node];
                         s0 = __float_as_int(box.h.w);
                         c0 = twig_left(hd.w) + twig_right(hd.w);
+                        cnt[2] += act && open ? 2 : 0;
+                    } else if (omask) {
+                        if (st.sp + 2 > kStackDepth) {
+                            overflow = true;
+                            break;
+                        }
+                        st.push({fc, omask, 0});
+                        node = fc + 1;
+                        mask = omask;
+                        continue;
                     }
-                    cnt[2] += act && open ? 2 : 0;
-                } else if (omask) {
-                    if (!st.push(fc, omask)) {
-                        overflow = true;
-                        break;
-                    }
-                    node = fc + 1;
-                    mask = omask;
-                    continue;
                 }
-            }
-            const bool lact = (lmask >> lane) & 1u;
-            if (kStaged && FP32) {
-                LeafStage& sg = stage[kStaged ? w : 0];
-                for (; c0 > 0; s0 += kWarp, c0 -= kWarp) {
-                    const int cn = min(kWarp, c0);
-                    stage_f32(sg, lane, b.ph, b.pl, s0, cn, s1, c1, false);
-                    __syncwarp();
-                    if (lact) {   // per run <= 32 terms in FP32, then one Kahan step
-                        for (int run = 0, first = 0; run < 2; run++) {
-                            const int at = run ? s1 : s0, k = run ? c1 : cn, np = rows_for(k);
-                            if (k == 0) break;
-                            cnt[0] += k - (i >= at && i < at + k);
-                            float part[3] = {0.f, 0.f, 0.f};
-                            if (soft && unit)
-                                rows_f32<DIM, false, true>(sg, first, np, nT, nL, e2h, part);
-                            else if (soft)
-                                rows_f32<DIM, false, false>(sg, first, np, nT, nL, e2h, part);
+                const bool lact = (lmask >> lane) & 1u;
+                if (c0) {
+                    const int block = staged ? kStage : kWarp;
+                    for (int bb = 0; bb < c0; bb += block) {
+                        const int cn = min(block, c0 - bb);
+                        for (int jj = lane; jj < cn; jj += kWarp) {
+                            const float4 h = b.ph[s0 + bb + jj], l = b.pl[s0 + bb + jj];
+                            if (staged) {
+                                stage[kStaged ? w : 0].put(jj, h, l);
+                            } else {
+                                sh[jj] = h;
+                                sl[jj] = l;
+                            }
+                        }
+                        __syncwarp();
+                        if (lact && sub == 0) cnt[0] += cn - (i >= s0 + bb && i < s0 + bb + cn);
+                        if (staged) {   // as the single-tree walk
+                            const LeafStage& sg = stage[kStaged ? w : 0];
+                            if (unit)
+                                leaf_block_soft<DIM, true>(lmask, lane, Th, Tl, sg, cn, box,
+                                                           e2h, e2l, ah, al);
                             else
-                                rows_f32<DIM, true, false>(sg, first, np, nT, nL, e2h, part);
-                            kahan_add_f32<DIM>(part, ah, al);
-                            first += np;
-                        }
-                    }
-                    __syncwarp();
-                }
-            } else if (c0) {
-                const int block = staged ? kStage : kWarp;
-                for (int bb = 0; bb < c0; bb += block) {
-                    const int cn = min(block, c0 - bb);
-                    for (int jj = lane; jj < cn; jj += kWarp) {
-                        const float4 h = b.ph[s0 + bb + jj], l = b.pl[s0 + bb + jj];
-                        if (staged) {
-                            stage[kStaged ? w : 0].put(jj, h, l);
-                        } else {
-                            sh[jj] = h;
-                            sl[jj] = l;
-                        }
-                    }
-                    __syncwarp();
-                    if (lact && sub == 0) cnt[0] += cn - (i >= s0 + bb && i < s0 + bb + cn);
-                    if (staged) {   // as the single-tree walk
-                        const LeafStage& sg = stage[kStaged ? w : 0];
-                        if (unit)
-                            leaf_block_soft<DIM, true>(lmask, lane, Th, Tl, sg, cn, box,
-                                                       e2h, e2l, ah, al);
-                        else
-                            leaf_block_soft<DIM, false>(lmask, lane, Th, Tl, sg, cn, box,
-                                                        e2h, e2l, ah, al);
-                    } else if (lact) {
-                        if (FP32) {   // <= 32 terms in FP32, then one Kahan step
-                            float2 pxy = make_float2(0.f, 0.f);
-                            float pz = 0.f;
-                            if (soft && unit) {
+                                leaf_block_soft<DIM, false>(lmask, lane, Th, Tl, sg, cn, box,
+                                                            e2h, e2l, ah, al);
+                        } else if (lact) {
+                            if (FP32) {   // <= 32 terms in FP32, then one Kahan step
+                                float2 pxy = make_float2(0.f, 0.f);
+                                float pz = 0.f;
+                                if (soft && unit) {
 #pragma unroll 8
-                                for (int q = sub; q < cn; q += LPT)
-                                    pair_f32_partial2<DIM, false, true>(
-                                        tx, sh[q], sl[q], e2h, pxy, pz);
-                            } else if (soft) {
+                                    for (int q = sub; q < cn; q += LPT)
+                                        pair_f32_partial2<DIM, false, true>(
+                                            tx, sh[q], sl[q], e2h, pxy, pz);
+                                } else if (soft) {
 #pragma unroll 8
-                                for (int q = sub; q < cn; q += LPT)
-                                    pair_f32_partial2<DIM, false, false>(
-                                        tx, sh[q], sl[q], e2h, pxy, pz);
+                                    for (int q = sub; q < cn; q += LPT)
+                                        pair_f32_partial2<DIM, false, false>(
+                                            tx, sh[q], sl[q], e2h, pxy, pz);
+                                } else {
+#pragma unroll 8
+                                    for (int q = sub; q < cn; q += LPT)
+                                        pair_f32_partial2<DIM, true, false>(
+                                            tx, sh[q], sl[q], e2h, pxy, pz);
+                                }
+                                const float part[3] = {pxy.x, pxy.y, pz};
+                                kahan_add_f32<DIM>(part, ah, al);
                             } else {
-#pragma unroll 8
-                                for (int q = sub; q < cn; q += LPT)
-                                    pair_f32_partial2<DIM, true, false>(
-                                        tx, sh[q], sl[q], e2h, pxy, pz);
-                            }
-                            const float part[3] = {pxy.x, pxy.y, pz};
-                            kahan_add_f32<DIM>(part, ah, al);
-                        } else {
-                            unsigned fb = 0;   // pairs left to FP64, taken after the loop
-                            if (soft && unit) {
-                                for (int q = sub; q < cn; q += LPT)
-                                    pair_ff_soft<DIM, true>(Th, Tl, sh[q], sl[q], e2h, e2l, ah, al);
-                            } else if (soft) {
-                                for (int q = sub; q < cn; q += LPT)
-                                    pair_ff_soft<DIM, false>(Th, Tl, sh[q], sl[q], e2h, e2l, ah, al);
-                            } else {
-                                for (int q = sub; q < cn; q += LPT)
-                                    fb |= (unsigned)!pair_ff<DIM, false>(Th, Tl, sh[q], sl[q], e2h,
-                                                                         e2l, ah, al) << q;
-                            }
-                            while (fb) {
-                                const int gi = s0 + bb + __ffs(fb) - 1;
-                                fb &= fb - 1;
-                                pair_fp64<DIM>(x, y, z, t.sx[gi], t.sy[gi],
-                                               DIM == 3 ? t.sz[gi] : 0.0, t.sm[gi], eps2, a64);
-                                cnt[4]++;
+                                unsigned fb = 0;   // pairs left to FP64, taken after the loop
+                                if (soft && unit) {
+                                    for (int q = sub; q < cn; q += LPT)
+                                        pair_ff_soft<DIM, true>(Th, Tl, sh[q], sl[q], e2h, e2l, ah, al);
+                                } else if (soft) {
+                                    for (int q = sub; q < cn; q += LPT)
+                                        pair_ff_soft<DIM, false>(Th, Tl, sh[q], sl[q], e2h, e2l, ah, al);
+                                } else {
+                                    for (int q = sub; q < cn; q += LPT)
+                                        fb |= (unsigned)!pair_ff<DIM, false>(Th, Tl, sh[q], sl[q], e2h,
+                                                                             e2l, ah, al) << q;
+                                }
+                                while (fb) {
+                                    const int gi = s0 + bb + __ffs(fb) - 1;
+                                    fb &= fb - 1;
+                                    pair_fp64<DIM>(x, y, z, t.sx[gi], t.sy[gi],
+                                                   DIM == 3 ? t.sz[gi] : 0.0, t.sm[gi], eps2, a64);
+                                    cnt[4]++;
+                                }
                             }
                         }
+                        __syncwarp();
                     }
-                    __syncwarp();
-                }
-                if (!FP32 && lact) {
+                    if (!FP32 && lact) {
 #pragma unroll
-                    for (int k = 0; k < DIM; k++) {
-                        const float hs = __fadd_rn(ah[k], al[k]);
-                        al[k] = __fsub_rn(al[k], __fsub_rn(hs, ah[k]));
-                        ah[k] = hs;
+                        for (int k = 0; k < DIM; k++) {
+                            const float hs = __fadd_rn(ah[k], al[k]);
+                            al[k] = __fsub_rn(al[k], __fsub_rn(hs, ah[k]));
+                            ah[k] = hs;
+                        }
                     }
                 }
+                if (st.sp == 0) break;
+                const StackEntry e = st.pop();
+                node = e.node;
+                mask = e.mask;
             }
-            if (st.empty()) break;
-            const int2 e = st.pop();
-            node = e.x;
-            mask = (unsigned)e.y;
         }
         if (overflow && lane == 0) atomicOr(a.err, kErrStackOverflow);
         // fold the lanes that share a target

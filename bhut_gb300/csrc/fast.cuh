@@ -353,7 +353,7 @@ constexpr float kFarScaleLo = 0.54433105395181735517 - (double)kFarScale;
 // and two independent chains per lane.
 // kFarRatio 16 / 32 / 64 / 256: 1M Plummer 137.0 / 134.8 / 133.6 / 132.4 ms;
 // error against FP64 sums in 2-D, 60k, 1.3e-12 / 1.3e-12 / 2.2e-12 / 6.9e-12
-// (FP64 monopoles and pair_ff_soft alone give 2.2e-12).
+// (2.2e-12 with pair_ff_soft for every leaf).
 constexpr float kFarRatio = 32.0f;
 struct FarLeaf {
     float s0;      // bias of r^2, at least max R
@@ -669,12 +669,12 @@ static __device__ __forceinline__ void leaf_box(const float4* __restrict__ ph, i
                     fmaf(0.5f * (hi[2] - lo[2]), s, o), 0.0f);
 }
 
-// Header of a node, one load per visit: leaf (-1, start, count, flag); internal
-// (first child, size, |com - box centre| as float bits, flag).  Flags: see
-// node_flag; kTwig and the counts at bits 8 and 16 for a twig, an internal
-// node whose children are leaves of neighbouring particles (at most 32 each,
-// with mass): a target that opens it takes both leaves, which need no visit of
-// their own.
+// Header of a node, one load per visit: leaf (-1, start, count, flag), any node
+// without mass (-1, start, 0, 0); internal (first child, size, |com - box
+// centre| as float bits, flag).  Flags: see node_flag; kTwig and the counts at
+// bits 8 and 16 for a twig, an internal node whose children are leaves of
+// neighbouring particles (at most 32 each, with mass): a target that opens it
+// takes both leaves, which need no visit of their own.
 constexpr int kNodeMass = 1, kNodeOutside = 2, kTwig = 4;
 static __device__ __forceinline__ int twig_left(int w) { return (w >> 8) & 0xff; }
 static __device__ __forceinline__ int twig_right(int w) { return (w >> 16) & 0xff; }
@@ -723,6 +723,7 @@ static __device__ __forceinline__ void put_node(const TreeDev& t, int64_t k, con
         hd = make_int4(fc, __float_as_int(__double2float_rn(__dmul_rn(t.size[k], f.s))),
                        __float_as_int(__double2float_ru(sqrt(dd) * f.s)), flag);
     }
+    if (!hd.w) hd = make_int4(-1, t.start[k], 0, 0);   // without mass: skipped (bh.py:514)
     o.nh[k] = h;
     o.nl[k] = l;
     o.nhdr[k] = hd;
@@ -965,12 +966,18 @@ struct OpenF32 {
         if (mac != 0.0f) return size >= theta * (dist - off);
         return dist == 0.0f || size >= theta * dist;
     }
-    // lanes outside `act` return anything
-    __device__ __forceinline__ bool operator()(float d2, float size, float off, bool act) const
+    // squares outside the band decide, the root inside it (lanes outside `act`
+    // return anything); two nodes share the rare branch
+    __device__ __forceinline__ bool near(float d2, float size, float off, bool& open) const
     {
         const float r = fmaf(off, mac, size * inv), r2 = r * r;
-        bool open = r2 >= d2;
-        if (act && !(fabsf(r2 - d2) > 0x1p-18f * d2)) open = opens(d2, size, off);
+        open = r2 >= d2;
+        return !(fabsf(r2 - d2) > 0x1p-18f * d2);
+    }
+    __device__ __forceinline__ bool operator()(float d2, float size, float off, bool act) const
+    {
+        bool open;
+        if (near(d2, size, off, open) && act) open = opens(d2, size, off);
         return open;
     }
 };
@@ -1007,6 +1014,180 @@ __device__ __forceinline__ void node_quad_f32(const float* Th, const float* Tl, 
         const float t = __fadd_rn(acc[k], y);
         cmp[k] = __fsub_rn(__fsub_rn(t, acc[k]), y);
         acc[k] = t;
+    }
+}
+
+// The warp's traversal stack (left children; the right child of an opened node
+// is visited next) of (node, lanes, lanes that open it) entries, two placements:
+//  STK 0: in shared memory, lane 0 writes, every lane reads (__syncwarp
+//         around each pop);
+//  STK 1: in registers, entry j held by lane j % 32 in register j / 32;
+//         a pop is three shuffles from the owning lane, a push a predicated
+//         register write; no shared memory, no __syncwarp.
+// Entries are warp-uniform, so every lane keeps the same depth `sp`.
+struct StackEntry {
+    int node;
+    unsigned mask, open;
+};
+template <int STK> struct WarpStack;
+
+template <> struct WarpStack<0> {
+    StackEntry* s;
+    int sp = 0, lane;
+    __device__ WarpStack(StackEntry* s_, int lane_) : s(s_), lane(lane_) {}
+    __device__ StackEntry pop()
+    {
+        __syncwarp();
+        const StackEntry e = s[--sp];
+        __syncwarp();
+        return e;
+    }
+    __device__ void push(const StackEntry& e)
+    {
+        if (lane == 0) s[sp] = e;
+        sp++;
+    }
+};
+
+template <> struct WarpStack<1> {
+    static_assert(kStackDepth <= 2 * kWarp, "register stack holds two entries per lane");
+    StackEntry e0{0, 0, 0}, e1{0, 0, 0};
+    int sp = 0, lane;
+    __device__ WarpStack(StackEntry*, int lane_) : lane(lane_) {}
+    __device__ StackEntry pop()
+    {
+        --sp;
+        const bool hi = sp >= kWarp;
+        return {__shfl_sync(0xffffffffu, hi ? e1.node : e0.node, sp & 31),
+                __shfl_sync(0xffffffffu, hi ? e1.mask : e0.mask, sp & 31),
+                __shfl_sync(0xffffffffu, hi ? e1.open : e0.open, sp & 31)};
+    }
+    __device__ void push(const StackEntry& e)
+    {
+        if (lane == (sp & 31)) {
+            if (sp < kWarp) e0 = e;
+            else e1 = e;
+        }
+        sp++;
+    }
+};
+
+// FP32 walk of a warp's targets (negated coordinates nT, nL for the rows) from
+// node `root`, shared by the single trees (FastTree) and the batches.  The
+// children of an opened node are tested together, so a node costs half a test
+// and half the loop around it; its left child waits in registers and goes to
+// the stack only when the right one is opened too.  Contributions reach a
+// target in the order of a walk that visits right before left.  The kernels
+// issue on 79 % of the clocks, so what counts is instructions: 2M galaxy, theta
+// 0.7, leaf 16, node by node 106.6 ms, by pairs 103.3, with one branch for both
+// roots and no separate test for mass 101.2 (1M of it: 38.5 G warp
+// instructions; rows about 12, monopoles 6, visits 19).  Separate kernels with
+// and without the small-r test: 100.9, batches 42.5 against 42.2, not kept.
+template <int DIM, class TREE, class STACK>
+__device__ __forceinline__ void walk_f32(const TREE& ft, int root, int lane, bool valid, int me,
+                                         bool outside, bool unit, const OpenF32& opener, float e2h,
+                                         const float* T, const float* Tl, float* acc, float* cmp,
+                                         STACK& st, LeafStage& stage, unsigned* cnt,
+                                         bool& overflow)
+{
+    const unsigned FULL = 0xffffffffu;
+    const bool soft = e2h >= 0x1p-126f;   // r^2 >= eps^2 is normal: no small-r test
+    const float2 nT[3] = {both(-T[0]), both(-T[1]), both(-T[2])};
+    const float2 nL[3] = {both(-Tl[0]), both(-Tl[1]), both(-Tl[2])};
+    const auto dist2 = [&](const float4& nh) {
+        float d2 = 0.0f;
+#pragma unroll
+        for (int k = 0; k < DIM; k++) {
+            const float d = __fsub_rn(comp(nh, k), T[k]);
+            d2 = fmaf(d, d, d2);
+        }
+        return d2;
+    };
+    StackEntry e{root, __ballot_sync(FULL, valid), 0};   // the node, lanes that reach and open it
+    StackEntry left{-1, 0, 0};                           // the sibling that comes next
+    int4 hd = ft.nhdr[root];                             // (first_child, start, count, flag)
+    e.open = __ballot_sync(FULL, opener(dist2(ft.nh[root]), __int_as_float(hd.y),
+                                        __int_as_float(hd.z), valid) && valid);
+    cnt[2] += valid;
+    while (true) {
+        // runs of particles to take: a leaf's blocks of 32, or a twig's right
+        // and left leaf (the order in which the leaves would be visited)
+        unsigned lmask = 0;
+        int s0 = hd.y, c0 = 0, s1 = 0, c1 = 0;
+        const int fc = hd.x;
+        if (fc < 0) {                     // (without mass: no particles, put_node)
+            lmask = e.mask;
+            c0 = hd.z;
+        } else {
+            if (((e.mask & ~e.open) >> lane) & 1u) {
+                if (ft.nq0)
+                    node_quad_f32<DIM>(T, Tl, ft.nh[e.node], ft.nl[e.node], ft.nq0[e.node],
+                                       ft.nq1[e.node], e2h, acc, cmp);
+                else
+                    pair_f32<DIM>(T, Tl, ft.nh[e.node], ft.nl[e.node], e2h, acc, cmp);
+                cnt[1]++;
+            }
+            if (e.open && (hd.w & kTwig)) {
+                lmask = e.open;
+                s1 = ft.nhdr[fc].y;
+                c1 = twig_left(hd.w);
+                s0 = s1 + c1;
+                c0 = twig_right(hd.w);
+                cnt[2] += (lmask >> lane) & 1u ? 2 : 0;
+            } else if (e.open) {
+                if (left.node >= 0) {
+                    if (st.sp + 3 > kStackDepth) { overflow = true; break; }
+                    st.push(left);
+                }
+                const int4 hl = ft.nhdr[fc];
+                hd = ft.nhdr[fc + 1];
+                const float dl = dist2(ft.nh[fc]), dr = dist2(ft.nh[fc + 1]);
+                const bool act = (e.open >> lane) & 1u;
+                cnt[2] += act ? 2 : 0;
+                bool ol, orr;
+                const bool nl = opener.near(dl, __int_as_float(hl.y), __int_as_float(hl.z), ol);
+                const bool nr = opener.near(dr, __int_as_float(hd.y), __int_as_float(hd.z), orr);
+                if (act && (nl || nr)) {
+                    if (nl) ol = opener.opens(dl, __int_as_float(hl.y), __int_as_float(hl.z));
+                    if (nr) orr = opener.opens(dr, __int_as_float(hd.y), __int_as_float(hd.z));
+                }
+                left = {fc, e.open, __ballot_sync(FULL, ol && act)};
+                e = {fc + 1, e.open, __ballot_sync(FULL, orr && act)};
+                continue;
+            }
+        }
+        for (; c0 > 0; s0 += kWarp, c0 -= kWarp) {
+            const int cn = min(kWarp, c0);
+            stage_f32(stage, lane, ft.ph, ft.pl, s0, cn, s1, c1, outside);
+            __syncwarp();
+            if ((lmask >> lane) & 1u) {
+                // per run <= 32 terms, then one Kahan step
+                for (int run = 0, first = 0; run < 2; run++) {
+                    const int at = run ? s1 : s0, k = run ? c1 : cn, np = rows_for(k);
+                    if (k == 0) break;
+                    cnt[0] += k - ((unsigned)(me - at) < (unsigned)k);
+                    float part[3] = {0.f, 0.f, 0.f};
+                    if (soft && unit)
+                        rows_f32<DIM, false, true>(stage, first, np, nT, nL, e2h, part);
+                    else if (soft)
+                        rows_f32<DIM, false, false>(stage, first, np, nT, nL, e2h, part);
+                    else
+                        rows_f32<DIM, true, false>(stage, first, np, nT, nL, e2h, part);
+                    kahan_add_f32<DIM>(part, acc, cmp);
+                    first += np;
+                }
+            }
+            __syncwarp();
+        }
+        if (left.node >= 0) {
+            e = left;
+            left.node = -1;
+        } else if (st.sp == 0) {
+            break;
+        } else {
+            e = st.pop();
+        }
+        hd = ft.nhdr[e.node];
     }
 }
 

@@ -535,124 +535,29 @@ __global__ void k_split_sum(const double* __restrict__ partial, int64_t nt, int 
 // test in FP32 on hi + lo displacements (each difference exact, rounded
 // once); per-target sums Kahan-compensated: every monopole, and every leaf
 // block of at most 32 pair terms (summed in FP32 first), is one Kahan step.
-// 2M galaxy, theta 0.7, leaf 16: 119 -> 109 ms with two sources to a row, the
-// opening test on squares and the right child from registers; of that about 71
-// ms are the walk (node loads, tests, monopoles), 16 staging leaves, the rest
-// pairs.  Prefetching the next nodes' headers: 122 to 126 ms, not kept.
+// Walk and rows are in fast.cuh (walk_f32, rows_f32), with the figures.  2M
+// galaxy, theta 0.7, leaf 16: 119 -> 101 ms with two sources to a row, the
+// opening test on squares, leaf pairs in one visit and children tested
+// together.  Prefetching the next nodes' headers: 122 to 126 ms, not kept.
 // FP64 stays in the tree build (bounding box, Morton keys, masses and
 // centres of mass, quadrupoles) and in the final scaling.
 // ---------------------------------------------------------------------------
-template <int DIM>
-__device__ __forceinline__ void walk_f32(const TreeDev& t, const FastTree& ft, const FastArgs& a,
-                                         int w, int lane, bool valid, bool outside, int64_t me_sorted,
-                                         const float* T, const float* Tl, float* acc, float* cmp,
-                                         int2 (*stack)[kStackDepth], LeafStage* stage,
-                                         unsigned* cnt, bool& overflow)
-{
-    const unsigned FULL = 0xffffffffu;
-    const bool soft = a.e2h >= 0x1p-126f;   // r^2 >= eps^2 is normal: no small-r test
-    const bool unit = ft.frame.unit != 0 && !outside;   // every particle mass exactly 1
-    const float2 nT[3] = {both(-T[0]), both(-T[1]), both(-T[2])};
-    const float2 nL[3] = {both(-Tl[0]), both(-Tl[1]), both(-Tl[2])};
-    const OpenF32 opener(a.theta, a.mac);
-    // (right child straight from registers, as in the fast form's walk)
-    int node = 0, sp = 0;
-    unsigned mask = __ballot_sync(FULL, valid);
-    while (true) {
-        const bool act = (mask >> lane) & 1u;
-        cnt[2] += act;
-        const int4 hd = ft.nhdr[node];   // (first_child, start, count, flag)
-        const float4 nh = ft.nh[node];
-        const int fc = hd.x;
-        // runs of particles to take: a leaf's blocks of 32, or a twig's right
-        // and left leaf (the order in which the leaves would be visited)
-        unsigned lmask = 0;
-        int s0 = hd.y, c0 = 0, s1 = 0, c1 = 0;
-        if (!hd.w) {
-        } else if (fc < 0) {
-            lmask = mask;
-            c0 = hd.z;
-        } else {
-            float d2 = 0.0f;
-#pragma unroll
-            for (int k = 0; k < DIM; k++) {
-                const float d = __fsub_rn(comp(nh, k), T[k]);
-                d2 = fmaf(d, d, d2);
-            }
-            const bool open = opener(d2, __int_as_float(hd.y), __int_as_float(hd.z), act);
-            const unsigned omask = __ballot_sync(FULL, act && open);
-            if (act && !open) {
-                if (ft.nq0)
-                    node_quad_f32<DIM>(T, Tl, nh, ft.nl[node], ft.nq0[node], ft.nq1[node], a.e2h,
-                                       acc, cmp);
-                else
-                    pair_f32<DIM>(T, Tl, nh, ft.nl[node], a.e2h, acc, cmp);
-                cnt[1]++;
-            }
-            if (omask && (hd.w & kTwig)) {
-                lmask = omask;
-                s1 = ft.nhdr[fc].y;
-                c1 = twig_left(hd.w);
-                s0 = s1 + c1;
-                c0 = twig_right(hd.w);
-                cnt[2] += act && open ? 2 : 0;
-            } else if (omask) {
-                if (sp + 2 > kStackDepth) { overflow = true; break; }
-                if (lane == 0) stack[w][sp] = make_int2(fc, (int)omask);
-                sp++;
-                node = fc + 1;
-                mask = omask;
-                continue;
-            }
-        }
-        for (; c0 > 0; s0 += kWarp, c0 -= kWarp) {
-            const int cn = min(kWarp, c0);
-            stage_f32(stage[w], lane, ft.ph, ft.pl, s0, cn, s1, c1, outside);
-            __syncwarp();
-            if ((lmask >> lane) & 1u) {
-                // per run <= 32 terms, then one Kahan step
-                for (int run = 0, first = 0; run < 2; run++) {
-                    const int at = run ? s1 : s0, k = run ? c1 : cn, np = rows_for(k);
-                    if (k == 0) break;
-                    cnt[0] += k - (me_sorted >= at && me_sorted < at + k);
-                    float part[3] = {0.f, 0.f, 0.f};
-                    if (soft && unit)
-                        rows_f32<DIM, false, true>(stage[w], first, np, nT, nL, a.e2h, part);
-                    else if (soft)
-                        rows_f32<DIM, false, false>(stage[w], first, np, nT, nL, a.e2h, part);
-                    else
-                        rows_f32<DIM, true, false>(stage[w], first, np, nT, nL, a.e2h, part);
-                    kahan_add_f32<DIM>(part, acc, cmp);
-                    first += np;
-                }
-            }
-            __syncwarp();
-        }
-        if (sp == 0) break;
-        __syncwarp();
-        const int2 e = stack[w][--sp];
-        __syncwarp();
-        node = e.x;
-        mask = (unsigned)e.y;
-    }
-}
-
-// Resident blocks per SM: the walk waits for loads (8 / 9 / 10 / 11 blocks at
-// 2M galaxy, theta 0.7, leaf 16: 109.9 / 111.1 / 106.5 / 111.7 ms; the kernel
-// issues on about 78 % of the clocks).  Twigs taken in one visit: 108.9 ms
-// without, 106.5 with.
+// Resident blocks per SM: 8 / 9 / 10 / 11 at 2M galaxy, theta 0.7, leaf 16:
+// 103.6 / 101.2 / 104.5 / 125 ms (more blocks leave fewer registers, and less
+// L1 beside the stages and stacks).
 #ifndef BHUT_F32_BLOCKS
-#define BHUT_F32_BLOCKS 10
+#define BHUT_F32_BLOCKS 9
 #endif
 template <int DIM>
 __global__ void __launch_bounds__(kFastThreads, BHUT_F32_BLOCKS)
 k_traverse_fp32(TreeDev t, FastTree ft, FastArgs a)
 {
-    __shared__ int2 stack[kFastWarps][kStackDepth];
+    __shared__ StackEntry stack[kFastWarps][kStackDepth];
     __shared__ LeafStage stage[kFastWarps];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned FULL = 0xffffffffu;
     const double conv = __dmul_rn(ft.frame.conv, a.G);
+    const OpenF32 opener(a.theta, a.mac);
     for (int64_t base = ((int64_t)blockIdx.x * kFastWarps + w) * kWarp; base < a.nt;
          base += (int64_t)gridDim.x * kFastWarps * kWarp) {
         const int64_t i = base + lane;
@@ -669,10 +574,11 @@ k_traverse_fp32(TreeDev t, FastTree ft, FastArgs a)
         outside = __any_sync(FULL, outside);
         float acc[3] = {0.f, 0.f, 0.f}, cmp[3] = {0.f, 0.f, 0.f};
         unsigned cnt[5] = {0, 0, 0, 0, 0};
-        const int64_t me_sorted = (valid && a.th == nullptr) ? i : -1;
+        const int me = valid && a.th == nullptr ? (int)i : -1;
         bool overflow = false;
-        walk_f32<DIM>(t, ft, a, w, lane, valid, outside, me_sorted, T, Tl, acc, cmp, stack, stage, cnt,
-                      overflow);
+        WarpStack<0> st(stack[w], lane);
+        walk_f32<DIM>(ft, 0, lane, valid, me, outside, ft.frame.unit != 0 && !outside, opener,
+                      a.e2h, T, Tl, acc, cmp, st, stage[w], cnt, overflow);
         if (overflow && lane == 0) atomicOr(a.err, kErrStackOverflow);
         if (a.stats) {
 #pragma unroll

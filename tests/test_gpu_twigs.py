@@ -67,6 +67,16 @@ def test_child_without_mass(dead, form):
     assert rel_l2(out, ref) < 30 * RTOL[form]      # (signs: sums may lose a factor)
 
 
+@pytest.mark.parametrize("form", ["fast", "fp32"])
+@pytest.mark.parametrize("n", [1, 5, 200])
+def test_no_mass_at_all(n, form):
+    pos, _ = workloads.gaussian(n, seed=n)
+    ref, counts = _solve(pos, np.zeros(n), "exact", 4, 3, 0.05)
+    out, c = _solve(pos, np.zeros(n), form, 4, 3, 0.05)
+    assert not out.any() and not ref.any()
+    assert c == counts
+
+
 @pytest.mark.parametrize("leaf", [1, 7, 16, 32])
 @pytest.mark.parametrize("form,eps", [("fp32", 0.05), ("fp32", 0.0), ("fast", 0.05), ("fast", 0.0)])
 def test_batch_equals_single(form, eps, leaf):
