@@ -56,25 +56,41 @@ inline unsigned grid_for(int64_t n, int block, unsigned cap = 152u * 16u)
 // Radix sort of (uint64 key, int32 value) pairs, stable, LSD, 8-bit digits
 // (sort.cu).
 // ---------------------------------------------------------------------------
-// Keys per tile: 2^BHUT_SORT_TILE_SHIFT (8 warps x 256 keys by default).
-// Smaller tiles give more blocks for the latency-bound rank/scatter step at
-// moderate n, at the price of larger count tables.
-#ifndef BHUT_SORT_TILE_SHIFT
-#define BHUT_SORT_TILE_SHIFT 11
+// Keys per tile (sort.cu): more tiles give more blocks for the latency-bound
+// rank and scatter steps, at the price of larger count tables.  Whole rebuilds,
+// us, by tiles of 256 / 512 / 1,024 / 2,048 keys:
+//   32,768   177 / 182 / 208 / 229      300,000    267 / 232 / 238 / 255
+//   100,000  205 / 194 / 211 / 236      500,000    350 / 299 / 286 / 288
+//   200,000  241 / 220 / 224 / 241      1,000,000  517 / 424 / 395 / 370
+#ifndef BHUT_SORT_SMALL_TILE_MAX
+#define BHUT_SORT_SMALL_TILE_MAX 320000
 #endif
-constexpr int kSortTileShift = BHUT_SORT_TILE_SHIFT;
-constexpr int kSortTile = 1 << kSortTileShift;
+// The fewest keys go without the scan launches: orders of 10,000 / 16,000 /
+// 24,000 / 32,768 keys 167 / 173 / 198 / 191 us, with them 201 / 205 / 209 /
+// 214 us; rebuilds 167 / 172 / 193 / 185 and 171 / 185 / 185 / 185 us.
+#ifndef BHUT_SORT_SUMS_MAX
+#define BHUT_SORT_SUMS_MAX 16384
+#endif
+constexpr int kSortShift = 11, kSortShiftSmall = 9;
 constexpr int kSortThreads = 256;
 constexpr int kSortPassesMax = 8;      // 64 key bits
 
-constexpr int64_t sort_tiles(int64_t n) { return (n + kSortTile - 1) / kSortTile; }
+constexpr bool sort_small_tiles(int64_t n) { return n <= BHUT_SORT_SMALL_TILE_MAX; }
+constexpr bool sort_sums(int64_t n) { return n <= BHUT_SORT_SUMS_MAX; }
+constexpr int64_t sort_tiles(int64_t n)
+{
+    const int shift = sort_small_tiles(n) ? kSortShiftSmall : kSortShift;
+    return (n + (1 << shift) - 1) >> shift;
+}
+constexpr int sort_tables(int64_t n) { return sort_sums(n) ? 3 : 2; }
 constexpr size_t sort_align(size_t x) { return (x + 255) & ~(size_t)255; }
-// Scratch of radix_sort_pairs for n keys: the ping-pong keys and values, two
-// bucket-major count tables (256 x tiles) and the per-pass digit totals.
+// Scratch of radix_sort_pairs for n keys: the ping-pong keys and values, two or
+// three count tables (256 x tiles) and the per-pass digit totals.  Not monotone
+// in n; largest below a limit L at L itself when L is above both rules' lines.
 constexpr size_t sort_scratch_bytes(int64_t n)
 {
     return sort_align(sizeof(uint64_t) * (size_t)n) + sort_align(sizeof(int32_t) * (size_t)n) +
-           2 * sort_align(sizeof(uint32_t) * 256 * (size_t)sort_tiles(n)) +
+           sort_tables(n) * sort_align(sizeof(uint32_t) * 256 * (size_t)sort_tiles(n)) +
            sort_align(sizeof(uint32_t) * 256 * kSortPassesMax);
 }
 // Sorts keys[0..n) ascending with values carried along.  `bits` is the

@@ -2,7 +2,7 @@
 //
 // Replaces np.argsort(codes, kind='stable') of bhut/utils/morton.py:135.  A
 // stable order of the keys is unique, so the permutation is bit-identical to
-// numpy's.  8-bit digits; keys are cut into tiles of kSortTile consecutive
+// numpy's.  8-bit digits; keys are cut into tiles of 512 or 2,048 consecutive
 // positions (of the order the pass reads).
 //
 //   k_sort_prep      one read of the keys: every pass's global digit totals
@@ -23,43 +23,47 @@
 //                    next pass's digit per destination tile (warp-aggregated
 //                    global atomics): the next pass needs no histogram launch.
 //
+// The fewest keys (sort_sums, common.cuh) go without the scan: each scatter
+// block adds up the few tiles' counts itself.  One launch per pass.
+//
 // No block waits on another block (no look-back): the only cross-block
-// dependencies are between launches.  Two launches per pass.
+// dependencies are between launches.  Two launches per pass otherwise.
 #include <atomic>
+#include <utility>
 
 #include "tree.cuh"
 
 // Points that one block orders (launch_order).  Whole rebuilds, us, by one
-// block / by passes: 1,000 points 126 / 177, 4,000 168 / 228, 8,000 237 / 248,
-// 12,000 282 / 246.
+// block / by passes: 1,500 points 117 / -, 3,000 142 / 144, 4,000 162 / 158,
+// 5,000 181 / 156, 8,000 208 / 157; orders alone: 3,000 139 / 169, 5,000 162 /
+// 161, 8,000 176 / 157.
 #ifndef BHUT_ORDER_SMALL
-#define BHUT_ORDER_SMALL 8192
+#define BHUT_ORDER_SMALL 4096
 #endif
 
 namespace bhut {
 
 namespace {
 
-constexpr int kItems = kSortTile / kSortThreads;       // keys per thread
 constexpr int kWarpsPerTile = kSortThreads / kWarp;    // 8
-constexpr int kWarpSpan = kSortTile / kWarpsPerTile;   // keys per warp
 constexpr int kScanThreads = 256;
-constexpr int kTileShift = kSortTileShift;             // log2(kSortTile)
-static_assert(kItems >= 1 && kItems * kSortThreads == kSortTile, "tile of whole warps");
+static_assert((1 << kSortShiftSmall) % kSortThreads == 0, "tiles of whole blocks");
 // resident scatter blocks per SM the register budget must allow (shared
-// memory allows three 59 KB tiles of 4,096 keys, five 34 KB tiles of 2,048)
-constexpr int kScatterMinBlocks = kSortTileShift >= 12 ? 3 : 4;
+// memory allows five 34 KB tiles of 2,048 keys)
+constexpr int kScatterMinBlocks = 4;
 static_assert(kScanThreads == kSortThreads, "the scan helper serves both kernels");
 
+template <int TILE>
 __device__ __forceinline__ int64_t item_pos(int64_t tile, int warp, int item, int lane)
 {
-    return tile * kSortTile + (int64_t)warp * kWarpSpan + item * kWarp + lane;
+    return tile * TILE + (int64_t)warp * (TILE / kWarpsPerTile) + item * kWarp + lane;
 }
 
 // Shared memory of the scatter kernel.
+template <int TILE>
 struct ScatterSmem {
-    uint64_t keys[kSortTile];
-    int32_t vals[kSortTile];
+    uint64_t keys[TILE];
+    int32_t vals[TILE];
     uint32_t warp_counts[kWarpsPerTile][256];
     uint32_t delta[256];      // global offset of the digit minus its local offset
     uint32_t local_off[256];
@@ -67,10 +71,12 @@ struct ScatterSmem {
 
 // k_sort_prep: block t reads tile t; per-tile counts of digit 0 and the
 // global totals of every pass's digit.
+template <int SHIFT>
 __global__ void __launch_bounds__(kSortThreads)
 k_sort_prep(const uint64_t* __restrict__ keys, int64_t n, int passes,
             uint32_t* __restrict__ counts0, int64_t tiles, uint32_t* __restrict__ totals)
 {
+    constexpr int kTile = 1 << SHIFT, kItems = kTile / kSortThreads;
     __shared__ uint32_t hist[kSortPassesMax][256];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t tile = blockIdx.x;
@@ -80,11 +86,11 @@ k_sort_prep(const uint64_t* __restrict__ keys, int64_t n, int passes,
     // or the few distinct high digits of clustered keys) is added once
 #pragma unroll 4
     for (int i = 0; i < kItems; i++) {
-        const int64_t pos = item_pos(tile, warp, i, lane);
+        const int64_t pos = item_pos<kTile>(tile, warp, i, lane);
         const bool valid = pos < n;
         const unsigned vmask = __ballot_sync(0xffffffffu, valid);
         // (a lane past the end borrows the tile's first key, which exists)
-        const uint64_t k = keys[valid ? pos : tile * kSortTile];
+        const uint64_t k = keys[valid ? pos : tile * kTile];
         for (int p = 0; p < passes; p++) {
             const unsigned d = (unsigned)(k >> (8 * p)) & 0xFFu;
             const bool same = __all_sync(0xffffffffu, d == __shfl_sync(0xffffffffu, d, 0));
@@ -168,20 +174,36 @@ k_sort_scan(uint32_t* __restrict__ counts, int64_t tiles, const uint32_t* __rest
 
 // k_sort_scatter: see the file comment.  `next_counts` (may be null) gets
 // the digit at `next_shift` of every key, per destination tile.
+//
+// SUMS (few tiles): no scan launch; `offsets` are the counts themselves, tile
+// by tile (entry tile * 256 + digit), which every block adds up, and the block
+// clears its part of `clear` (may be null), the table of the pass after next.
+template <int SHIFT, bool SUMS>
 __global__ void __launch_bounds__(kSortThreads, kScatterMinBlocks)
 k_sort_scatter(const uint64_t* __restrict__ keys_in, const int32_t* __restrict__ vals_in,
                uint64_t* __restrict__ keys_out, int32_t* __restrict__ vals_out, int64_t n,
                int shift, const uint32_t* __restrict__ offsets, int64_t tiles,
-               uint32_t* __restrict__ next_counts, int next_shift)
+               uint32_t* __restrict__ next_counts, int next_shift, uint32_t* __restrict__ clear)
 {
+    constexpr int kTile = 1 << SHIFT, kItems = kTile / kSortThreads;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    ScatterSmem& sm = *reinterpret_cast<ScatterSmem*>(smem_raw);
+    ScatterSmem<kTile>& sm = *reinterpret_cast<ScatterSmem<kTile>*>(smem_raw);
     __shared__ uint32_t warp_sums[kSortThreads / kWarp];
     const unsigned FULL = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t tile = blockIdx.x;
 #pragma unroll
     for (int w = 0; w < kWarpsPerTile; w++) sm.warp_counts[w][tid] = 0;
+    uint32_t before_tile = 0, of_digit = 0;   // keys of digit `tid`
+    if (SUMS) {
+#pragma unroll 8
+        for (int t = 0; t < (int)tiles; t++) {
+            const uint32_t c = offsets[t * 256 + tid];
+            of_digit += c;
+            before_tile += t < tile ? c : 0u;
+        }
+        if (clear) clear[tile * 256 + tid] = 0u;
+    }
     __syncthreads();
 
     uint64_t k[kItems];
@@ -189,7 +211,7 @@ k_sort_scatter(const uint64_t* __restrict__ keys_in, const int32_t* __restrict__
     const unsigned lt_mask = (1u << lane) - 1u;
 #pragma unroll
     for (int i = 0; i < kItems; i++) {
-        const int64_t p = item_pos(tile, warp, i, lane);
+        const int64_t p = item_pos<kTile>(tile, warp, i, lane);
         const bool valid = p < n;
         k[i] = valid ? keys_in[p] : ~0ull;
         const unsigned d = (unsigned)(k[i] >> shift) & 0xFFu;
@@ -219,16 +241,18 @@ k_sort_scatter(const uint64_t* __restrict__ keys_in, const int32_t* __restrict__
     }
     const uint32_t loc = block_exclusive_scan(run, nullptr, warp_sums);
     sm.local_off[tid] = loc;
-    sm.delta[tid] = offsets[(int64_t)tid * tiles + tile] - loc;
+    const uint32_t to = SUMS ? block_exclusive_scan(of_digit, nullptr, warp_sums) + before_tile
+                             : offsets[(int64_t)tid * tiles + tile];
+    sm.delta[tid] = to - loc;
     __syncthreads();
     // reorder the tile by digit in shared memory (stable)
 #pragma unroll
     for (int i = 0; i < kItems; i++) {
-        const int64_t p = item_pos(tile, warp, i, lane);
+        const int64_t p = item_pos<kTile>(tile, warp, i, lane);
         if (p < n) {
             const unsigned d = (unsigned)(k[i] >> shift) & 0xFFu;
             const uint32_t lpos = sm.local_off[d] + sm.warp_counts[warp][d] + rank[i];
-            if (lpos < (uint32_t)kSortTile) {   // always true; guards shared memory
+            if (lpos < (uint32_t)kTile) {   // always true; guards shared memory
                 sm.keys[lpos] = k[i];
                 sm.vals[lpos] = vals_in[p];    // (read here: fewer live registers)
             }
@@ -237,7 +261,7 @@ k_sort_scatter(const uint64_t* __restrict__ keys_in, const int32_t* __restrict__
     __syncthreads();
     // write out in digit runs: position j of the reordered tile goes to
     // delta[digit] + j
-    const int64_t cnt = min((int64_t)kSortTile, n - tile * kSortTile);
+    const int64_t cnt = min((int64_t)kTile, n - tile * kTile);
 #pragma unroll 4
     for (int j = tid; j < cnt; j += kSortThreads) {
         const uint64_t key = sm.keys[j];
@@ -248,30 +272,54 @@ k_sort_scatter(const uint64_t* __restrict__ keys_in, const int32_t* __restrict__
         vals_out[dst] = sm.vals[j];
         if (next_counts) {   // warp-aggregated: one atomic per (digit, tile) in the warp
             const unsigned nd = (unsigned)(key >> next_shift) & 0xFFu;
-            const unsigned dtile = dst >> kTileShift;
+            const unsigned dtile = dst >> SHIFT;
             const unsigned peers = __match_any_sync(__activemask(), (dtile << 8) | nd);
             if ((peers & ((1u << lane) - 1u)) == 0)
-                atomicAdd(&next_counts[(int64_t)nd * tiles + dtile], (unsigned)__popc(peers));
+                atomicAdd(&next_counts[SUMS ? (int64_t)dtile * 256 + nd : (int64_t)nd * tiles + dtile],
+                          (unsigned)__popc(peers));
         }
     }
+}
+
+// k_sort_count: digit 0 of every key per tile, for the first pass with SUMS;
+// clears the second pass's table.
+template <int SHIFT>
+__global__ void __launch_bounds__(kSortThreads)
+k_sort_count(const uint64_t* __restrict__ keys, int n, uint32_t* __restrict__ counts,
+             uint32_t* __restrict__ clear)
+{
+    __shared__ uint32_t hist[256];
+    const int tid = threadIdx.x, tile = blockIdx.x;
+    hist[tid] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < (1 << SHIFT) / kSortThreads; i++) {
+        const int p = (tile << SHIFT) + i * kSortThreads + tid;
+        if (p < n) atomicAdd(&hist[(unsigned)keys[p] & 0xffu], 1u);
+    }
+    __syncthreads();
+    counts[tile * 256 + tid] = hist[tid];
+    clear[tile * 256 + tid] = 0u;
 }
 
 struct SortLayout {
     uint64_t* keys_alt;
     int32_t* vals_alt;
-    uint32_t* counts[2];
+    uint32_t* counts[3];
     uint32_t* totals;
 };
 
 SortLayout carve(void* scratch, int64_t n)
 {
-    const int64_t tiles = sort_tiles(n);
     char* s = (char*)scratch;
     SortLayout L;
     L.keys_alt = (uint64_t*)s; s += sort_align(sizeof(uint64_t) * (size_t)n);
     L.vals_alt = (int32_t*)s;  s += sort_align(sizeof(int32_t) * (size_t)n);
-    L.counts[0] = (uint32_t*)s; s += sort_align(sizeof(uint32_t) * 256 * (size_t)tiles);
-    L.counts[1] = (uint32_t*)s; s += sort_align(sizeof(uint32_t) * 256 * (size_t)tiles);
+    const size_t table = sizeof(uint32_t) * 256 * (size_t)sort_tiles(n);
+    for (int k = 0; k < sort_tables(n); k++) {
+        L.counts[k] = (uint32_t*)s;
+        s += sort_align(table);
+    }
     L.totals = (uint32_t*)s;
     return L;
 }
@@ -282,7 +330,7 @@ SortLayout carve(void* scratch, int64_t n)
 // Small inputs: Morton keys, stable sort and Morton-ordered copies by one block.
 //
 // Up to a few thousand points the passes above take as long as their launches
-// (two a pass, 18 with the keys and the gather).  One block holds the keys in
+// (one a pass, 11 with the keys and the gather).  One block holds the keys in
 // registers and ranks, scatters and reads them back through shared memory,
 // eight bits at a time as above; places past the last point carry the largest
 // key and stay behind all others.
@@ -440,8 +488,7 @@ int order_small(const double* pos, const double* mass, int n, const double* box,
 {
     if (n <= 1024) return run_order_small<DIM, 1>(pos, mass, n, box, keys, perm, sx, sy, sz, sm, s);
     if (n <= 2048) return run_order_small<DIM, 2>(pos, mass, n, box, keys, perm, sx, sy, sz, sm, s);
-    if (n <= 4096) return run_order_small<DIM, 4>(pos, mass, n, box, keys, perm, sx, sy, sz, sm, s);
-    return run_order_small<DIM, 8>(pos, mass, n, box, keys, perm, sx, sy, sz, sm, s);
+    return run_order_small<DIM, 4>(pos, mass, n, box, keys, perm, sx, sy, sz, sm, s);
 }
 
 }  // namespace
@@ -450,7 +497,7 @@ int launch_order(const double* pos, const double* mass, int64_t n, int dim, cons
                  uint64_t* keys, int32_t* perm, double* sx, double* sy, double* sz, double* sm,
                  void* scratch, cudaStream_t s)
 {
-    static_assert(BHUT_ORDER_SMALL <= kSmallThreads * 8, "the largest block");
+    static_assert(BHUT_ORDER_SMALL <= kSmallThreads * 4, "the largest block");
     if (n <= BHUT_ORDER_SMALL)
         return dim == 3 ? order_small<3>(pos, mass, (int)n, box, keys, perm, sx, sy, sz, sm, s)
                         : order_small<2>(pos, mass, (int)n, box, keys, perm, sx, sy, sz, sm, s);
@@ -458,6 +505,94 @@ int launch_order(const double* pos, const double* mass, int64_t n, int dim, cons
     BHUT_TRY(radix_sort_pairs(keys, perm, n, dim == 3 ? 63 : 42, scratch, s));
     return sx ? launch_gather(pos, mass, perm, n, dim, sx, sy, sz, sm, s) : kOk;
 }
+
+namespace {
+
+// An odd number of passes ends in the other buffers.
+int copy_back(uint64_t* keys, int32_t* vals, const uint64_t* kin, const int32_t* vin, int64_t n,
+              cudaStream_t stream)
+{
+    if (kin == keys) return kOk;
+    BHUT_CUDA(cudaMemcpyAsync(keys, kin, sizeof(uint64_t) * (size_t)n, cudaMemcpyDeviceToDevice, stream));
+    BHUT_CUDA(cudaMemcpyAsync(vals, vin, sizeof(int32_t) * (size_t)n, cudaMemcpyDeviceToDevice, stream));
+    return kOk;
+}
+
+struct SortArgs {
+    uint64_t* keys;
+    int32_t* vals;
+    int64_t n, tiles;
+    int passes;
+    SortLayout L;
+    cudaStream_t stream;
+};
+
+// One launch a pass (sort_sums).
+int sort_with_sums(const SortArgs& a)
+{
+    constexpr int S = kSortShiftSmall, smem = (int)sizeof(ScatterSmem<1 << S>);
+    static_assert(smem <= 48 * 1024, "within the default limit");
+    const unsigned tiles = (unsigned)a.tiles;
+    const SortLayout& L = a.L;
+    k_sort_count<S><<<tiles, kSortThreads, 0, a.stream>>>(a.keys, (int)a.n, L.counts[0], L.counts[1]);
+    uint64_t *kin = a.keys, *kout = L.keys_alt;
+    int32_t *vin = a.vals, *vout = L.vals_alt;
+    for (int pass = 0; pass < a.passes; pass++) {
+        k_sort_scatter<S, true><<<tiles, kSortThreads, smem, a.stream>>>(
+            kin, vin, kout, vout, a.n, 8 * pass, L.counts[pass % 3], a.tiles,
+            pass + 1 < a.passes ? L.counts[(pass + 1) % 3] : nullptr, 8 * (pass + 1),
+            pass + 2 < a.passes ? L.counts[(pass + 2) % 3] : nullptr);
+        std::swap(kin, kout);
+        std::swap(vin, vout);
+    }
+    BHUT_CUDA(cudaGetLastError());
+    note_launches(1 + (int64_t)a.passes);
+    return copy_back(a.keys, a.vals, kin, vin, a.n, a.stream);
+}
+
+// A scan and a scatter a pass.
+template <int SHIFT>
+int sort_with_scans(const SortArgs& a)
+{
+    // the scatter's shared memory may exceed the default limit, and wants all
+    // of the unified L1/shared storage (several tiles per SM): once per device
+    const auto scatter = k_sort_scatter<SHIFT, false>;
+    constexpr int smem = (int)sizeof(ScatterSmem<1 << SHIFT>);
+    {
+        static std::atomic<bool> smem_set[64];
+        int dev = 0;
+        BHUT_CUDA(cudaGetDevice(&dev));
+        if (dev < 0 || dev >= 64 || !smem_set[dev].load(std::memory_order_acquire)) {
+            BHUT_CUDA(cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           smem));
+            BHUT_CUDA(cudaFuncSetAttribute(scatter, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                           (int)cudaSharedmemCarveoutMaxShared));
+            if (dev >= 0 && dev < 64) smem_set[dev].store(true, std::memory_order_release);
+        }
+    }
+    const unsigned tiles = (unsigned)a.tiles;
+    const SortLayout& L = a.L;
+    BHUT_CUDA(cudaMemsetAsync(L.totals, 0, sizeof(uint32_t) * 256 * kSortPassesMax, a.stream));
+    k_sort_prep<SHIFT><<<tiles, kSortThreads, 0, a.stream>>>(a.keys, a.n, a.passes, L.counts[0],
+                                                             a.tiles, L.totals);
+    uint64_t *kin = a.keys, *kout = L.keys_alt;
+    int32_t *vin = a.vals, *vout = L.vals_alt;
+    for (int pass = 0; pass < a.passes; pass++) {
+        const bool last = pass + 1 == a.passes;
+        uint32_t* cur = L.counts[pass & 1];
+        uint32_t* nxt = last ? nullptr : L.counts[(pass + 1) & 1];
+        k_sort_scan<<<256, kScanThreads, 0, a.stream>>>(cur, a.tiles, L.totals + 256 * pass, nxt);
+        scatter<<<tiles, kSortThreads, smem, a.stream>>>(
+            kin, vin, kout, vout, a.n, 8 * pass, cur, a.tiles, nxt, 8 * (pass + 1), nullptr);
+        std::swap(kin, kout);
+        std::swap(vin, vout);
+    }
+    BHUT_CUDA(cudaGetLastError());
+    note_launches(1 + 2ll * a.passes);
+    return copy_back(a.keys, a.vals, kin, vin, a.n, a.stream);
+}
+
+}  // namespace
 
 int radix_sort_pairs(uint64_t* keys, int32_t* vals, int64_t n, int bits, void* scratch,
                      cudaStream_t stream)
@@ -469,48 +604,10 @@ int radix_sort_pairs(uint64_t* keys, int32_t* vals, int64_t n, int bits, void* s
         set_error("radix sort: %d key bits out of range", bits);
         return kInvalid;
     }
-    // the scatter's shared memory exceeds the default limit: raise it once
-    // per device
-    {
-        static std::atomic<bool> smem_set[64];
-        int dev = 0;
-        BHUT_CUDA(cudaGetDevice(&dev));
-        if (dev < 0 || dev >= 64 || !smem_set[dev].load(std::memory_order_acquire)) {
-            BHUT_CUDA(cudaFuncSetAttribute(k_sort_scatter,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)sizeof(ScatterSmem)));
-            // all of the unified L1/shared storage as shared memory (several
-            // tiles per SM)
-            BHUT_CUDA(cudaFuncSetAttribute(k_sort_scatter,
-                                           cudaFuncAttributePreferredSharedMemoryCarveout,
-                                           (int)cudaSharedmemCarveoutMaxShared));
-            if (dev >= 0 && dev < 64) smem_set[dev].store(true, std::memory_order_release);
-        }
-    }
-    const int64_t tiles = sort_tiles(n);
-    const SortLayout L = carve(scratch, n);
-    BHUT_CUDA(cudaMemsetAsync(L.totals, 0, sizeof(uint32_t) * 256 * kSortPassesMax, stream));
-    k_sort_prep<<<(unsigned)tiles, kSortThreads, 0, stream>>>(keys, n, passes, L.counts[0], tiles,
-                                                              L.totals);
-    uint64_t *kin = keys, *kout = L.keys_alt;
-    int32_t *vin = vals, *vout = L.vals_alt;
-    for (int pass = 0; pass < passes; pass++) {
-        const bool last = pass + 1 == passes;
-        uint32_t* cur = L.counts[pass & 1];
-        uint32_t* nxt = last ? nullptr : L.counts[(pass + 1) & 1];
-        k_sort_scan<<<256, kScanThreads, 0, stream>>>(cur, tiles, L.totals + 256 * pass, nxt);
-        k_sort_scatter<<<(unsigned)tiles, kSortThreads, sizeof(ScatterSmem), stream>>>(
-            kin, vin, kout, vout, n, 8 * pass, cur, tiles, nxt, 8 * (pass + 1));
-        uint64_t* tk = kin; kin = kout; kout = tk;
-        int32_t* tv = vin; vin = vout; vout = tv;
-    }
-    BHUT_CUDA(cudaGetLastError());
-    note_launches(1 + 2ll * passes);
-    if (kin != keys) {
-        BHUT_CUDA(cudaMemcpyAsync(keys, kin, sizeof(uint64_t) * (size_t)n, cudaMemcpyDeviceToDevice, stream));
-        BHUT_CUDA(cudaMemcpyAsync(vals, vin, sizeof(int32_t) * (size_t)n, cudaMemcpyDeviceToDevice, stream));
-    }
-    return kOk;
+    const SortArgs a{keys, vals, n, sort_tiles(n), passes, carve(scratch, n), stream};
+    static_assert(BHUT_SORT_SUMS_MAX <= BHUT_SORT_SMALL_TILE_MAX, "sums add up small tiles");
+    if (sort_sums(n)) return sort_with_sums(a);
+    return sort_small_tiles(n) ? sort_with_scans<kSortShiftSmall>(a) : sort_with_scans<kSortShift>(a);
 }
 
 }  // namespace bhut
