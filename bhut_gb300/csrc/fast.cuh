@@ -90,6 +90,14 @@ static __device__ __forceinline__ void split_grid(double u, bool fine, float& h,
     l = __double2float_rn(r);
 }
 
+// Sum of a 32-bit count over the warp (two reductions, so that it cannot wrap).
+static __device__ __forceinline__ unsigned long long warp_sum(unsigned v)
+{
+    const unsigned lo = __reduce_add_sync(0xffffffffu, v & 0xffffu);
+    const unsigned hi = __reduce_add_sync(0xffffffffu, v >> 16);
+    return lo + ((unsigned long long)hi << 16);
+}
+
 // A node's header flag: 0 without mass (skipped), 1, or 3 when its centre of
 // mass lies outside the box (masses of both signs): its coordinates are not
 // on the grid and its monopole is taken in FP64.

@@ -488,18 +488,22 @@ k_traverse_fast(TreeDev t, FastTree ft, FastArgs a, int levels, double* __restri
                                                   Tl, band_abs, ah, al, a64, stack, stage, cnt,
                                                   overflow, levels, path);
         if (overflow && lane == 0) atomicOr(a.err, kErrStackOverflow);
-        if (a.stats) {
+        // a share of a split may have had nothing to do: then no counts, and
+        // zero sums without the scaling in FP64
+        const bool busy = !SPLIT || __any_sync(FULL, (cnt[0] | cnt[1] | cnt[2]) != 0);
+        if (a.stats && busy) {
 #pragma unroll
             for (int k = 0; k < 5; k++) {
-                unsigned long long v = cnt[k];   // per-target counts fit 32 bits
-                for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(FULL, v, o);
+                const unsigned long long v = warp_sum(cnt[k]);
                 if (lane == 0 && v) atomicAdd(&a.stats[k], v);
             }
         }
 #pragma unroll
         for (int k = 0; k < DIM; k++) {
-            const double v = __dadd_rn(
-                __dmul_rn(__dadd_rn((double)ah[k], (double)al[k]), conv), __dmul_rn(a64[k], a.G));
+            double v = 0.0;
+            if (busy)
+                v = __dadd_rn(__dmul_rn(__dadd_rn((double)ah[k], (double)al[k]), conv),
+                              __dmul_rn(a64[k], a.G));
             if (SPLIT) sum[SPLIT ? w : 0][SPLIT ? k : 0][lane] = v;
             else if (valid) a.out[(a.out_idx ? a.out_idx[i] : i) * DIM + k] = v;
         }
@@ -517,16 +521,32 @@ k_traverse_fast(TreeDev t, FastTree ft, FastArgs a, int levels, double* __restri
     }
 }
 
-__global__ void k_split_sum(const double* __restrict__ partial, int64_t nt, int dim, int shares,
-                            const int32_t* __restrict__ out_idx, double* __restrict__ out)
+// kSumRows threads per output, each with every kSumRows-th share: one thread
+// for all of 256 shares took 32 us for 2,000 targets.
+constexpr int kSumRows = 8;
+__global__ void __launch_bounds__(kWarp * kSumRows)
+k_split_sum(const double* __restrict__ partial, int64_t nt, int dim, int shares,
+            const int32_t* __restrict__ out_idx, double* __restrict__ out)
 {
-    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nt * dim;
-         j += (int64_t)gridDim.x * blockDim.x) {
-        double v = partial[j];
+    __shared__ double part[kSumRows][kWarp];
+    for (int64_t base = blockIdx.x * (int64_t)kWarp; base < nt * dim;
+         base += (int64_t)gridDim.x * kWarp) {
+        const int64_t j = base + threadIdx.x;
+        double v = 0.0;
+        if (j < nt * dim) {
 #pragma unroll 8
-        for (int y = 1; y < shares; y++) v = __dadd_rn(v, partial[(int64_t)y * nt * dim + j]);
-        const int64_t i = j / dim;
-        out[(out_idx ? out_idx[i] : i) * dim + j % dim] = v;
+            for (int y = threadIdx.y; y < shares; y += kSumRows)
+                v = __dadd_rn(v, partial[(int64_t)y * nt * dim + j]);
+        }
+        part[threadIdx.y][threadIdx.x] = v;
+        __syncthreads();
+        if (threadIdx.y == 0 && j < nt * dim) {
+            for (int y = 1; y < min(kSumRows, shares); y++)
+                v = __dadd_rn(v, part[y][threadIdx.x]);
+            const int64_t i = j / dim;
+            out[(out_idx ? out_idx[i] : i) * dim + j % dim] = v;
+        }
+        __syncthreads();
     }
 }
 
@@ -583,8 +603,7 @@ k_traverse_fp32(TreeDev t, FastTree ft, FastArgs a)
         if (a.stats) {
 #pragma unroll
             for (int k = 0; k < 3; k++) {
-                unsigned long long v = cnt[k];
-                for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(FULL, v, o);
+                const unsigned long long v = warp_sum(cnt[k]);
                 if (lane == 0 && v) atomicAdd(&a.stats[k], v);
             }
         }
@@ -624,7 +643,8 @@ int launch_fast_targets(const double* tx, const double* ty, const double* tz, in
 int launch_split_sum(const double* partial, int64_t nt, int dim, int shares,
                      const int32_t* out_idx, double* out, cudaStream_t s)
 {
-    k_split_sum<<<grid_for(nt * dim, 128), 128, 0, s>>>(partial, nt, dim, shares, out_idx, out);
+    k_split_sum<<<grid_for(nt * dim, kWarp), dim3(kWarp, kSumRows), 0, s>>>(partial, nt, dim, shares,
+                                                                           out_idx, out);
     BHUT_CUDA(cudaGetLastError());
     note_launches(1);
     return kOk;
