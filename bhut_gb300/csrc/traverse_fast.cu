@@ -39,19 +39,29 @@ constexpr int kFastWarps = 4;
 constexpr int kFastThreads = kFastWarps * kWarp;
 constexpr int kSplitMaxLevels = 10;
 // Tuning (overridable at build time): resident blocks per SM of the fast form
-// (4 / 5 / 6 cap the registers at 128 / 96 / 80).  Self solves with softening,
-// 5 / 6 / 7 blocks: 1M Plummer 134.6 / 131.1 / 135.6 ms, 200k 21.8 / 22.0 /
-// 23.4 ms, but 100k, about one wave, 9.8 / 9.9 / 10.3 and a 100k uniform cube
-// 4.31 / 4.67 / 4.95 ms: so 6 from a few waves on and 5 below.  Without
-// softening (the checks cost registers) 3 / 4 / 5 / 6: 250k 32.3 / 30.4 / 31.0
-// / 32.4 ms, 100k cube 5.2 / 5.0 / 4.6 / - ms.  Split, 4 / 5 / 6: 250k targets
-// of 1M 28.7 / 27.1 / 26.0 ms, 2-D 60k self 1.28 / 1.18 / 1.09; without
-// softening 30k cube 1.12 / 1.07 / 1.10.
+// (they cap the registers: 5 / 6 / 7 / 8 at 96 / 80 / 72 / 64).
+//   3-D, softened, not split: 5 / 6 / 7: 1M Plummer 134.6 / 131.1 / 135.6 ms,
+//     200k 21.8 / 22.0 / 23.4, but about one wave, 100k, 9.8 / 9.9 / 10.3 and
+//     100k uniform cube 4.31 / 4.67 / 4.95: MORE from a few waves on.
+//   3-D, unsoftened (the checks cost registers): 3 / 4 / 5 / 6: 250k 32.3 /
+//     30.4 / 31.0 / 32.4 ms, 100k cube 5.2 / 5.0 / 4.6 / -.
+//   3-D, split: 4 / 5 / 6 / 7: 250k targets of 1M 28.7 / 27.1 / 26.0 / 25.9 ms,
+//     2,000 - / - / 0.89 / 0.91; unsoftened 30k cube 1.12 / 1.07 / 1.10 / -.
+//   2-D, softened: 6 / 7 / 8 / 9: 1M 19.7 / 19.5 / 19.2 / 20.0 ms, 100k targets
+//     of 1M 4.62 / 4.45 / 4.32 / 4.37, 60k split 1.03 / 0.99 / 0.96 / -; 200k
+//     (two waves) 5 / 6: 3.31 / 3.45.
+//   2-D, unsoftened: 5 / 6 / 7: 300k 5.08 / 5.02 / 4.88 ms, 60k 1.22 / 1.15 / 1.11.
 #ifndef BHUT_FAST_BLOCKS
 #define BHUT_FAST_BLOCKS 5
 #endif
 #ifndef BHUT_FAST_BLOCKS_MORE
 #define BHUT_FAST_BLOCKS_MORE 6
+#endif
+#ifndef BHUT_FAST_BLOCKS_2D
+#define BHUT_FAST_BLOCKS_2D 8
+#endif
+#ifndef BHUT_FAST_BLOCKS_2D_CHECK
+#define BHUT_FAST_BLOCKS_2D_CHECK 7
 #endif
 // Split traversals (split_levels): split while fewer warps than this walk
 // and their subtrees hold more nodes than that.  Swept on GB300:
@@ -693,20 +703,21 @@ int launch_traverse_fast(const TreeDev& t, const FastTree& ft, const float4* th,
     } else {
         const bool soft = a.e2h >= 2.0f * kTinyR;
         constexpr int B = BHUT_FAST_BLOCKS, MORE = BHUT_FAST_BLOCKS_MORE;
+        constexpr int B2 = BHUT_FAST_BLOCKS_2D, C2 = BHUT_FAST_BLOCKS_2D_CHECK;
         const bool d3 = t.dim == 3;
         const int shares = levels > 0 ? (1 << levels) / kFastWarps : 0;
         const unsigned g = shares ? (unsigned)warps * (unsigned)shares : grid;
         const auto kernel =
-            shares                     ? (soft ? (d3 ? k_traverse_fast<3, true, true, MORE>
-                                                     : k_traverse_fast<2, true, true, MORE>)
-                                               : (d3 ? k_traverse_fast<3, false, true, B>
-                                                     : k_traverse_fast<2, false, true, B>))
-            : !soft                    ? (d3 ? k_traverse_fast<3, false, false, B>
-                                             : k_traverse_fast<2, false, false, B>)
-            : warps >= 3 * kWaveWarps  ? (d3 ? k_traverse_fast<3, true, false, MORE>
-                                             : k_traverse_fast<2, true, false, MORE>)
-                                       : (d3 ? k_traverse_fast<3, true, false, B>
-                                             : k_traverse_fast<2, true, false, B>);
+            shares                    ? (soft ? (d3 ? k_traverse_fast<3, true, true, MORE>
+                                                    : k_traverse_fast<2, true, true, B2>)
+                                              : (d3 ? k_traverse_fast<3, false, true, B>
+                                                    : k_traverse_fast<2, false, true, C2>))
+            : !soft                   ? (d3 ? k_traverse_fast<3, false, false, B>
+                                            : k_traverse_fast<2, false, false, C2>)
+            : warps >= 3 * kWaveWarps ? (d3 ? k_traverse_fast<3, true, false, MORE>
+                                            : k_traverse_fast<2, true, false, B2>)
+                                      : (d3 ? k_traverse_fast<3, true, false, B>
+                                            : k_traverse_fast<2, true, false, B>);
         kernel<<<g, kFastThreads, 0, s>>>(t, ft, a, levels, partial);
         if (shares > 1) BHUT_TRY(launch_split_sum(partial, nt, t.dim, shares, out_idx, out, s));
     }
