@@ -414,9 +414,9 @@ __global__ void k_seg_ff_particles(TreeDev t, bool fine, const int32_t* __restri
          i += (int64_t)gridDim.x * blockDim.x) {
         const FastFrame& f = frames[sys_of[i]];
         float4 h, l;
-        split_grid(__dmul_rn(__dsub_rn(t.sx[i], f.c[0]), f.s), fine, h.x, l.x);
-        split_grid(__dmul_rn(__dsub_rn(t.sy[i], f.c[1]), f.s), fine, h.y, l.y);
-        if (dim == 3) split_grid(__dmul_rn(__dsub_rn(t.sz[i], f.c[2]), f.s), fine, h.z, l.z);
+        split_grid(t.sx[i], f.c[0], f.s, fine, h.x, l.x);
+        split_grid(t.sy[i], f.c[1], f.s, fine, h.y, l.y);
+        if (dim == 3) split_grid(t.sz[i], f.c[2], f.s, fine, h.z, l.z);
         else h.z = l.z = 0.0f;
         if (f.unit) { h.w = 1.0f; l.w = 0.0f; }   // every mass is m0: exactly 1 in units of m0
         else split_plain(__dmul_rn(t.sm[i], f.ms), h.w, l.w);

@@ -114,9 +114,9 @@ __global__ void k_ff_particles(const double* __restrict__ sx, const double* __re
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
         float4 h, l;
-        split_grid(__dmul_rn(__dsub_rn(sx[i], f.c[0]), f.s), fine, h.x, l.x);
-        split_grid(__dmul_rn(__dsub_rn(sy[i], f.c[1]), f.s), fine, h.y, l.y);
-        if (dim == 3) split_grid(__dmul_rn(__dsub_rn(sz[i], f.c[2]), f.s), fine, h.z, l.z);
+        split_grid(sx[i], f.c[0], f.s, fine, h.x, l.x);
+        split_grid(sy[i], f.c[1], f.s, fine, h.y, l.y);
+        if (dim == 3) split_grid(sz[i], f.c[2], f.s, fine, h.z, l.z);
         else h.z = l.z = 0.0f;
         if (f.unit) { h.w = 1.0f; l.w = 0.0f; }   // every mass is m0: exactly 1 in units of m0
         else split_plain(__dmul_rn(sm[i], f.ms), h.w, l.w);
@@ -150,8 +150,13 @@ __global__ void k_ff_targets(const double* __restrict__ tx, const double* __rest
         bool inside = amax <= 1.0;
         float hh[3], ll[3];
         for (int d = 0; d < 3; d++) {
-            if (inside) split_grid(u[d], fine, hh[d], ll[d]);
-            else split_plain(u[d], hh[d], ll[d]);
+            if (inside) {
+                const float2 p = split_grid_fp64(u[d], fine);
+                hh[d] = p.x;
+                ll[d] = p.y;
+            } else {
+                split_plain(u[d], hh[d], ll[d]);
+            }
         }
         th[i] = make_float4(hh[0], hh[1], hh[2], inside ? 0.0f : 1.0f);
         tl[i] = make_float4(ll[0], ll[1], ll[2], __double2float_ru(amax));
