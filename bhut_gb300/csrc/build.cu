@@ -212,8 +212,11 @@ k_bbox(const double* __restrict__ pos, const double* __restrict__ mass, int64_t 
 // ---------------------------------------------------------------------------
 // K2: Morton keys (input order) and the identity payload for the sort.
 // ---------------------------------------------------------------------------
+// (48 and 40 registers: the blocks that those allow; with 52 and 42, 4M points
+// took 67 and 50 us instead of 62 and 42.)
 template <int dim>
-__global__ void k_morton(const double* __restrict__ pos, int64_t n,
+__global__ void __launch_bounds__(256, dim == 3 ? 5 : 6)
+k_morton(const double* __restrict__ pos, int64_t n,
                          const double* __restrict__ box, uint64_t* __restrict__ keys,
                          int32_t* __restrict__ idx)
 {
@@ -525,18 +528,109 @@ __device__ __forceinline__ void hand_over(int32_t node, int32_t* frontier, unsig
     else atomicOr(err, kErrBadNode);
 }
 
-// Node operations of a bottom-up pass: the moments (build and refit modes;
-// four lanes to a node) or the quadrupoles (one).
+// One lane to a node, for trees that keep the FP64 pipe busy: the lanes of a
+// warp then hold 32 nodes, and an axis' addition is one instruction for all of
+// them (four lanes to a node: for eight).  Same operations and order.
 template <int DIM>
+__device__ void put_node_solo(int32_t id, bool refit, const uint64_t* klo, const uint64_t* khi,
+                              const double* acc, double total, const NodeOut& o)
+{
+    if (!refit) {
+        double ext = 0.0;
+        for (int d = 0; d < DIM; d++) {
+            const double lo = __longlong_as_double((long long)ord_inv(klo[d]));
+            const double hi = __longlong_as_double((long long)ord_inv(khi[d]));
+            o.lo[3 * id + d] = lo;
+            o.hi[3 * id + d] = hi;
+            o.center[DIM * id + d] = __dmul_rn(__dadd_rn(lo, hi), 0.5);
+            const double e = __dsub_rn(hi, lo);
+            if (d == 0 || __double_as_longlong(e) > __double_as_longlong(ext)) ext = e;
+        }
+        const double half = __dmul_rn(ext, 0.5);
+        o.half[id] = half;
+        o.size[id] = __dmul_rn(2.0, half);
+    }
+    double com[3] = {0.0, 0.0, 0.0};
+    for (int d = 0; d < DIM; d++) com[d] = total > 0 ? __ddiv_rn(acc[d], total) : o.center[DIM * id + d];
+    o.cm[id] = NodeCM{com[0], com[1], com[2], total};
+}
+
+template <int DIM>
+__device__ void leaf_solo(int32_t id, bool refit, const TreeDev& t, const int32_t* __restrict__ start,
+                          const int32_t* __restrict__ count, const NodeOut& o)
+{
+    const int64_t s = start[id], c = count[id];
+    auto ld = [&](int64_t i) { return t.sm[s + i]; };
+    const double total = __dadd_rn(0.0, pairwise_sum(ld, c));
+    const double* axes[3] = {t.sx, t.sy, t.sz};
+    uint64_t klo[3] = {~0ull, ~0ull, ~0ull}, khi[3] = {0ull, 0ull, 0ull};
+    double acc[3] = {0.0, 0.0, 0.0};
+#pragma unroll 4
+    for (int64_t i = s; i < s + c; i++) {
+        const double mi = t.sm[i];
+#pragma unroll
+        for (int d = 0; d < DIM; d++) {
+            const double v = axes[d][i];
+            const uint64_t k = ord_key((uint64_t)__double_as_longlong(v));
+            klo[d] = k < klo[d] ? k : klo[d];
+            khi[d] = k > khi[d] ? k : khi[d];
+            acc[d] = __dadd_rn(acc[d], __dmul_rn(mi, v));
+        }
+    }
+    put_node_solo<DIM>(id, refit, klo, khi, acc, total, o);
+}
+
+template <int DIM>
+__device__ void internal_solo(int32_t id, int32_t fc, bool refit, const NodeOut& o)
+{
+    double a[4], b[4], acc[3] = {0.0, 0.0, 0.0};
+    for (int k = 0; k < 4; k++) {
+        a[k] = __ldcg(reinterpret_cast<const double*>(&o.cm[fc]) + k);
+        b[k] = __ldcg(reinterpret_cast<const double*>(&o.cm[fc + 1]) + k);
+    }
+    uint64_t klo[3] = {0, 0, 0}, khi[3] = {0, 0, 0};
+    if (!refit) {
+        for (int d = 0; d < DIM; d++) {
+            const uint64_t l0 = ord_key((uint64_t)__double_as_longlong(__ldcg(&o.lo[3 * fc + d])));
+            const uint64_t l1 = ord_key((uint64_t)__double_as_longlong(__ldcg(&o.lo[3 * (fc + 1) + d])));
+            const uint64_t h0 = ord_key((uint64_t)__double_as_longlong(__ldcg(&o.hi[3 * fc + d])));
+            const uint64_t h1 = ord_key((uint64_t)__double_as_longlong(__ldcg(&o.hi[3 * (fc + 1) + d])));
+            klo[d] = l1 < l0 ? l1 : l0;
+            khi[d] = h1 > h0 ? h1 : h0;
+        }
+    }
+    double total = refit ? 0.0 : __dadd_rn(0.0, __dadd_rn(a[3], b[3]));
+    if (!refit || a[3] > 0) {
+        if (refit) total = __dadd_rn(total, a[3]);
+        for (int d = 0; d < DIM; d++) acc[d] = __dadd_rn(acc[d], __dmul_rn(a[3], a[d]));
+    }
+    if (!refit || b[3] > 0) {
+        if (refit) total = __dadd_rn(total, b[3]);
+        for (int d = 0; d < DIM; d++) acc[d] = __dadd_rn(acc[d], __dmul_rn(b[3], b[d]));
+    }
+    put_node_solo<DIM>(id, refit, klo, khi, acc, total, o);
+}
+
+// Node operations of a bottom-up pass: the moments (build and refit modes;
+// four lanes to a node or one) or the quadrupoles (one).
+template <int DIM, int LANES>
 struct MomentOps {
-    static constexpr int kLanes = 4;
+    static constexpr int kLanes = LANES;
     TreeDev t;
     NodeOut o;
     bool refit;
     const int32_t* start;
     const int32_t* count;
-    __device__ void leaf(int32_t id) const { leaf_node<DIM>(Quad(), id, refit, t, start, count, o); }
-    __device__ void internal(int32_t p, int32_t fc) const { internal_node<DIM>(Quad(), p, fc, refit, o); }
+    __device__ void leaf(int32_t id) const
+    {
+        if (LANES == 4) leaf_node<DIM>(Quad(), id, refit, t, start, count, o);
+        else leaf_solo<DIM>(id, refit, t, start, count, o);
+    }
+    __device__ void internal(int32_t p, int32_t fc) const
+    {
+        if (LANES == 4) internal_node<DIM>(Quad(), p, fc, refit, o);
+        else internal_solo<DIM>(p, fc, refit, o);
+    }
 };
 
 template <class Ops>
@@ -686,7 +780,8 @@ int launch_climb(const Ops& ops, const TreeDev& t, const int32_t* leaf_list, int
         BHUT_CUDA(cudaMemsetAsync(frontier_count, 0, sizeof(unsigned), s));
     }
     const unsigned groups = (unsigned)((entries + kBuThreads - 1) / kBuThreads);
-    k_bottom_up<Ops><<<groups < 152u * 8u ? groups : 152u * 8u, kBuThreads * Ops::kLanes, 0, s>>>(
+    constexpr unsigned cap = 152u * 2048u / (kBuThreads * Ops::kLanes);   // all resident
+    k_bottom_up<Ops><<<groups < cap ? groups : cap, kBuThreads * Ops::kLanes, 0, s>>>(
         ops, t, leaf_list, entries, first_child, start, count, parent, frontier,
         frontier_count, err);
     if (!one)
@@ -857,19 +952,35 @@ int launch_topology(const TopoTables& tt, int32_t* first_child, int32_t* start, 
     return kOk;
 }
 
+// Leaf-list entries up to which four lanes work on a node (3-D; 2-D, where a
+// fourth lane has nothing to add): below, a level's dependent FP64 additions
+// are the time, above the FP64 pipe.  Rebuild / refit, us, by four lanes / one:
+//   3-D, leaf 32: 500k 296 / 153 and 298 / 156, 1M 378 / 176 and 385 / 186,
+//                 2M 592 / 261 and 562 / 225, 4M 1,062 / 462 and 950 / 370;
+//   2-D, leaf 32: 250k 214 / 146 and 205 / 132, 1M 325 / 172 and 309 / 157,
+//                 2M 496 / 246 and 436 / 195.
+#ifndef BHUT_QUAD_ENTRIES
+#define BHUT_QUAD_ENTRIES 40000
+#endif
+#ifndef BHUT_QUAD_ENTRIES_2D
+#define BHUT_QUAD_ENTRIES_2D 6000
+#endif
 int launch_bottom_up(const TreeDev& t, const int32_t* leaf_list, int64_t entries,
                      const int32_t* first_child, const int32_t* start, const int32_t* count,
                      const int32_t* parent, unsigned* arrive, NodeOut o, bool refit,
                      int32_t* frontier, unsigned* frontier_count, unsigned* err, bool ordered,
                      cudaStream_t s)
 {
+    const auto climb = [&](auto ops) {
+        return launch_climb(ops, t, leaf_list, entries, first_child, start, count, parent, arrive,
+                            frontier, frontier_count, err, ordered, s);
+    };
+    const bool quad = entries <= (t.dim == 3 ? BHUT_QUAD_ENTRIES : BHUT_QUAD_ENTRIES_2D);
     if (t.dim == 3)
-        return launch_climb(MomentOps<3>{t, o, refit, start, count}, t, leaf_list,
-                            entries, first_child, start, count, parent, arrive, frontier,
-                            frontier_count, err, ordered, s);
-    return launch_climb(MomentOps<2>{t, o, refit, start, count}, t, leaf_list,
-                        entries, first_child, start, count, parent, arrive, frontier,
-                        frontier_count, err, ordered, s);
+        return quad ? climb(MomentOps<3, 4>{t, o, refit, start, count})
+                    : climb(MomentOps<3, 1>{t, o, refit, start, count});
+    return quad ? climb(MomentOps<2, 4>{t, o, refit, start, count})
+                : climb(MomentOps<2, 1>{t, o, refit, start, count});
 }
 
 int launch_outside_root(const double* pos, int64_t n, int dim, const double* center0,

@@ -48,7 +48,7 @@ def test_batch_of_ragged_systems_equals_single_trees(sizes):
 @pytest.mark.parametrize("dim", [3, 2])
 @pytest.mark.parametrize("n", [1, 2, 31, 1023, 1024, 1025, 2049, 4097, 8191, 8192, 8193])
 def test_small_orders_equal_the_oracle(oracle_mod, n, dim):
-    """Points ordered by one block (up to 8,192) and by passes: keys with many
+    """Points ordered by one block (the smallest) and by passes: keys with many
     ties (a coarse lattice, and all points in one) and distinct ones."""
     rng = np.random.default_rng(n)
     for pos in (rng.standard_normal((n, dim)), rng.integers(0, 4, (n, dim)).astype(float),
