@@ -264,19 +264,19 @@ def measure_gemm_peak(torch, dtype) -> float:
     return 2.0 * n ** 3 / best / 1e12
 
 
-# Instructions of one float-float pair (or monopole) term of the fast form,
-# counted from bhut_gb300/csrc/fast.cuh (pair_ff_soft, 3-D, target inside
-# the box, softening bounding R from below as in this workload): exact
-# displacement and squares 21, cross term and r^2 low part 4, three
-# non-negative FastTwoSums into r^2 21 (6 of them min/max on the ALU pipe),
-# MUFU rsqrt 1, refinement and cube 10, three float-float products and
-# magnitude-ordered two-sum accumulations 36 (9 compare/select on the ALU
-# pipe) -> 93 for a leaf pair in the unit-mass frame (every particle the same
-# mass), 97 with the mass product (monopoles, or unequal masses).  Of these,
-# 77 / 81 run on the FP32 (FMA) pipe.  The fp32 form's counts live in
-# bhut_gb300.reports.
-FF_INSTR_UNIT_PAIR, FF_INSTR_MASS_PAIR = 93, 97
-FF_FMA_UNIT_PAIR, FF_FMA_MASS_PAIR = 77, 81
+# Operations of one float-float pair (or monopole) term of the fast form,
+# counted from bhut_gb300/csrc/fast.cuh (3-D, target inside the box, softening
+# bounding R from below as in this workload).
+#  * A pair of a distant leaf (far_pairs, most of them; two pairs go through
+#    each f32x2 instruction): displacement 6, squares and cross terms into a
+#    biased r^2 18, rsqrt, refinement and cube 11, forces into biased sums 18
+#    -> 53 on the FP32 (FMA) pipe, 3 on the ALU pipe and a MUFU rsqrt; the mass
+#    product (unequal masses) adds 4 and 1.  A pair of a near leaf
+#    (pair_ff_soft) takes 77 + 15 + 1 and is counted as a distant one here.
+#  * A monopole (pair_ff_soft with the mass product): 81 + 15 + 1.
+# The fp32 form's counts live in bhut_gb300.reports.
+FF_INSTR_UNIT_PAIR, FF_INSTR_MASS_PAIR, FF_INSTR_MONOPOLE = 57, 62, 97
+FF_FMA_UNIT_PAIR, FF_FMA_MASS_PAIR, FF_FMA_MONOPOLE = 53, 57, 81
 ARITH = {"exact": "IEEE FP64",
          "fast": "float-float on the FP32 pipe (about 48-bit significand); FP64 bounding box, "
                  "keys, centres of mass and rare fallbacks",
@@ -392,12 +392,12 @@ def run_ours(args, ws, rank, local):
             unit = bool(m[0] > 0 and np.all(m == m[0]))
             ipair = FF_INSTR_UNIT_PAIR if unit else FF_INSTR_MASS_PAIR
             fpair = FF_FMA_UNIT_PAIR if unit else FF_FMA_MASS_PAIR
-            ops = ipair * p2p + FF_INSTR_MASS_PAIR * m2p
-            fma_ops = fpair * p2p + FF_FMA_MASS_PAIR * m2p
-            rule = (f"{ipair} pair-term instructions per leaf pair{' (unit-mass frame)' if unit else ''}"
-                    f", {FF_INSTR_MASS_PAIR} per monopole (FP32 + ALU + MUFU; one warp "
-                    "instruction per clock per SM sub-partition is both the issue limit and "
-                    "the FFMA rate below)")
+            ops = ipair * p2p + FF_INSTR_MONOPOLE * m2p
+            fma_ops = fpair * p2p + FF_FMA_MONOPOLE * m2p
+            rule = (f"{ipair} operations per leaf pair{' (unit-mass frame)' if unit else ''}"
+                    f", {FF_INSTR_MONOPOLE} per monopole (FP32 + ALU + MUFU; leaf pairs counted "
+                    "as distant ones, whose FP32 operations go two to an f32x2 instruction at "
+                    "the pipe's FFMA rate below)")
         else:
             from bhut_gb300 import reports
             ops = reports.fp32_ops(p2p, m2p, "mono")
@@ -413,7 +413,7 @@ def run_ours(args, ws, rank, local):
             "kernel": "k_traverse_fast" if args.form == "fast" else "k_traverse_fp32",
             "achieved": achieved32,
             "peak": fma_rate,
-            "unit": "T instr/s" if args.form == "fast" else "T FP32-pipe ops/s",
+            "unit": "T ops/s" if args.form == "fast" else "T FP32-pipe ops/s",
             "frac": achieved32 / fma_rate,
             "traffic": traffic,
             "peak_source": "independent FP32 FMA chains on every SM, measured in this run "
@@ -423,7 +423,7 @@ def run_ours(args, ws, rank, local):
             "work_per_launch": ops,
             "work_rule": f"{rule} x evaluations counted by the kernel",
             **({"fp32_pipe_frac": fma_ops / trav_s / 1e12 / fma_rate,
-                "fp32_pipe_rule": f"{fpair} FP32-pipe ops per leaf pair, {FF_FMA_MASS_PAIR} per "
+                "fp32_pipe_rule": f"{fpair} FP32-pipe ops per leaf pair, {FF_FMA_MONOPOLE} per "
                                   "monopole, against the same FFMA rate"}
                if args.form == "fast" else {}),
             "fp64_equivalent": {"achieved": achieved64, "peak": peak64, "unit": "TFLOP/s",

@@ -788,7 +788,6 @@ void launch_batch_traverse(int stk, cudaStream_t s, const BatchDev& bd, const Ba
             <<<persistent_grid<DIM, FP32, TPW, 0>(), kBatchThreads, 0, s>>>(bd, a);
 }
 
-inline size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
 }  // namespace
 

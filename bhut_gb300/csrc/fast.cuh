@@ -381,8 +381,8 @@ static __device__ __forceinline__ int nth_set_bit(unsigned m, int r)
 //   * the leaf's force sums start at +-B, B a power of two above twice any
 //     term plus what the terms can take off it, on the side of the box
 //     (terms of the other sign come from |d_k| <= h_k - |g_k| only); B comes
-//     off exactly after the leaf.  6 operations per component instead of 9 and three of the
-//     ALU pipe;
+//     off exactly after the leaf.  6 operations per component instead of 9 and
+//     three of the ALU pipe;
 //   * the displacement stays (d, l) without renormalisation: |l| <= 2^-23,
 //     and the products with l are rounded once at 2^-24 of themselves, i.e.
 //     2^-47 / D of the pair -- the error that the coordinates have anyway;
@@ -853,30 +853,6 @@ __device__ __forceinline__ void pair_f32(const float* Th, const float* Tl, float
 }
 
 
-// FP32 pair term added to a plain FP32 partial sum p (no compensation): the
-// leaf loop sums at most 32 such terms and then adds the partial to the
-// Kahan-compensated per-target accumulator with kahan_add_f32 (blocked
-// Kahan summation).  Same displacement, r^2 and force as pair_f32.
-// CHECK = false: the caller guarantees e2 >= 2^-126; r^2 is an FMA chain of
-// non-negative terms started at e2, so r^2 >= e2 and the test is compiled out
-// (same result bit for bit).
-template <int DIM, bool CHECK = true>
-__device__ __forceinline__ void pair_f32_partial(const float* Th, const float* Tl, float4 sh,
-                                                 float4 sl, float e2, float* p)
-{
-    const float d0 = __fadd_rn(__fsub_rn(sh.x, Th[0]), __fsub_rn(sl.x, Tl[0]));
-    const float d1 = __fadd_rn(__fsub_rn(sh.y, Th[1]), __fsub_rn(sl.y, Tl[1]));
-    const float d2 = DIM == 3 ? __fadd_rn(__fsub_rn(sh.z, Th[2]), __fsub_rn(sl.z, Tl[2])) : 0.0f;
-    float r2 = fmaf(d1, d1, fmaf(d0, d0, e2));
-    if (DIM == 3) r2 = fmaf(d2, d2, r2);
-    const bool ok = !CHECK || r2 >= 0x1p-126f;
-    const float ri = rsqrt_mufu(ok ? r2 : 1.0f);
-    const float f = ok ? sh.w * (ri * ri * ri) : 0.0f;
-    p[0] = fmaf(f, d0, p[0]);
-    p[1] = fmaf(f, d1, p[1]);
-    if (DIM == 3) p[2] = fmaf(f, d2, p[2]);
-}
-
 // A target's negated hi and lo coordinates, x and y packed for the f32x2
 // instructions of pair_f32_partial2.
 struct TargetF32x2 {
@@ -894,12 +870,15 @@ static __device__ __forceinline__ TargetF32x2 target_f32x2(const float* T, const
     return t;
 }
 
-// pair_f32_partial with the x and y components in Blackwell's f32x2
-// instructions (FADD2 / FFMA2: two IEEE single operations per issue slot).
-// Every operation and its order are those of pair_f32_partial (x - y is
-// x + (-y) exactly), so the result is the same bit for bit.  UNIT: the
-// source's mass is exactly 1 (the unit-mass frame) and the product with it
-// is skipped, also exactly.
+// FP32 pair term added to a plain FP32 partial sum (pxy, pz): the leaf loop
+// sums at most 32 such terms and then adds the partial to the Kahan-compensated
+// per-target accumulator with kahan_add_f32 (blocked Kahan summation).  Same
+// displacement, r^2 and force as pair_f32, with the x and y components in
+// Blackwell's f32x2 instructions (FADD2 / FFMA2: two IEEE single operations per
+// issue slot; x - y is x + (-y) exactly).  CHECK = false: the caller guarantees
+// e2 >= 2^-126; r^2 is an FMA chain of non-negative terms started at e2, so
+// r^2 >= e2 and the test is compiled out.  UNIT: the source's mass is exactly 1
+// (the unit-mass frame) and the product with it is skipped, also exactly.
 template <int DIM, bool CHECK, bool UNIT>
 __device__ __forceinline__ void pair_f32_partial2(const TargetF32x2& t, float4 sh, float4 sl,
                                                   float e2, float2& pxy, float& pz)
@@ -917,12 +896,11 @@ __device__ __forceinline__ void pair_f32_partial2(const TargetF32x2& t, float4 s
     if (DIM == 3) pz = fmaf(f, dz, pz);
 }
 
-// Rows first .. first + np - 1 of a staged block (two sources to a row) for a target
-// with negated coordinates (nT, nL): displacements, r^2 and w = r^-3 of both
+// Rows first .. first + np - 1 of a staged block (two sources to a row) for a
+// target with negated coordinates (nT, nL): displacements, r^2 and w = r^-3 of both
 // sources in f32x2 instructions, the forces added to the partial sum p one
 // source after the other.  Every operation and its order are those of
-// pair_f32_partial (x - y is x + (-y) exactly), so the sums are the same bit
-// for bit.  UNIT: masses are exactly 1 and their products are skipped, also
+// pair_f32_partial2, so the sums are the same bit for bit.  UNIT: masses are exactly 1 and their products are skipped, also
 // exactly.  np is a multiple of four; places past the last source hold
 // stand-ins that add exactly zero.
 template <int DIM, bool CHECK, bool UNIT>

@@ -37,7 +37,6 @@ BHUT_FN uint64_t bits(double x)
 BHUT_FN double from_bits(uint64_t b) { return __longlong_as_double((long long)b); }
 BHUT_FN uint32_t fbits(float x) { return __float_as_uint(x); }
 BHUT_FN float from_fbits(uint32_t b) { return __uint_as_float(b); }
-BHUT_FN uint64_t mul_hi(uint64_t a, uint64_t b) { return __umul64hi(a, b); }
 BHUT_FN float fma32(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 BHUT_FN float add32(float a, float b) { return __fadd_rn(a, b); }
 BHUT_FN float mul32(float a, float b) { return __fmul_rn(a, b); }

@@ -367,10 +367,9 @@ def build_report(n: int = 1_000_000, reps: int = 10, leaf: int = 32, seed: int =
 # Sub-records of the benchmark line (bench.py): each bounded in time
 # ---------------------------------------------------------------------------
 # FP32-pipe operations per evaluation, counted from bhut_gb300/csrc/fast.cuh:
-# a pair term into a leaf partial (pair_f32_partial2: displacement 9,
-# r^2 + eps^2 3, cube 2, m * w 1 -- none in the unit-mass frame -- three
-# FMAs 3; the x and y operations run as f32x2 instructions, two operations
-# per issue), a Kahan-added monopole (pair_f32: the same 15 plus a Kahan step
+# a pair term into a leaf partial (rows_f32: displacement 9, r^2 + eps^2 3,
+# cube 2, m * w 1 -- none in the unit-mass frame -- three FMAs 3; all but the
+# FMAs run as f32x2 instructions, two sources per issue), a Kahan-added monopole (pair_f32: the same 15 plus a Kahan step
 # per component 12), a Kahan-added monopole + quadrupole node (node_quad_f32:
 # displacement 9, r^2 3, powers 3, Q d 9, d.Q d 3, force factor 4, per
 # component 6 -> 49), each plus one MUFU rsqrt.  Every workload here has
@@ -541,13 +540,13 @@ def c1_record(*, n: int = 10_000, theta: float = 0.5, eps: float = 0.01, G: floa
                    "d2h_bytes_per_call": int(acc.nbytes)},
            "interactions_per_solve": {"p2p": p2p, "m2p": m2p, "node_visits": visits}}
     if fma_rate:
-        instr = 93 * p2p + 97 * m2p
+        instr = 57 * p2p + 97 * m2p   # operations of the terms, as in bench.py
         rec["roofline"] = {"bound": "fp32", "kernel": "k_traverse_fast",
                            "achieved": instr / t_trav / 1e12, "peak": fma_rate,
-                           "unit": "T instr/s", "frac": instr / t_trav / 1e12 / fma_rate,
-                           "note": "10,000 targets at 4 lanes each (k_traverse_fast_lpt) are "
-                                   "1,250 warps for 152 SMs: latency-bound at this size (the "
-                                   "traversal time includes the launch)"}
+                           "unit": "T ops/s", "frac": instr / t_trav / 1e12 / fma_rate,
+                           "note": "10,000 targets are 313 warps of 32; the walk is split over "
+                                   "the tree's top levels among several warps per 32 targets "
+                                   "and stays latency-bound (the time includes the launches)"}
     return rec, np.asarray(acc), (pos, m)
 
 
