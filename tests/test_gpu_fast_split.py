@@ -69,3 +69,16 @@ def test_split_repeats_itself(nt):
     a = tree.accelerations(pos[:nt], softening=0.01)
     assert np.array_equal(a, tree.accelerations(pos[:nt], softening=0.01))
     tree.close()
+
+
+@pytest.mark.parametrize("form", ["fast", "exact"])
+@pytest.mark.parametrize("n,leaf", [(2, 1), (3, 1), (4, 1), (65, 32), (97, 32), (130, 32), (300, 8)])
+def test_smallest_trees(oracle_mod, n, leaf, form):
+    """Trees of two to a few leaves: paths that end above their last level."""
+    pos, m = workloads.gaussian(n, seed=n)
+    tree = bh.Tree(pos, m, leaf_size=leaf, form=form).build()
+    a = tree.accelerations(theta=0.5, softening=0.05)
+    ref = oracle_mod.accelerations(oracle_mod.build_tree(pos, m, leaf), pos, m, theta=0.5,
+                                   softening=0.05)
+    assert rel_l2(a, ref) < (RTOL if form == "fast" else 1e-13)
+    tree.close()
