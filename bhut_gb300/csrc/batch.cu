@@ -889,6 +889,18 @@ int plan_tasks(bhut_batch* b)
     return kOk;
 }
 
+// Boxes of leaf pairs, which form "fast" alone writes and reads.  The form may
+// change after a layout was planned, so a solve asks for them too; a captured
+// solve holds their address.
+int ensure_twigs(bhut_batch* b)
+{
+    if (b->form != BHUT_FORM_FAST) return kOk;
+    const void* before = b->twig.p;
+    BHUT_TRY(b->twig.ensure(sizeof(LeafBox) * (size_t)b->mtot, b->stream));
+    if (b->twig.p != before) drop_graph(b);
+    return kOk;
+}
+
 // Host plan: node and leaf counts of every system, buffers, task list.
 int plan_layout(bhut_batch* b, const int64_t* offsets, int64_t nsys)
 {
@@ -949,7 +961,7 @@ int plan_layout(bhut_batch* b, const int64_t* offsets, int64_t nsys)
     BHUT_TRY(b->frontier.ensure(sizeof(int32_t) * b->ltot, s));
     BHUT_TRY(b->nh.ensure(sizeof(float4) * mtot, s));
     BHUT_TRY(b->nl.ensure(sizeof(float4) * mtot, s));
-    BHUT_TRY(b->twig.ensure(sizeof(LeafBox) * (b->form == BHUT_FORM_FAST ? mtot : 1), s));
+    BHUT_TRY(ensure_twigs(b));
     BHUT_TRY(b->quad.ensure(sizeof(double) * 6 * mtot, s));
     BHUT_TRY(b->nq0.ensure(sizeof(float4) * mtot, s));
     BHUT_TRY(b->nq1.ensure(sizeof(float2) * mtot, s));
@@ -1279,6 +1291,7 @@ int bhut_batch_solve(bhut_batch* b, double theta, double softening, double G, do
     if (!(theta >= 0)) { set_error("theta must be non-negative, got %g", theta); return kInvalid; }
     if (!(softening >= 0)) { set_error("softening must be non-negative, got %g", softening); return kInvalid; }
     BHUT_TRY(ensure_topology(b));
+    BHUT_TRY(ensure_twigs(b));
     const bool dev_out = is_device_pointer(out);
     double* dst = dev_out ? out : b->out.as<double>();
     {
