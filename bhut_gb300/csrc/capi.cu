@@ -154,7 +154,8 @@ struct bhut_tree {
     // traversal targets
     DevBuf tpos, tkeys, tperm, tx, ty, tz, tbox, out, split_partial;
     // float-float copies for the fast form
-    FastFrame frame{};        // from hbox
+    double fbox[kBoxDoubles] = {};   // what frames them: hbox with the current masses (frame_refit)
+    FastFrame frame{};        // from fbox
     DevBuf ph, pl, nh, nl, twig, th, tl, quad, nq0, nq1, nhdr;
     bool ff_valid = false;
     bool ff_quad = false;
@@ -336,6 +337,7 @@ int do_build(bhut_tree* t, int64_t n)
         BHUT_TRY(read_box(t, t->box, t->hbox));
     }
     t->box_in_valid = false;
+    std::copy(t->hbox, t->hbox + kBoxDoubles, t->fbox);
     // replay a captured graph of this exact buffer set; capture one when the
     // same buffer set comes back (a handle built once, as by
     // accelerations(), launches its kernels directly); two are kept: staging
@@ -472,6 +474,14 @@ bool outside_root(const double* root, const double* box, int dim)
     return most > 1.1 * half;
 }
 
+// A refit keeps the build's box and with it the frame's geometry; the unit of
+// mass follows the masses of the refit.
+void frame_refit(bhut_tree* t)
+{
+    t->fbox[6] = t->hbox_in[6];     // largest |mass|
+    t->fbox[15] = t->hbox_in[15];   // all masses equal
+}
+
 // Writes a device result either straight into a device out pointer or via a
 // device buffer and a copy to host memory.
 struct OutTarget {
@@ -507,7 +517,7 @@ int prepare_fast(bhut_tree* t)
     const bool fine = t->form == BHUT_FORM_FAST;
     if (t->ff_valid && t->ff_quad == want_quad && t->ff_fine == fine) return kOk;
     cudaStream_t s = t->stream;
-    t->frame = frame_of_box(t->hbox, t->dim);
+    t->frame = frame_of_box(t->fbox, t->dim);
     BHUT_TRY(t->ph.ensure(sizeof(float4) * t->n, s));
     BHUT_TRY(t->pl.ensure(sizeof(float4) * t->n, s));
     BHUT_TRY(t->nh.ensure(sizeof(float4) * t->m, s));
@@ -787,6 +797,7 @@ int bhut_tree_refit(bhut_tree* t, const double* positions, const double* masses,
                               t->frontier.as<int32_t>(),
                               t->counters.as<unsigned>() + 6, t->err.as<unsigned>(),
                               !t->imported(), s));
+    frame_refit(t);
     t->ff_valid = false;
     return check_err_word(t, "refit");
 }
@@ -815,6 +826,7 @@ int bhut_tree_refit_only(bhut_tree* t, const double* positions, const double* ma
                               t->frontier.as<int32_t>(),
                               t->counters.as<unsigned>() + 6, t->err.as<unsigned>(),
                               !t->imported(), s));
+    frame_refit(t);
     t->ff_valid = false;
     return check_err_word(t, "refit");
 }
@@ -1364,6 +1376,7 @@ int bhut_tree_import(bhut_tree* t, const double* positions, const double* masses
                                     t->box_partial.as<double>(), t->counters.as<unsigned>(),
                                     t->box.as<double>(), t->err.as<unsigned>(), s);
     if (rc == kOk) rc = read_box(t, t->box, t->hbox);
+    std::copy(t->hbox, t->hbox + kBoxDoubles, t->fbox);
     unsigned nleaves = 0;
     if (rc == kOk) {
         cudaError_t e = cudaMemcpyAsync(&nleaves, leaves, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
