@@ -154,7 +154,7 @@ struct bhut_tree {
     // traversal targets
     DevBuf tpos, tkeys, tperm, tx, ty, tz, tbox, out, split_partial;
     // float-float copies for the fast form
-    double fbox[kBoxDoubles] = {};   // what frames them: hbox with the current masses (frame_refit)
+    double fbox[kBoxDoubles] = {};   // what frames them: hbox, changed by refits (frame_refit)
     FastFrame frame{};        // from fbox
     DevBuf ph, pl, nh, nl, twig, th, tl, quad, nq0, nq1, nhdr;
     bool ff_valid = false;
@@ -474,10 +474,20 @@ bool outside_root(const double* root, const double* box, int dim)
     return most > 1.1 * half;
 }
 
-// A refit keeps the build's box and with it the frame's geometry; the unit of
-// mass follows the masses of the refit.
+// A refit keeps the build's box and with it the frame's geometry, as long as
+// the frame maps every particle into [-1, 1] (beyond, hi parts are no longer
+// exact on their grid: 5e-8 relative L2 at a hundred times the box); only
+// refit_only and imported trees can leave it, and are framed by the box of
+// their particles then.  The unit of mass follows the masses of the refit.
 void frame_refit(bhut_tree* t)
 {
+    std::copy(t->hbox, t->hbox + kBoxDoubles, t->fbox);
+    const FastFrame f = frame_of_box(t->hbox, t->dim);
+    bool inside = true;
+    for (int d = 0; d < t->dim; d++)
+        inside = inside && std::fabs((t->hbox_in[d] - f.c[d]) * f.s) <= 1.0 &&
+                 std::fabs((t->hbox_in[3 + d] - f.c[d]) * f.s) <= 1.0;
+    if (!inside) std::copy(t->hbox_in, t->hbox_in + 6, t->fbox);
     t->fbox[6] = t->hbox_in[6];     // largest |mass|
     t->fbox[15] = t->hbox_in[15];   // all masses equal
 }
