@@ -998,7 +998,7 @@ struct OpenF32 {
     // return anything); two nodes share the rare branch
     __device__ __forceinline__ bool near(float d2, float size, float off, bool& open) const
     {
-        const float r = fmaf(off, mac, size * inv), r2 = r * r;
+        const float r = fmaf(off, mac, size * inv), r2 = r * fabsf(r);   // (negative: never opens)
         open = r2 >= d2;
         return !(fabsf(r2 - d2) > 0x1p-18f * d2);
     }

@@ -107,14 +107,17 @@ static __device__ __forceinline__ bool pair_exact(double dx, double dy, double d
 // size / sqrt(s) >= theta (bh.py:576-601) for s = |x - com|^2 as np.linalg.norm
 // sums it (fma chain, OpenBLAS ddot).  The squares decide outside 2^-39 of
 // each other (both sides are within a few 2^-53 of the exact ones, and
-// positive doubles order as integers); inside, or outside the normal range,
+// positive doubles order as integers); inside, or outside the normal range, or
+// for a negative theta or size (tree statistics and imported trees take both),
 // the reference's own square root and division.
 static __device__ __forceinline__ bool opens(double s, double size, double theta)
 {
     const int64_t a = (int64_t)fp64int::bits(__dmul_rn(size, size));
     const int64_t b = (int64_t)fp64int::bits(__dmul_rn(__dmul_rn(theta, theta), s));
     const int64_t gap = a - b;
-    if ((gap > 8192 || gap < -8192) && fp64int::normal_positive(a) && fp64int::normal_positive(b))
+    const bool negative = (int64_t)(fp64int::bits(size) | fp64int::bits(theta)) < 0;
+    if ((gap > 8192 || gap < -8192) && !negative && fp64int::normal_positive(a) &&
+        fp64int::normal_positive(b))
         return gap > 0;
     const double d = __dsqrt_rn(s);
     return d == 0.0 || __ddiv_rn(size, d) >= theta;

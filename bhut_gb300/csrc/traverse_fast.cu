@@ -313,7 +313,8 @@ __device__ __forceinline__ void walk(const TreeDev& t, const FastTree& ft, const
                 h2 = fmaf(d, d, h2);
             }
             const float size_f = __int_as_float(hd.y);
-            const float s2 = size_f * size_f, td2 = theta2 * h2;
+            // (an imported tree may hold negative sizes, which open nothing)
+            const float s2 = size_f * fabsf(size_f), td2 = theta2 * h2;
             bool open = act && s2 >= td2;
             if (act && (FAR || !(fabsf(s2 - td2) > fmaf(0x1p-14f, td2, 0x1p-28f * theta2)))) {
                 float d2 = 0.0f;
