@@ -279,6 +279,10 @@ __device__ __forceinline__ void walk(const TreeDev& t, const FastTree& ft, const
 {
     const unsigned FULL = 0xffffffffu;
     const float theta_f = (float)a.theta, theta2 = theta_f * theta_f;
+    // absolute part of the squares' band; squares of such a theta leave the
+    // range in which their products keep 2^-14: never decided by them
+    const bool squares = theta_f == 0.0f || (theta_f >= 0x1p-30f && theta_f <= 0x1p+30f);
+    const float band2 = squares ? 0x1p-28f * theta2 : INFINITY;
     const double eps2 = __dmul_rn(a.eps, a.eps);
     const int64_t me = base + lane;              // the lane's target
     bool own = !SPLIT || path == 0;              // this warp works on the node
@@ -316,7 +320,7 @@ __device__ __forceinline__ void walk(const TreeDev& t, const FastTree& ft, const
             // (an imported tree may hold negative sizes, which open nothing)
             const float s2 = size_f * fabsf(size_f), td2 = theta2 * h2;
             bool open = act && s2 >= td2;
-            if (act && (FAR || !(fabsf(s2 - td2) > fmaf(0x1p-14f, td2, 0x1p-28f * theta2)))) {
+            if (act && (FAR || !(fabsf(s2 - td2) > fmaf(0x1p-14f, td2, band2)))) {
                 float d2 = 0.0f;
 #pragma unroll
                 for (int k = 0; k < DIM; k++) {
