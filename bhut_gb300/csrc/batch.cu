@@ -801,9 +801,9 @@ struct BufB {
     {
         if (need <= bytes && p) return kOk;
         if (p) { cudaFreeAsync(p, s); p = nullptr; bytes = 0; }
-        cudaError_t e = cudaMallocAsync(&p, need < 256 ? 256 : need, s);
-        if (e != cudaSuccess) { p = nullptr; return cuda_status(e, "cudaMallocAsync"); }
-        bytes = need < 256 ? 256 : need;
+        const size_t want = need < 256 ? 256 : need;
+        BHUT_TRY(device_alloc(&p, want, s));
+        bytes = want;
         return kOk;
     }
     void release(cudaStream_t s) { if (p) cudaFreeAsync(p, s); p = nullptr; bytes = 0; }

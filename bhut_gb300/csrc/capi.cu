@@ -42,6 +42,18 @@ int cuda_status(cudaError_t e, const char* what)
 // Destroys the idle trees kept for reuse (bhut_tree_destroy); false: none.
 bool release_idle_trees();
 
+int device_alloc(void** p, size_t bytes, cudaStream_t s)
+{
+    cudaError_t e = cudaMallocAsync(p, bytes, s);
+    if (e == cudaErrorMemoryAllocation && release_idle_trees()) {
+        cudaGetLastError();
+        e = cudaMallocAsync(p, bytes, s);
+    }
+    if (e == cudaSuccess) return kOk;
+    *p = nullptr;
+    return cuda_status(e, "cudaMallocAsync");
+}
+
 // ---- device buffers -----------------------------------------------------------
 struct DevBuf {
     void* p = nullptr;
@@ -54,16 +66,8 @@ struct DevBuf {
             p = nullptr;
             bytes = 0;
         }
-        size_t want = need < 256 ? 256 : need;
-        cudaError_t e = cudaMallocAsync(&p, want, s);
-        if (e == cudaErrorMemoryAllocation && release_idle_trees()) {
-            cudaGetLastError();
-            e = cudaMallocAsync(&p, want, s);
-        }
-        if (e != cudaSuccess) {
-            p = nullptr;
-            return cuda_status(e, "cudaMallocAsync");
-        }
+        const size_t want = need < 256 ? 256 : need;
+        BHUT_TRY(device_alloc(&p, want, s));
         bytes = want;
         return kOk;
     }
@@ -612,8 +616,8 @@ int traverse(bhut_tree* t, const double* tx, const double* ty, const double* tz,
 // instead of being destroyed: a one-shot solve of a few thousand particles
 // spends more on creating a stream and some forty buffers, and on giving them
 // back, than on its kernels (1,000 particles: 195 of 690 us).  Bounded to
-// kIdleTrees of kIdleBytes each; given back when an allocation of the library
-// fails.  A tree in the pool holds no results: everything but stream, buffers
+// kIdleTrees of kIdleBytes each; given back when an allocation of the library,
+// a batch's too, fails and by bhut_pool_trim.  A tree in the pool holds no results: everything but stream, buffers
 // and pinned memory is reset.
 constexpr size_t kIdleTrees = 4, kIdleBytes = 32u << 20;
 
@@ -1429,6 +1433,7 @@ int bhut_pool_trim(void)
     BHUT_CUDA(cudaGetDevice(&dev));
     cudaMemPool_t pool;
     BHUT_CUDA(cudaDeviceGetDefaultMemPool(&pool, dev));
+    release_idle_trees();
     BHUT_CUDA(cudaDeviceSynchronize());
     BHUT_CUDA(cudaMemPoolTrimTo(pool, 0));
     return kOk;

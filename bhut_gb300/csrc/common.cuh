@@ -31,6 +31,9 @@ void set_error(const char* fmt, ...);
 // Counts kernel launches made by the library (reported by bhut_launch_count).
 void note_launches(long long k);
 int cuda_status(cudaError_t e, const char* what);
+// Stream-ordered device memory for the handles' buffers (capi.cu); without
+// memory the trees kept for reuse are given back first.
+int device_alloc(void** p, size_t bytes, cudaStream_t s);
 
 #define BHUT_CUDA(call)                                              \
     do {                                                             \

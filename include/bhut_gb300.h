@@ -322,8 +322,9 @@ BHUT_API int bhut_measure_fp32_peak(double *tflops);
  * engine's device buffers (current device). */
 BHUT_API int bhut_pool_usage(int64_t *used, int64_t *reserved);
 
-/* Returns the pool's reserved but unused device memory to the driver
- * (synchronises the device); the server calls it after retiring requests. */
+/* Returns the pool's reserved but unused device memory, the buffers of ended
+ * trees that are kept for reuse among it, to the driver (synchronises the
+ * device); the server calls it after retiring requests. */
 BHUT_API int bhut_pool_trim(void);
 
 #ifdef __cplusplus
