@@ -612,6 +612,65 @@ int traverse(bhut_tree* t, const double* tx, const double* ty, const double* tz,
     return kOk;
 }
 
+// Pinned blocks of the trees (bhut_tree::pin), cut from slabs of kPinSlab that
+// stay with the process: pinning and unpinning take 140 and 180 us, and
+// unpinning waits for the whole device (a handle's end took 22 ms beside
+// another stream that was busy that long; 0.1 ms).  A slab without users goes
+// back with bhut_pool_trim.
+constexpr size_t kPinBytes = 512, kPinSlab = 64;
+static_assert(sizeof(double) * kBoxDoubles + kStatusBytes <= kPinBytes, "a tree's pinned block");
+
+struct Pins {
+    std::mutex m;
+    std::vector<char*> free, slabs;
+};
+
+Pins& pins()
+{
+    static Pins* p = new Pins;   // never destroyed, as idle_trees
+    return *p;
+}
+
+cudaError_t take_pin(double** out)
+{
+    Pins& p = pins();
+    std::lock_guard<std::mutex> lock(p.m);
+    if (p.free.empty()) {
+        p.slabs.reserve(p.slabs.size() + 1);
+        p.free.reserve((p.slabs.size() + 1) * kPinSlab);   // giving back allocates nothing
+        void* slab = nullptr;
+        const cudaError_t e = cudaHostAlloc(&slab, kPinBytes * kPinSlab, cudaHostAllocPortable);
+        if (e != cudaSuccess) return e;
+        p.slabs.push_back((char*)slab);
+        for (size_t k = 0; k < kPinSlab; k++) p.free.push_back((char*)slab + k * kPinBytes);
+    }
+    *out = (double*)p.free.back();
+    p.free.pop_back();
+    return cudaSuccess;
+}
+
+void give_pin(double* pin)
+{
+    if (!pin) return;
+    Pins& p = pins();
+    std::lock_guard<std::mutex> lock(p.m);
+    p.free.push_back((char*)pin);
+}
+
+void trim_pins()
+{
+    Pins& p = pins();
+    std::lock_guard<std::mutex> lock(p.m);
+    for (size_t k = p.slabs.size(); k-- > 0;) {
+        char* slab = p.slabs[k];
+        const auto of_slab = [&](char* b) { return b >= slab && b < slab + kPinBytes * kPinSlab; };
+        if ((size_t)std::count_if(p.free.begin(), p.free.end(), of_slab) < kPinSlab) continue;
+        p.free.erase(std::remove_if(p.free.begin(), p.free.end(), of_slab), p.free.end());
+        p.slabs.erase(p.slabs.begin() + (std::ptrdiff_t)k);
+        cudaFreeHost(slab);
+    }
+}
+
 // Small trees on streams of their own are kept for the next bhut_tree_create
 // instead of being destroyed: a one-shot solve of a few thousand particles
 // spends more on creating a stream and some forty buffers, and on giving them
@@ -685,7 +744,7 @@ void free_tree(bhut_tree* t)
     for (DevBuf* b : t->buffers()) b->release(t->stream);
     cudaStreamSynchronize(t->stream);
     for (BuildGraph& g : t->graphs) g.reset();
-    if (t->pin) cudaFreeHost(t->pin);
+    give_pin(t->pin);
     if (t->own_stream) cudaStreamDestroy(t->stream);
     delete t;
 }
@@ -739,7 +798,7 @@ int bhut_tree_create(int dim, int leaf_size, void* stream, bhut_tree** out)
     int st = t->counters.ensure(sizeof(unsigned) * 8, t->stream);
     if (st == kOk) st = t->err.ensure(kStatusBytes, t->stream);
     if (st == kOk) {
-        cudaError_t e = cudaMallocHost(&t->pin, sizeof(double) * kBoxDoubles + kStatusBytes);
+        cudaError_t e = take_pin(&t->pin);
         if (e == cudaSuccess)
             e = cudaMemsetAsync(t->counters.p, 0, sizeof(unsigned) * 8, t->stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(t->err.p, 0, kStatusBytes, t->stream);
@@ -1434,6 +1493,7 @@ int bhut_pool_trim(void)
     cudaMemPool_t pool;
     BHUT_CUDA(cudaDeviceGetDefaultMemPool(&pool, dev));
     release_idle_trees();
+    trim_pins();
     BHUT_CUDA(cudaDeviceSynchronize());
     BHUT_CUDA(cudaMemPoolTrimTo(pool, 0));
     return kOk;
