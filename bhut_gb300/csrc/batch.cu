@@ -27,6 +27,7 @@
 // loop.  All launches of a solve can be captured in one CUDA graph.
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/bhut_gb300.h"
@@ -470,8 +471,30 @@ struct BatchArgs {
 #ifndef BHUT_BATCH_BLOCKS
 #define BHUT_BATCH_BLOCKS 8
 #endif
+// ... and of form fast, which without a bound takes 150 registers (3 blocks) in
+// 3-D, 128 (4) in 2-D and 102 (4) with two lanes per target.  Geometric mean and
+// worst of 576 solves (2 to 120 systems of 33 to 100,000, leaves of 1 to 256,
+// softened and not), relative to one walk of 120 / 92 / 96 registers that does
+// not merge leaf pairs: 3-D 3 / 4 / 5 blocks 0.83 (1.31) / 0.79 (1.10) / 0.87
+// (1.48); 2-D 4 / 5 / 6 blocks 0.73 (1.25) / 0.75 (1.12) / 0.80 (1.25); two lanes
+// per target 4 / 5 / 6 blocks 0.85 (1.21) / 0.85 (1.18) / 0.83 (1.09).
+#ifndef BHUT_BATCH_FAST_BLOCKS
+#define BHUT_BATCH_FAST_BLOCKS 4
+#endif
+#ifndef BHUT_BATCH_FAST_BLOCKS_2D
+#define BHUT_BATCH_FAST_BLOCKS_2D 5
+#endif
+#ifndef BHUT_BATCH_FAST_BLOCKS_16
+#define BHUT_BATCH_FAST_BLOCKS_16 6
+#endif
+constexpr int batch_blocks(int dim, bool fp32, int tpw)
+{
+    if (fp32) return BHUT_BATCH_BLOCKS;
+    return dim == 2 ? BHUT_BATCH_FAST_BLOCKS_2D
+                    : (tpw == 32 ? BHUT_BATCH_FAST_BLOCKS : BHUT_BATCH_FAST_BLOCKS_16);
+}
 template <int DIM, bool FP32, int TPW, int STK>
-__global__ void __launch_bounds__(kBatchThreads, FP32 ? BHUT_BATCH_BLOCKS : 1)
+__global__ void __launch_bounds__(kBatchThreads, batch_blocks(DIM, FP32, TPW))
 k_batch_traverse(BatchDev b, BatchArgs a)
 {
     constexpr int LPT = kWarp / TPW;            // lanes per target
@@ -535,176 +558,184 @@ k_batch_traverse(BatchDev b, BatchArgs a)
             walk_f32<DIM>(b, root, lane, valid, valid ? (int)i : -1, false, unit, opener, e2h, Th, Tl,
                           ah, al, st, stage[w], cnt, overflow);
         } else {
-            int node = root;
-            unsigned mask = __ballot_sync(FULL, valid);
-            while (true) {
-                const bool act = (mask >> lane) & 1u;
-                cnt[2] += act && sub == 0;
-                const int4 hd = b.nhdr[node];   // (first_child, start, count, flag)
-                const float4 nhv = b.nh[node];
-                const int fc = hd.x;
-                const bool staged = kStaged && soft;
-                LeafBox box;
-                unsigned lmask = 0;   // lanes that take the particles [s0, s0 + c0)
-                int s0 = hd.y, c0 = 0;
-                if (!hd.w) {
-                } else if (fc < 0) {
-                    lmask = mask;
-                    c0 = hd.z;
-                    if (staged) {
-                        box.c = nhv;
-                        box.h = b.nl[node];
-                    }
-                } else {
-                    bool open = false;
-                    float4 nlv = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (FP32) {   // hi coordinates only, as the single-tree walk
-                        float d2 = 0.0f;
+            // form fast has one walk for systems with a large softening and one for
+            // the others (a branch within one walk keeps the registers of both
+            // alive: 3,000-particle systems without softening took up to 1.4
+            // times as long)
+            const auto walk = [&](auto tag) {
+                constexpr bool staged = decltype(tag)::value;
+                int node = root;
+                unsigned mask = __ballot_sync(FULL, valid);
+                while (true) {
+                    const bool act = (mask >> lane) & 1u;
+                    cnt[2] += act && sub == 0;
+                    const int4 hd = b.nhdr[node];   // (first_child, start, count, flag)
+                    const float4 nhv = b.nh[node];
+                    const int fc = hd.x;
+                    LeafBox box;
+                    unsigned lmask = 0;   // lanes that take the particles [s0, s0 + c0)
+                    int s0 = hd.y, c0 = 0;
+                    if (!hd.w) {
+                    } else if (fc < 0) {
+                        lmask = mask;
+                        c0 = hd.z;
+                        if (staged) {
+                            box.c = nhv;
+                            box.h = b.nl[node];
+                        }
+                    } else {
+                        bool open = false;
+                        float4 nlv = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (FP32) {   // hi coordinates only, as the single-tree walk
+                            float d2 = 0.0f;
 #pragma unroll
-                        for (int k = 0; k < DIM; k++) {
-                            const float d = __fsub_rn(comp(nhv, k), Th[k]);
-                            d2 = fmaf(d, d, d2);
-                        }
-                        open = opener(d2, __int_as_float(hd.y), __int_as_float(hd.z), act);
-                    } else if (act) {
-                        nlv = b.nl[node];
-                        float d2 = 0.0f;
-#pragma unroll
-                        for (int k = 0; k < DIM; k++) {
-                            const float d = __fadd_rn(__fsub_rn(comp(nhv, k), Th[k]),
-                                                      __fsub_rn(comp(nlv, k), Tl[k]));
-                            d2 = fmaf(d, d, d2);
-                        }
-                        const float dist = d2 > 0.0f ? d2 * rsqrtf(d2) : 0.0f;
-                        const float size_f = __int_as_float(hd.y);
-                        const float td = theta_f * dist;
-                        const float band = theta_f * fmaf(kBandRel, dist, 2.0f * kBandAbs);
-                        if (size_f >= td + band) open = true;
-                        else if (size_f < td - band) open = false;
-                        else {
-                            open = open_exact64<DIM>(x, y, z, t.cm[node], t.size[node], a.theta);
-                            cnt[3]++;
-                        }
-                    }
-                    const unsigned omask = __ballot_sync(FULL, act && open);
-                    if (act && !open && sub == 0) {
-                        if (FP32) {
+                            for (int k = 0; k < DIM; k++) {
+                                const float d = __fsub_rn(comp(nhv, k), Th[k]);
+                                d2 = fmaf(d, d, d2);
+                            }
+                            open = opener(d2, __int_as_float(hd.y), __int_as_float(hd.z), act);
+                        } else if (act) {
                             nlv = b.nl[node];
-                            if (b.nq0)
-                                node_quad_f32<DIM>(Th, Tl, nhv, nlv, b.nq0[node], b.nq1[node], e2h,
-                                                   ah, al);
-                            else
-                                pair_f32<DIM>(Th, Tl, nhv, nlv, e2h, ah, al);
-                        } else if (soft && !(hd.w & kNodeOutside)) {
-                            pair_ff_soft<DIM, false>(Th, Tl, nhv, nlv, e2h, e2l, ah, al);
-                        } else if ((hd.w & kNodeOutside) || !pair_ff<DIM, false>(Th, Tl, nhv, nlv, e2h, e2l, ah, al)) {
-                            const NodeCM cm = t.cm[node];
-                            pair_fp64<DIM>(x, y, z, cm.x, cm.y, cm.z, cm.w, eps2, a64);
-                            cnt[4]++;
-                        }
-                        cnt[1]++;
-                    }
-                    if (staged && omask && (hd.w & kTwig)) {
-                        lmask = omask;
-                        box = b.twig[node];
-                        s0 = __float_as_int(box.h.w);
-                        c0 = twig_left(hd.w) + twig_right(hd.w);
-                        cnt[2] += act && open ? 2 : 0;
-                    } else if (omask) {
-                        if (st.sp + 2 > kStackDepth) {
-                            overflow = true;
-                            break;
-                        }
-                        st.push({fc, omask, 0});
-                        node = fc + 1;
-                        mask = omask;
-                        continue;
-                    }
-                }
-                const bool lact = (lmask >> lane) & 1u;
-                if (c0) {
-                    const int block = staged ? kStage : kWarp;
-                    for (int bb = 0; bb < c0; bb += block) {
-                        const int cn = min(block, c0 - bb);
-                        for (int jj = lane; jj < cn; jj += kWarp) {
-                            const float4 h = b.ph[s0 + bb + jj], l = b.pl[s0 + bb + jj];
-                            if (staged) {
-                                stage[kStaged ? w : 0].put(jj, h, l);
-                            } else {
-                                sh[jj] = h;
-                                sl[jj] = l;
-                            }
-                        }
-                        __syncwarp();
-                        if (lact && sub == 0) cnt[0] += cn - (i >= s0 + bb && i < s0 + bb + cn);
-                        if (staged) {   // as the single-tree walk
-                            const LeafStage& sg = stage[kStaged ? w : 0];
-                            if (unit)
-                                leaf_block_soft<DIM, true>(lmask, lane, Th, Tl, sg, cn, box,
-                                                           e2h, e2l, ah, al);
-                            else
-                                leaf_block_soft<DIM, false>(lmask, lane, Th, Tl, sg, cn, box,
-                                                            e2h, e2l, ah, al);
-                        } else if (lact) {
-                            if (FP32) {   // <= 32 terms in FP32, then one Kahan step
-                                float2 pxy = make_float2(0.f, 0.f);
-                                float pz = 0.f;
-                                if (soft && unit) {
-#pragma unroll 8
-                                    for (int q = sub; q < cn; q += LPT)
-                                        pair_f32_partial2<DIM, false, true>(
-                                            tx, sh[q], sl[q], e2h, pxy, pz);
-                                } else if (soft) {
-#pragma unroll 8
-                                    for (int q = sub; q < cn; q += LPT)
-                                        pair_f32_partial2<DIM, false, false>(
-                                            tx, sh[q], sl[q], e2h, pxy, pz);
-                                } else {
-#pragma unroll 8
-                                    for (int q = sub; q < cn; q += LPT)
-                                        pair_f32_partial2<DIM, true, false>(
-                                            tx, sh[q], sl[q], e2h, pxy, pz);
-                                }
-                                const float part[3] = {pxy.x, pxy.y, pz};
-                                kahan_add_f32<DIM>(part, ah, al);
-                            } else {
-                                unsigned fb = 0;   // pairs left to FP64, taken after the loop
-                                if (soft && unit) {
-                                    for (int q = sub; q < cn; q += LPT)
-                                        pair_ff_soft<DIM, true>(Th, Tl, sh[q], sl[q], e2h, e2l, ah, al);
-                                } else if (soft) {
-                                    for (int q = sub; q < cn; q += LPT)
-                                        pair_ff_soft<DIM, false>(Th, Tl, sh[q], sl[q], e2h, e2l, ah, al);
-                                } else {
-                                    for (int q = sub; q < cn; q += LPT)
-                                        fb |= (unsigned)!pair_ff<DIM, false>(Th, Tl, sh[q], sl[q], e2h,
-                                                                             e2l, ah, al) << q;
-                                }
-                                while (fb) {
-                                    const int gi = s0 + bb + __ffs(fb) - 1;
-                                    fb &= fb - 1;
-                                    pair_fp64<DIM>(x, y, z, t.sx[gi], t.sy[gi],
-                                                   DIM == 3 ? t.sz[gi] : 0.0, t.sm[gi], eps2, a64);
-                                    cnt[4]++;
-                                }
-                            }
-                        }
-                        __syncwarp();
-                    }
-                    if (!FP32 && lact) {
+                            float d2 = 0.0f;
 #pragma unroll
-                        for (int k = 0; k < DIM; k++) {
-                            const float hs = __fadd_rn(ah[k], al[k]);
-                            al[k] = __fsub_rn(al[k], __fsub_rn(hs, ah[k]));
-                            ah[k] = hs;
+                            for (int k = 0; k < DIM; k++) {
+                                const float d = __fadd_rn(__fsub_rn(comp(nhv, k), Th[k]),
+                                                          __fsub_rn(comp(nlv, k), Tl[k]));
+                                d2 = fmaf(d, d, d2);
+                            }
+                            const float dist = d2 > 0.0f ? d2 * rsqrtf(d2) : 0.0f;
+                            const float size_f = __int_as_float(hd.y);
+                            const float td = theta_f * dist;
+                            const float band = theta_f * fmaf(kBandRel, dist, 2.0f * kBandAbs);
+                            if (size_f >= td + band) open = true;
+                            else if (size_f < td - band) open = false;
+                            else {
+                                open = open_exact64<DIM>(x, y, z, t.cm[node], t.size[node], a.theta);
+                                cnt[3]++;
+                            }
+                        }
+                        const unsigned omask = __ballot_sync(FULL, act && open);
+                        if (act && !open && sub == 0) {
+                            if (FP32) {
+                                nlv = b.nl[node];
+                                if (b.nq0)
+                                    node_quad_f32<DIM>(Th, Tl, nhv, nlv, b.nq0[node], b.nq1[node], e2h,
+                                                       ah, al);
+                                else
+                                    pair_f32<DIM>(Th, Tl, nhv, nlv, e2h, ah, al);
+                            } else if (soft && !(hd.w & kNodeOutside)) {
+                                pair_ff_soft<DIM, false>(Th, Tl, nhv, nlv, e2h, e2l, ah, al);
+                            } else if ((hd.w & kNodeOutside) || !pair_ff<DIM, false>(Th, Tl, nhv, nlv, e2h, e2l, ah, al)) {
+                                const NodeCM cm = t.cm[node];
+                                pair_fp64<DIM>(x, y, z, cm.x, cm.y, cm.z, cm.w, eps2, a64);
+                                cnt[4]++;
+                            }
+                            cnt[1]++;
+                        }
+                        if (staged && omask && (hd.w & kTwig)) {
+                            lmask = omask;
+                            box = b.twig[node];
+                            s0 = __float_as_int(box.h.w);
+                            c0 = twig_left(hd.w) + twig_right(hd.w);
+                            cnt[2] += act && open ? 2 : 0;
+                        } else if (omask) {
+                            if (st.sp + 2 > kStackDepth) {
+                                overflow = true;
+                                break;
+                            }
+                            st.push({fc, omask, 0});
+                            node = fc + 1;
+                            mask = omask;
+                            continue;
                         }
                     }
+                    const bool lact = (lmask >> lane) & 1u;
+                    if (c0) {
+                        const int block = staged ? kStage : kWarp;
+                        for (int bb = 0; bb < c0; bb += block) {
+                            const int cn = min(block, c0 - bb);
+                            for (int jj = lane; jj < cn; jj += kWarp) {
+                                const float4 h = b.ph[s0 + bb + jj], l = b.pl[s0 + bb + jj];
+                                if (staged) {
+                                    stage[kStaged ? w : 0].put(jj, h, l);
+                                } else {
+                                    sh[jj] = h;
+                                    sl[jj] = l;
+                                }
+                            }
+                            __syncwarp();
+                            if (lact && sub == 0) cnt[0] += cn - (i >= s0 + bb && i < s0 + bb + cn);
+                            if (staged) {   // as the single-tree walk
+                                const LeafStage& sg = stage[kStaged ? w : 0];
+                                if (unit)
+                                    leaf_block_soft<DIM, true>(lmask, lane, Th, Tl, sg, cn, box,
+                                                               e2h, e2l, ah, al);
+                                else
+                                    leaf_block_soft<DIM, false>(lmask, lane, Th, Tl, sg, cn, box,
+                                                                e2h, e2l, ah, al);
+                            } else if (lact) {
+                                if (FP32) {   // <= 32 terms in FP32, then one Kahan step
+                                    float2 pxy = make_float2(0.f, 0.f);
+                                    float pz = 0.f;
+                                    if (soft && unit) {
+#pragma unroll 8
+                                        for (int q = sub; q < cn; q += LPT)
+                                            pair_f32_partial2<DIM, false, true>(
+                                                tx, sh[q], sl[q], e2h, pxy, pz);
+                                    } else if (soft) {
+#pragma unroll 8
+                                        for (int q = sub; q < cn; q += LPT)
+                                            pair_f32_partial2<DIM, false, false>(
+                                                tx, sh[q], sl[q], e2h, pxy, pz);
+                                    } else {
+#pragma unroll 8
+                                        for (int q = sub; q < cn; q += LPT)
+                                            pair_f32_partial2<DIM, true, false>(
+                                                tx, sh[q], sl[q], e2h, pxy, pz);
+                                    }
+                                    const float part[3] = {pxy.x, pxy.y, pz};
+                                    kahan_add_f32<DIM>(part, ah, al);
+                                } else {
+                                    unsigned fb = 0;   // pairs left to FP64, taken after the loop
+                                    if (soft && unit) {
+                                        for (int q = sub; q < cn; q += LPT)
+                                            pair_ff_soft<DIM, true>(Th, Tl, sh[q], sl[q], e2h, e2l, ah, al);
+                                    } else if (soft) {
+                                        for (int q = sub; q < cn; q += LPT)
+                                            pair_ff_soft<DIM, false>(Th, Tl, sh[q], sl[q], e2h, e2l, ah, al);
+                                    } else {
+                                        for (int q = sub; q < cn; q += LPT)
+                                            fb |= (unsigned)!pair_ff<DIM, false>(Th, Tl, sh[q], sl[q], e2h,
+                                                                                 e2l, ah, al) << q;
+                                    }
+                                    while (fb) {
+                                        const int gi = s0 + bb + __ffs(fb) - 1;
+                                        fb &= fb - 1;
+                                        pair_fp64<DIM>(x, y, z, t.sx[gi], t.sy[gi],
+                                                       DIM == 3 ? t.sz[gi] : 0.0, t.sm[gi], eps2, a64);
+                                        cnt[4]++;
+                                    }
+                                }
+                            }
+                            __syncwarp();
+                        }
+                        if (!FP32 && lact) {
+#pragma unroll
+                            for (int k = 0; k < DIM; k++) {
+                                const float hs = __fadd_rn(ah[k], al[k]);
+                                al[k] = __fsub_rn(al[k], __fsub_rn(hs, ah[k]));
+                                ah[k] = hs;
+                            }
+                        }
+                    }
+                    if (st.sp == 0) break;
+                    const StackEntry e = st.pop();
+                    node = e.node;
+                    mask = e.mask;
                 }
-                if (st.sp == 0) break;
-                const StackEntry e = st.pop();
-                node = e.node;
-                mask = e.mask;
-            }
+            };
+            if (kStaged && soft) walk(std::bool_constant<kStaged>());
+            else walk(std::false_type());
         }
         if (overflow && lane == 0) atomicOr(a.err, kErrStackOverflow);
         // fold the lanes that share a target
