@@ -578,7 +578,7 @@ int traverse(bhut_tree* t, const double* tx, const double* ty, const double* tz,
     // (form fp32 keeps one order of its sums)
     const int levels = t->form == BHUT_FORM_FP32
                            ? 0
-                           : split_levels(nt, t->m, self_targets, t->form == BHUT_FORM_EXACT);
+                           : split_levels(nt, t->m, t->n, self_targets, t->form == BHUT_FORM_EXACT);
     const int64_t part = split_partial_doubles(nt, t->dim, levels);
     if (part > 0) BHUT_TRY(t->split_partial.ensure(sizeof(double) * part, t->stream));
     switch (t->form) {

@@ -83,6 +83,14 @@ constexpr int kSplitMaxLevels = 10;
 #ifndef BHUT_SPLIT_WARPS
 #define BHUT_SPLIT_WARPS 49152
 #endif
+// Trees of one or two long leaves have no nodes to split by: their first two
+// levels pay while a warp has this many particles (a split shares a leaf's
+// blocks).  Self solves of 500 / 1,000 / 4,000 / 12,000 particles in one or two
+// leaves 90 / 138 / 426 / 1,171 us unsplit, 55 / 75 / 149 / 628 split, 40 targets
+// 157 / 202 / 478 / 1,230 and 127 / 137 / 219 / 426; by 32 to 128 particles the same.
+#ifndef BHUT_SPLIT_PARTICLES
+#define BHUT_SPLIT_PARTICLES 64
+#endif
 // Form "exact" (pairs are dearer, the walk matters less): ms for none / 12501 /
 // 25000 / 50001 warps, Plummer: 10k self 10.5 / 2.0 / 2.0 / 2.0, 30k 32.4 /
 // 14.6 / 13.7 / 13.3, 60k 62.6 / 42.4 / 40.9 / 40.8, 100k 95.7 / 85.3 / 86.5 /
@@ -262,8 +270,8 @@ __device__ __forceinline__ void leaf_block_check(unsigned mask, int lane, const 
 // fallback); UNIT: leaf pairs skip the mass product (unit masses).
 // SPLIT: 2^levels warps share the targets; a warp follows the bits of `path`
 // (highest first) through the top `levels` levels and walks the subtree it
-// reaches.  A node of those levels is worked on (leaf, monopoles, counts) by
-// the warp whose remaining bits are zero.
+// reaches.  A node of those levels is worked on (monopoles, counts) by the warp
+// whose remaining bits are zero, a leaf's particles by all that reach it.
 // A twig (put_node) that some lane opens is worked on like a leaf: its two
 // leaves, always visited by the same lanes, cost one visit, one staging and
 // one set of bounds instead of two (1M Plummer 142.7 ms without, 137.0 with,
@@ -304,7 +312,13 @@ __device__ __forceinline__ void walk(const TreeDev& t, const FastTree& ft, const
         if (!hd.w) {                      // mass == 0 skip (bh.py:514)
         } else if (fc < 0) {
             lmask = mask;
-            c = own ? hd.z : 0;
+            c = hd.z;
+            if (SPLIT && levels > 0) {    // runs of whole blocks for the warps that reach it
+                const int run = (((c - 1) >> levels) / kStage + 1) * kStage;
+                const int first = min(c, (path & ((1 << levels) - 1)) * run);
+                s += first;
+                c = min(run, c - first);
+            }
         } else {
             // The hi parts alone decide outside a band of 2^-14 of d^2 plus
             // 2^-28 (the lo parts move d by delta <= 2^-22, and 2 d delta <=
@@ -678,14 +692,15 @@ int launch_split_sum(const double* partial, int64_t nt, int dim, int shares,
 
 // Levels of the tree to split a traversal of nt targets by (0: none, else
 // 2 to kSplitMaxLevels), and the doubles of `partial` it needs.
-int split_levels(int64_t nt, int64_t nodes, bool self, bool exact)
+int split_levels(int64_t nt, int64_t nodes, int64_t particles, bool self, bool exact)
 {
     const int64_t groups = (nt + kWarp - 1) / kWarp;
     if (self && groups >= (exact ? 2 : 1) * kWaveWarps) return 0;
     const int64_t warps = exact ? BHUT_SPLIT_WARPS_EXACT : BHUT_SPLIT_WARPS;
     int levels = 0;
     while (levels < kSplitMaxLevels && (groups << levels) < warps &&
-           (nodes >> levels) > (levels < 2 ? BHUT_SPLIT_NODES_FIRST : BHUT_SPLIT_NODES))
+           ((nodes >> levels) > (levels < 2 ? BHUT_SPLIT_NODES_FIRST : BHUT_SPLIT_NODES) ||
+            (!exact && levels < 2 && (particles >> levels) > 2 * BHUT_SPLIT_PARTICLES)))
         levels++;
     return levels < 2 ? 0 : levels;
 }

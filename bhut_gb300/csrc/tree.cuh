@@ -300,7 +300,7 @@ int launch_traverse_fast(const TreeDev& t, const FastTree& ft, const float4* th,
                          int levels, double* partial);
 // Few targets: 2^levels warps per 32 targets (0: one), the doubles of scratch
 // that takes, and the sum of the blocks' partial results.
-int split_levels(int64_t nt, int64_t nodes, bool self, bool exact);
+int split_levels(int64_t nt, int64_t nodes, int64_t particles, bool self, bool exact);
 int64_t split_partial_doubles(int64_t nt, int dim, int levels);
 int launch_split_sum(const double* partial, int64_t nt, int dim, int shares,
                      const int32_t* out_idx, double* out, cudaStream_t s);
