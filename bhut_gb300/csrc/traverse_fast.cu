@@ -31,6 +31,8 @@
 //    nodes inside a small error band are decided by the exact FP64 test of
 //    k_traverse_exact (bh.py:576-601).  Every lane therefore evaluates
 //    exactly the reference's interaction set for its target.
+#include <cmath>
+
 #include "fast.cuh"
 
 namespace bhut {
@@ -195,6 +197,7 @@ struct FastArgs {
     unsigned* err;
     unsigned long long* stats;
     int mac;                 // 0: reference criterion, 1: offset criterion (fp32 form)
+    float theta2, band2;     // theta^2 and the absolute band of the test on squares (form fast)
 };
 
 // leaf_block_soft for the checked path (targets inside the box, softening
@@ -286,11 +289,7 @@ __device__ __forceinline__ void walk(const TreeDev& t, const FastTree& ft, const
                                      int levels = 0, int path = 0)
 {
     const unsigned FULL = 0xffffffffu;
-    const float theta_f = (float)a.theta, theta2 = theta_f * theta_f;
-    // absolute part of the squares' band; squares of such a theta leave the
-    // range in which their products keep 2^-14: never decided by them
-    const bool squares = theta_f == 0.0f || (theta_f >= 0x1p-30f && theta_f <= 0x1p+30f);
-    const float band2 = squares ? 0x1p-28f * theta2 : INFINITY;
+    const float theta_f = (float)a.theta;
     const double eps2 = __dmul_rn(a.eps, a.eps);
     const int64_t me = base + lane;              // the lane's target
     bool own = !SPLIT || path == 0;              // this warp works on the node
@@ -332,9 +331,9 @@ __device__ __forceinline__ void walk(const TreeDev& t, const FastTree& ft, const
             }
             const float size_f = __int_as_float(hd.y);
             // (an imported tree may hold negative sizes, which open nothing)
-            const float s2 = size_f * fabsf(size_f), td2 = theta2 * h2;
+            const float s2 = size_f * fabsf(size_f), td2 = a.theta2 * h2;
             bool open = act && s2 >= td2;
-            if (act && (FAR || !(fabsf(s2 - td2) > fmaf(0x1p-14f, td2, band2)))) {
+            if (act && (FAR || !(fabsf(s2 - td2) > fmaf(0x1p-14f, td2, a.band2)))) {
                 float d2 = 0.0f;
 #pragma unroll
                 for (int k = 0; k < DIM; k++) {
@@ -726,6 +725,12 @@ int launch_traverse_fast(const TreeDev& t, const FastTree& ft, const float4* th,
     a.e2h = (float)eps_scaled_sq;
     a.e2l = (float)(eps_scaled_sq - (double)a.e2h);
     a.out = out; a.err = err; a.stats = stats; a.mac = mac;
+    // A theta whose products would leave the range in which they keep 2^-14 gets an
+    // infinite band: the squares then decide nothing.  (Kernel arguments: chosen
+    // in the walk, the band cost a register and 0.5 to 1 % of the time.)
+    const float tf = (float)theta;
+    a.theta2 = tf * tf;
+    a.band2 = tf == 0.0f || (tf >= 0x1p-30f && tf <= 0x1p+30f) ? 0x1p-28f * a.theta2 : INFINITY;
     int64_t warps = (nt + kWarp - 1) / kWarp;
     unsigned grid = grid_for(warps, kFastWarps, 152u * 64u);
     if (fp32) {
