@@ -900,16 +900,20 @@ __device__ __forceinline__ void pair_f32_partial2(const TargetF32x2& t, float4 s
 // target with negated coordinates (nT, nL): displacements, r^2 and w = r^-3 of both
 // sources in f32x2 instructions, the forces added to the partial sum p one
 // source after the other.  Every operation and its order are those of
-// pair_f32_partial2, so the sums are the same bit for bit.  UNIT: masses are exactly 1 and their products are skipped, also
-// exactly.  np is a multiple of four; places past the last source hold
-// stand-ins that add exactly zero.
+// pair_f32_partial2, so the sums are the same bit for bit.  UNIT: masses are
+// exactly 1 and their products are skipped, also exactly.  np is even; places
+// past the last source hold stand-ins that add exactly zero.  (In steps of four
+// rows, leaves of 33 to 64 particles took up to 1.22 times as long as one source
+// at a time, for the stand-ins and registers spilled: 300k galaxy in leaves of 48
+// 20.7 ms, by two rows 20.0, one by one 19.5; 256 systems in leaves of 16 41.8,
+// 39.8 and, without leaf pairs, 56.8.)
 template <int DIM, bool CHECK, bool UNIT>
 __device__ __forceinline__ void rows_f32(const LeafStage& st, int first, int np, const float2* nT,
                                          const float2* nL, float e2, float* p)
 {
-    for (int r0 = first; r0 < first + np; r0 += 4)
+    for (int r0 = first; r0 < first + np; r0 += 2)
 #pragma unroll
-    for (int r = r0; r < r0 + 4; r++) {
+    for (int r = r0; r < r0 + 2; r++) {
         const float4 A = st.a[r], B = st.b[r];
         const float2 dx = __fadd2_rn(__fadd2_rn(make_float2(A.x, A.y), nT[0]),
                                      __fadd2_rn(make_float2(B.x, B.y), nL[0]));
@@ -941,7 +945,7 @@ __device__ __forceinline__ void rows_f32(const LeafStage& st, int first, int np,
 
 
 // Rows that rows_f32 takes for c sources.
-static __device__ __forceinline__ int rows_for(int c) { return ((c + 7) >> 3) << 2; }
+static __device__ __forceinline__ int rows_for(int c) { return ((c + 3) >> 2) << 1; }
 
 // Stages two runs of at most 32 sources for rows_f32, the second (which may be
 // empty) in the rows after the first's.  Stand-ins fill the rows: for targets
