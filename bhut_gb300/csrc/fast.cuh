@@ -746,7 +746,8 @@ static __device__ __forceinline__ void put_node(const TreeDev& t, int64_t k, con
     split_plain(__dmul_rn(c.w, f.ms), h.w, l.w);
     int4 hd;
     if (fc < 0) {
-        leaf_box(ph, t.start[k], t.count[k], h, l);   // (LeafBox in a leaf's place)
+        // (a LeafBox in a leaf's place; form "fp32" reads neither)
+        if (fine) leaf_box(ph, t.start[k], t.count[k], h, l);
         hd = make_int4(fc, t.start[k], t.count[k], c.w != 0.0 ? kNodeMass : 0);
     } else {
         // distance between the centre of mass and the AABB centre (offset MAC)
