@@ -5,9 +5,12 @@
 // _barnes_hut_single_target_external (:83-146).  One warp owns 32
 // Morton-contiguous targets and walks the tree with a shared stack of
 // (node, lane mask) entries: a lane that accepts a node adds its monopole and
-// drops out of that subtree, so every lane visits exactly the nodes, in
-// exactly the order, of the reference's own traversal for its target
-// (right child first, bh.py:531-537).  Per-pair arithmetic is the Numba leaf
+// drops out of that subtree, so every lane visits exactly the nodes of the
+// reference's own traversal for its target, right child first (bh.py:531-537).
+// Contributions are summed in that order within the subtrees at the depth
+// top_levels (a function of the node count alone), and these sums in pairs,
+// child by child, up to the root: whichever levels the warps of a call split,
+// a target's value depends on the tree only.  Per-pair arithmetic is the Numba leaf
 // loop (bh.py:226-280) with explicit round-to-nearest intrinsics and IEEE
 // sqrt/division, so P2P terms match the reference's bit for bit; monopoles
 // use r2^1.5 = r2 * sqrt(r2) in place of pow (kernels.py:66), within 2 ulp.
@@ -23,6 +26,12 @@ namespace bhut {
 
 constexpr int kTravWarps = 4;
 constexpr int kTravThreads = kTravWarps * kWarp;
+
+// Resident blocks per SM of k_traverse_exact, at the registers that they allow.
+// 3-D, split: without a bound (101 registers, 4 blocks) / 5 / 6: 100k Plummer
+// 93.2 / 85.7 / 82.5 ms, 10k 1.97 / 1.83 / 1.76; not split, 5 / 6: 200k 140 / 145.
+// 2-D, 6 / 7: 50k 3.68 / 3.60, 10k 0.80 / 0.78, targets of either 0 to 6 % less / more.
+constexpr int exact_blocks(int dim, bool split) { return dim == 3 && !split ? 5 : 6; }
 
 // Products of a pair on the integer pipes: the squares and the force
 // components (tuning: 0 takes the FP64 pipe; 100k Plummer traversal both 95.9
@@ -157,15 +166,20 @@ __device__ __forceinline__ void monopole_exact(double dx, double dy, double dz, 
 
 // SPLIT: 2^levels warps share 32 targets as in k_traverse_fast (few targets;
 // a warp follows the bits of its path through the top levels and walks the
-// subtree it reaches), so a target's pair terms are the same bit for bit but
-// are summed per subtree first.
+// subtree it reaches); levels <= top.
+//
+// The walk keeps the place (d, idx) of the unit that it is summing: a node above
+// depth `top`, or a subtree at that depth.  At a unit's end the sum waits in
+// saved[d] when it is a right child's, for its left sibling's; a left child's is
+// added to it and the pair is the parent's.  Lanes without a part in a unit add
+// zeros.
 template <int DIM, bool SPLIT>
-__global__ void __launch_bounds__(kTravThreads)
+__global__ void __launch_bounds__(kTravThreads, exact_blocks(DIM, SPLIT))
 k_traverse_exact(TreeDev t, const double* __restrict__ tx, const double* __restrict__ ty,
                  const double* __restrict__ tz, const int32_t* __restrict__ self_id,
                  const int32_t* __restrict__ out_idx, int64_t nt, double theta, double eps,
                  double G, double* __restrict__ out, unsigned* __restrict__ err,
-                 unsigned long long* __restrict__ stats, int levels0,
+                 unsigned long long* __restrict__ stats, int levels0, int top,
                  double* __restrict__ partial)
 {
     __shared__ int2 stack[kTravWarps][kStackDepth];
@@ -186,13 +200,15 @@ k_traverse_exact(TreeDev t, const double* __restrict__ tx, const double* __restr
          g * kWarp < nt; g += step) {
         const int64_t i = g * kWarp + lane;
         const int path = SPLIT ? share * kTravWarps + w : 0;
-        int levels = levels0;
         bool own = path == 0;                                // works on the node
         const bool valid = i < nt;
         const double x = valid ? tx[i] : 0.0, y = valid ? ty[i] : 0.0;
         const double z = (valid && DIM == 3) ? tz[i] : 0.0;
         const int32_t me = (valid && self_id) ? self_id[i] : -1;
         double ax = 0.0, ay = 0.0, az = 0.0;
+        double saved[kTopLevels + 1][DIM];
+        int d = 0, idx = 0, sp0 = 0;
+        bool fresh = true;                                   // the next node begins a unit
         unsigned long long n_p2p = 0, n_m2p = 0, n_visit = 0;
         const unsigned live = __ballot_sync(FULL, valid);
         if (lane == 0) stack[w][0] = make_int2(0, (int)live);
@@ -202,14 +218,16 @@ k_traverse_exact(TreeDev t, const double* __restrict__ tx, const double* __restr
         while (sp > 0) {
             const int2 e = stack[w][--sp];
             __syncwarp();
+            if (fresh) sp0 = sp;
+            unsigned omask = 0;
             const int node = e.x;
             const unsigned mask = (unsigned)e.y;
             const bool act = (mask >> lane) & 1u;
             n_visit += act && own;
             const NodeCM cm = t.cm[node];
-            if (cm.w == 0.0) continue;                       // bh.py:514
             const int fc = t.first_child[node];
-            if (fc < 0) {                                    // leaf: bh.py:520-524
+            if (cm.w == 0.0) {                               // bh.py:514
+            } else if (fc < 0) {                             // leaf: bh.py:520-524
                 const int s = t.start[node], c = own ? t.count[node] : 0;
                 double lx = 0.0, ly = 0.0, lz = 0.0;
                 for (int b = 0; b < c; b += kWarp) {
@@ -249,16 +267,16 @@ k_traverse_exact(TreeDev t, const double* __restrict__ tx, const double* __restr
                     if (DIM == 3) dz = __dsub_rn(cm.z, z);
                     open = opens(norm2_fma<DIM>(dx, dy, dz), t.size[node], theta);
                 }
-                const unsigned omask = __ballot_sync(FULL, act && open);
+                omask = __ballot_sync(FULL, act && open);
                 if (act && !open && own) {
                     monopole_exact<DIM>(dx, dy, dz, cm.w, eps2, G, ax, ay, az);
                     n_m2p++;
                 }
-                if (SPLIT && omask && levels > 0) {
-                    levels--;
-                    own = (path & ((1 << levels) - 1)) == 0;
+                if (SPLIT && omask && d < levels0) {
+                    const int rest = levels0 - 1 - d;        // bits of the path below the child
+                    own = (path & ((1 << rest) - 1)) == 0;
                     if (lane == 0)
-                        stack[w][sp] = make_int2(fc + ((path >> levels) & 1), (int)omask);
+                        stack[w][sp] = make_int2(fc + ((path >> rest) & 1), (int)omask);
                     sp++;
                     __syncwarp();
                 } else if (omask) {
@@ -270,6 +288,26 @@ k_traverse_exact(TreeDev t, const double* __restrict__ tx, const double* __restr
                     sp += 2;
                     __syncwarp();
                 }
+            }
+            if (omask && d < top) {                          // on to its (right) child
+                idx = 2 * idx + 1;                           // (above levels0 not looked at)
+                d++;
+                fresh = true;
+            } else if ((fresh = sp == sp0)) {                // the unit's end
+                double v[3] = {ax, ay, az};
+                for (; d > levels0 && !(idx & 1); idx >>= 1, d--) {
+#pragma unroll
+                    for (int k = 0; k < DIM; k++) v[k] = __dadd_rn(saved[d][k], v[k]);
+                }
+                const bool wait = d > levels0;
+                if (wait) {
+#pragma unroll
+                    for (int k = 0; k < DIM; k++) saved[d][k] = v[k];
+                }
+                idx--;
+                ax = wait ? 0.0 : v[0];
+                ay = wait ? 0.0 : v[1];
+                az = wait ? 0.0 : v[2];
             }
         }
         if (overflow && lane == 0) atomicOr(err, kErrStackOverflow);
@@ -291,9 +329,8 @@ k_traverse_exact(TreeDev t, const double* __restrict__ tx, const double* __restr
             if (DIM == 3) sum[SPLIT ? w : 0][SPLIT ? DIM - 1 : 0][lane] = az;
             __syncthreads();
             if (w < DIM && valid) {
-                double v = sum[0][SPLIT ? w : 0][lane];
-                for (int u = 1; u < kTravWarps; u++)
-                    v = __dadd_rn(v, sum[SPLIT ? u : 0][SPLIT ? w : 0][lane]);
+                const auto of = [&](int u) { return sum[SPLIT ? u : 0][SPLIT ? w : 0][lane]; };
+                const double v = __dadd_rn(__dadd_rn(of(0), of(1)), __dadd_rn(of(2), of(3)));
                 if (shares > 1) partial[((int64_t)share * nt + i) * DIM + w] = v;
                 else out[(out_idx ? out_idx[i] : i) * DIM + w] = v;
             }
@@ -389,6 +426,8 @@ int launch_traverse_exact(const TreeDev& t, const double* tx, const double* ty, 
                           unsigned long long* stats, cudaStream_t s, int levels, double* partial)
 {
     if (nt <= 0) return kOk;
+    const int top = top_levels(t.m);
+    if (levels > top) { set_error("split deeper than the sums of form exact"); return kInternal; }
     const int64_t groups = (nt + kWarp - 1) / kWarp;
     const int shares = levels > 0 ? (1 << levels) / kTravWarps : 1;
     const unsigned grid = levels > 0 ? (unsigned)(groups * shares)
@@ -397,10 +436,10 @@ int launch_traverse_exact(const TreeDev& t, const double* tx, const double* ty, 
                        ? (levels > 0 ? k_traverse_exact<3, true> : k_traverse_exact<3, false>)
                        : (levels > 0 ? k_traverse_exact<2, true> : k_traverse_exact<2, false>);
     kernel<<<grid, kTravThreads, 0, s>>>(t, tx, ty, tz, self_id, out_idx, nt, theta, eps, G, out,
-                                         err, stats, levels, partial);
+                                         err, stats, levels, top, partial);
     BHUT_CUDA(cudaGetLastError());
     note_launches(1);
-    return shares > 1 ? launch_split_sum(partial, nt, t.dim, shares, out_idx, out, s) : kOk;
+    return shares > 1 ? launch_split_sum(partial, nt, t.dim, shares, true, out_idx, out, s) : kOk;
 }
 
 // ---------------------------------------------------------------------------

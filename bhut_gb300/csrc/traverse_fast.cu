@@ -39,7 +39,6 @@ namespace bhut {
 
 constexpr int kFastWarps = 4;
 constexpr int kFastThreads = kFastWarps * kWarp;
-constexpr int kSplitMaxLevels = 10;
 // Tuning (overridable at build time): resident blocks per SM of the fast form
 // (they cap the registers: 5 / 6 / 7 / 8 at 96 / 80 / 72 / 64).
 //   3-D, softened, not split: 5 / 6 / 7: 1M Plummer 134.6 / 131.1 / 135.6 ms,
@@ -562,8 +561,10 @@ k_traverse_fast(TreeDev t, FastTree ft, FastArgs a, int levels, double* __restri
 }
 
 // kSumRows threads per output, each with every kSumRows-th share: one thread
-// for all of 256 shares took 32 us for 2,000 targets.
+// for all of 256 shares took 32 us for 2,000 targets.  PAIRS (form exact): each
+// with a run of shares, added in pairs as the tree's levels are.
 constexpr int kSumRows = 8;
+template <bool PAIRS>
 __global__ void __launch_bounds__(kWarp * kSumRows)
 k_split_sum(const double* __restrict__ partial, int64_t nt, int dim, int shares,
             const int32_t* __restrict__ out_idx, double* __restrict__ out)
@@ -573,7 +574,16 @@ k_split_sum(const double* __restrict__ partial, int64_t nt, int dim, int shares,
          base += (int64_t)gridDim.x * kWarp) {
         const int64_t j = base + threadIdx.x;
         double v = 0.0;
-        if (j < nt * dim) {
+        if (PAIRS && j < nt * dim) {
+            const int run = max(shares / kSumRows, 1), y0 = threadIdx.y * run;
+            double wait[kTopLevels];   // sums of whole runs of 2^k shares
+            for (int y = 0; y0 < shares && y < run; y++) {
+                v = partial[(int64_t)(y0 + y) * nt * dim + j];
+                int k = 0;
+                for (; (y >> k) & 1; k++) v = __dadd_rn(wait[k], v);
+                wait[k] = v;
+            }
+        } else if (j < nt * dim) {
 #pragma unroll 8
             for (int y = threadIdx.y; y < shares; y += kSumRows)
                 v = __dadd_rn(v, partial[(int64_t)y * nt * dim + j]);
@@ -581,8 +591,18 @@ k_split_sum(const double* __restrict__ partial, int64_t nt, int dim, int shares,
         part[threadIdx.y][threadIdx.x] = v;
         __syncthreads();
         if (threadIdx.y == 0 && j < nt * dim) {
-            for (int y = 1; y < min(kSumRows, shares); y++)
-                v = __dadd_rn(v, part[y][threadIdx.x]);
+            if (PAIRS) {
+                double p[kSumRows];
+                for (int y = 0; y < kSumRows; y++) p[y] = part[y][threadIdx.x];
+#pragma unroll
+                for (int o = 1; o < kSumRows; o *= 2)
+#pragma unroll
+                    for (int y = 0; y < kSumRows; y += 2 * o) p[y] = __dadd_rn(p[y], p[y + o]);
+                v = p[0];
+            } else {
+                for (int y = 1; y < min(kSumRows, shares); y++)
+                    v = __dadd_rn(v, part[y][threadIdx.x]);
+            }
             const int64_t i = j / dim;
             out[(out_idx ? out_idx[i] : i) * dim + j % dim] = v;
         }
@@ -680,26 +700,41 @@ int launch_fast_targets(const double* tx, const double* ty, const double* tz, in
     return kOk;
 }
 
-int launch_split_sum(const double* partial, int64_t nt, int dim, int shares,
+int launch_split_sum(const double* partial, int64_t nt, int dim, int shares, bool pairs,
                      const int32_t* out_idx, double* out, cudaStream_t s)
 {
-    k_split_sum<<<grid_for(nt * dim, kWarp), dim3(kWarp, kSumRows), 0, s>>>(partial, nt, dim, shares,
-                                                                           out_idx, out);
+    const auto kernel = pairs ? k_split_sum<true> : k_split_sum<false>;
+    kernel<<<grid_for(nt * dim, kWarp), dim3(kWarp, kSumRows), 0, s>>>(partial, nt, dim, shares,
+                                                                      out_idx, out);
     BHUT_CUDA(cudaGetLastError());
     note_launches(1);
     return kOk;
 }
 
+// Whether a tree of so many nodes has work for another level of a split.
+static bool splits_further(int64_t nodes, int levels)
+{
+    return levels < kTopLevels &&
+           (nodes >> levels) > (levels < 2 ? BHUT_SPLIT_NODES_FIRST : BHUT_SPLIT_NODES);
+}
+
+int top_levels(int64_t nodes)
+{
+    int levels = 0;
+    while (splits_further(nodes, levels)) levels++;
+    return levels;
+}
+
 // Levels of the tree to split a traversal of nt targets by (0: none, else
-// 2 to kSplitMaxLevels), and the doubles of `partial` it needs.
+// 2 to kTopLevels), and the doubles of `partial` it needs.
 int split_levels(int64_t nt, int64_t nodes, int64_t particles, bool self, bool exact)
 {
     const int64_t groups = (nt + kWarp - 1) / kWarp;
     if (self && groups >= (exact ? 2 : 1) * kWaveWarps) return 0;
     const int64_t warps = exact ? BHUT_SPLIT_WARPS_EXACT : BHUT_SPLIT_WARPS;
     int levels = 0;
-    while (levels < kSplitMaxLevels && (groups << levels) < warps &&
-           ((nodes >> levels) > (levels < 2 ? BHUT_SPLIT_NODES_FIRST : BHUT_SPLIT_NODES) ||
+    while ((groups << levels) < warps &&
+           (splits_further(nodes, levels) ||
             (!exact && levels < 2 && (particles >> levels) > 2 * BHUT_SPLIT_PARTICLES)))
         levels++;
     return levels < 2 ? 0 : levels;
@@ -756,7 +791,7 @@ int launch_traverse_fast(const TreeDev& t, const FastTree& ft, const float4* th,
                                       : (d3 ? k_traverse_fast<3, true, false, B>
                                             : k_traverse_fast<2, true, false, B>);
         kernel<<<g, kFastThreads, 0, s>>>(t, ft, a, levels, partial);
-        if (shares > 1) BHUT_TRY(launch_split_sum(partial, nt, t.dim, shares, out_idx, out, s));
+        if (shares > 1) BHUT_TRY(launch_split_sum(partial, nt, t.dim, shares, false, out_idx, out, s));
     }
     BHUT_CUDA(cudaGetLastError());
     note_launches(1);

@@ -301,8 +301,12 @@ int launch_traverse_fast(const TreeDev& t, const FastTree& ft, const float4* th,
 // Few targets: 2^levels warps per 32 targets (0: one), the doubles of scratch
 // that takes, and the sum of the blocks' partial results.
 int split_levels(int64_t nt, int64_t nodes, int64_t particles, bool self, bool exact);
+// Levels of a tree of so many nodes whose sums form exact adds in pairs; a split
+// of that form is no deeper.
+constexpr int kTopLevels = 10;
+int top_levels(int64_t nodes);
 int64_t split_partial_doubles(int64_t nt, int dim, int levels);
-int launch_split_sum(const double* partial, int64_t nt, int dim, int shares,
+int launch_split_sum(const double* partial, int64_t nt, int dim, int shares, bool pairs,
                      const int32_t* out_idx, double* out, cudaStream_t s);
 // TreeData arrays as the reference lays them out (bhut/tree/node.py:15-77):
 // int64 indices, com (m, dim), for compute_tree_statistics.
