@@ -52,12 +52,12 @@ constexpr int kBatchThreads = kBatchWarps * kWarp;
 // min x, y, z and of max x, y, z, the bits of max |mass|, flags (bit 0: a
 // mass differs from the system's first, bit 1: a particle lies beyond 1.1x
 // the system's root box).
-constexpr int kSegAcc = 8;
+constexpr int64_t kSegAcc = 8;   // (64 bits: so is every offset by system)
 constexpr int kSegChunk = 4096;   // particles per block of the chunked box
 // Per-system box (kSegBox doubles): min (0..2), max (3..5), max |m| (6),
 // equal positive masses (7), RN(1 / extent) (8..10), zero extent on some
 // axis (11), extent (12..14; 1 for a zero extent).
-constexpr int kSegBox = 16;
+constexpr int64_t kSegBox = 16;
 
 __global__ void k_seg_acc_init(uint64_t* __restrict__ acc, int64_t ns)
 {
@@ -237,7 +237,7 @@ __global__ void k_seg_outside(const double* __restrict__ pos, const int64_t* __r
                               uint8_t* __restrict__ flag)
 {
     const int s = blockIdx.x;
-    const double* r = roots + 4 * s;
+    const double* r = roots + 4 * (int64_t)s;
     const double lim = __dmul_rn(1.1, r[3]);
     bool out = false;
     for (int64_t i = off[s] + threadIdx.x; i < off[s + 1]; i += blockDim.x) {
@@ -266,7 +266,7 @@ __global__ void k_seg_keep_outside(const double* __restrict__ pos, int64_t n, in
          i += (int64_t)gridDim.x * blockDim.x) {
         const int s = sys_of[i];
         if (!keep[s]) continue;
-        const double* r = roots + 4 * s;
+        const double* r = roots + 4 * (int64_t)s;
         const double lim = __dmul_rn(1.1, r[3]);
         double mx = fabs(__dsub_rn(pos[i * dim], r[0]));
         for (int d = 1; d < dim; d++) {

@@ -386,9 +386,9 @@ __device__ __forceinline__ void put_box(const Quad& w, int32_t id, uint64_t klo,
     if (w.q < DIM) {
         const double lo = __longlong_as_double((long long)ord_inv(klo));
         const double hi = __longlong_as_double((long long)ord_inv(khi));
-        o.lo[3 * id + w.q] = lo;
-        o.hi[3 * id + w.q] = hi;
-        o.center[DIM * id + w.q] = __dmul_rn(__dadd_rn(lo, hi), 0.5);
+        o.lo[node_at(3, id, w.q)] = lo;
+        o.hi[node_at(3, id, w.q)] = hi;
+        o.center[node_at(DIM, id, w.q)] = __dmul_rn(__dadd_rn(lo, hi), 0.5);
         e = __dsub_rn(hi, lo);
     }
     double ext = w.from(e, 0);   // extents order as integers (not negative)
@@ -410,7 +410,7 @@ __device__ __forceinline__ void put_moments(const Quad& w, int32_t id, double ac
                                             const NodeOut& o)
 {
     double v = 0.0;
-    if (w.q < DIM) v = total > 0 ? __ddiv_rn(acc, total) : o.center[DIM * id + w.q];
+    if (w.q < DIM) v = total > 0 ? __ddiv_rn(acc, total) : o.center[node_at(DIM, id, w.q)];
     else if (w.q == 3) v = total;
     reinterpret_cast<double*>(&o.cm[id])[w.q] = v;
 }
@@ -449,6 +449,12 @@ __device__ void leaf_node(const Quad& w, int32_t id, bool refit, const TreeDev& 
     put_moments<DIM>(w, id, acc, total, o);
 }
 
+// A child's bound, written by another thread, as an ordered integer.
+static __device__ __forceinline__ uint64_t bound_key(const double* bound, int32_t id, int axis)
+{
+    return ord_key((uint64_t)__double_as_longlong(__ldcg(&bound[node_at(3, id, axis)])));
+}
+
 // Internal node from its two children (build.py:276-292 in build mode,
 // refit.py:173-192 in refit mode), written by other threads (L2, not L1).
 template <int DIM>
@@ -460,10 +466,8 @@ __device__ void internal_node(const Quad& w, int32_t id, int32_t fc, bool refit,
     if (!refit) {
         uint64_t klo = 0, khi = 0;
         if (w.q < DIM) {
-            const uint64_t l0 = ord_key((uint64_t)__double_as_longlong(__ldcg(&o.lo[3 * fc + w.q])));
-            const uint64_t l1 = ord_key((uint64_t)__double_as_longlong(__ldcg(&o.lo[3 * (fc + 1) + w.q])));
-            const uint64_t h0 = ord_key((uint64_t)__double_as_longlong(__ldcg(&o.hi[3 * fc + w.q])));
-            const uint64_t h1 = ord_key((uint64_t)__double_as_longlong(__ldcg(&o.hi[3 * (fc + 1) + w.q])));
+            const uint64_t l0 = bound_key(o.lo, fc, w.q), l1 = bound_key(o.lo, fc + 1, w.q);
+            const uint64_t h0 = bound_key(o.hi, fc, w.q), h1 = bound_key(o.hi, fc + 1, w.q);
             klo = l1 < l0 ? l1 : l0;
             khi = h1 > h0 ? h1 : h0;
         }
@@ -540,9 +544,9 @@ __device__ void put_node_solo(int32_t id, bool refit, const uint64_t* klo, const
         for (int d = 0; d < DIM; d++) {
             const double lo = __longlong_as_double((long long)ord_inv(klo[d]));
             const double hi = __longlong_as_double((long long)ord_inv(khi[d]));
-            o.lo[3 * id + d] = lo;
-            o.hi[3 * id + d] = hi;
-            o.center[DIM * id + d] = __dmul_rn(__dadd_rn(lo, hi), 0.5);
+            o.lo[node_at(3, id, d)] = lo;
+            o.hi[node_at(3, id, d)] = hi;
+            o.center[node_at(DIM, id, d)] = __dmul_rn(__dadd_rn(lo, hi), 0.5);
             const double e = __dsub_rn(hi, lo);
             if (d == 0 || __double_as_longlong(e) > __double_as_longlong(ext)) ext = e;
         }
@@ -551,7 +555,8 @@ __device__ void put_node_solo(int32_t id, bool refit, const uint64_t* klo, const
         o.size[id] = __dmul_rn(2.0, half);
     }
     double com[3] = {0.0, 0.0, 0.0};
-    for (int d = 0; d < DIM; d++) com[d] = total > 0 ? __ddiv_rn(acc[d], total) : o.center[DIM * id + d];
+    for (int d = 0; d < DIM; d++)
+        com[d] = total > 0 ? __ddiv_rn(acc[d], total) : o.center[node_at(DIM, id, d)];
     o.cm[id] = NodeCM{com[0], com[1], com[2], total};
 }
 
@@ -591,10 +596,8 @@ __device__ void internal_solo(int32_t id, int32_t fc, bool refit, const NodeOut&
     uint64_t klo[3] = {0, 0, 0}, khi[3] = {0, 0, 0};
     if (!refit) {
         for (int d = 0; d < DIM; d++) {
-            const uint64_t l0 = ord_key((uint64_t)__double_as_longlong(__ldcg(&o.lo[3 * fc + d])));
-            const uint64_t l1 = ord_key((uint64_t)__double_as_longlong(__ldcg(&o.lo[3 * (fc + 1) + d])));
-            const uint64_t h0 = ord_key((uint64_t)__double_as_longlong(__ldcg(&o.hi[3 * fc + d])));
-            const uint64_t h1 = ord_key((uint64_t)__double_as_longlong(__ldcg(&o.hi[3 * (fc + 1) + d])));
+            const uint64_t l0 = bound_key(o.lo, fc, d), l1 = bound_key(o.lo, fc + 1, d);
+            const uint64_t h0 = bound_key(o.hi, fc, d), h1 = bound_key(o.hi, fc + 1, d);
             klo[d] = l1 < l0 ? l1 : l0;
             khi[d] = h1 > h0 ? h1 : h0;
         }

@@ -226,6 +226,13 @@ struct MortonBox {
     }
 };
 
+// Entry `axis` of node id in an array of `width` values a node (64 bits: three
+// times a node id passes 2^31 from 715,827,883 nodes).
+static __host__ __device__ __forceinline__ int64_t node_at(int width, int32_t id, int axis)
+{
+    return (int64_t)width * id + axis;
+}
+
 // Node arrays written by the bottom-up pass.
 struct NodeOut {
     NodeCM* cm;        // (com, mass)
