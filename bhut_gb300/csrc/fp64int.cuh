@@ -102,14 +102,6 @@ BHUT_FN Parts product(const Parts& a, const Parts& b)
     return Parts{hi & ~0x7ffull, a.sign ^ b.sign, e, a.zero || b.zero};
 }
 
-// The double of parts within the normal range (m rounded to 53 bits or not).
-BHUT_FN double whole(const Parts& a)
-{
-    const uint32_t top = (uint32_t)(a.m >> 43) + ((uint32_t)(a.e - 1) << 20);
-    const uint64_t r = ((uint64_t)top << 32) | (uint32_t)(a.m >> 11);
-    return from_bits((a.zero ? 0ull : r) | ((uint64_t)a.sign << 32));
-}
-
 // RN(a b) as a double (the carry of the rounding runs into the exponent).
 BHUT_FN double mul(const Parts& a, const Parts& b)
 {

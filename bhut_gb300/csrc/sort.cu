@@ -33,10 +33,12 @@
 
 #include "tree.cuh"
 
-// Points that one block orders (launch_order).  Whole rebuilds, us, by one
-// block / by passes: 1,500 points 117 / -, 3,000 142 / 144, 4,000 162 / 158,
-// 5,000 181 / 156, 8,000 208 / 157; orders alone: 3,000 139 / 169, 5,000 162 /
-// 161, 8,000 176 / 157.
+// Points that one block orders (launch_order).  One block / passes, 3-D, us: whole
+// rebuilds (captured) of 1,000 points 120 / 133, 2,000 130 / 134, 3,000 147 / 151,
+// 4,000 156 / 145; orders 112 / 145, 115 / 149, 128 / 159, 137 / 147; one-shot
+// solves of host arrays 211 / 250, 226 / 263, 270 / 296, 302 / 319.  2-D alike: a
+// rebuild's graph hides the launches of the passes, so it alone would have the line
+// at 3,500.  5,000 points: orders 162 / 161, rebuilds 181 / 156.
 #ifndef BHUT_ORDER_SMALL
 #define BHUT_ORDER_SMALL 4096
 #endif

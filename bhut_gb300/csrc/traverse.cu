@@ -33,22 +33,6 @@ constexpr int kTravThreads = kTravWarps * kWarp;
 // 2-D, 6 / 7: 50k 3.68 / 3.60, 10k 0.80 / 0.78, targets of either 0 to 6 % less / more.
 constexpr int exact_blocks(int dim, bool split) { return dim == 3 && !split ? 5 : 6; }
 
-// Products of a pair on the integer pipes: the squares and the force
-// components (tuning: 0 takes the FP64 pipe; 100k Plummer traversal both 95.9
-// ms, squares alone 103.3, forces alone 104.9, neither 122.4).
-#ifndef BHUT_INT_SQUARES
-#define BHUT_INT_SQUARES 1
-#endif
-#ifndef BHUT_INT_FORCE
-#define BHUT_INT_FORCE 1
-#endif
-template <bool INT>
-static __device__ __forceinline__ double mul_rn(const fp64int::Parts& a, const fp64int::Parts& b,
-                                                double x, double y)
-{
-    return INT ? fp64int::mul(a, b) : __dmul_rn(x, y);
-}
-
 // v, kept in registers (a product of two kernel arguments would otherwise be
 // formed again for every pair).
 static __device__ __forceinline__ double held(double v)
@@ -89,19 +73,19 @@ static __device__ __forceinline__ bool pair_exact(double dx, double dy, double d
     const auto X = parts(dx), Y = parts(dy), Z = parts(DIM == 3 ? dz : 0.0), M = parts(gm);
     bool ok = within(X, -250, 250) && within(Y, -250, 250) && within(Z, -250, 250) &&
               within(M, -200, 200);
-    double r2 = mul_rn<BHUT_INT_SQUARES>(X, X, dx, dx);
-    r2 = __dadd_rn(r2, mul_rn<BHUT_INT_SQUARES>(Y, Y, dy, dy));
-    if (DIM == 3) r2 = __dadd_rn(r2, mul_rn<BHUT_INT_SQUARES>(Z, Z, dz, dz));
+    // (100k Plummer traversal with all products in integers 95.9 ms, the squares
+    // alone 103.3, the forces alone 104.9, neither 122.4)
+    double r2 = fp64int::mul(X, X);
+    r2 = __dadd_rn(r2, fp64int::mul(Y, Y));
+    if (DIM == 3) r2 = __dadd_rn(r2, fp64int::mul(Z, Z));
     r2 = __dadd_rn(r2, eps2);
     const auto R = parts(r2);
     if (ok && R.zero) return false;   // (never -0)
     ok = ok && within(R, -340, 300);
     const auto I = fp64int::rsqrt(R);
     const auto W = fp64int::product(M, fp64int::product(fp64int::product(I, I), I));
-    const double f = BHUT_INT_FORCE ? 0.0 : fp64int::whole(W);
-    double3 F = make_double3(mul_rn<BHUT_INT_FORCE>(W, X, f, dx),
-                             mul_rn<BHUT_INT_FORCE>(W, Y, f, dy),
-                             DIM == 3 ? mul_rn<BHUT_INT_FORCE>(W, Z, f, dz) : 0.0);
+    double3 F = make_double3(fp64int::mul(W, X), fp64int::mul(W, Y),
+                             DIM == 3 ? fp64int::mul(W, Z) : 0.0);
     if (!ok) {   // something beyond those ranges
         double3 G;
         if (!pair_fp64_force<DIM>(dx, dy, dz, gm, eps2, &G)) return false;

@@ -76,11 +76,15 @@ constexpr int kFastThreads = kFastWarps * kWarp;
 //   1M self                139      -      -      -    139    181
 //   nodes                 4 / 8 / 16 / 32: 10k self 0.42 / 0.35 / 0.34 / 0.33,
 //                         1,000 self 0.10 / 0.10 / 0.11 / 0.20
-// Self targets that fill the GPU once (kWaveWarps) are not split: neighbours
-// then share what the walk reads, and a split gives it up (100k uniform cube
-// without softening 5.04 ms unsplit, 5.87 to 6.58 split; 100k Plummer 10.3,
-// 9.3 to 10.0).  External targets vary more from group to group, and the
-// shorter walks balance.
+// Self targets that fill the GPU once (kWaveWarps: the wave of the 3-D softened
+// kernel, which the others take over) are not split: neighbours then share what
+// the walk reads, and a split gives it up.  ms, not split / split, softened and
+// not, at 98k, 130k and 195k: uniform cube 4.1 / 3.9, 6.0 / 6.4, 8.7 / 10.6 and
+// 4.3 / 4.4, 6.5 / 7.2, 9.0 / 12.3; Plummer 9.2 / 7.9, 14.0 / 12.3, 19.6 / 19.5 and
+// 9.5 / 8.9, 14.4 / 13.6, 20.1 / 21.5; 2-D Gaussian 1.67 / 1.83, 2.48 / 2.69, 3.20
+// / 3.92.  So the line is right for even distributions and in 2-D, and gives 10 to
+// 15 % away just beyond it where the targets' work varies.  External targets vary
+// more from group to group, and the shorter walks balance.
 #ifndef BHUT_SPLIT_WARPS
 #define BHUT_SPLIT_WARPS 49152
 #endif
@@ -388,7 +392,7 @@ __device__ __forceinline__ void walk(const TreeDev& t, const FastTree& ft, const
                 mask = omask;
                 continue;
             }
-                        if (!FAR && omask && (hd.w & kTwig)) {   // both leaves here
+            if (!FAR && omask && (hd.w & kTwig)) {   // both leaves here
                 box = ft.twig[node];
                 lmask = omask;
                 s = __float_as_int(box.h.w);

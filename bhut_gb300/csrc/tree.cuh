@@ -292,8 +292,8 @@ int launch_traverse_exact(const TreeDev& t, const double* tx, const double* ty, 
                           const int32_t* self_id, const int32_t* out_idx, int64_t nt, double theta,
                           double eps, double G, double* out, unsigned* err,
                           unsigned long long* stats, cudaStream_t s, int levels, double* partial);
-// `fine`: the lo parts of form "fast" (split_grid), else those of "fp32".
 FastFrame frame_of_box(const double* box, int dim);   // box on the host
+// `fine`: the lo parts of form "fast" (split_grid), else those of "fp32".
 int launch_fast_prepare(const FastFrame& frame, bool fine, const TreeDev& t, const double* center,
                         const double* quad, float4* ph, float4* pl, const NodeCopies& o,
                         cudaStream_t s);
