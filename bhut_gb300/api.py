@@ -9,10 +9,11 @@ and the result comes back as a CUDA tensor on the same device.
 
 One keyword is added to both entry points: ``form`` selects the traversal
 arithmetic -- ``"exact"`` (FP64; pair terms bit-identical to the reference's
-Numba loop), ``"fast"`` (FP64-accurate float-float arithmetic on the FP32
-pipe) or ``"fp32"`` (the FP32/Kahan precision form).  ``criterion`` accepts,
-besides the reference's ``"bh"``, ``"bh_offset"`` (open when
-|x - com| < size/theta + |com - box centre|), available with ``form="fp32"``;
+Numba loop, summed in an order that depends on the tree alone), ``"fast"``
+(FP64-accurate float-float arithmetic on the FP32 pipe) or ``"fp32"`` (the
+FP32/Kahan precision form).  ``criterion`` accepts, besides the reference's
+``"bh"``, ``"bh_offset"`` (open when |x - com| < size/theta + |com - box
+centre|), available with ``form="fp32"``;
 ``multipole`` accepts, besides ``"mono"``, ``"quad"`` (monopole plus traceless
 quadrupole per node), also with ``form="fp32"`` only.
 """
@@ -531,9 +532,11 @@ class Tree:
                              G: float = 1.0) -> list:
         """Chunks in, chunks out: the map_blocks path of bhut/api.py:690-731
         without Dask.  The chunks are evaluated in ONE traversal launch over
-        their concatenation (each target's result does not depend on which
-        other targets share the launch) and the result is returned split
-        into chunks of the same lengths, as CUDA tensors for CUDA chunks."""
+        their concatenation and the result is returned split into chunks of
+        the same lengths, as CUDA tensors for CUDA chunks.  In forms
+        ``"exact"`` and ``"fp32"`` a target's result does not depend on which
+        other targets share the launch; in form ``"fast"`` the rounding of
+        its sums does (some 1e-13 of it, more where its terms cancel)."""
         chunks = [_to_f64(c) for c in target_chunks]
         if not chunks:
             return []

@@ -89,7 +89,10 @@ BHUT_API int bhut_tree_rebuild(bhut_tree *t, const double *positions, const doub
 BHUT_API int bhut_tree_accel_self(bhut_tree *t, double theta, double softening, double G, double *out);
 
 /* Accelerations at m external targets (m, dim), out (m, dim).  Replaces
- * barnes_hut_accelerations_targets (bhut/traverse/bh.py:30-146). */
+ * barnes_hut_accelerations_targets (bhut/traverse/bh.py:30-146).  In forms
+ * exact and fp32 a target's result does not depend on the call's other
+ * targets; in form fast the rounding of its sums does (some 1e-13 of it,
+ * more where its terms cancel). */
 BHUT_API int bhut_tree_accel_targets(bhut_tree *t, const double *targets, int64_t m, double theta,
                             double softening, double G, double *out);
 

@@ -1,5 +1,5 @@
-"""A target's value in form exact depends on the tree alone: not on how many
-targets a call has, nor on which."""
+"""A target's value in forms exact and fp32 depends on the tree alone: not on how
+many targets a call has, nor on which."""
 import numpy as np
 import pytest
 
@@ -14,11 +14,12 @@ def _engine(engine_lib):
     yield
 
 
+@pytest.mark.parametrize("form", ["exact", "fp32"])
 @pytest.mark.parametrize("n,dim,leaf", [(1, 3, 32), (40, 2, 1), (500, 3, 8), (3000, 3, 32), (20_000, 2, 16),
                                         (70_000, 3, 32), (200_000, 3, 64)])
-def test_targets_by_call_size(n, dim, leaf):
+def test_targets_by_call_size(n, dim, leaf, form):
     pos, m = workloads.gaussian(n, seed=n, dim=dim)
-    tree = bh.Tree(pos, m, leaf_size=leaf, dim=dim, form="exact").build()
+    tree = bh.Tree(pos, m, leaf_size=leaf, dim=dim, form=form).build()
     rng = np.random.default_rng(0)
     t = np.concatenate([pos[rng.integers(0, n, 2000)] * 1.01, rng.uniform(-9, 9, (500, dim))])
     kw = dict(theta=0.6, softening=0.02)
