@@ -675,9 +675,9 @@ void trim_pins()
 // instead of being destroyed: a one-shot solve of a few thousand particles
 // spends more on creating a stream and some forty buffers, and on giving them
 // back, than on its kernels (1,000 particles: 195 of 690 us).  Bounded to
-// kIdleTrees of kIdleBytes each; given back when an allocation of the library,
-// a batch's too, fails and by bhut_pool_trim.  A tree in the pool holds no results: everything but stream, buffers
-// and pinned memory is reset.
+// kIdleTrees of kIdleBytes each; given back when an allocation of the library, a
+// batch's too, fails and by bhut_pool_trim.  A tree in the pool holds no results:
+// everything but stream, buffers and pinned memory is reset.
 constexpr size_t kIdleTrees = 4, kIdleBytes = 32u << 20;
 
 struct IdleTrees {
